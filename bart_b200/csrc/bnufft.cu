@@ -3130,20 +3130,41 @@ static int net_ensure_ws(bnufft_precnet_s* n, long P, long nblk)
 	return BNUFFT_OK;
 }
 
-// weight and bias gradients of layer l into grad
-template <int CIN, int COUT, typename AT, typename GT>
-static int net_wgrad(bnufft_precnet_s* n, int l, const AT* a, const GT* g, int X, int Y, long nimg, cudaStream_t st)
+// most blocks of a weight-gradient launch (persistent, two to four per SM):
+// the partial vectors to reduce
+enum { NET_WG_BLOCKS = 4 * 148 };
+
+static int net_wgrad_reduce(bnufft_precnet_s* n, int l, unsigned nblk, cudaStream_t st)
 {
-	size_t smem = sizeof(float) * (NET_HALO_Y * NET_HALO_X * CIN + NET_TILE_Y * NET_TILE_X * COUT);
-	dim3 grid = net_tiles(X, Y, nimg);
-	long nblk = (long)grid.x * grid.y * grid.z;
-	const int O = COUT * 9 * CIN + COUT;
-	TRY(prep_kernel(k_wgrad<CIN, COUT, AT, GT>, smem));
-	k_wgrad<CIN, COUT, AT, GT><<<grid, NET_THREADS, smem, st>>>(a, g, X, Y, n->part);
-	LAUNCHED();
-	k_wgrad_reduce<<<(O + 255) / 256, 256, 0, st>>>(n->part, nblk, O, n->grad + NetLayout::woff(l));
+	const int O = NetLayout::size(l);
+	k_wgrad_reduce<<<(O + 31) / 32, 256, 0, st>>>(n->part, (int)nblk, O, n->grad + NetLayout::woff(l));
 	LAUNCHED();
 	return BNUFFT_OK;
+}
+
+// weight and bias gradients of layer l (2..5: 32 -> 32 channels) into grad
+static int net_wgrad32(bnufft_precnet_s* n, int l, const bf16* a, const bf16* g, int X, int Y, long nimg, cudaStream_t st)
+{
+	const dim3 t = net_tiles(X, Y, nimg);
+	const long ntiles = (long)t.x * t.y * t.z;
+	const unsigned nblk = (unsigned)std::min<long>(ntiles, NET_WG_BLOCKS / 2);
+	TRY(prep_kernel(k_wgrad32, WG_SMEM));
+	k_wgrad32<<<nblk, WG_THREADS, WG_SMEM, st>>>(a, g, X, Y, (int)t.x, (int)t.y, ntiles, n->part);
+	LAUNCHED();
+	return net_wgrad_reduce(n, l, nblk, st);
+}
+
+// the same for the layers with 2 channels on one side (OUT6: layer 6, else
+// layer 1): w the 32-channel tensor, t the complex image
+template <bool OUT6>
+static int net_wgrad_thin(bnufft_precnet_s* n, const bf16* w, const float2* t, int X, int Y, long nimg, cudaStream_t st)
+{
+	const int tx = (X + NET_TILE_X - 1) / NET_TILE_X;
+	const long nrows = (long)tx * Y * nimg;
+	const unsigned nblk = (unsigned)std::min<long>((nrows + WT_WARPS - 1) / WT_WARPS, NET_WG_BLOCKS);
+	k_wgrad_thin<OUT6><<<nblk, 32 * WT_WARPS, 0, st>>>(w, t, X, Y, tx, nrows, n->part);
+	LAUNCHED();
+	return net_wgrad_reduce(n, OUT6 ? 5 : 0, nblk, st);
 }
 
 extern "C" int bnufft_precnet_nparams(void) { return NET_N; }
@@ -3248,7 +3269,7 @@ extern "C" int bnufft_precnet_forward(bnufft_precnet_t n, void* out, const void*
 
 	const long P = X * Y * nimg;
 	dim3 grid = net_tiles((int)X, (int)Y, nimg);
-	TRY(net_ensure_ws(n, P, (long)grid.x * grid.y * grid.z));
+	TRY(net_ensure_ws(n, P, std::min<long>((long)grid.x * grid.y * grid.z, NET_WG_BLOCKS)));
 	size_t b = sizeof(float2) * P;
 	Staged i, o;
 	TRY(stage_in(i, in, b, st));
@@ -3285,7 +3306,7 @@ static int net_train(bnufft_precnet_t n, const void* in, const void* target, con
 	const long P = X * Y * nimg;
 	const int x = (int)X, y = (int)Y;
 	dim3 grid = net_tiles(x, y, nimg);
-	TRY(net_ensure_ws(n, P, (long)grid.x * grid.y * grid.z));
+	TRY(net_ensure_ws(n, P, std::min<long>((long)grid.x * grid.y * grid.z, NET_WG_BLOCKS)));
 	size_t b = sizeof(float2) * P;
 	Staged si, stg;
 	TRY(stage_in(si, in, b, st));
@@ -3310,7 +3331,7 @@ static int net_train(bnufft_precnet_t n, const void* in, const void* target, con
 	}
 
 	// backward: layer 6, then 5..2 on the tensor cores, then layer 1
-	TRY((net_wgrad<NET_C, 2, bf16, float>(n, 5, n->act[4], (const float*)n->gout, x, y, nimg, st)));
+	TRY(net_wgrad_thin<true>(n, n->act[4], n->gout, x, y, nimg, st));
 	k_net_out_bwd<<<pb, NET_THREADS, 0, st>>>(n->gout, n->act[4], x, y, P, n->pr + NetLayout::woff(5), n->gu0);
 	LAUNCHED();
 	bf16* gu = n->gu0;
@@ -3318,13 +3339,13 @@ static int net_train(bnufft_precnet_t n, const void* in, const void* target, con
 
 	for (int l = 4; l >= 1; l--) {
 
-		TRY((net_wgrad<NET_C, NET_C, bf16, bf16>(n, l, n->act[l - 1], gu, x, y, nimg, st)));
+		TRY(net_wgrad32(n, l, n->act[l - 1], gu, x, y, nimg, st));
 		TRY(launch_conv32<1>(n, gu, n->wt + (l - 1) * 9216, n->wt_tc + (l - 1) * 9216, nullptr, n->act[l - 1], gn, x,
 				y, nimg, nullptr, nullptr, st));
 		std::swap(gu, gn);
 	}
 
-	TRY((net_wgrad<2, NET_C, float, bf16>(n, 0, (const float*)inp, gu, x, y, nimg, st)));
+	TRY(net_wgrad_thin<false>(n, gu, inp, x, y, nimg, st));
 
 	if (grads)
 		CUDA_TRY(cudaMemcpyAsync(grads, n->grad, sizeof(float) * NET_N, cudaMemcpyDefault, st));

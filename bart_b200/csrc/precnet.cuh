@@ -14,8 +14,8 @@
 // Training uses the same kernels plus the backward passes: the data
 // gradient of a 32 -> 32 layer is the forward kernel with the weights
 // transposed and the taps flipped, masked by the ReLU of the layer below;
-// weight gradients are FP32 sums over pixels, per block, then reduced in a
-// fixed order (bit-reproducible).
+// weight gradients are FP32 sums over pixels, per block (layers 2-5 on the
+// tensor cores), then reduced in a fixed order (bit-reproducible).
 //
 // Parameter vector (float32), per layer l = 1..6: W_l[cout][tap][cin]
 // (tap = 3 ky + kx), then b_l[cout].
@@ -420,91 +420,321 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out_bwd(const float2* __res
 	}
 }
 
-__device__ __forceinline__ float net_load(const bf16* p) { return __bfloat162float(*p); }
-__device__ __forceinline__ float net_load(const float* p) { return *p; }
-
-// Weight and bias gradients of a 3x3 layer, per block of a 32 x 8 pixel tile:
+// Weight and bias gradients -----------------------------------------------------
+//
+// Both kernels are persistent: a block takes image tiles blockIdx.x,
+// blockIdx.x + gridDim.x, ... and keeps its sums in registers over all of
+// them, so it writes one partial vector of the layer's parameters at the end
+// (a few hundred vectors to reduce instead of one per tile), in a fixed order:
+// the gradients are the same bits every run.
 //   part[blk][(co * 9 + tap) * CIN + ci] = sum_p g[p][co] a[p + off(tap)][ci]
-//   part[blk][COUT * 9 * CIN + co]        = sum_p g[p][co]
-// a: [P][CIN], g: [P][COUT] (bf16 or float). grid (ceil(X/32), ceil(Y/8), nimg).
-template <int CIN, int COUT, typename AT, typename GT>
-__global__ void __launch_bounds__(NET_THREADS) k_wgrad(const AT* __restrict__ a, const GT* __restrict__ g, int X, int Y,
-		float* __restrict__ part)
+//   part[blk][COUT * 9 * CIN + co]       = sum_p g[p][co]
+
+// 32 -> 32 channels on the tensor cores (mma.sync, bf16 in, float32 sums).
+// Per tile of 32 x 8 pixels the gradient rows and the activations' halo lie
+// in shared memory pixel by pixel; ldmatrix.trans reads both as MMA operands
+// with the pixels as K. Warp w owns tap w: its 32 x 32 sums are 32 registers.
+// The next tile arrives by cp.async while this one is summed. Bound by the
+// tile traffic (1.33 x 64 + 64 B per pixel) and shared-memory reads; the
+// FP32-pipe kernel it replaces took two shared-memory loads per FMA (1019 us
+// per layer of seven 256^2 images; their whole gradient pass 5.37 -> 0.74 ms,
+// with the thin layers and the reduction below).
+constexpr int WG_WARPS = 9;
+constexpr int WG_THREADS = 32 * WG_WARPS;
+constexpr int WG_STAGE = (NET_HALO_X * NET_HALO_Y + NET_TILE_X * NET_TILE_Y) * NET_SA_STRIDE;	// bf16 per buffer
+constexpr size_t WG_SMEM = 2 * sizeof(bf16) * WG_STAGE;
+
+__device__ __forceinline__ void ldsm_x4_t(uint32_t (&r)[4], uint32_t addr)
 {
-	extern __shared__ float wg_smem[];
-	float* sa = wg_smem;					// [10][34][CIN]
-	float* sg = sa + NET_HALO_Y * NET_HALO_X * CIN;		// [8][32][COUT]
-	constexpr int O = COUT * 9 * CIN;
+	asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+		: "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr));
+}
 
-	const int x0 = blockIdx.x * NET_TILE_X;
-	const int y0 = blockIdx.y * NET_TILE_Y;
-	const long ibase = (long)blockIdx.z * X * Y;
+// 16 bytes global -> shared, zeros where !ok (nothing is read there)
+__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, bool ok)
+{
+	const int n = ok ? 16 : 0;
+	asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" :: "r"(dst), "l"(src), "r"(n));
+}
 
-	for (int i = threadIdx.x; i < NET_HALO_Y * NET_HALO_X * CIN; i += NET_THREADS) {
+__global__ void __launch_bounds__(WG_THREADS, 2) k_wgrad32(const bf16* __restrict__ a, const bf16* __restrict__ g,
+		int X, int Y, int tx, int ty, long ntiles, float* __restrict__ part)
+{
+	extern __shared__ __align__(16) unsigned char wg_smem[];
+	const uint32_t s0 = (uint32_t)__cvta_generic_to_shared(wg_smem);
+	constexpr int HALO = NET_HALO_X * NET_HALO_Y;
+	constexpr uint32_t PIX = NET_SA_STRIDE * 2;		// bytes per pixel
+	constexpr uint32_t STAGE = WG_STAGE * 2;
+	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+	const int ky = warp / 3, kx = warp % 3;
 
-		int ci = i % CIN;
-		int pix = i / CIN;
-		int gy = y0 + pix / NET_HALO_X - 1;
-		int gx = x0 + pix % NET_HALO_X - 1;
-		sa[i] = ((gy >= 0) && (gy < Y) && (gx >= 0) && (gx < X)) ? net_load(a + (ibase + (long)gy * X + gx) * CIN + ci) : 0.f;
+	auto load = [&](long tile, int buf) {
+		const int x0 = (int)(tile % tx) * NET_TILE_X;
+		const int y0 = (int)((tile / tx) % ty) * NET_TILE_Y;
+		const long ibase = (tile / ((long)tx * ty)) * (long)X * Y;
+		const uint32_t sa = s0 + buf * STAGE, sg = sa + HALO * PIX;
+
+		for (int i = threadIdx.x; i < HALO * 4; i += WG_THREADS) {
+
+			const int q = i & 3, pix = i >> 2;
+			const int gy = y0 + pix / NET_HALO_X - 1, gx = x0 + pix % NET_HALO_X - 1;
+			const bool ok = (gy >= 0) && (gy < Y) && (gx >= 0) && (gx < X);
+			cp_async16_zfill(sa + pix * PIX + q * 16, ok ? a + (ibase + (long)gy * X + gx) * NET_C + q * 8 : a, ok);
+		}
+
+		for (int i = threadIdx.x; i < NET_TILE_X * NET_TILE_Y * 4; i += WG_THREADS) {
+
+			const int q = i & 3, pix = i >> 2;
+			const int gy = y0 + pix / NET_TILE_X, gx = x0 + pix % NET_TILE_X;
+			const bool ok = (gy < Y) && (gx < X);
+			cp_async16_zfill(sg + pix * PIX + q * 16, ok ? g + (ibase + (long)gy * X + gx) * NET_C + q * 8 : g, ok);
+		}
+
+		asm volatile("cp.async.commit_group;\n" ::: "memory");
+	};
+
+	float acc[2][4][4], bacc[2][4];
+#pragma unroll
+	for (int mt = 0; mt < 2; mt++) {
+#pragma unroll
+		for (int e = 0; e < 4; e++) {
+
+			bacc[mt][e] = 0.f;
+#pragma unroll
+			for (int nt = 0; nt < 4; nt++)
+				acc[mt][nt][e] = 0.f;
+		}
 	}
 
-	for (int i = threadIdx.x; i < NET_TILE_Y * NET_TILE_X * COUT; i += NET_THREADS) {
+	// lane's row of the 8x8 matrices of one ldmatrix: gradient matrices are
+	// (pixels 0-7, co 0-7), (0-7, 8-15), (8-15, 0-7), (8-15, 8-15) of a 16 x 16
+	// block, activation ones (0-7, ci 0-7), (8-15, 0-7), (0-7, 8-15), (8-15, 8-15)
+	const int mrow = lane & 7, msel = lane >> 3;
+	const uint32_t goff = ((msel >> 1) * 8 + mrow) * PIX + (msel & 1) * 16;
+	const uint32_t aoff = ((msel & 1) * 8 + mrow + ky * NET_HALO_X + kx) * PIX + (msel >> 1) * 16;
+	int buf = 0;
 
-		int co = i % COUT;
-		int pix = i / COUT;
-		int gy = y0 + pix / NET_TILE_X;
-		int gx = x0 + pix % NET_TILE_X;
-		sg[i] = ((gy < Y) && (gx < X)) ? net_load(g + (ibase + (long)gy * X + gx) * COUT + co) : 0.f;
+	if (blockIdx.x < ntiles)
+		load(blockIdx.x, 0);
+
+	for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+
+		if (tile + gridDim.x < ntiles) {
+
+			load(tile + gridDim.x, buf ^ 1);
+			asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+
+		} else {
+
+			asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+		}
+
+		__syncthreads();
+		const uint32_t sa = s0 + buf * STAGE + aoff, sg = s0 + buf * STAGE + HALO * PIX + goff;
+#pragma unroll 2
+		for (int k = 0; k < NET_TILE_X * NET_TILE_Y / 16; k++) {
+
+			const int py = k / 2, px = (k % 2) * 16;
+			uint32_t fa[2][4], fb[2][4];
+			ldsm_x4_t(fa[0], sg + (py * NET_TILE_X + px) * PIX);
+			ldsm_x4_t(fa[1], sg + (py * NET_TILE_X + px) * PIX + 32);
+			ldsm_x4_t(fb[0], sa + (py * NET_HALO_X + px) * PIX);
+			ldsm_x4_t(fb[1], sa + (py * NET_HALO_X + px) * PIX + 32);
+#pragma unroll
+			for (int mt = 0; mt < 2; mt++) {
+#pragma unroll
+				for (int nt = 0; nt < 4; nt++)
+					mma_bf16(acc[mt][nt], fa[mt][0], fa[mt][1], fa[mt][2], fa[mt][3], fb[nt / 2][2 * (nt & 1)],
+							fb[nt / 2][2 * (nt & 1) + 1]);
+
+				if (4 == warp)	// the bias gradient: a column of ones
+					mma_bf16(bacc[mt], fa[mt][0], fa[mt][1], fa[mt][2], fa[mt][3], 0x3f803f80u, 0x3f803f80u);
+			}
+		}
+
+		__syncthreads();	// before the next load overwrites this buffer
+		buf ^= 1;
+	}
+
+	float* dst = part + (long)blockIdx.x * (NET_C * 9 * NET_C + NET_C);
+	const int r = lane >> 2, t = lane & 3;
+#pragma unroll
+	for (int mt = 0; mt < 2; mt++) {
+#pragma unroll
+		for (int hh = 0; hh < 2; hh++) {
+
+			const int co = mt * 16 + hh * 8 + r;
+#pragma unroll
+			for (int nt = 0; nt < 4; nt++)
+				*(float2*)(dst + (co * 9 + warp) * NET_C + nt * 8 + 2 * t)
+					= make_float2(acc[mt][nt][2 * hh], acc[mt][nt][2 * hh + 1]);
+
+			if ((4 == warp) && (0 == t))
+				dst[NET_C * 9 * NET_C + co] = bacc[mt][2 * hh];
+		}
+	}
+}
+
+// Layers 1 and 6 (2 channels on one side) on the FP32 pipes: lane = channel of
+// the 32-channel tensor w, whose pixels are read once each; the 3 x 3 window
+// of the complex (2-channel) image t around a pixel slides along x in
+// registers, so a pixel costs one 2-byte load and three broadcast 8-byte
+// loads for 36 FMAs. A warp takes rows of 32 pixels.
+//   OUT6 (layer 6): w = activations at q, t = output gradient: tap k of pixel q
+//          meets t at q - off(k); outputs [co 2][tap][ci = lane], bias from t
+//   else (layer 1): w = output gradient at p, t = input: tap k meets t at
+//          p + off(k); outputs [co = lane][tap][ci 2], bias from w
+constexpr int WT_WARPS = 8;
+
+template <bool OUT6>
+__global__ void __launch_bounds__(32 * WT_WARPS) k_wgrad_thin(const bf16* __restrict__ w, const float2* __restrict__ t,
+		int X, int Y, int tx, long nrows, float* __restrict__ part)
+{
+	constexpr int O = 2 * 9 * NET_C;
+	constexpr int OB = OUT6 ? 2 : NET_C;		// bias gradients
+	__shared__ float red[WT_WARPS][O + NET_C];
+	__shared__ float2 win[WT_WARPS][3][NET_TILE_X + 2];
+	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+	float2 acc[9];
+	float2 bsum = make_float2(0.f, 0.f);
+#pragma unroll
+	for (int k = 0; k < 9; k++)
+		acc[k] = make_float2(0.f, 0.f);
+
+	// work rows: 32 pixels of one image row; tx of them per image row
+	for (long row = (long)blockIdx.x * WT_WARPS + warp; row < nrows; row += (long)gridDim.x * WT_WARPS) {
+
+		const int x0 = (int)(row % tx) * NET_TILE_X;
+		const long iy = row / tx;			// image row over all images
+		const int y = (int)(iy % Y);
+		const long base = (iy - y) * X;
+		__syncwarp();
+
+		for (int i = lane; i < 3 * (NET_TILE_X + 2); i += 32) {
+
+			const int dy = i / (NET_TILE_X + 2), dx = i % (NET_TILE_X + 2);
+			const int yy = y + dy - 1, xx = x0 + dx - 1;
+			win[warp][dy][dx] = ((yy >= 0) && (yy < Y) && (xx >= 0) && (xx < X)) ? t[base + (long)yy * X + xx]
+					: make_float2(0.f, 0.f);
+		}
+
+		__syncwarp();
+		const bf16* wp = w + (base + (long)y * X + x0) * NET_C + lane;
+		const int n = min(NET_TILE_X, X - x0);
+		float2 c0[3], c1[3], c2[3];			// window columns x - 1, x, x + 1
+#pragma unroll
+		for (int d = 0; d < 3; d++) {
+
+			c0[d] = win[warp][d][0];
+			c1[d] = win[warp][d][1];
+		}
+#pragma unroll 8
+		for (int px = 0; px < NET_TILE_X; px++) {
+
+			const float v = (px < n) ? __bfloat162float(wp[(long)px * NET_C]) : 0.f;
+#pragma unroll
+			for (int d = 0; d < 3; d++)
+				c2[d] = win[warp][d][px + 2];
+#pragma unroll
+			for (int d = 0; d < 3; d++) {
+
+				const int r0 = OUT6 ? 3 * (2 - d) + 2 : 3 * d;		// the tap that meets row d, column x - 1
+				const int r1 = OUT6 ? 3 * (2 - d) + 1 : 3 * d + 1;
+				const int r2 = OUT6 ? 3 * (2 - d) : 3 * d + 2;
+				acc[r0].x = fmaf(v, c0[d].x, acc[r0].x);
+				acc[r0].y = fmaf(v, c0[d].y, acc[r0].y);
+				acc[r1].x = fmaf(v, c1[d].x, acc[r1].x);
+				acc[r1].y = fmaf(v, c1[d].y, acc[r1].y);
+				acc[r2].x = fmaf(v, c2[d].x, acc[r2].x);
+				acc[r2].y = fmaf(v, c2[d].y, acc[r2].y);
+			}
+
+			if (!OUT6)
+				bsum.x += v;
+#pragma unroll
+			for (int d = 0; d < 3; d++) {
+
+				c0[d] = c1[d];
+				c1[d] = c2[d];
+			}
+		}
+
+		if (OUT6) {	// lane's pixel of the row: the bias gradient (summed over lanes below)
+
+			const float2 v = win[warp][1][lane + 1];
+
+			if (lane < n) {
+
+				bsum.x += v.x;
+				bsum.y += v.y;
+			}
+		}
+	}
+
+#pragma unroll
+	for (int k = 0; k < 9; k++) {
+
+		red[warp][OUT6 ? k * NET_C + lane : (lane * 9 + k) * 2] = acc[k].x;
+		red[warp][OUT6 ? (9 + k) * NET_C + lane : (lane * 9 + k) * 2 + 1] = acc[k].y;
+	}
+
+	if (OUT6) {
+
+		for (int o = 16; o > 0; o >>= 1) {
+
+			bsum.x += __shfl_xor_sync(0xffffffffu, bsum.x, o);
+			bsum.y += __shfl_xor_sync(0xffffffffu, bsum.y, o);
+		}
+
+		if (0 == lane) {
+
+			red[warp][O] = bsum.x;
+			red[warp][O + 1] = bsum.y;
+		}
+
+	} else {
+
+		red[warp][O + lane] = bsum.x;
 	}
 
 	__syncthreads();
 
-	float* dst = part + (long)(blockIdx.x + gridDim.x * (blockIdx.y + (long)gridDim.y * blockIdx.z)) * (O + COUT);
+	for (int o = threadIdx.x; o < O + OB; o += 32 * WT_WARPS) {
 
-	for (int o = threadIdx.x; o < O + COUT; o += NET_THREADS) {
+		float s = 0.f;
+#pragma unroll
+		for (int k = 0; k < WT_WARPS; k++)
+			s += red[k][o];
 
-		float acc = 0.f;
-
-		if (o < O) {
-
-			const int co = o / (9 * CIN);
-			const int tap = (o / CIN) % 9;
-			const int ci = o % CIN;
-			const int ky = tap / 3;
-			const int kx = tap % 3;
-#pragma unroll 4
-			for (int py = 0; py < NET_TILE_Y; py++)
-				for (int px = 0; px < NET_TILE_X; px++)
-					acc = fmaf(sg[(py * NET_TILE_X + px) * COUT + co],
-						sa[((py + ky) * NET_HALO_X + px + kx) * CIN + ci], acc);
-
-		} else {
-
-			const int co = o - O;
-
-			for (int pix = 0; pix < NET_TILE_Y * NET_TILE_X; pix++)
-				acc += sg[pix * COUT + co];
-		}
-
-		dst[o] = acc;
+		part[(long)blockIdx.x * (O + OB) + o] = s;
 	}
 }
 
-// grad[o] = sum over blocks of part[blk][o], in block order
-__global__ void k_wgrad_reduce(const float* __restrict__ part, long nblk, int O, float* __restrict__ grad)
+// grad[o] = sum over blocks of part[blk][o] in float64: 32 outputs per block,
+// eight slices of the partials, combined in a fixed order
+__global__ void __launch_bounds__(256) k_wgrad_reduce(const float* __restrict__ part, int nblk, int O,
+		float* __restrict__ grad)
 {
-	const int o = blockIdx.x * blockDim.x + threadIdx.x;
-
-	if (o >= O)
-		return;
-
+	__shared__ double sh[8][32];
+	const int o = blockIdx.x * 32 + threadIdx.x % 32, sl = threadIdx.x / 32;
 	double acc = 0.;
 
-	for (long k = 0; k < nblk; k++)
-		acc += part[k * O + o];
+	if (o < O) {
+#pragma unroll 4
+		for (int k = sl; k < nblk; k += 8)
+			acc += part[(long)k * O + o];
+	}
 
-	grad[o] = (float)acc;
+	sh[sl][threadIdx.x % 32] = acc;
+	__syncthreads();
+
+	if ((0 == sl) && (o < O)) {
+
+		for (int k = 1; k < 8; k++)
+			acc += sh[k][threadIdx.x];
+
+		grad[o] = (float)acc;
+	}
 }
 
 // gout = c (out - target), loss partials sum |out - target|^2 per block

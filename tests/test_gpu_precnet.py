@@ -83,6 +83,27 @@ def test_gradients_vs_oracle():
         assert rel(g[bo:e], go[bo:e]) < 1e-2, li
 
 
+@pytest.mark.parametrize("X,Y,n", [(1, 1, 1), (5, 3, 2), (32, 8, 1), (33, 9, 3), (31, 130, 1), (320, 250, 1)])
+def test_gradients_tile_edges(X, Y, n):
+    """Weight and bias gradients where the 32 x 8 pixel tiles and 32-pixel rows
+    of the persistent kernels end: one pixel, a tile exactly and one pixel
+    more, several images, more tiles (320) than blocks. The kernels sum exact
+    bf16 products in float32; the tolerance is that of test_gradients_vs_oracle
+    (an activation or a gradient may round to its other bf16 neighbour, 2^-8)."""
+    rng = np.random.default_rng(X * 1000 + Y + n)
+    p = _params(rng)
+    x, t = _img(rng, X, Y, n), _img(rng, X, Y, n)
+    net = precnet.PrecNet(p)
+    g = np.zeros(po.NPARAMS, dtype=np.float32)
+    loss = net.train_step(x, t, X, Y, n, 0.0, grads=g)
+    net.free()
+    lo, go = po.loss_and_grad(p, po.to_channels(x), po.to_channels(t), bf16_mode=True)
+    assert abs(loss - lo) <= 1e-4 * lo
+    for li, (wo, bo, e) in enumerate(po.offsets()):
+        assert rel(g[wo:bo], go[wo:bo]) < 1e-2, li
+        assert rel(g[bo:e], go[bo:e]) < 1e-2, li
+
+
 def test_gradients_bit_reproducible():
     rng = np.random.default_rng(6)
     p = _params(rng)
