@@ -88,8 +88,10 @@ def test_gradients_tile_edges(X, Y, n):
     """Weight and bias gradients where the 32 x 8 pixel tiles and 32-pixel rows
     of the persistent kernels end: one pixel, a tile exactly and one pixel
     more, several images, more tiles (320) than blocks. The kernels sum exact
-    bf16 products in float32; the tolerance is that of test_gradients_vs_oracle
-    (an activation or a gradient may round to its other bf16 neighbour, 2^-8)."""
+    bf16 products in float32, so they differ from the oracle only where an
+    activation or gradient rounds to its other bf16 neighbour (2^-8 relative);
+    a layer's gradient has up to five such roundings behind it, and few pixels
+    average nothing out: 5 * 2^-8."""
     rng = np.random.default_rng(X * 1000 + Y + n)
     p = _params(rng)
     x, t = _img(rng, X, Y, n), _img(rng, X, Y, n)
@@ -100,8 +102,8 @@ def test_gradients_tile_edges(X, Y, n):
     lo, go = po.loss_and_grad(p, po.to_channels(x), po.to_channels(t), bf16_mode=True)
     assert abs(loss - lo) <= 1e-4 * lo
     for li, (wo, bo, e) in enumerate(po.offsets()):
-        assert rel(g[wo:bo], go[wo:bo]) < 1e-2, li
-        assert rel(g[bo:e], go[bo:e]) < 1e-2, li
+        assert rel(g[wo:bo], go[wo:bo]) < 5 * 2.0 ** -8, li
+        assert rel(g[bo:e], go[bo:e]) < 5 * 2.0 ** -8, li
 
 
 def test_gradients_bit_reproducible():
