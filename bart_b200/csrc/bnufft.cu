@@ -756,15 +756,17 @@ struct Bins {
 	// output-stationary scatter (k_grid6_tiles): bins are its tiles
 	int tg_cfg = -1;		// kernel shape (TG_*), -1: not used
 	long ntiles = 0;
-	int* bin_start = nullptr;	// [nbins + 1]
+	int* hit_start = nullptr;	// [ntiles + 1]
+	int* hits = nullptr;		// samples that meet each tile
 	int* work_tile = nullptr;	// [nwork_max]
 	int* work_chunk = nullptr;
 	int* work_start = nullptr;	// [ntiles + 1]; work_start[ntiles] = work items
-	unsigned char* multi = nullptr;	// [ntiles]
+	int* multi = nullptr;		// [ntiles + 1] tiles with several work items; their number in [ntiles]
 	long nwork_max = 0;		// upper bound of work items (launch size)
-	int cand = 512;			// candidates per work item
+	int chunk = 256;		// hits per work item
 	float4* foot = nullptr;		// [M][FOOT_F4] footprints of the sorted samples
-	float2* kperm = nullptr;	// [M][kperm_c] k-space in bin order (large problems)
+	bool gather = false;		// they serve the degridding (k_degrid6_quads)
+	float2* kperm = nullptr;	// [M][kperm_c] k-space in bin order, a sample's coils side by side
 	long kperm_c = 0;
 };
 
@@ -798,7 +800,7 @@ struct OpCtx {
 
 static void free_bins(Bins& b, cudaStream_t st)
 {
-	void* ptrs[] = { b.perm, b.traj, b.sub_bin, b.sub_first, b.sub_count, b.sub_start, b.bin_start, b.work_tile,
+	void* ptrs[] = { b.perm, b.traj, b.sub_bin, b.sub_first, b.sub_count, b.sub_start, b.hit_start, b.hits, b.work_tile,
 			b.work_chunk, b.work_start, b.multi, b.foot, b.kperm };
 
 	for (void* q : ptrs)
@@ -1073,18 +1075,31 @@ static int op_spectrum_adjoint(OpCtx& op, const float2* grid, const float2* maps
 			dh.p, dh.part, dh.done, dh.nblocks);
 }
 
+// grid -> k-space of C channels, times the plan's weights
 static int degrid(OpCtx& op, const float2* grid, long C, float2* ksp, cudaStream_t st)
 {
-	if (op.bins.perm && (6.f == op.g.width)) {
+	const long M = op.g.M;
+
+	if (op.bins.foot && op.bins.gather) {
 
 		const Bins& b = op.bins;
 		cudaEvent_t pe = prof_begin("degrid", st);
-		unsigned nb = (unsigned)((op.g.M + BIN_THREADS - 1) / BIN_THREADS);
+		const long nb = (4 * M + BIN_THREADS - 1) / BIN_THREADS;
+		// channels per block: all of them (the weights are read once), fewer
+		// (in fours) when the samples alone give less than a few blocks per SM
+		int cpb = (int)C;
+
+		while ((cpb > 4) && (nb * ((C + cpb - 1) / cpb) < 8 * 148))
+			cpb = std::max(4, (cpb / 2 + 3) / 4 * 4);
+
+		const dim3 blocks((unsigned)nb, (unsigned)((C + cpb - 1) / cpb));
 
 		if (op.g.G[2] > 1)
-			k_degrid6<6><<<nb, BIN_THREADS, 0, st>>>(b.traj, b.perm, op.g.M, grid_geom(op.g), (int)C, grid, ksp, op.kb);
+			k_degrid6_quads<6><<<blocks, BIN_THREADS, 0, st>>>(b.foot, b.perm, M, grid_geom(op.g), (int)C, cpb, grid, ksp,
+					op.wgt, (int)op.wgt_c);
 		else
-			k_degrid6<1><<<nb, BIN_THREADS, 0, st>>>(b.traj, b.perm, op.g.M, grid_geom(op.g), (int)C, grid, ksp, op.kb);
+			k_degrid6_quads<1><<<blocks, BIN_THREADS, 0, st>>>(b.foot, b.perm, M, grid_geom(op.g), (int)C, cpb, grid, ksp,
+					op.wgt, (int)op.wgt_c);
 
 		prof_end(pe, st);
 		LAUNCHED();
@@ -1092,16 +1107,53 @@ static int degrid(OpCtx& op, const float2* grid, long C, float2* ksp, cudaStream
 	}
 
 	int cpc = (int)std::min<long>(C, 8);
-	dim3 blocks((unsigned)((op.g.M + 127) / 128), (unsigned)((C + cpc - 1) / cpc));
+	dim3 blocks((unsigned)((M + 127) / 128), (unsigned)((C + cpc - 1) / cpc));
 	cudaEvent_t pe = prof_begin("degrid", st);
-	k_degrid<<<blocks, 128, 0, st>>>(op.traj, op.g.M, grid_geom(op.g), (int)C, cpc, grid, ksp, op.kb);
+	k_degrid<<<blocks, 128, 0, st>>>(op.traj, M, grid_geom(op.g), (int)C, cpc, grid, ksp, op.kb);
 	prof_end(pe, st);
+	LAUNCHED();
+
+	if (op.wgt) {
+
+		k_weight<<<vec_blocks(M * C), RED_THREADS, 0, st>>>(ksp, ksp, op.wgt, M, C, op.wgt_c, 0);
+		LAUNCHED();
+	}
+
+	return BNUFFT_OK;
+}
+
+// channels of a row of the bin-ordered k-space (16-byte copies: even)
+static long tg_row(long C) { return (C > 1) ? (C + 1) / 2 * 2 : 1; }
+
+template <int TX, int LY, int LZ, int CT>
+static int launch_tiles(const OpCtx& op, const TileWork& tw, int C, const float2* ksp, float2* grid, cudaStream_t st)
+{
+	constexpr int NL = LY * LZ, CW = 32 / NL * CT;
+	constexpr size_t smem = sizeof(float) * TG_WARPS * TgStage<NL, CW>::FLOATS;
+	const Bins& b = op.bins;
+	const unsigned nblk = (unsigned)((b.nwork_max * ((C + CW - 1) / CW) + TG_WARPS - 1) / TG_WARPS);
+	auto kern = k_grid6_tiles<TX, LY, LZ, CT>;
+	TRY(prep_kernel(kern, smem));
+	kern<<<nblk, 32 * TG_WARPS, smem, st>>>(op.g.M, grid_geom(op.g), b.bg, tw, C, (int)tg_row(C), ksp, grid);
 	LAUNCHED();
 	return BNUFFT_OK;
 }
 
+// k-space of C channels, times the conjugate of the plan's weights -> grid
 static int grid_adj(OpCtx& op, const float2* ksp, long C, float2* grid, cudaStream_t st)
 {
+	const bool tiles = !op.csr.row_ptr && op.bins.perm && (op.bins.tg_cfg >= 0);
+
+	if (op.wgt && !tiles) {
+
+		if (!op.wbuf)
+			CUDA_TRY(cudaMallocAsync(&op.wbuf, sizeof(float2) * op.g.M * C, st));
+
+		k_weight<<<vec_blocks(op.g.M * C), RED_THREADS, 0, st>>>(op.wbuf, ksp, op.wgt, op.g.M, C, op.wgt_c, 1);
+		LAUNCHED();
+		ksp = op.wbuf;
+	}
+
 	if (op.csr.row_ptr) {	// deterministic: fixed-order gather per cell
 
 		int cpc = (int)std::min<long>(C, 8);
@@ -1113,64 +1165,51 @@ static int grid_adj(OpCtx& op, const float2* ksp, long C, float2* grid, cudaStre
 		return BNUFFT_OK;
 	}
 
-	if (op.bins.perm && (op.bins.tg_cfg >= 0)) {	// output-stationary tiles: no clearing pass
+	if (tiles) {	// output-stationary tiles: no clearing pass
 
 		Bins& b = op.bins;
 		const GridGeom gg = grid_geom(op.g);
-		TileWork tw = { b.bin_start, b.work_tile, b.work_chunk, b.work_start + b.ntiles, b.multi, b.foot, b.cand };
-		int sorted = 0;
+		const long Cp = tg_row(C);
+		TileWork tw = { b.hit_start, b.hits, b.work_tile, b.work_chunk, b.work_start + b.ntiles, b.foot, b.chunk };
 
-		// k-space in bin order (one pass), so the tiles read their samples'
-		// values coalesced
-		if (C > 1) {
+		if (b.kperm_c < Cp) {	// more channels than the plan was made for (not while capturing)
 
-			if (b.kperm_c < C) {	// more channels than the plan was made for (not while capturing)
+			if (b.kperm)
+				cudaFreeAsync(b.kperm, st);
 
-				if (b.kperm)
-					cudaFreeAsync(b.kperm, st);
-
-				b.kperm = nullptr;
-				b.kperm_c = 0;
-				CUDA_TRY(cudaMallocAsync(&b.kperm, sizeof(float2) * op.g.M * C, st));
-				b.kperm_c = C;
-			}
-
-			k_permute_ksp<<<vec_blocks(op.g.M * C, 256, 16 * 148), 256, 0, st>>>(b.kperm, ksp, b.perm, op.g.M, (int)C);
-			LAUNCHED();
-			ksp = b.kperm;
-			sorted = 1;
+			b.kperm = nullptr;
+			b.kperm_c = 0;
+			CUDA_TRY(cudaMallocAsync(&b.kperm, sizeof(float2) * op.g.M * Cp, st));
+			b.kperm_c = Cp;
 		}
 
-		cudaEvent_t pe = prof_begin("grid", st);
-		k_zero_tiles<<<(unsigned)std::min<long>(b.ntiles, 8 * 148), 256, 0, st>>>(grid, gg, b.bg, b.multi, b.ntiles, (int)C);
+		const dim3 pb((unsigned)((op.g.M + 31) / 32), (unsigned)((Cp + 31) / 32));
+		k_permute_ksp<<<pb, 256, 0, st>>>(b.kperm, ksp, b.perm, op.g.M, (int)C, (int)Cp, op.wgt, (int)op.wgt_c);
 		LAUNCHED();
-		int t[3];
-		tg_shape(b.tg_cfg, t);
-		const int gpw = 32 / (t[1] * t[2]);
-		const int ct = (TG_3D_C8 == b.tg_cfg) ? 4 : ((TG_2D_C8 == b.tg_cfg) || (TG_2D_C4 == b.tg_cfg) ? 2 : 1);
-		const long ncq = (C + gpw * ct - 1) / (gpw * ct);
-		const unsigned nblk = (unsigned)((b.nwork_max * ncq + TG_WARPS - 1) / TG_WARPS);
+		cudaEvent_t pe = prof_begin("grid", st);
+		k_zero_tiles<<<(unsigned)std::min<long>((b.ntiles * C + 7) / 8, 8 * 148), 256, 0, st>>>(grid, gg, b.bg, b.multi,
+				b.multi + b.ntiles, (int)C);
+		LAUNCHED();
 
 		switch (b.tg_cfg) {
 		case TG_2D_C1:
-			k_grid6_tiles<16, 32, 1, 1><<<nblk, 32 * TG_WARPS, 0, st>>>(b.perm, op.g.M, gg, b.bg, tw, (int)C, ksp, sorted, grid);
+			TRY((launch_tiles<16, 32, 1, 1>(op, tw, (int)C, b.kperm, grid, st)));
 			break;
 		case TG_2D_C4:
-			k_grid6_tiles<16, 16, 1, 2><<<nblk, 32 * TG_WARPS, 0, st>>>(b.perm, op.g.M, gg, b.bg, tw, (int)C, ksp, sorted, grid);
+			TRY((launch_tiles<16, 16, 1, 2>(op, tw, (int)C, b.kperm, grid, st)));
 			break;
 		case TG_2D_C8:
-			k_grid6_tiles<16, 8, 1, 2><<<nblk, 32 * TG_WARPS, 0, st>>>(b.perm, op.g.M, gg, b.bg, tw, (int)C, ksp, sorted, grid);
+			TRY((launch_tiles<16, 8, 1, 2>(op, tw, (int)C, b.kperm, grid, st)));
 			break;
 		case TG_3D_C1:
-			k_grid6_tiles<8, 8, 4, 1><<<nblk, 32 * TG_WARPS, 0, st>>>(b.perm, op.g.M, gg, b.bg, tw, (int)C, ksp, sorted, grid);
+			TRY((launch_tiles<8, 8, 4, 1>(op, tw, (int)C, b.kperm, grid, st)));
 			break;
 		default:
-			k_grid6_tiles<8, 4, 4, 4><<<nblk, 32 * TG_WARPS, 0, st>>>(b.perm, op.g.M, gg, b.bg, tw, (int)C, ksp, sorted, grid);
+			TRY((launch_tiles<8, 4, 4, 4>(op, tw, (int)C, b.kperm, grid, st)));
 			break;
 		}
 
 		prof_end(pe, st);
-		LAUNCHED();
 		return BNUFFT_OK;
 	}
 
@@ -1293,8 +1332,23 @@ static int build_csr(OpCtx& op, cudaStream_t st)
 	return BNUFFT_OK;
 }
 
-// Sort the samples by bin and cut bins into sub-blocks (plan time).
-static int build_bins(OpCtx& op, cudaStream_t st)
+// tiles that one sample can meet at most: its six cells per axis meet two
+// tiles of at least six cells, three shorter ones, and on periodic grids one
+// more where the last tile is cut short
+static long tg_max_hits(const Geom& g, const BinGeom& bg)
+{
+	long n = 1;
+
+	for (int a = 0; a < 3; a++)
+		if (g.G[a] > 1)
+			n *= ((bg.bs[a] < 6) || (g.periodic && (0 != g.G[a] % bg.bs[a]))) ? 3 : 2;
+
+	return n;
+}
+
+// Sort the samples by bin and cut bins into sub-blocks (plan time). gather:
+// the plan also degrids.
+static int build_bins(OpCtx& op, cudaStream_t st, bool gather)
 {
 	const Geom& g = op.g;
 	Bins& b = op.bins;
@@ -1348,6 +1402,9 @@ static int build_bins(OpCtx& op, cudaStream_t st)
 
 	if ((g.M >= (1L << 31)) || (nbins >= (1L << 31)))
 		return fail(BNUFFT_ERR_UNSUPPORTED, "binning: %ld samples, %ld bins", g.M, nbins);
+
+	if ((b.tg_cfg >= 0) && (g.M * tg_max_hits(g, bg) >= (1L << 31)))	// hit lists are indexed with ints
+		b.tg_cfg = -1;
 
 	unsigned *keys = nullptr, *keys2 = nullptr;
 	int *vals = nullptr, *counts = nullptr, *bin_start = nullptr, *nsub = nullptr, *sub_start = nullptr;
@@ -1414,60 +1471,71 @@ static int build_bins(OpCtx& op, cudaStream_t st)
 	// coil tiles per pass: as many as fit in ~110 KB of shared memory
 	b.cc = (int)std::max(1L, std::min(8L, (110L * 1024) / (long)(sizeof(float2) * bg.ncells)));
 
-	// work items of the output-stationary scatter: each tile's candidates
-	// (the samples of its neighbour bins) in chunks of b.cand
-	if (b.tg_cfg >= 0) {
+	// the samples' footprints (start cells and weights): they depend on
+	// the trajectory only, so every apply reads them instead of recomputing
+	// 18 table lookups per sample. The degridding needs sides of at least 16
+	// cells and z offsets that fit an int; other sizes take k_degrid.
+	b.gather = gather && (6.f == g.width) && (g.gsz < (1L << 31));
 
-		const long nt = nbins;
-		const int nneigh = (g.G[2] > 1) ? 27 : 9;
-		int* nwork = nullptr;
-		void* wtmp = nullptr;
-		size_t wtmp_bytes = 0;
-		b.ntiles = nt;
-		b.bin_start = bin_start;
-		bin_start = nullptr;	// kept by the plan
-		b.cand = (g.G[2] > 1) ? 1024 : 256;	// measured best (256..1024 tried)
+	for (int a = 0; a < 3; a++)
+		b.gather = b.gather && ((1 == g.G[a]) || (g.G[a] >= 16));
 
-		if (const char* e = getenv("BNUFFT_GRID_CAND"))	// tuning knob: candidates per work item
-			b.cand = std::max(64, std::min(4096, atoi(e)));
+	if ((b.tg_cfg >= 0) || b.gather) {
 
-		b.nwork_max = nt + (M * nneigh + b.cand - 1) / b.cand;
-
-		if (b.nwork_max >= (1L << 31))
-			return fail(BNUFFT_ERR_UNSUPPORTED, "gridding: %ld work items", b.nwork_max);
-
-		CUDA_TRY(cudaMallocAsync(&nwork, sizeof(int) * (nt + 1), st));
-		CUDA_TRY(cudaMallocAsync(&b.work_start, sizeof(int) * (nt + 1), st));
-		CUDA_TRY(cudaMallocAsync(&b.multi, nt, st));
-		CUDA_TRY(cudaMallocAsync(&b.work_tile, sizeof(int) * b.nwork_max, st));
-		CUDA_TRY(cudaMallocAsync(&b.work_chunk, sizeof(int) * b.nwork_max, st));
-		CUDA_TRY(cudaMemsetAsync(nwork + nt, 0, sizeof(int), st));
-		k_tile_cand<<<vec_blocks(nt), RED_THREADS, 0, st>>>(b.bin_start, bg, g.periodic, nt, b.cand, nwork, b.multi);
-		LAUNCHED();
-		CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, wtmp_bytes, nwork, b.work_start, (int)(nt + 1), st));
-		CUDA_TRY(cudaMallocAsync(&wtmp, wtmp_bytes, st));
-		CUDA_TRY(cub::DeviceScan::ExclusiveSum(wtmp, wtmp_bytes, nwork, b.work_start, (int)(nt + 1), st));
-		g_launches.fetch_add(1, std::memory_order_relaxed);
-		k_work_fill<<<vec_blocks(nt), RED_THREADS, 0, st>>>(b.work_start, nt, b.work_tile, b.work_chunk);
-		LAUNCHED();
-		cudaFreeAsync(nwork, st);
-		cudaFreeAsync(wtmp, st);
-
-		// the samples' footprints (start cells and weights): they depend on
-		// the trajectory only, so every apply reads them instead of
-		// recomputing 18 table lookups per sample and tile
 		CUDA_TRY(cudaMallocAsync(&b.foot, sizeof(float4) * FOOT_F4 * M, st));
 		k_foot<<<vec_blocks(M, 128, 8 * 148), 128, 0, st>>>(b.traj, M, grid_geom(g), op.kb, b.foot);
 		LAUNCHED();
+	}
+
+	// the output-stationary scatter: the samples that meet each tile, and the
+	// work items (chunks of them)
+	if (b.tg_cfg >= 0) {
+
+		const long nt = nbins;
+		int *nwork = nullptr, *cursor = nullptr;
+		void* wtmp = nullptr;
+		size_t wtmp_bytes = 0;
+		b.ntiles = nt;
+		b.chunk = (g.G[2] > 1) ? 256 : 64;
+
+		if (const char* e = getenv("BNUFFT_GRID_CHUNK"))	// tuning knob: hits per work item
+			b.chunk = std::max(32, std::min(4096, atoi(e)));
+
+		b.nwork_max = nt + (M * tg_max_hits(g, bg) + b.chunk - 1) / b.chunk;
+		CUDA_TRY(cudaMallocAsync(&nwork, sizeof(int) * (nt + 1), st));
+		CUDA_TRY(cudaMallocAsync(&cursor, sizeof(int) * (nt + 1), st));
+		CUDA_TRY(cudaMallocAsync(&b.hit_start, sizeof(int) * (nt + 1), st));
+		CUDA_TRY(cudaMallocAsync(&b.hits, sizeof(int) * M * tg_max_hits(g, bg), st));
+		CUDA_TRY(cudaMallocAsync(&b.work_start, sizeof(int) * (nt + 1), st));
+		CUDA_TRY(cudaMallocAsync(&b.multi, sizeof(int) * (nt + 1), st));
+		CUDA_TRY(cudaMallocAsync(&b.work_tile, sizeof(int) * b.nwork_max, st));
+		CUDA_TRY(cudaMallocAsync(&b.work_chunk, sizeof(int) * b.nwork_max, st));
+		CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, wtmp_bytes, cursor, b.hit_start, (int)(nt + 1), st));
+		CUDA_TRY(cudaMallocAsync(&wtmp, wtmp_bytes, st));
+		CUDA_TRY(cudaMemsetAsync(cursor, 0, sizeof(int) * (nt + 1), st));
+		CUDA_TRY(cudaMemsetAsync(b.multi + nt, 0, sizeof(int), st));
+		k_tile_hits<<<vec_blocks(M), RED_THREADS, 0, st>>>(b.foot, M, grid_geom(g), bg, cursor, nullptr);
+		LAUNCHED();
+		CUDA_TRY(cub::DeviceScan::ExclusiveSum(wtmp, wtmp_bytes, cursor, b.hit_start, (int)(nt + 1), st));
+		CUDA_TRY(cudaMemcpyAsync(cursor, b.hit_start, sizeof(int) * nt, cudaMemcpyDeviceToDevice, st));
+		k_tile_hits<<<vec_blocks(M), RED_THREADS, 0, st>>>(b.foot, M, grid_geom(g), bg, cursor, b.hits);
+		LAUNCHED();
+		k_tile_work<<<vec_blocks(nt + 1), RED_THREADS, 0, st>>>(b.hit_start, nt, b.chunk, nwork);
+		LAUNCHED();
+		CUDA_TRY(cub::DeviceScan::ExclusiveSum(wtmp, wtmp_bytes, nwork, b.work_start, (int)(nt + 1), st));
+		g_launches.fetch_add(2, std::memory_order_relaxed);
+		k_work_fill<<<vec_blocks(nt), RED_THREADS, 0, st>>>(b.work_start, nt, b.work_tile, b.work_chunk, b.multi,
+				b.multi + nt);
+		LAUNCHED();
+		cudaFreeAsync(nwork, st);
+		cudaFreeAsync(cursor, st);
+		cudaFreeAsync(wtmp, st);
 
 		// the bin-ordered k-space of the applies, allocated here so that
 		// applies allocate nothing (their solves can then be captured into
 		// graphs and nested as child graphs)
-		if (op.coils > 1) {
-
-			CUDA_TRY(cudaMallocAsync(&b.kperm, sizeof(float2) * M * op.coils, st));
-			b.kperm_c = op.coils;
-		}
+		b.kperm_c = tg_row(op.coils);
+		CUDA_TRY(cudaMallocAsync(&b.kperm, sizeof(float2) * M * b.kperm_c, st));
 	}
 
 	void* frees[] = { keys, keys2, vals, counts, bin_start, nsub, tmp };
@@ -1484,15 +1552,7 @@ static int op_forward(OpCtx& op, const float2* cim, const float2* maps, long C, 
 {
 	TRY(alloc_work(op.w, op.g, C, st));
 	TRY(op_spectrum(op, cim, maps, true, C, op.w.grid, st));
-	TRY(degrid(op, op.w.grid, C, ksp, st));
-
-	if (op.wgt) {
-
-		k_weight<<<vec_blocks(op.g.M * C), RED_THREADS, 0, st>>>(ksp, ksp, op.wgt, op.g.M, C, op.wgt_c, 0);
-		LAUNCHED();
-	}
-
-	return BNUFFT_OK;
+	return degrid(op, op.w.grid, C, ksp, st);
 }
 
 // adjoint NUFFT: ksp [M, C] -> cim [npix, C] (maps: partial coil sums)
@@ -1500,16 +1560,6 @@ static int op_adjoint(OpCtx& op, const float2* ksp, const float2* maps, long C, 
 		const DotHook& dh = DotHook())
 {
 	TRY(alloc_work(op.w, op.g, C, st));
-
-	if (op.wgt) {
-
-		if (!op.wbuf)
-			CUDA_TRY(cudaMallocAsync(&op.wbuf, sizeof(float2) * op.g.M * C, st));
-
-		k_weight<<<vec_blocks(op.g.M * C), RED_THREADS, 0, st>>>(op.wbuf, ksp, op.wgt, op.g.M, C, op.wgt_c, 1);
-		LAUNCHED();
-		ksp = op.wbuf;
-	}
 
 	TRY(grid_adj(op, ksp, C, op.w.grid, st));
 	return op_spectrum_adjoint(op, op.w.grid, maps, true, C, cpg, out, st, dh);
@@ -1632,7 +1682,7 @@ static int compute_psf(const Geom& g, const float2* traj_c, const float* kb, flo
 	in.kb = kb;
 	TRY(init_rolloff(in, st));
 
-	TRY(build_bins(in, st));
+	TRY(build_bins(in, st, false));
 
 	if (deterministic)
 		TRY(build_csr(in, st));
@@ -2130,7 +2180,7 @@ static int upload_traj(bnufft_plan_s* p, const void* traj, cudaStream_t st, bool
 
 	// the chained NUFFT (os != 2) grids with the generic per-sample kernels
 	if ((BNUFFT_OK == s) && !p->op.g.chain)
-		s = build_bins(p->op, st);
+		s = build_bins(p->op, st, true);
 
 	if ((BNUFFT_OK == s) && p->conf.deterministic) {
 

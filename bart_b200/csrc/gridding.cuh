@@ -6,9 +6,9 @@
 // (dense bins at the k-space centre become several sub-blocks, so the work
 // is balanced). The sorted trajectory is stored as float4 (coalesced loads).
 //
-// Degridding (gather): one thread per sample in bin order; neighbouring
-// threads read overlapping taps, so the gathers hit L1, and the weights are
-// computed once per sample for all coils.
+// Degridding (gather): four lanes per sample in bin order; neighbouring
+// samples read overlapping taps, so the gathers hit L1, and the weights are
+// read once per sample for all coils.
 // Gridding (scatter), default: one thread per sample in bin order with one
 // global float2 atomic per tap (bin order keeps a block's atomics within a
 // few L2 lines). Alternative (BNUFFT_GRIDDING=tiles): a block takes one
@@ -237,111 +237,6 @@ __device__ __forceinline__ void axis_taps6(float k, int N, int periodic, const f
 	}
 }
 
-// Degridding, width 6: one thread per sample in bin order (coalesced float4
-// trajectory loads, neighbouring threads share taps in L1), weights computed
-// once and reused for every coil. TZ = 6 for 3D, 1 for 2D.
-template <int TZ>
-__global__ void __launch_bounds__(BIN_THREADS, 2) k_degrid6(const float4* __restrict__ traj_sorted,
-		const int* __restrict__ perm, long M, GridGeom g, int C,
-		const float2* __restrict__ grid, float2* __restrict__ ksp, const float* __restrict__ kbg)
-{
-	__shared__ float kb[KB_TABLE_N + 1];
-
-	for (int i = threadIdx.x; i <= KB_TABLE_N; i += blockDim.x)
-		kb[i] = kbg[i];
-
-	__syncthreads();
-
-	long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-
-	if (i >= M)
-		return;
-
-	float4 k = traj_sorted[i];
-	Taps6 tx, ty, tz;
-	axis_taps6<0>(k.x, g.N[0], g.periodic, kb, 0, tx);
-	axis_taps6<0>(k.y, g.N[1], g.periodic, kb, 0, ty);
-	axis_taps6<0>(k.z, g.N[2], g.periodic, kb, 0, tz);
-	const long m = perm[i];
-
-	// the x taps as an 8-cell window from an even cell: each (z, y) row is
-	// read with 4 float4 loads instead of 6 float2 gathers (the gather is
-	// bound by L1 requests); windows that wrap around the row read per tap
-	int lo = INT_MAX, hi = INT_MIN;
-#pragma unroll
-	for (int e = 0; e < 6; e++) {
-
-		if (0.f != tx.w[e]) {
-
-			lo = min(lo, tx.cell[e]);
-			hi = max(hi, tx.cell[e]);
-		}
-	}
-
-	const int base = lo & ~1;
-	const bool vec = (lo <= hi) && (hi - base < 8);
-	float wx8[8];
-#pragma unroll
-	for (int j = 0; j < 8; j++) {
-
-		float w = 0.f;	// taps with weight only (see k_grid6_atomic)
-#pragma unroll
-		for (int e = 0; e < 6; e++)
-			w = ((0.f != tx.w[e]) && (tx.cell[e] == base + j)) ? tx.w[e] : w;
-
-		wx8[j] = vec ? w : 0.f;
-	}
-
-	for (int c = 0; c < C; c++) {
-
-		const float2* gc = grid + g.gsz * c;
-		float2 acc = make_float2(0.f, 0.f);
-#pragma unroll 1
-		for (int a = 0; a < TZ; a++) {
-
-			float dz = tz.w[a];
-			long oz = (long)tz.cell[a] * g.G[1];
-#pragma unroll
-			for (int b = 0; b < 6; b++) {
-
-				float dzy = __fmul_rn(dz, ty.w[b]);
-				long oy = (oz + ty.cell[b]) * g.G[0];
-
-				if (vec) {
-#pragma unroll
-					for (int q = 0; q < 4; q++) {
-
-						// slots past the last tap hold no weight and are not
-						// read (the window may pass the end of the row)
-						if ((0.f == wx8[2 * q]) && (0.f == wx8[2 * q + 1]))
-							continue;
-
-						float d0 = __fmul_rn(dzy, wx8[2 * q]);
-						float d1 = __fmul_rn(dzy, wx8[2 * q + 1]);
-						float4 v = *(const float4*)(gc + oy + base + 2 * q);
-						acc.x = fmaf(v.x, d0, acc.x);
-						acc.y = fmaf(v.y, d0, acc.y);
-						acc.x = fmaf(v.z, d1, acc.x);
-						acc.y = fmaf(v.w, d1, acc.y);
-					}
-
-				} else {
-#pragma unroll
-					for (int e = 0; e < 6; e++) {
-
-						float d = __fmul_rn(dzy, tx.w[e]);
-						float2 v = gc[oy + tx.cell[e]];
-						acc.x = fmaf(v.x, d, acc.x);
-						acc.y = fmaf(v.y, d, acc.y);
-					}
-				}
-			}
-		}
-
-		ksp[m + M * c] = acc;
-	}
-}
-
 // Gridding, width 6: per sub-block, accumulate into shared-memory tiles of cc
 // coils with shared-memory atomics, then flush touched cells with one global
 // float2 atomic each. The grid must be zeroed.
@@ -567,44 +462,6 @@ __global__ void __launch_bounds__(BIN_THREADS, 2) k_grid6_atomic(const float4* _
 	}
 }
 
-// Gridding, width 6, output-stationary (the default scatter) ------------------
-//
-// The grid is cut into tiles that are the sample bins (TX x LY x LZ cells of
-// the centred oversampled grid). One warp job owns one tile and a group of
-// coils: lane (line, grp) holds the TX x-cells of tile line (y, z) = line
-// for CT coils in registers, so it accumulates without atomics. A sample's
-// taps lie within 3 cells of its centred position 2k + N on every axis
-// (cells 2w + s, |w - pos_s| <= 1.5), so the samples that reach a tile are
-// in the tile's bin and its 3^d - 1 neighbours: the warp scans those bins'
-// sorted samples 32 at a time, keeps the ones whose footprint meets the tile
-// (ballot + compaction into shared memory, with their weights and coil
-// values), and adds each kept sample to its lanes' cells. The x offset of a
-// sample is the same for the whole warp, so a switch on it selects a fully
-// unrolled update of exactly the taps inside the tile; lanes whose line is
-// outside the sample's y/z window skip it.
-//
-// Work items: a tile's candidates (the samples of its neighbourhood, in a
-// fixed bin order) are cut into chunks (TileWork.cand); tiles with one chunk
-// write their cells with plain stores (empty tiles write zeros, so the grid
-// needs no clearing), tiles with several chunks (the dense k-space centre)
-// add their chunks with atomics into cells that k_zero_tiles cleared.
-// Weights are those of axis_taps6 (bit-identical to the reference's
-// grid_point_gen, src/noncart/grid.c:403-465) and the combined weight the
-// same float32 product ((1 * wz) * wy) * wx.
-
-enum { TG_WARPS = 4 };
-
-struct TileWork {
-
-	const int* bin_start;		// [nbins + 1] sorted sample range of each bin
-	const int* work_tile;		// [nwork] tile of a work item
-	const int* work_chunk;		// [nwork] chunk of the tile's candidates
-	const int* nwork_dev;		// number of work items
-	const unsigned char* multi;	// [ntiles] 1 if the tile has several work items
-	const float4* foot;		// [M][FOOT_F4] footprints of the sorted samples
-	int cand;			// candidates per work item
-};
-
 // Footprint record of a sorted sample (built once per trajectory by
 // k_foot): float4 0 holds the centred start cells lo of the x, y, z taps
 // (as int bits); float4s 1..5 the weights of cells lo .. lo + 5 per axis,
@@ -714,6 +571,290 @@ __global__ void k_foot(const float4* __restrict__ traj_sorted, long M, GridGeom 
 	}
 }
 
+// Degridding, width 6: four lanes (a quad) per sample, in bin order. The six x
+// taps are at most seven consecutive cells; lane q of the quad reads cells
+// 2q, 2q + 1 of the 8-cell window that starts at an even cell, so a tap row is
+// one 64-byte access of the quad (a thread per sample needed four separate
+// ones, and the gather is bound by the L1's lines per request). Weights come
+// from the plan's footprint records and stay in registers for all channels of
+// the block (grid.y splits the channels in chunks of cpb where the samples
+// alone do not fill the GPU). Four channels are summed side by side and
+// exchanged within the quad so that lane q ends up with channel c + q. The
+// optional weights multiply (wgt, wgt_c channels) happens on the way out.
+// Needs even grid sides of at least 16 cells (2N grids of N >= 8).
+// One B200, 8-coil 128^3 kooshball: 9.17 ms before.
+template <int CC, int TZ>
+__device__ __forceinline__ void degrid6_quad(const float2* __restrict__ gc, long gsz, const float* __restrict__ f,
+		const int (&zoff)[TZ], const int (&row)[6], const float (&wy)[6], float w0, float w1, bool act,
+		float2 (&acc)[CC])
+{
+#pragma unroll
+	for (int c = 0; c < CC; c++)
+		acc[c] = make_float2(0.f, 0.f);
+
+	if (!act)	// both cells of this lane are outside the footprint
+		return;
+
+#pragma unroll 1
+	for (int a = 0; a < TZ; a++) {
+
+		const float dz = f[16 + a];
+		int zo = zoff[0];
+#pragma unroll
+		for (int k = 1; k < TZ; k++)
+			zo = (k == a) ? zoff[k] : zo;
+#pragma unroll
+		for (int b = 0; b < 6; b++) {
+
+			const float dzy = __fmul_rn(dz, wy[b]);
+			const float d0 = __fmul_rn(dzy, w0), d1 = __fmul_rn(dzy, w1);
+			const long o = (long)zo + row[b];
+#pragma unroll
+			for (int c = 0; c < CC; c++) {
+
+				const float4 v = *(const float4*)(gc + gsz * c + o);
+				acc[c].x = fmaf(v.x, d0, acc[c].x);
+				acc[c].y = fmaf(v.y, d0, acc[c].y);
+				acc[c].x = fmaf(v.z, d1, acc[c].x);
+				acc[c].y = fmaf(v.w, d1, acc[c].y);
+			}
+		}
+	}
+}
+
+__device__ __forceinline__ float2 shfl_xor2(float2 v, int m)
+{
+	return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+}
+
+// grid cell index of centred cell c of an axis of G = 2N cells; cells outside a
+// non-periodic grid (their weight is 0) are moved inside
+__device__ __forceinline__ int cell_of(int c, int N, int G, int periodic)
+{
+	if (1 == G)
+		return 0;
+
+	if (periodic) {
+
+		c %= G;
+		c = (c < 0) ? c + G : c;
+
+	} else {
+
+		c = min(max(c, 0), G - 1);
+	}
+
+	c += N;
+	return (c >= G) ? c - G : c;
+}
+
+template <int TZ>
+__global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* __restrict__ foot,
+		const int* __restrict__ perm, long M, GridGeom g, int C, int cpb, const float2* __restrict__ grid,
+		float2* __restrict__ ksp, const float2* __restrict__ wgt, int wgt_c)
+{
+	const int q = threadIdx.x & 3;
+	const long s = ((long)blockIdx.x * BIN_THREADS + threadIdx.x) / 4;
+	const long i = min(s, M - 1);		// surplus quads repeat the last sample and write nothing
+	const float4 h = foot[i * FOOT_F4];
+	const float* f = (const float*)(foot + i * FOOT_F4);
+	const long m = perm[i];
+
+	// this lane's two cells of the x window
+	int lo = __float_as_int(h.x);
+
+	if (g.periodic) {
+
+		lo %= g.G[0];
+		lo = (lo < 0) ? lo + g.G[0] : lo;
+
+	} else {
+
+		lo = min(max(lo, -6), g.G[0]);	// further out all weights are 0
+	}
+
+	const int u = lo + g.N[0];
+	int e = (u & ~1) + 2 * q;
+	const int t = e - u;			// -1 .. 6
+	e = (e >= g.G[0]) ? e - g.G[0] : e;
+	const float w0 = ((t >= 0) && (t < 6)) ? f[4 + t] : 0.f;
+	const float w1 = (t < 5) ? f[5 + t] : 0.f;
+	int row[6], zoff[TZ];
+	float wy[6];
+#pragma unroll
+	for (int b = 0; b < 6; b++) {
+
+		row[b] = cell_of(__float_as_int(h.y) + b, g.N[1], g.G[1], g.periodic) * g.G[0] + e;
+		wy[b] = f[10 + b];
+	}
+
+	// planes of up to 2^31 cells (z offsets of larger grids do not fit an int: the launcher checks)
+#pragma unroll
+	for (int a = 0; a < TZ; a++)
+		zoff[a] = (TZ > 1) ? cell_of(__float_as_int(h.z) + a, g.N[2], g.G[2], g.periodic) * g.G[1] * g.G[0] : 0;
+
+	const bool act = (0.f != w0) || (0.f != w1);
+	const bool valid = (s < M);
+	const int c0 = blockIdx.y * cpb, c1 = min(C, c0 + cpb);
+	int c = c0;
+
+	for (; c + 3 < c1; c += 4) {
+
+		float2 acc[4];
+		degrid6_quad<4, TZ>(grid + g.gsz * c, g.gsz, f, zoff, row, wy, w0, w1, act, acc);
+		float2 k0 = (q & 2) ? acc[2] : acc[0], k1 = (q & 2) ? acc[3] : acc[1];
+		k0 = cadd(k0, shfl_xor2((q & 2) ? acc[0] : acc[2], 2));
+		k1 = cadd(k1, shfl_xor2((q & 2) ? acc[1] : acc[3], 2));
+		float2 r = cadd((q & 1) ? k1 : k0, shfl_xor2((q & 1) ? k0 : k1, 1));
+
+		if (valid) {
+
+			if (wgt)
+				r = cmul(r, wgt[m + M * ((c + q) % wgt_c)]);
+
+			ksp[m + M * (c + q)] = r;
+		}
+	}
+
+	for (; c < c1; c++) {
+
+		float2 acc[1];
+		degrid6_quad<1, TZ>(grid + g.gsz * c, g.gsz, f, zoff, row, wy, w0, w1, act, acc);
+		float2 r = cadd(acc[0], shfl_xor2(acc[0], 2));
+		r = cadd(r, shfl_xor2(r, 1));
+
+		if (valid && (0 == q)) {
+
+			if (wgt)
+				r = cmul(r, wgt[m + M * (c % wgt_c)]);
+
+			ksp[m + M * c] = r;
+		}
+	}
+}
+
+// Gridding, width 6, output-stationary (the default scatter) ------------------
+//
+// The grid is cut into tiles of TX x LY x LZ cells of the centred oversampled
+// grid. One warp job owns one tile (or a chunk of its samples) and a group of
+// coils: lane (line, grp) holds the TX x-cells of tile line (y, z) = line for
+// CT coils in registers, so it accumulates without atomics. The samples whose
+// footprint meets a tile (their hits: a sample has 2.1 in a 16 x 8 tile, 8.2
+// in an 8 x 4 x 4 one) are listed per tile at plan time; before, a job tested
+// every sample of the 3^d neighbour bins (9 or 27 per sample), which took half
+// of its instructions. A job takes its hits 32 at a time: footprint records
+// and coil values (k-space in bin order, a sample's coils side by side) arrive
+// by cp.async while the previous batch accumulates, the warp fills a table of
+// every hit's weight on every tile line, and then adds hit after hit, the next
+// one's weights and values loaded ahead. The x offset of a sample is the same
+// for the whole warp, so a switch on it selects a fully unrolled update of
+// exactly the taps inside the tile; lanes whose line is outside the sample's
+// y/z window skip it. Bound by instruction issue.
+//
+// Work items: tiles with one chunk of hits write their cells with plain stores
+// (empty tiles write zeros, so the grid needs no clearing), tiles with several
+// chunks (the dense k-space centre) add their chunks with atomics into cells
+// that k_zero_tiles cleared. Cells travel in pairs (16 bytes): tile edges and
+// grid sides are even. Weights are those of axis_taps6 (bit-identical to the
+// reference's grid_point_gen, src/noncart/grid.c:403-465) and the combined
+// weight the same float32 product ((1 * wz) * wy) * wx.
+
+enum { TG_WARPS = 4 };
+
+struct TileWork {
+
+	const int* hit_start;		// [ntiles + 1]
+	const int* hits;		// sorted-sample indices by tile
+	const int* work_tile;		// [nwork] tile of a work item
+	const int* work_chunk;		// [nwork] chunk of the tile's hits
+	const int* nwork_dev;		// number of work items
+	const float4* foot;		// [M][FOOT_F4] footprints of the sorted samples
+	int chunk;			// hits per work item
+};
+
+// The tiles of one axis (nb tiles of edge t) that cells lo .. lo + 5 meet:
+// first tile and count (0: none); tiles past the last one wrap around
+__device__ __forceinline__ int2 axis_tiles(int lo, int t, int nb, int G, int periodic)
+{
+	if (1 == G)
+		return make_int2(0, 1);
+
+	if (periodic) {
+
+		lo %= G;
+		lo = (lo < 0) ? lo + G : lo;
+		const int first = lo / t, hi = lo + 5;
+		return make_int2(first, (hi < G) ? hi / t - first + 1 : nb - first + (hi - G) / t + 1);
+	}
+
+	if ((lo < -5) || (lo >= G))
+		return make_int2(0, 0);
+
+	const int first = max(lo, 0) / t;
+	return make_int2(first, min(lo + 5, G - 1) / t - first + 1);
+}
+
+// Hits per tile (hits == nullptr: count into cursor) or the hit lists
+// themselves (cursor starts as the tiles' first positions). The order within
+// a tile's list is that of the atomics.
+__global__ void k_tile_hits(const float4* __restrict__ foot, long M, GridGeom g, BinGeom bg, int* __restrict__ cursor,
+		int* __restrict__ hits)
+{
+	for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (long)gridDim.x * blockDim.x) {
+
+		const float4 f = foot[i * FOOT_F4];
+		const int2 ax = axis_tiles(__float_as_int(f.x), bg.bs[0], bg.nb[0], g.G[0], g.periodic);
+		const int2 ay = axis_tiles(__float_as_int(f.y), bg.bs[1], bg.nb[1], g.G[1], g.periodic);
+		const int2 az = axis_tiles(__float_as_int(f.z), bg.bs[2], bg.nb[2], g.G[2], g.periodic);
+
+		for (int a = 0; a < az.y; a++) {
+
+			const int z = (az.x + a) % bg.nb[2];
+
+			for (int b = 0; b < ay.y; b++) {
+
+				const int y = (ay.x + b) % bg.nb[1];
+
+				for (int c = 0; c < ax.y; c++) {
+
+					const int x = (ax.x + c) % bg.nb[0];
+					const int p = atomicAdd(&cursor[x + bg.nb[0] * (y + bg.nb[1] * z)], 1);
+
+					if (hits)
+						hits[p] = (int)i;
+				}
+			}
+		}
+	}
+}
+
+// work items (chunks of hits) per tile
+__global__ void k_tile_work(const int* __restrict__ hit_start, long ntiles, int chunk, int* __restrict__ nwork)
+{
+	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t <= ntiles; t += (long)gridDim.x * blockDim.x)
+		nwork[t] = (t < ntiles) ? max(1, (hit_start[t + 1] - hit_start[t] + chunk - 1) / chunk) : 0;
+}
+
+// work item table: tile t owns items work_start[t] .. work_start[t + 1] - 1;
+// tiles with several are listed in multi (count nmulti, cleared before)
+__global__ void k_work_fill(const int* __restrict__ work_start, long ntiles, int* __restrict__ work_tile,
+		int* __restrict__ work_chunk, int* __restrict__ multi, int* __restrict__ nmulti)
+{
+	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += (long)gridDim.x * blockDim.x) {
+
+		const int w0 = work_start[t], w1 = work_start[t + 1];
+
+		for (int w = w0; w < w1; w++) {
+
+			work_tile[w] = (int)t;
+			work_chunk[w] = w - w0;
+		}
+
+		if (w1 - w0 > 1)
+			multi[atomicAdd(nmulti, 1)] = (int)t;
+	}
+}
+
 // offset of a footprint start relative to a tile origin, along an axis of
 // G cells: periodic grids take the representative nearest to the tile
 __device__ __forceinline__ int foot_rel(int lo, int origin, int G, int periodic)
@@ -743,19 +884,10 @@ __device__ __forceinline__ int dft_index(int c, int N, int G)
 	return (c >= G) ? c - G : c;
 }
 
-// one staged sample of a warp job
-template <int CW>
-struct __align__(16) TgSample {
-
-	float w[24];		// x, y, z weights of cells lo .. lo + 5 (6 each)
-	int rx, ry, rz, pad;
-	float2 v[CW];
-};
-
 // acc[i][c] += (wyz * wx[t]) * v[c] for the taps t whose cell i = RX + t is
 // inside the tile (RX a compile-time offset)
 template <int TX, int CT, int RX>
-__device__ __forceinline__ void tg_accum_x(float2 (&acc)[TX][CT], const float* wx, float wyz, const float2* v)
+__device__ __forceinline__ void tg_accum_x(float2 (&acc)[TX][CT], const float (&wx)[6], float wyz, const float2 (&v)[CT])
 {
 #pragma unroll
 	for (int t = 0; t < 6; t++) {
@@ -774,10 +906,11 @@ __device__ __forceinline__ void tg_accum_x(float2 (&acc)[TX][CT], const float* w
 }
 
 // the update for a sample at x offset rx (-5 .. TX - 1, at most 15)
-#define BN_TG_CASE(R) case R: tg_accum_x<TX, CT, R>(acc, wx, wyz, v); break;
+#define BN_TG_CASE(R) case R: if constexpr (R < TX) tg_accum_x<TX, CT, R>(acc, wx, wyz, v); break;
 
 template <int TX, int CT>
-__device__ __forceinline__ void tg_switch(int rx, float2 (&acc)[TX][CT], const float* wx, float wyz, const float2* v)
+__device__ __forceinline__ void tg_switch(int rx, float2 (&acc)[TX][CT], const float (&wx)[6], float wyz,
+		const float2 (&v)[CT])
 {
 	static_assert(TX <= 16, "x offsets up to 15");
 
@@ -792,117 +925,66 @@ __device__ __forceinline__ void tg_switch(int rx, float2 (&acc)[TX][CT], const f
 
 #undef BN_TG_CASE
 
-// grid cells of the tiles that several work items add into: zeroed first
-__global__ void k_zero_tiles(float2* __restrict__ grid, GridGeom g, BinGeom bg, const unsigned char* __restrict__ multi,
-		long ntiles, int C)
+// grid cells of the tiles that several work items add into: zeroed first, a
+// warp per tile and channel
+__global__ void k_zero_tiles(float2* __restrict__ grid, GridGeom g, BinGeom bg, const int* __restrict__ multi,
+		const int* __restrict__ nmulti, int C)
 {
-	const long per = (long)bg.bs[0] * bg.bs[1] * bg.bs[2];
+	const int lane = threadIdx.x % 32;
+	const long n = (long)*nmulti * C;
+	const int half = bg.bs[0] / 2, pairs = half * bg.bs[1] * bg.bs[2];
 
-	for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+	for (long j = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32; j < n; j += (long)gridDim.x * blockDim.x / 32) {
 
-		if (!multi[t])
-			continue;
+		const int t = multi[j / C], c = (int)(j % C);
+		const int bx = t % bg.nb[0], by = (t / bg.nb[0]) % bg.nb[1], bz = t / (bg.nb[0] * bg.nb[1]);
 
-		const int bx = (int)(t % bg.nb[0]), by = (int)((t / bg.nb[0]) % bg.nb[1]), bz = (int)(t / ((long)bg.nb[0] * bg.nb[1]));
+		for (int e = lane; e < pairs; e += 32) {
 
-		for (long e = threadIdx.x; e < per * C; e += blockDim.x) {
-
-			const int c = (int)(e / per);
-			const long l = e - (long)c * per;
-			const int cx = bx * bg.bs[0] + (int)(l % bg.bs[0]);
-			const int cy = by * bg.bs[1] + (int)((l / bg.bs[0]) % bg.bs[1]);
-			const int cz = bz * bg.bs[2] + (int)(l / ((long)bg.bs[0] * bg.bs[1]));
+			const int cx = bx * bg.bs[0] + 2 * (e % half);
+			const int cy = by * bg.bs[1] + (e / half) % bg.bs[1];
+			const int cz = bz * bg.bs[2] + e / (half * bg.bs[1]);
 
 			if ((cx >= g.G[0]) || (cy >= g.G[1]) || (cz >= g.G[2]))
 				continue;
 
 			const long cell = dft_index(cx, g.N[0], g.G[0]) + (long)g.G[0] * (dft_index(cy, g.N[1], g.G[1])
 					+ (long)g.G[1] * dft_index(cz, g.N[2], g.G[2]));
-			grid[cell + g.gsz * c] = make_float2(0.f, 0.f);
+			*(float4*)(grid + cell + g.gsz * c) = make_float4(0.f, 0.f, 0.f, 0.f);
 		}
 	}
 }
 
-// candidates of tile (tx, ty, tz): the neighbour bins in the order dz, dy,
-// dx = -1..1 (singleton axes: 0 only; non-periodic edges skipped)
-__device__ __forceinline__ int tg_neighbour(int b, int d, int nb, int periodic)
+__device__ __forceinline__ void cp_async(uint32_t dst, const void* src, int bytes)
 {
-	int n = b + d;
-
-	if (periodic)
-		return (n < 0) ? n + nb : ((n >= nb) ? n - nb : n);
-
-	return ((n < 0) || (n >= nb)) ? -1 : n;
+	if (16 == bytes)
+		asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" :: "r"(dst), "l"(src));
+	else
+		asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" :: "r"(dst), "l"(src));
 }
 
-// candidates per tile and the work items (chunks of cand) per tile
-__global__ void k_tile_cand(const int* __restrict__ bin_start, BinGeom bg, int periodic, long ntiles, int cand,
-		int* __restrict__ nwork, unsigned char* __restrict__ multi)
-{
-	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += (long)gridDim.x * blockDim.x) {
+// shared memory of one warp: two batches of 32 hit records (footprint and CW
+// coil values) and the batch's weight table [32][NL]
+template <int NL, int CW>
+struct TgStage {
 
-		const int bx = (int)(t % bg.nb[0]), by = (int)((t / bg.nb[0]) % bg.nb[1]), bz = (int)(t / ((long)bg.nb[0] * bg.nb[1]));
-		const int rz = (bg.nb[2] > 1) ? 1 : 0, ry = (bg.nb[1] > 1) ? 1 : 0;
-		long n = 0;
-
-		for (int dz = -rz; dz <= rz; dz++) {
-
-			const int z = tg_neighbour(bz, dz, bg.nb[2], periodic);
-
-			if (z < 0)
-				continue;
-
-			for (int dy = -ry; dy <= ry; dy++) {
-
-				const int y = tg_neighbour(by, dy, bg.nb[1], periodic);
-
-				if (y < 0)
-					continue;
-
-				for (int dx = -1; dx <= 1; dx++) {
-
-					const int x = tg_neighbour(bx, dx, bg.nb[0], periodic);
-
-					if (x < 0)
-						continue;
-
-					const long b = x + (long)bg.nb[0] * (y + (long)bg.nb[1] * z);
-					n += bin_start[b + 1] - bin_start[b];
-				}
-			}
-		}
-
-		const long w = (n + cand - 1) / cand;
-		nwork[t] = (int)((w < 1) ? 1 : w);
-		multi[t] = (w > 1) ? 1 : 0;
-	}
-}
-
-// work item table: tile t owns items work_start[t] .. work_start[t + 1] - 1
-__global__ void k_work_fill(const int* __restrict__ work_start, long ntiles, int* __restrict__ work_tile,
-		int* __restrict__ work_chunk)
-{
-	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += (long)gridDim.x * blockDim.x)
-		for (int w = work_start[t]; w < work_start[t + 1]; w++) {
-
-			work_tile[w] = (int)t;
-			work_chunk[w] = w - work_start[t];
-		}
-}
+	static constexpr int REC = 4 * FOOT_F4 + ((2 * CW + 3) / 4) * 4;	// floats per hit record
+	static constexpr int FLOATS = 2 * 32 * REC + 32 * NL;
+};
 
 // TX x-cells per lane, LY x LZ lines per tile (LY * LZ divides 32), CT coils
-// per lane: a warp job covers CW = (32 / (LY * LZ)) * CT coils. ksp_sorted:
-// ksp is in bin order (sample i of the sorted trajectory at ksp[i + M c]),
-// else in the caller's order (ksp[perm[i] + M c]).
+// per lane: a warp job covers CW = (32 / (LY * LZ)) * CT coils. ksp: [M][Cp] in
+// bin order, Cp even (1 for one coil), zeros past the last coil.
 template <int TX, int LY, int LZ, int CT>
-__global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(const int* __restrict__ perm, long M, GridGeom g,
-		BinGeom bg, TileWork tw, int C, const float2* __restrict__ ksp, int ksp_sorted, float2* __restrict__ grid)
+__global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(long M, GridGeom g, BinGeom bg, TileWork tw, int C,
+		int Cp, const float2* __restrict__ ksp, float2* __restrict__ grid)
 {
 	constexpr int NL = LY * LZ;
 	constexpr int GPW = 32 / NL;
 	constexpr int CW = GPW * CT;
 	static_assert(NL * GPW == 32, "lines per tile must divide 32");
-	__shared__ TgSample<CW> stage[TG_WARPS][32];
+	using ST = TgStage<NL, CW>;
+	extern __shared__ __align__(16) float tg_smem[];
 
 	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 	const int ncq = (C + CW - 1) / CW;	// coil chunks
@@ -913,14 +995,16 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(const int* __r
 	if (wi >= *tw.nwork_dev)	// warp-uniform; the warps share no barrier
 		return;
 
+	float* rec = tg_smem + warp * ST::FLOATS;
+	float* wt = rec + 2 * 32 * ST::REC;
 	const int tile = tw.work_tile[wi];
-	const int chunk = tw.work_chunk[wi];
 	const int bx = tile % bg.nb[0], by = (tile / bg.nb[0]) % bg.nb[1], bz = tile / (bg.nb[0] * bg.nb[1]);
 	const int ox = bx * TX, oy = by * LY, oz = bz * LZ;
-	const int j = lane % LY, k = (lane / LY) % LZ, grp = lane / NL;
+	const int line = lane % NL, grp = lane / NL;
 	const int cw0 = cq * CW;		// first coil of the job
 	const int c0 = cw0 + grp * CT;		// first coil of this lane
-	TgSample<CW>* sg = stage[warp];
+	const int h0 = tw.hit_start[tile], h1 = tw.hit_start[tile + 1];
+	const int first = h0 + tw.work_chunk[wi] * tw.chunk, last = min(h1, first + tw.chunk);
 
 	float2 acc[TX][CT];
 #pragma unroll
@@ -929,133 +1013,140 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(const int* __r
 		for (int c = 0; c < CT; c++)
 			acc[i][c] = make_float2(0.f, 0.f);
 
-	const long cand0 = (long)chunk * tw.cand, cand1 = cand0 + tw.cand;
-	const int rz = (bg.nb[2] > 1) ? 1 : 0, ry = (bg.nb[1] > 1) ? 1 : 0;
-	long off = 0;
+	// lane's record of a batch: footprint and coil values, 16 bytes at a time
+	// (8 for a single coil); coils past the padded row stay zero
+	const int nv = (1 == CW) ? 1 : min(CW, Cp - cw0);
 
-	for (int dz = -rz; (dz <= rz) && (off < cand1); dz++) {
+	if (CW > 1)
+		for (int b = 0; b < 2; b++)
+			for (int k = nv; k < CW; k++)
+				*(float2*)(rec + (b * 32 + lane) * ST::REC + 4 * FOOT_F4 + 2 * k) = make_float2(0.f, 0.f);
 
-		const int nz = tg_neighbour(bz, dz, bg.nb[2], g.periodic);
+	auto fetch = [&](int i, int buf) {
+		if (i >= 0) {
 
-		if (nz < 0)
-			continue;
-
-		for (int dy = -ry; (dy <= ry) && (off < cand1); dy++) {
-
-			const int ny = tg_neighbour(by, dy, bg.nb[1], g.periodic);
-
-			if (ny < 0)
-				continue;
-
-			for (int dx = -1; (dx <= 1) && (off < cand1); dx++) {
-
-				const int nx = tg_neighbour(bx, dx, bg.nb[0], g.periodic);
-
-				if (nx < 0)
-					continue;
-
-				const long b = nx + (long)bg.nb[0] * (ny + (long)bg.nb[1] * nz);
-				const int s0 = tw.bin_start[b], s1 = tw.bin_start[b + 1];
-				const long a = max(off, cand0), e = min(off + (long)(s1 - s0), cand1);
-				const int i0 = s0 + (int)(a - off), i1 = s0 + (int)(e - off);
-				off += s1 - s0;
-
-				// batches of 32 candidates; the next batch's footprint start
-				// and coil values are loaded while this batch accumulates
-				float4 f0n = make_float4(0.f, 0.f, 0.f, 0.f);
-				float2 vn[CW];
-
-				auto fetch = [&](int i) {
-					if (i < i1) {
-
-						f0n = tw.foot[(long)i * FOOT_F4];
-						const long m = ksp_sorted ? (long)i : (long)perm[i];
+			const uint32_t dst = (uint32_t)__cvta_generic_to_shared(rec + (buf * 32 + lane) * ST::REC);
+			const float4* f = tw.foot + (long)i * FOOT_F4;
 #pragma unroll
-						for (int c = 0; c < CW; c++)
-							vn[c] = (cw0 + c < C) ? ksp[m + M * (cw0 + c)] : make_float2(0.f, 0.f);
-					}
-				};
+			for (int k = 0; k < FOOT_F4; k++)
+				cp_async(dst + 16 * k, f + k, 16);
 
-				fetch(i0 + lane);
+			const float2* v = ksp + (long)i * Cp + cw0;
 
-				for (int base = i0; base < i1; base += 32) {
+			if (1 == CW) {
 
-					const int i = base + lane;
-					const float4 f0 = f0n;
-					float2 vc[CW];
+				cp_async(dst + 16 * FOOT_F4, v, 8);
+
+			} else {
 #pragma unroll
-					for (int c = 0; c < CW; c++)
-						vc[c] = vn[c];
-
-					fetch(i + 32);
-					bool hit = false;
-					int lx = 0, ly = 0, lz = 0;
-
-					if (i < i1) {
-
-						lx = foot_rel(__float_as_int(f0.x), ox, g.G[0], g.periodic);
-						ly = foot_rel(__float_as_int(f0.y), oy, g.G[1], g.periodic);
-						lz = foot_rel(__float_as_int(f0.z), oz, g.G[2], g.periodic);
-						hit = (lx > -6) && (lx < TX) && (ly > -6) && (ly < LY) && (lz > -6) && (lz < LZ);
-					}
-
-					const unsigned mask = __ballot_sync(0xffffffffu, hit);
-					const int n = __popc(mask);
-
-					if (hit) {
-
-						TgSample<CW>& d = sg[__popc(mask & ((1u << lane) - 1u))];
-						const float4* f = tw.foot + (long)i * FOOT_F4;
-#pragma unroll
-						for (int q = 0; q < 5; q++)
-							*(float4*)(d.w + 4 * q) = f[1 + q];
-						d.rx = lx;
-						d.ry = ly;
-						d.rz = lz;
-#pragma unroll
-						for (int c = 0; c < CW; c++)
-							d.v[c] = vc[c];
-					}
-
-					__syncwarp();
-
-					for (int q = 0; q < n; q++) {
-
-						const TgSample<CW>& d = sg[q];
-						const int ty = j - d.ry, tz = k - d.rz;
-
-						if ((ty < 0) || (ty >= 6) || (tz < 0) || (tz >= 6))
-							continue;
-
-						const float wyz = __fmul_rn(d.w[12 + tz], d.w[6 + ty]);
-
-						if (0.f == wyz)
-							continue;
-
-						float2 v[CT];
-#pragma unroll
-						for (int c = 0; c < CT; c++)
-							v[c] = d.v[grp * CT + c];
-
-						tg_switch<TX, CT>(d.rx, acc, d.w, wyz, v);
-					}
-
-					__syncwarp();
-				}
+				for (int k = 0; k < CW; k += 2)
+					if (k < nv)
+						cp_async(dst + 16 * FOOT_F4 + 8 * k, v + k, 16);
 			}
 		}
+
+		asm volatile("cp.async.commit_group;\n" ::: "memory");
+	};
+
+	int buf = 0;
+	int inext = (first + lane < last) ? tw.hits[first + lane] : -1;
+	fetch(inext, 0);
+	inext = (first + 32 + lane < last) ? tw.hits[first + 32 + lane] : -1;
+
+	for (int base = first; base < last; base += 32) {
+
+		fetch(inext, buf ^ 1);
+		inext = (base + 64 + lane < last) ? tw.hits[base + 64 + lane] : -1;
+		asm volatile("cp.async.wait_group 1;\n" ::: "memory");
+		float* rb = rec + buf * 32 * ST::REC;
+		const int n = min(32, last - base);
+
+		if (lane < n) {	// this lane's own record: offsets relative to the tile
+
+			int* r = (int*)(rb + lane * ST::REC);
+			r[0] = foot_rel(r[0], ox, g.G[0], g.periodic);
+			r[1] = foot_rel(r[1], oy, g.G[1], g.periodic);
+			r[2] = foot_rel(r[2], oz, g.G[2], g.periodic);
+		}
+
+		__syncwarp();
+#pragma unroll 4
+		for (int e = lane; e < n * NL; e += 32) {
+
+			const int l = e % NL;
+			const float* r = rb + (e / NL) * ST::REC;
+			const int ty = l % LY - __float_as_int(r[1]), tz = l / LY - __float_as_int(r[2]);
+			const bool in = (ty >= 0) && (ty < 6) && (tz >= 0) && (tz < 6);
+			wt[e] = in ? __fmul_rn(r[16 + tz], r[10 + ty]) : 0.f;
+		}
+
+		__syncwarp();
+
+		// one hit's inputs: the line's weight, the x weights and offset, the values
+		auto load = [&](int q, float& wyz, float (&wx)[6], int& rx, float2 (&v)[CT]) {
+			const float* r = rb + q * ST::REC;
+			wyz = wt[q * NL + line];
+			rx = __float_as_int(r[0]);
+			const float4 a = *(const float4*)(r + 4);
+			const float2 b = *(const float2*)(r + 8);
+			wx[0] = a.x, wx[1] = a.y, wx[2] = a.z, wx[3] = a.w, wx[4] = b.x, wx[5] = b.y;
+			const float2* vp = (const float2*)(r + 4 * FOOT_F4) + grp * CT;
+
+			if constexpr (0 == CT % 2) {
+#pragma unroll
+				for (int c = 0; c < CT; c += 2) {
+
+					const float4 t = *(const float4*)(vp + c);
+					v[c] = make_float2(t.x, t.y);
+					v[c + 1] = make_float2(t.z, t.w);
+				}
+
+			} else {
+#pragma unroll
+				for (int c = 0; c < CT; c++)
+					v[c] = vp[c];
+			}
+		};
+
+		float wyz, wx[6];
+		int rx;
+		float2 v[CT];
+		load(0, wyz, wx, rx, v);
+
+		for (int q = 0; q < n; q++) {
+
+			float wyzn, wxn[6];
+			int rxn;
+			float2 vn[CT];
+			load(min(q + 1, n - 1), wyzn, wxn, rxn, vn);
+
+			if (0.f != wyz)
+				tg_switch<TX, CT>(rx, acc, wx, wyz, v);
+
+			wyz = wyzn;
+			rx = rxn;
+#pragma unroll
+			for (int t = 0; t < 6; t++)
+				wx[t] = wxn[t];
+#pragma unroll
+			for (int c = 0; c < CT; c++)
+				v[c] = vn[c];
+		}
+
+		__syncwarp();	// before the batch after next overwrites this buffer
+		buf ^= 1;
 	}
 
-	// this lane's line: TX cells from ox along x, at (oy + j, oz + k)
-	const int cy = oy + j, cz = oz + k;
+	// this lane's line: TX cells from ox along x
+	const int cy = oy + line % LY, cz = oz + line / LY;
 
 	if ((cy >= g.G[1]) || (cz >= g.G[2]))
 		return;
 
-	const bool add = tw.multi[tile];
+	const bool add = (h1 - h0 > tw.chunk);
 	const long row = (long)g.G[0] * (dft_index(cy, g.N[1], g.G[1]) + (long)g.G[1] * dft_index(cz, g.N[2], g.G[2]));
 #pragma unroll
-	for (int i = 0; i < TX; i++) {
+	for (int i = 0; i < TX; i += 2) {
 
 		const int cx = ox + i;
 
@@ -1069,24 +1160,47 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(const int* __r
 			if (c0 + c >= C)
 				break;
 
-			float2* dst = grid + cell + g.gsz * (c0 + c);
+			float4* dst = (float4*)(grid + cell + g.gsz * (c0 + c));
+			const float4 v = make_float4(acc[i][c].x, acc[i][c].y, acc[i + 1][c].x, acc[i + 1][c].y);
 
 			if (add)
-				atomicAdd(dst, acc[i][c]);
+				atomicAdd(dst, v);
 			else
-				*dst = acc[i][c];
+				*dst = v;
 		}
 	}
 }
 
-// ksp [M, C] into bin order: dst[i + M c] = src[perm[i] + M c]
-__global__ void k_permute_ksp(float2* __restrict__ dst, const float2* __restrict__ src, const int* __restrict__ perm,
-		long M, int C)
+// ksp [M, C] into bin order with a sample's coils side by side:
+// dst[i][c] = src[perm[i] + M c], zeros for C <= c < Cp; times the conjugate
+// of the weights (w, wc channels) if given. grid (ceil(M / 32), ceil(Cp / 32)).
+__global__ void __launch_bounds__(256) k_permute_ksp(float2* __restrict__ dst, const float2* __restrict__ src,
+		const int* __restrict__ perm, long M, int C, int Cp, const float2* __restrict__ w, int wc)
 {
-	for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < M * C; e += (long)gridDim.x * blockDim.x) {
+	__shared__ float2 t[32][33];
+	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+	const long i0 = (long)blockIdx.x * 32;
+	const int cb = blockIdx.y * 32, cn = min(32, Cp - cb);
+	const long m = (i0 + lane < M) ? perm[i0 + lane] : 0;
 
-		const long c = e / M, i = e - c * M;
-		dst[e] = src[perm[i] + M * c];
+	for (int c = warp; c < cn; c += 8) {
+
+		float2 v = (cb + c < C) ? src[m + M * (cb + c)] : make_float2(0.f, 0.f);
+
+		if (w && (cb + c < C))
+			v = cmulc(v, w[m + M * ((cb + c) % wc)]);
+
+		t[c][lane] = v;
+	}
+
+	__syncthreads();
+
+	for (int e = threadIdx.x; e < 32 * cn; e += 256) {
+
+		const int i = e / cn, c = e % cn;
+
+		if (i0 + i < M)
+			dst[(i0 + i) * Cp + cb + c] = t[c][i];
 	}
 }
 
