@@ -18,7 +18,9 @@
 #include <string>
 #include <vector>
 
-#include "../../include/bnufft.h"
+#include "host.cuh"
+#include "passes.cuh"
+#include "fft_smooth.cuh"
 #include "nufft_kernels.cuh"
 #include "cg_kernels.cuh"
 #include "gridding.cuh"
@@ -36,9 +38,9 @@ using namespace bn;
 // ----------------------------------------------------------------------------
 
 static thread_local std::string g_err;
-static std::atomic<long> g_launches{0};
+std::atomic<long> bn::g_launches{0};
 
-static int fail(int code, const char* fmt, ...)
+int bn::fail(int code, const char* fmt, ...)
 {
 	char buf[512];
 	va_list ap;
@@ -48,15 +50,6 @@ static int fail(int code, const char* fmt, ...)
 	g_err = buf;
 	return code;
 }
-
-#define CUDA_TRY(call) do { cudaError_t e_ = (call); if (cudaSuccess != e_) \
-	return fail(BNUFFT_ERR_CUDA, "%s:%d %s: %s", __FILE__, __LINE__, #call, cudaGetErrorString(e_)); } while (0)
-
-#define LAUNCHED() do { g_launches.fetch_add(1, std::memory_order_relaxed); \
-	cudaError_t e_ = cudaGetLastError(); if (cudaSuccess != e_) \
-	return fail(BNUFFT_ERR_CUDA, "%s:%d launch: %s", __FILE__, __LINE__, cudaGetErrorString(e_)); } while (0)
-
-#define TRY(call) do { int s_ = (call); if (BNUFFT_OK != s_) return s_; } while (0)
 
 // Optional timing of one kernel class (bnufft_prof_start): a pair of CUDA
 // events on the launching stream around every launch of that class.
@@ -69,7 +62,7 @@ static std::atomic<bool> g_prof_active{false};
 // passes run for the preconditioner carry this class prefix ("precond_")
 static thread_local bool t_prof_precond = false;
 
-static cudaEvent_t prof_begin(const char* kind, cudaStream_t st)
+cudaEvent_t bn::prof_begin(const char* kind, cudaStream_t st)
 {
 	if (!g_prof_active.load(std::memory_order_relaxed))
 		return nullptr;
@@ -103,7 +96,7 @@ static cudaEvent_t prof_begin(const char* kind, cudaStream_t st)
 	return b;
 }
 
-static void prof_end(cudaEvent_t e, cudaStream_t st)
+void bn::prof_end(cudaEvent_t e, cudaStream_t st)
 {
 	if (e)
 		cudaEventRecord(e, st);
@@ -253,7 +246,7 @@ static void twiddles_host(int L, float2* h)
 	}
 }
 
-static int get_twiddles(int L, const float2** out)
+int bn::get_twiddles(int L, const float2** out)
 {
 	int dev;
 	CUDA_TRY(cudaGetDevice(&dev));
@@ -262,7 +255,7 @@ static int get_twiddles(int L, const float2** out)
 	while ((1 << lg) < L)
 		lg++;
 
-	if ((dev >= 0) && (dev < 64) && (lg < 16)) {
+	if ((dev >= 0) && (dev < 64) && (lg < 16) && ((1 << lg) == L)) {
 
 		const float2* f = g_tw_fast[dev][lg].load(std::memory_order_acquire);
 
@@ -330,15 +323,15 @@ static int get_kb_table(float os, float width, const float** out)
 // (Bluestein on a power-of-two FFT of at most 4096)
 static bool supported_len(int L) { return (L >= 2) && ((L <= 2048) || ((L <= 4096) && (0 == (L & (L - 1))))); }
 
-// dynamic shared memory of a column pass (ColLayout) / row pass (RowLayout), twiddles included
-static size_t pass_smem(int L, int B) { return sizeof(float2) * (size_t)L * (size_t)(smem_stride(B) + 1); }
-static size_t rows_smem(int L, int B) { return sizeof(float2) * ((size_t)B * (size_t)(L + L / 8) + (size_t)L); }
-
 // sequences per block (B in {4, 8, 16}, B * L / 8 threads <= 1024): as many
 // as fit, fewer when the launch would have too few blocks to fill the GPU
 static int choose_B(int L, long nseq)
 {
-	int B = std::min(16, 8192 / L);
+	int B = 16;
+
+	while (B * L > 8192)
+		B /= 2;
+
 	int Bmin = std::min(16, std::max(4, 256 / L));	// at least one warp per block
 
 	while ((B > Bmin) && ((nseq + B - 1) / B < 2 * 148))
@@ -354,13 +347,11 @@ static std::map<std::pair<const void*, int>, bool> g_attr_done;
 static thread_local std::pair<const void*, int> g_attr_last[8];
 static thread_local int g_attr_next = 0;
 
-template <typename K>
-static int prep_kernel(K kernel, size_t smem)
+int bn::opt_in_smem(const void* kernel)
 {
-	(void)smem;
 	int dev;
 	CUDA_TRY(cudaGetDevice(&dev));
-	auto key = std::make_pair((const void*)kernel, dev);
+	auto key = std::make_pair(kernel, dev);
 
 	for (auto& k : g_attr_last)	// per-thread memo of recent kernels
 		if (k == key)
@@ -379,111 +370,21 @@ static int prep_kernel(K kernel, size_t smem)
 	return BNUFFT_OK;
 }
 
-template <int L, int B>
-static int launch_rows_fwd_LB(const float2* img, const float2* maps, const float* ax, const float* ayz,
-		int X, long YZ, long R, float2* out, cudaStream_t st, const int* done, const Dft& d)
+// FFT lengths with a pass kernel: powers of two and the mixed lengths
+static const int FFT_LENGTHS[] = { 16, 32, 64, 128, 192, 256, 320, 384, 448, 512, 576, 640, 768, 1024, 2048, 4096 };
+
+// the shortest of them >= n (pow2: of the powers of two); 0: none
+static int fft_length(int n, bool pow2 = false)
 {
-	const float2* tw;
-	TRY(get_twiddles(L, &tw));
-	size_t smem = rows_smem(L, B);
-	auto kern = (d.n == L) ? k_rows_fwd<L, B, false> : k_rows_fwd<L, B, true>;
-	TRY(prep_kernel(kern, smem));
-	cudaEvent_t pe = prof_begin("rows_fwd", st);
-	kern<<<(unsigned)((R + B - 1) / B), B * L / 8, smem, st>>>(img, maps, ax, ayz, X, YZ, R, out, tw, done, d);
-	prof_end(pe, st);
-	LAUNCHED();
-	return BNUFFT_OK;
+	for (int l : FFT_LENGTHS)
+		if ((l >= n) && (!pow2 || !is_mix(l)))
+			return l;
+
+	return 0;
 }
 
-template <int L, int B, int MODE>
-static int launch_cols_LB(const float2* in, long ies, long ios, int n_in, int wrap_in,
-		float2* out, long oes, long oos, int n_out, int wrap_out, int W, long O,
-		const float2* psf, long pes, long pmod, long pos, const int* done, cudaStream_t st, const Dft& d)
-{
-	const float2* tw;
-	TRY(get_twiddles(L, &tw));
-	size_t smem = pass_smem(L, B);
-
-	if ((d.n == L) && cols_double_buffered(MODE, false, L, B))
-		smem += sizeof(float2) * (size_t)L * (size_t)smem_stride(B);	// the second exchange buffer
-
-	auto kern = (d.n == L) ? k_cols<L, B, MODE, false> : k_cols<L, B, MODE, true>;
-	TRY(prep_kernel(kern, smem));
-
-	if (O > 65535)
-		return fail(BNUFFT_ERR_UNSUPPORTED, "column pass with %ld outer sequences", O);
-
-	dim3 grid((unsigned)((W + B - 1) / B), (unsigned)O);
-	cudaEvent_t pe = prof_begin((2 == MODE) ? "cols_toeplitz" : ((1 == MODE) ? "cols_inv" : "cols_fwd"), st);
-	kern<<<grid, B * L / 8, smem, st>>>(in, ies, ios, n_in, wrap_in, out, oes, oos, n_out, wrap_out,
-			W, psf, pes, pmod, pos, tw, done, d);
-	prof_end(pe, st);
-	LAUNCHED();
-	return BNUFFT_OK;
-}
-
-template <int L, int B>
-static int launch_rows_inv_LB(const float2* in, const float2* maps, const float* ax, const float* ayz,
-		int X, long YZ, int C, int cpg, float2* out, const float2* pdot, double* dot_part, const int* done,
-		cudaStream_t st, const Dft& d)
-{
-	const float2* tw;
-	TRY(get_twiddles(L, &tw));
-	int groups = (C + cpg - 1) / cpg;
-	size_t smem = rows_smem(L, B);
-	auto kern = (d.n == L) ? k_rows_inv<L, B, false> : k_rows_inv<L, B, true>;
-	TRY(prep_kernel(kern, smem));
-	dim3 grid((unsigned)((YZ + B - 1) / B), (unsigned)groups);
-	cudaEvent_t pe = prof_begin("rows_inv", st);
-	kern<<<grid, B * L / 8, smem, st>>>(in, maps, ax, ayz, X, YZ, C, cpg, out, tw, pdot, dot_part, done, d);
-	prof_end(pe, st);
-	LAUNCHED();
-	return BNUFFT_OK;
-}
-
-template <int L, int B>
-static int launch_rows_fwd_cg_LB(const float2* bvec, const float2* r, const float2* p_prev, float2* p_cur,
-		const float2* maps, const float* ax, const float* ayz, int X, long YZ, long R, float2* out,
-		CgScalars* stt, int it, const double* rs_part, int nrs, double* pp_part, cudaStream_t st, const Dft& d)
-{
-	const float2* tw;
-	TRY(get_twiddles(L, &tw));
-	size_t smem = rows_smem(L, B);
-	auto kern = (d.n == L) ? k_rows_fwd_cg<L, B, false> : k_rows_fwd_cg<L, B, true>;
-	TRY(prep_kernel(kern, smem));
-	cudaEvent_t pe = prof_begin("rows_fwd", st);
-	kern<<<(unsigned)((R + B - 1) / B), B * L / 8, smem, st>>>(bvec, r, p_prev, p_cur, maps, ax, ayz,
-			X, YZ, R, out, tw, stt, it, rs_part, nrs, pp_part, d);
-	prof_end(pe, st);
-	LAUNCHED();
-	return BNUFFT_OK;
-}
-
-// run CALL with compile-time LL (FFT length) and BB (sequences per block)
-#define DISPATCH_LB(L, B, CALL) \
-	switch (L) { \
-	case 16: { constexpr int LL = 16; DISPATCH_B(B, CALL) } \
-	case 32: { constexpr int LL = 32; DISPATCH_B(B, CALL) } \
-	case 64: { constexpr int LL = 64; DISPATCH_B(B, CALL) } \
-	case 128: { constexpr int LL = 128; DISPATCH_B(B, CALL) } \
-	case 256: { constexpr int LL = 256; DISPATCH_B(B, CALL) } \
-	case 512: { constexpr int LL = 512; DISPATCH_B(B, CALL) } \
-	case 1024: { constexpr int LL = 1024; DISPATCH_B(B, CALL) } \
-	case 2048: { constexpr int LL = 2048; DISPATCH_B(B, CALL) } \
-	case 4096: { constexpr int LL = 4096; DISPATCH_B(B, CALL) } \
-	default: return fail(BNUFFT_ERR_UNSUPPORTED, "FFT length %d (powers of two 16..4096 are built)", L); }
-
-#define DISPATCH_B(B, CALL) \
-	switch (B) { \
-	case 2: { constexpr int BB = 2; if constexpr (LL >= 4096 && BB * LL / 8 <= 1024) return CALL; break; } \
-	case 4: { constexpr int BB = 4; if constexpr (BB * LL / 8 <= 1024 && BB * LL / 8 >= 32) return CALL; break; } \
-	case 8: { constexpr int BB = 8; if constexpr (BB * LL / 8 <= 1024 && BB * LL / 8 >= 32) return CALL; break; } \
-	case 16: { constexpr int BB = 16; if constexpr (BB * LL / 8 <= 1024 && BB * LL / 8 >= 32) return CALL; break; } \
-	} \
-	return fail(BNUFFT_ERR_ARG, "no FFT pass instance for L=%d B=%d", L, B);
-
-// DFT of logical length n: the power-of-two FFT of length n itself, or
-// Bluestein's algorithm on the power-of-two length P >= 2n - 1 with its
+// DFT of logical length n: the FFT of length n itself, or
+// Bluestein's algorithm on the shortest FFT length P >= 2n - 1 with its
 // chirp and filter tables (computed once per device and length on the host
 // in float64: chirp exp(-i pi (j^2 mod 2n) / n), filters by a float64 FFT)
 struct DftTables {
@@ -498,6 +399,36 @@ static std::map<std::pair<int, int>, DftTables> g_dft;
 static void fft_host(std::vector<std::complex<double>>& a)	// in place, forward, unnormalised
 {
 	const size_t n = a.size();
+
+	if (0 != (n & (n - 1))) {	// not a power of two: halves while even, then the sum itself
+
+		std::vector<std::complex<double>> h[2];
+
+		if (0 == n % 2) {
+
+			for (size_t i = 0; i < n; i++)
+				h[i % 2].push_back(a[i]);
+
+			fft_host(h[0]);
+			fft_host(h[1]);
+		}
+
+		std::vector<std::complex<double>> out(n);
+
+		for (size_t k = 0; k < n; k++) {
+
+			auto w = [&](size_t j) { return std::polar(1., -2. * M_PI * (double)(j % n) / (double)n); };
+
+			if (0 == n % 2)
+				out[k] = h[0][k % (n / 2)] + w(k) * h[1][k % (n / 2)];
+			else
+				for (size_t i = 0; i < n; i++)
+					out[k] += w(i * k) * a[i];
+		}
+
+		a = out;
+		return;
+	}
 
 	for (size_t i = 1, j = 0; i < n; i++) {
 
@@ -534,18 +465,15 @@ static int get_dft(int n, Dft* d, int* P)
 	d->n = n;
 	d->chirp = d->bf = d->bi = nullptr;
 
-	if ((n >= 16) && (n <= 4096) && (0 == (n & (n - 1)))) {
+	if (n == fft_length(n)) {
 
 		*P = n;
 		return BNUFFT_OK;
 	}
 
-	int p = 16;
+	const int p = fft_length(2 * n - 1);
 
-	while (p < 2 * n - 1)
-		p *= 2;
-
-	if ((n < 2) || (p > 4096))
+	if ((n < 2) || (0 == p))
 		return fail(BNUFFT_ERR_UNSUPPORTED, "DFT length %d (powers of two up to 4096, other lengths up to 2048)", n);
 
 	int dev;
@@ -601,22 +529,135 @@ static int get_dft(int n, Dft* d, int* P)
 	return BNUFFT_OK;
 }
 
-// The passes below take the logical DFT length n (the grid length) and run
-// the power-of-two FFT of length P (n itself or Bluestein's)
+// Radices of a smooth length n that is no built length (fft_smooth.cuh): the
+// fewest of 2..13, of those the ones with the smallest largest radix. false:
+// n is a built length, has a larger prime factor, or is too long for the
+// passes' shared memory.
+static unsigned magic_of(int m) { return (m > 1) ? (unsigned)(((1ull << 32) + m - 1) / (unsigned)m) : 0u; }
+
+static void smooth_search(int n, int most, int depth, int* cur, int* best, int& nbest)
+{
+	if (1 == n) {
+
+		if ((0 == nbest) || (depth < nbest) || ((depth == nbest) && (cur[0] < best[0]))) {
+
+			std::copy(cur, cur + depth, best);
+			nbest = depth;
+		}
+
+		return;
+	}
+
+	if ((depth == SM_STAGES) || (nbest && (depth >= nbest)))
+		return;
+
+	for (int r = std::min(n, most); r >= 2; r--)
+		if (0 == n % r) {
+
+			cur[depth] = r;
+			smooth_search(n / r, r, depth + 1, cur, best, nbest);
+		}
+}
+
+static bool smooth_plan(int n, SmoothPlan* d)
+{
+	if ((n < 16) || (n > 1024) || (n == fft_length(n)))
+		return false;
+
+	int cur[SM_STAGES], best[SM_STAGES], nbest = 0;
+	smooth_search(n, 13, 0, cur, best, nbest);
+
+	if (0 == nbest)
+		return false;
+
+	d->n = n;
+	d->nst = nbest;
+	d->n_magic = magic_of(n);
+
+	for (int s = 0, ns = 1; s < nbest; s++) {
+
+		d->radix[s] = best[s];
+		d->ns[s] = ns;
+		d->ns_magic[s] = magic_of(ns);
+		d->nb_magic[s] = magic_of(n / best[s]);
+		ns *= best[s];
+	}
+
+	return true;
+}
+
+// sequences per block of a smooth pass: eight, four where two exchange buffers
+// of eight would leave one block per SM
+static int smooth_B(int n) { return (n <= 448) ? 8 : 4; }
+static size_t smooth_rows_smem(int n, int B, int X) { return sizeof(float2) * (2ul * B * sm_row(n) + n + (size_t)B * X); }
+static size_t smooth_cols_smem(int n, int B) { return sizeof(float2) * (size_t)n * (2 * (B | 1) + 1); }
+
+template <bool CG>
+static int smooth_rows_fwd(const SmoothPlan& d, const float2* img, const float2* r, const float2* p_prev, float2* p_cur,
+		const float2* maps, const float* ax, const float* ayz, int X, long YZ, long R, float2* out, const int* done,
+		CgScalars* stt, int it, const double* rs_part, int nrs, double* pp_part, int* nblocks, cudaStream_t st)
+{
+	const float2* tw;
+	TRY(get_twiddles(d.n, &tw));
+	const int B = smooth_B(d.n);
+	const size_t smem = smooth_rows_smem(d.n, B, 0);
+	const unsigned nb = (unsigned)((R + B - 1) / B);
+	auto kern = (8 == B) ? k_srows_fwd<CG, 8> : k_srows_fwd<CG, 4>;
+	TRY(prep_kernel(kern, smem));
+
+	if (nblocks)
+		*nblocks = (int)nb;
+
+	cudaEvent_t pe = prof_begin("rows_fwd", st);
+	kern<<<nb, SM_THREADS, smem, st>>>(img, r, p_prev, p_cur, maps, ax, ayz, X, YZ, R, out, tw, done, stt, it, rs_part, nrs,
+			pp_part, d);
+	prof_end(pe, st);
+	LAUNCHED();
+	return BNUFFT_OK;
+}
+
+// The passes below take the logical DFT length n (the grid length) and run its
+// FFT (a built length, or a smooth one) or Bluestein's on a built length
 static int rows_fwd(int n, const float2* img, const float2* maps, const float* ax, const float* ayz,
 		int X, long YZ, long R, float2* out, cudaStream_t st, const int* done = nullptr)
 {
+	SmoothPlan sp;
+
+	if (smooth_plan(n, &sp))
+		return smooth_rows_fwd<false>(sp, img, nullptr, nullptr, nullptr, maps, ax, ayz, X, YZ, R, out, done, nullptr, 0,
+				nullptr, 0, nullptr, nullptr, st);
+
 	Dft d;
 	int L;
 	TRY(get_dft(n, &d, &L));
 	int B = choose_B(L, R);
-	DISPATCH_LB(L, B, (launch_rows_fwd_LB<LL, BB>(img, maps, ax, ayz, X, YZ, R, out, st, done, d)));
+	return pass_table(L)->rows_fwd(L, B, img, maps, ax, ayz, X, YZ, R, out, st, done, d);
 }
 
 static int cols(int n, int mode, const float2* in, long ies, long ios, int n_in, int wrap_in,
 		float2* out, long oes, long oos, int n_out, int wrap_out, int W, long O,
 		const float2* psf, long pes, long pmod, long pos, cudaStream_t st, const int* done = nullptr)
 {
+	SmoothPlan sp;
+
+	// (single columns, W = 1, would leave most of a block's columns empty)
+	if ((2 != mode) && (W >= 4) && (O <= 65535) && smooth_plan(n, &sp)) {
+
+		const float2* tw;
+		TRY(get_twiddles(n, &tw));
+		const int B = smooth_B(n);
+		const size_t smem = smooth_cols_smem(n, B);
+		auto kern = (8 == B) ? ((0 == mode) ? k_scols<false, 8> : k_scols<true, 8>)
+				: ((0 == mode) ? k_scols<false, 4> : k_scols<true, 4>);
+		TRY(prep_kernel(kern, smem));
+		cudaEvent_t pe = prof_begin((1 == mode) ? "cols_inv" : "cols_fwd", st);
+		kern<<<dim3((unsigned)((W + B - 1) / B), (unsigned)O), SM_THREADS, smem, st>>>(in, ies, ios, n_in, wrap_in, out, oes,
+				oos, n_out, wrap_out, W, tw, done, sp);
+		prof_end(pe, st);
+		LAUNCHED();
+		return BNUFFT_OK;
+	}
+
 	Dft d;
 	int L;
 	TRY(get_dft(n, &d, &L));
@@ -663,41 +704,65 @@ static int cols(int n, int mode, const float2* in, long ies, long ios, int n_in,
 		}
 	}
 
-	if (0 == mode)
-		DISPATCH_LB(L, B, (launch_cols_LB<LL, BB, 0>(in, ies, ios, n_in, wrap_in, out, oes, oos, n_out, wrap_out, W, O, psf, pes, pmod, pos, done, st, d)))
-	else if (1 == mode)
-		DISPATCH_LB(L, B, (launch_cols_LB<LL, BB, 1>(in, ies, ios, n_in, wrap_in, out, oes, oos, n_out, wrap_out, W, O, psf, pes, pmod, pos, done, st, d)))
-	else
-		DISPATCH_LB(L, B, (launch_cols_LB<LL, BB, 2>(in, ies, ios, n_in, wrap_in, out, oes, oos, n_out, wrap_out, W, O, psf, pes, pmod, pos, done, st, d)))
+	return pass_table(L)->cols(L, B, mode, in, ies, ios, n_in, wrap_in, out, oes, oos, n_out, wrap_out, W, O, psf, pes, pmod,
+			pos, done, st, d);
 }
 
 static int rows_inv(int n, const float2* in, const float2* maps, const float* ax, const float* ayz,
 		int X, long YZ, int C, int cpg, float2* out, cudaStream_t st,
 		const float2* pdot = nullptr, double* dot_part = nullptr, const int* done = nullptr, int* nblocks = nullptr)
 {
+	int groups = (C + cpg - 1) / cpg;
+	SmoothPlan sp;
+
+	if (smooth_plan(n, &sp)) {
+
+		const float2* tw;
+		TRY(get_twiddles(n, &tw));
+		const int B = smooth_B(n);
+		const size_t smem = smooth_rows_smem(n, B, maps ? X : 0);
+		auto kern = (8 == B) ? k_srows_inv<8> : k_srows_inv<4>;
+		TRY(prep_kernel(kern, smem));
+		const dim3 grid((unsigned)((YZ + B - 1) / B), (unsigned)groups);
+
+		if (nblocks)
+			*nblocks = (int)(grid.x * grid.y);
+
+		cudaEvent_t pe = prof_begin("rows_inv", st);
+		kern<<<grid, SM_THREADS, smem, st>>>(in, maps, ax, ayz, X, YZ, C, cpg, out, tw, pdot, dot_part, done, magic_of(X), sp);
+		prof_end(pe, st);
+		LAUNCHED();
+		return BNUFFT_OK;
+	}
+
 	Dft d;
 	int L;
 	TRY(get_dft(n, &d, &L));
-	int groups = (C + cpg - 1) / cpg;
 	int B = choose_B(L, YZ * groups);
 
 	if (nblocks)
 		*nblocks = (int)(((YZ + B - 1) / B) * groups);
 
-	DISPATCH_LB(L, B, (launch_rows_inv_LB<LL, BB>(in, maps, ax, ayz, X, YZ, C, cpg, out, pdot, dot_part, done, st, d)));
+	return pass_table(L)->rows_inv(L, B, in, maps, ax, ayz, X, YZ, C, cpg, out, pdot, dot_part, done, st, d);
 }
 
 static int rows_fwd_cg(int n, const float2* bvec, const float2* r, const float2* p_prev, float2* p_cur,
 		const float2* maps, const float* ax, const float* ayz, int X, long YZ, long R, float2* out,
 		CgScalars* stt, int it, const double* rs_part, int nrs, double* pp_part, int* nblocks, cudaStream_t st)
 {
+	SmoothPlan sp;
+
+	if (smooth_plan(n, &sp))
+		return smooth_rows_fwd<true>(sp, bvec, r, p_prev, p_cur, maps, ax, ayz, X, YZ, R, out, nullptr, stt, it, rs_part, nrs,
+				pp_part, nblocks, st);
+
 	Dft d;
 	int L;
 	TRY(get_dft(n, &d, &L));
 	int B = choose_B(L, R);
 	*nblocks = (int)((R + B - 1) / B);
-	DISPATCH_LB(L, B, (launch_rows_fwd_cg_LB<LL, BB>(bvec, r, p_prev, p_cur, maps, ax, ayz, X, YZ, R, out,
-			stt, it, rs_part, nrs, pp_part, st, d)));
+	return pass_table(L)->rows_fwd_cg(L, B, bvec, r, p_prev, p_cur, maps, ax, ayz, X, YZ, R, out,
+			stt, it, rs_part, nrs, pp_part, st, d);
 }
 
 static unsigned vec_blocks(long n, int threads = RED_THREADS, int maxb = 4 * 148)
@@ -1921,8 +1986,8 @@ struct bnufft_plan_s {
 	long MrMs = 0;
 	float2* basis = nullptr;	// [T, K], element t + T k
 	float2* pinv = nullptr;	// circulant preconditioner 1/pre, [N0, N1*N2] DFT order (on demand)
-	// Toeplitz normal on a power-of-two circulant embedding when 2N is not a
-	// power of two: geometry with G = E >= 2N and the PSF re-embedded there
+	// Toeplitz normal on a circulant embedding of a built FFT length when 2N is
+	// none: geometry with G = E >= 2N and the PSF re-embedded there
 	bool embed = false;
 	OpCtx toe;
 	float2* psf_t = nullptr;
@@ -2002,42 +2067,31 @@ __global__ static void k_toe_embed(float2* __restrict__ qe, const float2* __rest
 	}
 }
 
-// Build p->toe / p->psf_t from p->psf (see the struct). With P the PSF on
-// the L = 2N grid, the normal operator is y = sum_m x_m L q[(n - m) mod L],
-// q = IDFT(P) / L per axis, and only |n - m| < N enters: on a length-E grid
-// the same operator has q' = (L / E) q on |d| < N, zero elsewhere, and
-// P' = DFT_E(q').
-static int build_toeplitz_embedding(bnufft_plan_s* p, cudaStream_t st)
+// Embedding lengths E >= 2N per axis: the shortest built FFT lengths (pow2: of
+// the powers of two). Returns whether they differ from 2N; false too where an
+// axis is too long for any.
+static bool embed_lengths(const Geom& g, bool pow2, int E[3])
 {
-	const Geom& g = p->op.g;
-	int E[3];
-	bool embed = false;
+	bool embed = false, ok = true;
 
 	for (int a = 0; a < 3; a++) {
 
-		E[a] = 1;
-
-		if (g.G[a] > 1) {
-
-			int e = 16;
-
-			while (e < g.G[a])
-				e *= 2;
-
-			E[a] = e;
-			embed |= (e != g.G[a]);
-		}
+		E[a] = (g.G[a] > 1) ? fft_length(g.G[a], pow2) : 1;
+		ok = ok && (E[a] > 0);
+		embed = embed || (E[a] != g.G[a]);
 	}
 
-	if (p->psf_t)
-		cudaFreeAsync(p->psf_t, st);
+	return embed && ok;
+}
 
-	p->psf_t = nullptr;
-	p->embed = false;
-
-	if (!embed || (E[0] > 4096) || (E[1] > 4096) || (E[2] > 4096))
-		return BNUFFT_OK;
-
+// The geometry on the embedding grid E and the PSF there (*psf_e, allocated
+// here) from p->psf. With P the PSF on the L = 2N grid, the normal operator is
+// y = sum_m x_m L q[(n - m) mod L], q = IDFT(P) / L per axis, and only
+// |n - m| < N enters: on a length-E grid the same operator has q' = (L / E) q
+// on |d| < N, zero elsewhere, and P' = DFT_E(q').
+static int embed_psf(bnufft_plan_s* p, const int E[3], OpCtx& ctx, float2** psf_e, cudaStream_t st)
+{
+	const Geom& g = p->op.g;
 	const long L0 = g.G[0], L1 = g.G[1], L2 = g.G[2];
 	const long ne = (long)E[0] * E[1] * E[2];
 	float2* q = nullptr;
@@ -2070,7 +2124,7 @@ static int build_toeplitz_embedding(bnufft_plan_s* p, cudaStream_t st)
 	k_toe_embed<<<vec_blocks(ne), RED_THREADS, 0, st>>>(qe, q, grid_geom(g), E[0], E[1], E[2], (float)(1. / (double)ne));
 	LAUNCHED();
 
-	// forward DFT on the embedding grid (powers of two)
+	// forward DFT on the embedding grid
 	const long E0 = E[0], E1 = E[1], E2 = E[2];
 	TRY(along_x((int)E0, 0, qe, qe, E1 * E2));
 
@@ -2081,18 +2135,34 @@ static int build_toeplitz_embedding(bnufft_plan_s* p, cudaStream_t st)
 		TRY(cols((int)E2, 0, qe, E0 * E1, 0, (int)E2, 0, qe, E0 * E1, 0, (int)E2, 0, (int)(E0 * E1), 1, nullptr, 0, 1, 0, st));
 
 	cudaFreeAsync(q, st);
-	p->psf_t = qe;
-
-	free_work(p->toe.w, st);
-	p->toe = OpCtx();
-	p->toe.g = g;
-	p->toe.g.gsz = ne;
+	*psf_e = qe;
+	free_work(ctx.w, st);
+	ctx = OpCtx();
+	ctx.g = g;
+	ctx.g.gsz = ne;
 
 	for (int a = 0; a < 3; a++)
-		p->toe.g.G[a] = E[a];
+		ctx.g.G[a] = E[a];
 
-	p->toe.kb = p->op.kb;
-	p->toe.traj = nullptr;
+	ctx.kb = p->op.kb;
+	ctx.traj = nullptr;
+	return BNUFFT_OK;
+}
+
+// p->toe / p->psf_t from p->psf (see the struct)
+static int build_toeplitz_embedding(bnufft_plan_s* p, cudaStream_t st)
+{
+	if (p->psf_t)
+		cudaFreeAsync(p->psf_t, st);
+
+	p->psf_t = nullptr;
+	p->embed = false;
+	int E[3];
+
+	if (!embed_lengths(p->op.g, false, E))
+		return BNUFFT_OK;
+
+	TRY(embed_psf(p, E, p->toe, &p->psf_t, st));
 	p->embed = true;
 	return BNUFFT_OK;
 }
@@ -3454,7 +3524,9 @@ struct bnufft_pics_s {
 					// preconditioner (BNUFFT_FCG_FUSE=0: not)
 	int ndir = 0;			// its <p, r> and ||p||^2 partials per launch
 	bnufft_precnet_t net = nullptr;	// learned correction (conf.precond == 2), not owned
-	float2* pinv_pad = nullptr;	// padded-circulant spectrum (conf.precond == 3), Toeplitz grid
+	float2* pinv_pad = nullptr;	// padded-circulant spectrum (conf.precond 2 and 3), on its grid:
+	bool pre_own = false;		// pre (a power-of-two embedding) or, if that is the same, the
+	OpCtx pre;			// Toeplitz operator's
 	double* mcn_part = nullptr;	// ||M_circ(r)||^2 partials
 	bf16* nact[2] = { nullptr, nullptr };	// its activations, ping-pong [npix][32]
 	long max_row_blocks;
@@ -3841,11 +3913,29 @@ static int build_precond_pad(bnufft_pics_s* ps, cudaStream_t st)
 	if (!p->psf)
 		return fail(BNUFFT_ERR_ARG, "the padded preconditioner needs the Toeplitz PSF");
 
-	const Geom& g = toe_ctx(p).g;
+	// the preconditioner is defined on the power-of-two circulant; the normal
+	// operator may run on a shorter one
+	int E[3];
+	const bool embed = embed_lengths(p->op.g, true, E);
+	const Geom& tg = toe_ctx(p).g;
+	float2* psf_e = nullptr;
+
+	if (embed && ((E[0] != tg.G[0]) || (E[1] != tg.G[1]) || (E[2] != tg.G[2]))) {
+
+		TRY(embed_psf(p, E, ps->pre, &psf_e, st));
+		TRY(alloc_work(ps->pre.w, ps->pre.g, 1, st));
+		ps->pre_own = true;
+	}
+
+	const Geom& g = ps->pre_own ? ps->pre.g : tg;
 	const float mu_lam = (float)(2.5 * ps->conf.lambda * std::pow(4., (double)g.nd) / (double)g.gsz);
 	CUDA_TRY(cudaMallocAsync(&ps->pinv_pad, sizeof(float2) * g.gsz, st));
-	k_precond_pad_spectrum<<<vec_blocks(g.gsz), RED_THREADS, 0, st>>>(ps->pinv_pad, toe_psf(p, st), g.gsz, mu_lam);
+	k_precond_pad_spectrum<<<vec_blocks(g.gsz), RED_THREADS, 0, st>>>(ps->pinv_pad, psf_e ? psf_e : toe_psf(p, st), g.gsz, mu_lam);
 	LAUNCHED();
+
+	if (psf_e)
+		cudaFreeAsync(psf_e, st);
+
 	return BNUFFT_OK;
 }
 
@@ -3856,7 +3946,7 @@ static int pics_precond_pad(bnufft_pics_s* ps, const float2* r, float2* z, const
 		int* nblocks, cudaStream_t st)
 {
 	bnufft_plan_s* p = ps->nufft;
-	OpCtx& op = toe_ctx(p);
+	OpCtx& op = ps->pre_own ? ps->pre : toe_ctx(p);
 	const Geom& g = op.g;
 	const int* done = &ps->scal->done;
 	long YZ = (long)g.N[1] * g.N[2];
@@ -4703,6 +4793,7 @@ extern "C" void bnufft_pics_free(bnufft_pics_t ps)
 		if (b)
 			cudaFreeAsync(b, st);
 
+	free_work(ps->pre.w, st);
 	bnufft_free(ps->nufft);
 	delete ps;
 }

@@ -1,6 +1,7 @@
 // Shared-memory Stockham FFT core for sm_100a.
 //
-// A thread block transforms B sequences of length L (power of two, 16..4096).
+// A thread block transforms B sequences of length L (power of two, 16..4096,
+// or one of the mixed lengths further down).
 // Each sequence is served by T = L/8 threads (index jt). Between stages the
 // data lives in shared memory in one of two layouts (ColLayout for column
 // passes, RowLayout for row passes; see below), chosen so that both the
@@ -346,6 +347,374 @@ __device__ __forceinline__ void fft_regs_db(float2 (&v)[8], float2* s, float2* s
 	__syncthreads();
 
 	fft_tail_db<L, LAY, 8, INV>(v, s, s2, b, jt, tw);
+}
+
+// Mixed lengths L = 64 R, R in {3, 5, 6, 7, 9, 10, 12} ------------------------
+//
+// They fill the gaps between the powers of two (192, 320, 384, 448, 576, 640,
+// 768), so that a transform of a given minimum length costs at most 1.3 times
+// the points it needs per axis instead of 2. Three stages with the same
+// L / 8 threads per sequence and the same shared-memory layouts:
+//   forward: radix 8, 8, then R (64 butterflies): the input is held as in the
+//            power-of-two transforms (positions jt + (L/8) m in v[m]), the
+//            spectrum as spec_pos says: butterfly j = jt + q L/8 (< 64) leaves
+//            positions j + 64 i in w[q R + i];
+//   inverse: the mirror image, radix R, 8, 8, from that spectrum order back to
+//            positions jt + (L/8) m.
+// So forward, product with a spectrum, inverse still chain in registers. The
+// powers of the last forward twiddle come from four table entries and at most
+// two products each.
+__host__ __device__ constexpr bool is_mix(int L) { return 0 != (L & (L - 1)); }
+
+// registers of the spectrum-side set of a thread
+__host__ __device__ constexpr int spec_regs(int L) { return is_mix(L) ? ((64 + L / 8 - 1) / (L / 8)) * (L / 64) : 8; }
+
+// position of register m of the spectrum-side set (>= L: none)
+template <int L, typename LAY>
+__device__ __forceinline__ int spec_pos(int m)
+{
+	if constexpr (is_mix(L)) {
+
+		const int j = LAY::jt() + (m / (L / 64)) * (L / 8);
+		return (j < 64) ? j + 64 * (m % (L / 64)) : L;
+
+	} else {
+
+		return LAY::jt() + (L / 8) * m;
+	}
+}
+
+template <bool INV>
+__device__ __forceinline__ void dft3(float2& x0, float2& x1, float2& x2)
+{
+	const float s = 0.86602540378443864676f;	// sin(pi / 3)
+	const float2 t = cadd(x1, x2), d = rot90<INV>(cscale(csub(x1, x2), s));
+	const float2 m = make_float2(fmaf(-0.5f, t.x, x0.x), fmaf(-0.5f, t.y, x0.y));
+	x0 = cadd(x0, t);
+	x1 = cadd(m, d);
+	x2 = csub(m, d);
+}
+
+// odd length n from the sums and differences of the pairs x[k], x[n - k]:
+// X[k] = x0 + sum_j cos(2 pi jk / n) t_j -+ i sum_j sin(2 pi jk / n) d_j
+template <int N, bool INV>
+__device__ __forceinline__ void dft_odd(float2 (&x)[N], const float (&c)[N], const float (&s)[N])
+{
+	constexpr int H = (N - 1) / 2;
+	float2 t[H + 1], d[H + 1];
+	float2 sum = x[0];
+#pragma unroll
+	for (int j = 1; j <= H; j++) {
+
+		t[j] = cadd(x[j], x[N - j]);
+		d[j] = csub(x[j], x[N - j]);
+		sum = cadd(sum, t[j]);
+	}
+
+	const float2 x0 = x[0];
+	x[0] = sum;
+#pragma unroll
+	for (int k = 1; k <= H; k++) {
+
+		float2 a = x0, b = make_float2(0.f, 0.f);
+#pragma unroll
+		for (int j = 1; j <= H; j++) {
+
+			a.x = fmaf(c[(j * k) % N], t[j].x, a.x);
+			a.y = fmaf(c[(j * k) % N], t[j].y, a.y);
+			b.x = fmaf(s[(j * k) % N], d[j].x, b.x);
+			b.y = fmaf(s[(j * k) % N], d[j].y, b.y);
+		}
+
+		b = rot90<INV>(b);
+		x[k] = cadd(a, b);
+		x[N - k] = csub(a, b);
+	}
+}
+
+// cos and sin of 2 pi k / 5, 2 pi k / 7 and 2 pi k / 9
+template <bool INV>
+__device__ __forceinline__ void dft5(float2 (&x)[5])
+{
+	constexpr float c1 = 0.30901699437494742410f, c2 = -0.80901699437494742410f;
+	constexpr float s1 = 0.95105651629515357212f, s2 = 0.58778525229247312917f;
+	const float c[5] = { 1.f, c1, c2, c2, c1 };
+	const float s[5] = { 0.f, s1, s2, -s2, -s1 };
+	dft_odd<5, INV>(x, c, s);
+}
+
+template <bool INV>
+__device__ __forceinline__ void dft7(float2 (&x)[7])
+{
+	constexpr float c1 = 0.62348980185873353053f, c2 = -0.22252093395631440429f, c3 = -0.90096886790241912624f;
+	constexpr float s1 = 0.78183148246802980871f, s2 = 0.97492791218182360702f, s3 = 0.43388373911755812048f;
+	const float c[7] = { 1.f, c1, c2, c3, c3, c2, c1 };
+	const float s[7] = { 0.f, s1, s2, s3, -s3, -s2, -s1 };
+	dft_odd<7, INV>(x, c, s);
+}
+
+// 3 x 3: columns x[a], x[a + 3], x[a + 6], twiddles W9^(a b), rows
+template <bool INV>
+__device__ __forceinline__ void dft9(float2 (&x)[9])
+{
+	const float sg = INV ? 1.f : -1.f;
+	const float2 w1 = make_float2(0.76604444311897803520f, sg * 0.64278760968653932632f);
+	const float2 w2 = make_float2(0.17364817766693034885f, sg * 0.98480775301220805937f);
+	const float2 w4 = make_float2(-0.93969262078590838405f, sg * 0.34202014332566873304f);
+#pragma unroll
+	for (int a = 0; a < 3; a++)
+		dft3<INV>(x[a], x[a + 3], x[a + 6]);
+
+	x[4] = cmul(x[4], w1);		// column 1, frequency 1
+	x[7] = cmul(x[7], w2);		// column 1, frequency 2
+	x[5] = cmul(x[5], w2);		// column 2, frequency 1
+	x[8] = cmul(x[8], w4);		// column 2, frequency 2
+	float2 y[9];
+#pragma unroll
+	for (int b = 0; b < 3; b++) {
+
+		float2 p = x[3 * b], q = x[3 * b + 1], r = x[3 * b + 2];
+		dft3<INV>(p, q, r);
+		y[b] = p;
+		y[b + 3] = q;
+		y[b + 6] = r;
+	}
+#pragma unroll
+	for (int k = 0; k < 9; k++)
+		x[k] = y[k];
+}
+
+// R = A B with coprime factors (prime-factor algorithm, no twiddles): input
+// index (B a + A b) mod R, output k from (k mod A, k mod B)
+template <int A, int B, bool INV>
+__device__ __forceinline__ void dft_pfa(float2 (&x)[A * B])
+{
+	float2 y[A][B];
+#pragma unroll
+	for (int b = 0; b < B; b++) {
+
+		float2 u[A];
+#pragma unroll
+		for (int a = 0; a < A; a++)
+			u[a] = x[(B * a + A * b) % (A * B)];
+
+		if constexpr (2 == A)
+			dft2<INV>(u);
+		else
+			dft4<INV>(u);
+#pragma unroll
+		for (int a = 0; a < A; a++)
+			y[a][b] = u[a];
+	}
+#pragma unroll
+	for (int a = 0; a < A; a++) {
+
+		if constexpr (3 == B)
+			dft3<INV>(y[a][0], y[a][1], y[a][2]);
+		else
+			dft5<INV>(y[a]);
+	}
+#pragma unroll
+	for (int k = 0; k < A * B; k++)
+		x[k] = y[k % A][k % B];
+}
+
+template <int R, bool INV>
+__device__ __forceinline__ void dft_mix(float2 (&x)[R])
+{
+	static_assert((3 == R) || (5 == R) || (6 == R) || (7 == R) || (9 == R) || (10 == R) || (12 == R), "built radices");
+
+	if constexpr (3 == R)
+		dft3<INV>(x[0], x[1], x[2]);
+	else if constexpr (5 == R)
+		dft5<INV>(x);
+	else if constexpr (7 == R)
+		dft7<INV>(x);
+	else if constexpr (9 == R)
+		dft9<INV>(x);
+	else if constexpr (6 == R)
+		dft_pfa<2, 3, INV>(x);
+	else if constexpr (10 == R)
+		dft_pfa<2, 5, INV>(x);
+	else
+		dft_pfa<4, 3, INV>(x);
+}
+
+// Forward transform of v (positions jt + (L/8) m) into the spectrum-side set
+// w. DB: two exchange buffers, one barrier per exchange (see fft_regs_db);
+// else s2 == s and a barrier on entry.
+template <int L, typename LAY, bool DB>
+__device__ __forceinline__ void mix_fwd(float2 (&v)[8], float2 (&w)[spec_regs(L)], float2* s, float2* s2,
+		const float2* tw, bool half_in)
+{
+	constexpr int R = L / 64, T = L / 8;
+	const int b = LAY::seq(), jt = LAY::jt();
+
+	if (half_in)
+		dft8_half<false>(v);
+	else
+		dft8<false>(v);
+
+	if (!DB)
+		__syncthreads();
+#pragma unroll
+	for (int i = 0; i < 8; i++)
+		s[LAY::idx(8 * jt + i, b)] = v[i];
+
+	__syncthreads();
+#pragma unroll
+	for (int i = 0; i < 8; i++)
+		v[i] = s[LAY::idx(jt + i * T, b)];
+
+	if (!DB)
+		__syncthreads();
+
+	const int k = jt % 8;
+	twiddle<L, 8, 8, false>(v, k, tw);
+	dft8<false>(v);
+#pragma unroll
+	for (int i = 0; i < 8; i++)
+		s2[LAY::idx((jt - k) * 8 + k + 8 * i, b)] = v[i];
+
+	__syncthreads();
+#pragma unroll
+	for (int q = 0; q < spec_regs(L) / R; q++) {
+
+		const int j = min(jt + q * T, 63);	// surplus threads repeat the last butterfly
+		float2 u[R];
+#pragma unroll
+		for (int i = 0; i < R; i++)
+			u[i] = s2[LAY::idx(j + 64 * i, b)];
+
+		// W_L^(i j): entries j, 2j, 4j, 8j and products
+		const float2 w1 = tw[j], w2 = tw[2 * j], w3 = cmul(w2, w1);
+		u[1] = cmul(u[1], w1);
+		u[2] = cmul(u[2], w2);
+
+		if constexpr (R > 3) {
+
+			const float2 w4 = tw[4 * j];
+			u[3] = cmul(u[3], w3);
+			u[4] = cmul(u[4], w4);
+
+			if constexpr (R > 5)
+				u[5] = cmul(u[5], cmul(w4, w1));
+
+			if constexpr (R > 6)
+				u[6] = cmul(u[6], cmul(w4, w2));
+
+			if constexpr (R > 7)
+				u[7] = cmul(u[7], cmul(w4, w3));
+		}
+
+		if constexpr (R > 8) {
+
+			const float2 w8 = tw[8 * j];
+			u[8] = cmul(u[8], w8);
+
+			if constexpr (R > 9)
+				u[9] = cmul(u[9], cmul(w8, w1));
+
+			if constexpr (R > 11) {
+
+				u[10] = cmul(u[10], cmul(w8, w2));
+				u[11] = cmul(u[11], cmul(w8, w3));
+			}
+		}
+
+		dft_mix<R, false>(u);
+#pragma unroll
+		for (int i = 0; i < R; i++)
+			w[q * R + i] = u[i];
+	}
+}
+
+// Inverse transform of the spectrum-side set w into v.
+template <int L, typename LAY, bool DB>
+__device__ __forceinline__ void mix_inv(float2 (&w)[spec_regs(L)], float2 (&v)[8], float2* s, float2* s2,
+		const float2* tw)
+{
+	constexpr int R = L / 64, T = L / 8;
+	const int b = LAY::seq(), jt = LAY::jt();
+
+	if (!DB)
+		__syncthreads();
+#pragma unroll
+	for (int q = 0; q < spec_regs(L) / R; q++) {
+
+		const int j = jt + q * T;
+		float2 u[R];
+#pragma unroll
+		for (int i = 0; i < R; i++)
+			u[i] = w[q * R + i];
+
+		dft_mix<R, true>(u);
+
+		if (j < 64) {
+#pragma unroll
+			for (int i = 0; i < R; i++)
+				s[LAY::idx(R * j + i, b)] = u[i];
+		}
+	}
+
+	__syncthreads();
+#pragma unroll
+	for (int i = 0; i < 8; i++)
+		v[i] = s[LAY::idx(jt + i * T, b)];
+
+	if (!DB)
+		__syncthreads();
+
+	const int k = jt % R;
+	twiddle<L, R, 8, true>(v, k, tw);
+	dft8<true>(v);
+#pragma unroll
+	for (int i = 0; i < 8; i++)
+		s2[LAY::idx((jt - k) * 8 + k + R * i, b)] = v[i];
+
+	__syncthreads();
+#pragma unroll
+	for (int i = 0; i < 8; i++)
+		v[i] = s2[LAY::idx(jt + i * T, b)];
+
+	twiddle<L, 8 * R, 8, true>(v, jt, tw);
+	dft8<true>(v);
+}
+
+// Forward and inverse transforms of any built length between the input-side
+// set v and the spectrum-side set w (the same registers for powers of two);
+// single exchange buffer, barrier on entry.
+template <int L, typename LAY>
+__device__ __forceinline__ void fft_fwd(float2 (&v)[8], float2 (&w)[spec_regs(L)], float2* s, const float2* tw,
+		bool half_in = false)
+{
+	if constexpr (is_mix(L)) {
+
+		mix_fwd<L, LAY, false>(v, w, s, s, tw, half_in);
+
+	} else {
+
+		fft_regs<L, LAY, false>(v, s, tw, half_in);
+#pragma unroll
+		for (int m = 0; m < 8; m++)
+			w[m] = v[m];
+	}
+}
+
+template <int L, typename LAY>
+__device__ __forceinline__ void fft_inv(float2 (&w)[spec_regs(L)], float2 (&v)[8], float2* s, const float2* tw)
+{
+	if constexpr (is_mix(L)) {
+
+		mix_inv<L, LAY, false>(w, v, s, s, tw);
+
+	} else {
+#pragma unroll
+		for (int m = 0; m < 8; m++)
+			v[m] = w[m];
+
+		fft_regs<L, LAY, true>(v, s, tw);
+	}
 }
 
 // stage-1 position of register m for this thread

@@ -337,6 +337,34 @@ def test_tiled_scatter_matches_atomic(N, spokes, coils, nd, periodic, monkeypatc
     assert rel(outs[0], want.reshape(cd, order="F")) < TOL
 
 
+@pytest.mark.parametrize("dims,coils", [
+    ((96, 160, 1), 2), ((192, 224, 1), 1), ((288, 320, 1), 1), ((384, 62, 1), 2),      # the mixed lengths
+    ((70, 132, 1), 3), ((104, 90, 1), 5), ((154, 54, 1), 1),    # radices 2 to 13
+    ((228, 34, 1), 1),                                          # 456 = 8 3 19 and 68 = 4 17: Bluestein
+    ((250, 500, 1), 1),                                         # four sequences per block
+    ((36, 40, 50), 2)])
+def test_grid_lengths_vs_oracle(dims, coils):
+    """Forward, adjoint and Toeplitz normal on grids of mixed lengths (64 times
+    3, 5, 6, 7, 9, 10, 12), of smooth lengths (products of radices up to 13)
+    and of lengths with a larger prime factor, on the two sides of a
+    rectangle, against the float64 oracle. Transforms of at most 1000 points
+    per axis add less than 1e-6 to the gridding's float32 sums."""
+    rng = np.random.default_rng(sum(dims))
+    t = rng.uniform(-0.5, 0.5, (3, 60, 50)) * np.array(dims)[:, None, None]
+    t[np.array(dims) == 1] = 0.0
+    t = t.astype(np.complex64)
+    cd, kd = list(dims) + [coils], [1, 60, 50, coils]
+    op = nufft_create2(kd, cd, list(t.shape), t, conf=NufftConf(toeplitz=True))
+    o = orc.NufftOracle(t.real.reshape(3, -1, order="F"), dims)
+    x = (rng.standard_normal(cd) + 1j * rng.standard_normal(cd)).astype(np.complex64)
+    y = (rng.standard_normal(kd) + 1j * rng.standard_normal(kd)).astype(np.complex64)
+    fwd, adj, nrm = (np.asarray(v).copy() for v in (op.forward(x), op.adjoint(y), op.normal(x)))
+    op.free()
+    assert rel(fwd.reshape(-1, coils, order="F"), o.forward(x)) < TOL
+    assert rel(adj, o.adjoint(y.reshape(-1, coils, order="F"))) < TOL
+    assert rel(nrm, o.normal_toeplitz(x)) < TOL
+
+
 @pytest.mark.parametrize("name", ["nufft2d_n64_chain", "nufft2d_n64_chain_weights", "nufft3d_n16_chain"])
 def test_chain_vs_reference(name):
     """Oversampling other than 2 (nufft -o 1.25 / 1.5 / 2.5: the reference's

@@ -5,6 +5,7 @@ import os
 import numpy as np
 import pytest
 
+from bart_b200 import synth
 from bart_b200.pics import Pics, PicsConf
 from conftest import golden, rel
 from oracle import nufft_oracle as orc
@@ -286,6 +287,37 @@ def test_padded_precond_matches_oracle():
     p.free()
     zo = orc.padded_precond(A.nufft, 0.01)(r.astype(np.complex128).reshape(N, N, 1, 1))[:, :, 0, 0]
     assert rel(z, (N * N) ** 2 * zo) < 1e-5
+
+
+@pytest.mark.parametrize("N", [72, 100])
+def test_padded_precond_keeps_power_of_two_grid(N):
+    """Where the normal operator runs on a shorter grid than the power of two
+    (2N = 144 on 192; 2N = 200 on 256, the same), the padded-circulant
+    preconditioner is still the power-of-two circulant's: its application
+    against the float64 one from the oracle's PSF, and the normal operator on
+    its own grid against the oracle."""
+    rng = np.random.default_rng(N)
+    traj = synth.radial_traj(N, 40)
+    sens = synth.coil_maps(N, 3, rng)
+    lam, L, E = 0.01, 2 * N, 256
+    p = Pics(traj, sens, conf=PicsConf(lam=lam, precond=3))
+    r = (rng.standard_normal((N, N)) + 1j * rng.standard_normal((N, N))).astype(np.complex64)
+    z = np.asarray(p.precond(np.asfortranarray(r))).reshape(N, N, order="F")
+    y = np.asarray(p.normal(np.asfortranarray(r))).reshape(N, N, order="F")
+    p.free()
+    A = orc.SenseOracle(traj.real.reshape(3, -1, order="F"), sens)
+    q = np.fft.ifft2(np.fft.ifftshift(A.nufft.psf()[:, :, 0])) / (N * N)
+    d = np.arange(-N + 1, N)
+    qe = np.zeros((E, E), dtype=np.complex128)
+    qe[np.ix_(d % E, d % E)] = q[np.ix_(d % L, d % L)]
+    P = np.abs(np.fft.fft2(qe)) * (L / E) ** 2
+    mu = max(2.5 * lam * 16.0 / E ** 2, 1e-3 * P[0, 0])
+    want = E * E * np.fft.ifft2(np.fft.fft2(r.astype(np.complex128), (E, E)) / (P + mu))[:N, :N]
+    assert rel(z, want) < 1e-5
+    s = sens[:, :, 0].astype(np.complex128)
+    cim = (r.astype(np.complex128)[:, :, None] * s)[:, :, None, :]
+    full = np.sum(np.conj(s) * A.nufft.normal_toeplitz(cim)[:, :, 0, :], axis=2)
+    assert rel(y, full) < 1e-5
 
 
 def test_fcg_folded_launches_match_unfolded():
