@@ -829,8 +829,13 @@ struct Bins {
 	int* multi = nullptr;		// [ntiles + 1] tiles with several work items; their number in [ntiles]
 	long nwork_max = 0;		// upper bound of work items (launch size)
 	int chunk = 256;		// hits per work item
+	bool det = false;		// deterministic: hits in sample order, partial tiles instead of atomics
+	int* slot = nullptr;		// [ntiles + 1] first partial of each tile with several work items
+	long nslots = 0;
+	float2* part = nullptr;		// [nslots][part_c][cells of a tile]
+	long part_c = 0;
 	float4* foot = nullptr;		// [M][FOOT_F4] footprints of the sorted samples
-	bool gather = false;		// they serve the degridding (k_degrid6_quads)
+	bool quads = false;		// they serve the quad kernels (degridding, single-channel scatter)
 	float2* kperm = nullptr;	// [M][kperm_c] k-space in bin order, a sample's coils side by side
 	long kperm_c = 0;
 };
@@ -866,7 +871,7 @@ struct OpCtx {
 static void free_bins(Bins& b, cudaStream_t st)
 {
 	void* ptrs[] = { b.perm, b.traj, b.sub_bin, b.sub_first, b.sub_count, b.sub_start, b.hit_start, b.hits, b.work_tile,
-			b.work_chunk, b.work_start, b.multi, b.foot, b.kperm };
+			b.work_chunk, b.work_start, b.multi, b.foot, b.kperm, b.slot, b.part };
 
 	for (void* q : ptrs)
 		if (q)
@@ -1145,7 +1150,7 @@ static int degrid(OpCtx& op, const float2* grid, long C, float2* ksp, cudaStream
 {
 	const long M = op.g.M;
 
-	if (op.bins.foot && op.bins.gather) {
+	if (op.bins.quads) {
 
 		const Bins& b = op.bins;
 		cudaEvent_t pe = prof_begin("degrid", st);
@@ -1187,8 +1192,18 @@ static int degrid(OpCtx& op, const float2* grid, long C, float2* ksp, cudaStream
 	return BNUFFT_OK;
 }
 
-// channels of a row of the bin-ordered k-space (16-byte copies: even)
-static long tg_row(long C) { return (C > 1) ? (C + 1) / 2 * 2 : 1; }
+// partial tiles of C channels (deterministic scatter)
+static int alloc_partials(Bins& b, long C, cudaStream_t st)
+{
+	const long cells = (long)b.bg.bs[0] * b.bg.bs[1] * b.bg.bs[2];
+	CUDA_TRY(cudaMallocAsync(&b.part, sizeof(float2) * std::max(1L, b.nslots * C * cells), st));
+	b.part_c = C;
+	return BNUFFT_OK;
+}
+
+// channels of a row of the bin-ordered k-space: jobs of several coils copy 16
+// bytes at a time, so their rows are even
+static long tg_row(int cfg, long C) { return ((TG_2D_C1 == cfg) || (TG_3D_C1 == cfg)) ? C : (C + 1) / 2 * 2; }
 
 template <int TX, int LY, int LZ, int CT>
 static int launch_tiles(const OpCtx& op, const TileWork& tw, int C, const float2* ksp, float2* grid, cudaStream_t st)
@@ -1199,7 +1214,7 @@ static int launch_tiles(const OpCtx& op, const TileWork& tw, int C, const float2
 	const unsigned nblk = (unsigned)((b.nwork_max * ((C + CW - 1) / CW) + TG_WARPS - 1) / TG_WARPS);
 	auto kern = k_grid6_tiles<TX, LY, LZ, CT>;
 	TRY(prep_kernel(kern, smem));
-	kern<<<nblk, 32 * TG_WARPS, smem, st>>>(op.g.M, grid_geom(op.g), b.bg, tw, C, (int)tg_row(C), ksp, grid);
+	kern<<<nblk, 32 * TG_WARPS, smem, st>>>(op.g.M, grid_geom(op.g), b.bg, tw, C, (int)tg_row(b.tg_cfg, C), ksp, grid);
 	LAUNCHED();
 	return BNUFFT_OK;
 }
@@ -1234,8 +1249,9 @@ static int grid_adj(OpCtx& op, const float2* ksp, long C, float2* grid, cudaStre
 
 		Bins& b = op.bins;
 		const GridGeom gg = grid_geom(op.g);
-		const long Cp = tg_row(C);
-		TileWork tw = { b.hit_start, b.hits, b.work_tile, b.work_chunk, b.work_start + b.ntiles, b.foot, b.chunk };
+		const long Cp = tg_row(b.tg_cfg, C);
+		TileWork tw = { b.hit_start, b.hits, b.work_tile, b.work_chunk, b.work_start + b.ntiles, b.foot, b.chunk, nullptr,
+				nullptr };
 
 		if (b.kperm_c < Cp) {	// more channels than the plan was made for (not while capturing)
 
@@ -1251,10 +1267,29 @@ static int grid_adj(OpCtx& op, const float2* ksp, long C, float2* grid, cudaStre
 		const dim3 pb((unsigned)((op.g.M + 31) / 32), (unsigned)((Cp + 31) / 32));
 		k_permute_ksp<<<pb, 256, 0, st>>>(b.kperm, ksp, b.perm, op.g.M, (int)C, (int)Cp, op.wgt, (int)op.wgt_c);
 		LAUNCHED();
+		if (b.det && (b.part_c < C)) {	// as above
+
+			if (b.part)
+				cudaFreeAsync(b.part, st);
+
+			b.part = nullptr;
+			b.part_c = 0;
+			TRY(alloc_partials(b, C, st));
+		}
+
 		cudaEvent_t pe = prof_begin("grid", st);
-		k_zero_tiles<<<(unsigned)std::min<long>((b.ntiles * C + 7) / 8, 8 * 148), 256, 0, st>>>(grid, gg, b.bg, b.multi,
+
+		if (b.det) {
+
+			tw.slot = b.slot;
+			tw.part = b.part;
+
+		} else {
+
+			k_zero_tiles<<<(unsigned)std::min<long>((b.ntiles * C + 7) / 8, 8 * 148), 256, 0, st>>>(grid, gg, b.bg, b.multi,
 				b.multi + b.ntiles, (int)C);
-		LAUNCHED();
+			LAUNCHED();
+		}
 
 		switch (b.tg_cfg) {
 		case TG_2D_C1:
@@ -1274,29 +1309,36 @@ static int grid_adj(OpCtx& op, const float2* ksp, long C, float2* grid, cudaStre
 			break;
 		}
 
+		if (b.det) {
+
+			k_sum_tiles<<<(unsigned)std::min<long>((b.ntiles * C + 7) / 8, 8 * 148), 256, 0, st>>>(grid, gg, b.bg, b.multi,
+					b.multi + b.ntiles, b.work_start, b.slot, b.part, (int)C);
+			LAUNCHED();
+		}
+
 		prof_end(pe, st);
 		return BNUFFT_OK;
 	}
 
 	CUDA_TRY(cudaMemsetAsync(grid, 0, sizeof(float2) * op.g.gsz * C, st));
 
-	if (op.bins.perm && (6.f == op.g.width) && (gridding_kind() >= 1)) {
+	if (op.bins.quads && (gridding_kind() >= 1)) {
 
 		const Bins& b = op.bins;
 		cudaEvent_t pe = prof_begin("grid", st);
-		unsigned nb = (unsigned)((op.g.M + BIN_THREADS - 1) / BIN_THREADS);
+		const unsigned nb = (unsigned)((4 * op.g.M + BIN_THREADS - 1) / BIN_THREADS);
 
 		if (op.g.G[2] > 1)
-			k_grid6_atomic<6><<<nb, BIN_THREADS, 0, st>>>(b.traj, b.perm, op.g.M, grid_geom(op.g), (int)C, ksp, grid, op.kb);
+			k_grid6_quads<6><<<nb, BIN_THREADS, 0, st>>>(b.foot, b.perm, op.g.M, grid_geom(op.g), (int)C, ksp, grid);
 		else
-			k_grid6_atomic<1><<<nb, BIN_THREADS, 0, st>>>(b.traj, b.perm, op.g.M, grid_geom(op.g), (int)C, ksp, grid, op.kb);
+			k_grid6_quads<1><<<nb, BIN_THREADS, 0, st>>>(b.foot, b.perm, op.g.M, grid_geom(op.g), (int)C, ksp, grid);
 
 		prof_end(pe, st);
 		LAUNCHED();
 		return BNUFFT_OK;
 	}
 
-	if (op.bins.perm && (6.f == op.g.width)) {
+	if (op.bins.perm && (6.f == op.g.width) && (0 == gridding_kind())) {
 
 		const Bins& b = op.bins;
 		int cc = (int)std::min<long>(b.cc, C);
@@ -1330,8 +1372,21 @@ static int grid_adj(OpCtx& op, const float2* ksp, long C, float2* grid, cudaStre
 	return BNUFFT_OK;
 }
 
+// the size limit of deterministic gridding (that of the CSR matrix)
+static int check_csr(const Geom& g)
+{
+	const long slots = (long)CSR_TAPS_AXIS * CSR_TAPS_AXIS * ((g.G[2] > 1) ? CSR_TAPS_AXIS : 1);
+
+	if ((g.M >= (1L << 31)) || ((unsigned long long)g.gsz * (unsigned long long)g.M >= (~0ull >> 1)) || (g.M * slots >= (1L << 31)))
+		return fail(BNUFFT_ERR_UNSUPPORTED, "deterministic gridding: %ld samples x %ld cells is too large", g.M, g.gsz);
+
+	return BNUFFT_OK;
+}
+
 // Build the CSR interpolation matrix of op's trajectory (stable sort by
 // cell * M + sample, so each row lists its samples in increasing order).
+// Deterministic gridding: with tiles (whose hits build_bins then listed in
+// order) there is nothing left to do; else the CSR matrix.
 static int build_csr(OpCtx& op, cudaStream_t st)
 {
 	const Geom& g = op.g;
@@ -1339,8 +1394,8 @@ static int build_csr(OpCtx& op, cudaStream_t st)
 	long slots = (long)CSR_TAPS_AXIS * CSR_TAPS_AXIS * slots_z;
 	long n = g.M * slots;
 
-	if ((g.M >= (1L << 31)) || ((unsigned long long)g.gsz * (unsigned long long)g.M >= (~0ull >> 1)) || (n >= (1L << 31)))
-		return fail(BNUFFT_ERR_UNSUPPORTED, "deterministic gridding: %ld samples x %ld cells is too large", g.M, g.gsz);
+	if (op.bins.det)
+		return BNUFFT_OK;
 
 	unsigned long long *keys = nullptr, *keys2 = nullptr;
 	float *vals = nullptr, *vals2 = nullptr;
@@ -1411,9 +1466,9 @@ static long tg_max_hits(const Geom& g, const BinGeom& bg)
 	return n;
 }
 
-// Sort the samples by bin and cut bins into sub-blocks (plan time). gather:
-// the plan also degrids.
-static int build_bins(OpCtx& op, cudaStream_t st, bool gather)
+// Sort the samples by bin and cut bins into sub-blocks (plan time). det: the
+// scatter is deterministic.
+static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 {
 	const Geom& g = op.g;
 	Bins& b = op.bins;
@@ -1432,13 +1487,15 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool gather)
 	// 144 us), while single-channel problems (little work per candidate
 	// sample) are faster with the global-atomic scatter (256^2, 402 spokes:
 	// 55 against 122 us); BNUFFT_GRIDDING=lines selects it everywhere
-	const bool tg_want = (2 == gridding_kind()) ? (op.coils >= 2) : (3 == gridding_kind());
+	// (deterministic: tiles for single channels too, and of one shape, so that a
+	// channel's sums do not depend on how many are gridded at once)
+	const bool tg_want = (2 == gridding_kind()) ? (det || (op.coils >= 2)) : (3 == gridding_kind());
 
 	if ((6.f == g.width) && (0 == op.bin_edge) && tg_want && (g.G[0] > 1) && (g.G[1] > 1)) {
 
 		const bool d3 = (g.G[2] > 1);
-		int cfg = d3 ? ((op.coils >= 2) ? TG_3D_C8 : TG_3D_C1)
-				: ((op.coils >= 5) ? TG_2D_C8 : ((op.coils >= 2) ? TG_2D_C4 : TG_2D_C1));
+		int cfg = d3 ? ((det || (op.coils >= 2)) ? TG_3D_C8 : TG_3D_C1)
+				: ((det || (op.coils >= 5)) ? TG_2D_C8 : ((op.coils >= 2) ? TG_2D_C4 : TG_2D_C1));
 		int t[3];
 		tg_shape(cfg, t);
 		bool ok = true;
@@ -1538,17 +1595,23 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool gather)
 
 	// the samples' footprints (start cells and weights): they depend on
 	// the trajectory only, so every apply reads them instead of recomputing
-	// 18 table lookups per sample. The degridding needs sides of at least 16
-	// cells and z offsets that fit an int; other sizes take k_degrid.
-	b.gather = gather && (6.f == g.width) && (g.gsz < (1L << 31));
+	// 18 table lookups per sample. The quad kernels need sides of at least 16
+	// cells and z offsets that fit an int; other sizes take the generic ones.
+	b.quads = (6.f == g.width) && (g.gsz < (1L << 31));
 
 	for (int a = 0; a < 3; a++)
-		b.gather = b.gather && ((1 == g.G[a]) || (g.G[a] >= 16));
+		b.quads = b.quads && ((1 == g.G[a]) || (g.G[a] >= 16));
 
-	if ((b.tg_cfg >= 0) || b.gather) {
+	short4* lo4 = nullptr;
+
+	if ((b.tg_cfg >= 0) || b.quads) {
 
 		CUDA_TRY(cudaMallocAsync(&b.foot, sizeof(float4) * FOOT_F4 * M, st));
-		k_foot<<<vec_blocks(M, 128, 8 * 148), 128, 0, st>>>(b.traj, M, grid_geom(g), op.kb, b.foot);
+
+		if (b.tg_cfg >= 0)
+			CUDA_TRY(cudaMallocAsync(&lo4, sizeof(short4) * M, st));
+
+		k_foot<<<vec_blocks(3 * M, 256, 8 * 148), 256, 0, st>>>(b.traj, M, grid_geom(g), op.kb, b.foot, lo4);
 		LAUNCHED();
 	}
 
@@ -1577,14 +1640,15 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool gather)
 		CUDA_TRY(cudaMallocAsync(&b.work_chunk, sizeof(int) * b.nwork_max, st));
 		CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, wtmp_bytes, cursor, b.hit_start, (int)(nt + 1), st));
 		CUDA_TRY(cudaMallocAsync(&wtmp, wtmp_bytes, st));
-		CUDA_TRY(cudaMemsetAsync(cursor, 0, sizeof(int) * (nt + 1), st));
+		CUDA_TRY(cudaMemsetAsync(cursor + nt, 0, sizeof(int), st));
 		CUDA_TRY(cudaMemsetAsync(b.multi + nt, 0, sizeof(int), st));
-		k_tile_hits<<<vec_blocks(M), RED_THREADS, 0, st>>>(b.foot, M, grid_geom(g), bg, cursor, nullptr);
+		const unsigned hb = (unsigned)std::min<long>(nt, 16 * 148);
+		k_tile_hits<<<hb, TH_THREADS, 0, st>>>(lo4, bin_start, grid_geom(g), bg, nt, cursor, nullptr, nullptr);
 		LAUNCHED();
 		CUDA_TRY(cub::DeviceScan::ExclusiveSum(wtmp, wtmp_bytes, cursor, b.hit_start, (int)(nt + 1), st));
-		CUDA_TRY(cudaMemcpyAsync(cursor, b.hit_start, sizeof(int) * nt, cudaMemcpyDeviceToDevice, st));
-		k_tile_hits<<<vec_blocks(M), RED_THREADS, 0, st>>>(b.foot, M, grid_geom(g), bg, cursor, b.hits);
+		k_tile_hits<<<hb, TH_THREADS, 0, st>>>(lo4, bin_start, grid_geom(g), bg, nt, nullptr, b.hit_start, b.hits);
 		LAUNCHED();
+		cudaFreeAsync(lo4, st);
 		k_tile_work<<<vec_blocks(nt + 1), RED_THREADS, 0, st>>>(b.hit_start, nt, b.chunk, nwork);
 		LAUNCHED();
 		CUDA_TRY(cub::DeviceScan::ExclusiveSum(wtmp, wtmp_bytes, nwork, b.work_start, (int)(nt + 1), st));
@@ -1592,6 +1656,21 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool gather)
 		k_work_fill<<<vec_blocks(nt), RED_THREADS, 0, st>>>(b.work_start, nt, b.work_tile, b.work_chunk, b.multi,
 				b.multi + nt);
 		LAUNCHED();
+
+		if (det) {
+
+			b.det = true;
+			CUDA_TRY(cudaMallocAsync(&b.slot, sizeof(int) * (nt + 1), st));
+			k_tile_slots<<<vec_blocks(nt + 1), RED_THREADS, 0, st>>>(nwork, nt, cursor);
+			LAUNCHED();
+			CUDA_TRY(cub::DeviceScan::ExclusiveSum(wtmp, wtmp_bytes, cursor, b.slot, (int)(nt + 1), st));
+			int total = 0;
+			CUDA_TRY(cudaMemcpyAsync(&total, b.slot + nt, sizeof(int), cudaMemcpyDeviceToHost, st));
+			CUDA_TRY(cudaStreamSynchronize(st));
+			b.nslots = total;
+			TRY(alloc_partials(b, op.coils, st));
+		}
+
 		cudaFreeAsync(nwork, st);
 		cudaFreeAsync(cursor, st);
 		cudaFreeAsync(wtmp, st);
@@ -1599,7 +1678,7 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool gather)
 		// the bin-ordered k-space of the applies, allocated here so that
 		// applies allocate nothing (their solves can then be captured into
 		// graphs and nested as child graphs)
-		b.kperm_c = tg_row(op.coils);
+		b.kperm_c = tg_row(b.tg_cfg, op.coils);
 		CUDA_TRY(cudaMallocAsync(&b.kperm, sizeof(float2) * M * b.kperm_c, st));
 	}
 
@@ -1747,7 +1826,10 @@ static int compute_psf(const Geom& g, const float2* traj_c, const float* kb, flo
 	in.kb = kb;
 	TRY(init_rolloff(in, st));
 
-	TRY(build_bins(in, st, false));
+	if (deterministic)
+		TRY(check_csr(in.g));
+
+	TRY(build_bins(in, st, deterministic));
 
 	if (deterministic)
 		TRY(build_csr(in, st));
@@ -2250,7 +2332,10 @@ static int upload_traj(bnufft_plan_s* p, const void* traj, cudaStream_t st, bool
 
 	// the chained NUFFT (os != 2) grids with the generic per-sample kernels
 	if ((BNUFFT_OK == s) && !p->op.g.chain)
-		s = build_bins(p->op, st, true);
+		s = p->conf.deterministic ? check_csr(p->op.g) : BNUFFT_OK;
+
+	if ((BNUFFT_OK == s) && !p->op.g.chain)
+		s = build_bins(p->op, st, 0 != p->conf.deterministic);
 
 	if ((BNUFFT_OK == s) && p->conf.deterministic) {
 

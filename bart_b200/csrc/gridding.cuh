@@ -9,9 +9,9 @@
 // Degridding (gather): four lanes per sample in bin order; neighbouring
 // samples read overlapping taps, so the gathers hit L1, and the weights are
 // read once per sample for all coils.
-// Gridding (scatter), default: one thread per sample in bin order with one
-// global float2 atomic per tap (bin order keeps a block's atomics within a
-// few L2 lines). Alternative (BNUFFT_GRIDDING=tiles): a block takes one
+// Gridding (scatter): output-stationary tiles for several channels, a quad of
+// lanes per sample with global atomics for one (bin order keeps a block's
+// atomics within a few L2 lines). Alternative (BNUFFT_GRIDDING=tiles): a block takes one
 // sub-block, accumulates its samples' taps into a zeroed shared-memory tile
 // (bin plus HALO cells per side, a chunk of coils) with shared-memory atomics
 // and flushes touched cells with one global atomic each; on B200 it measured
@@ -352,116 +352,6 @@ __global__ void __launch_bounds__(BIN_THREADS, 2) k_grid6_binned(const float4* _
 	}
 }
 
-// Gridding, width 6, without tiles: one thread per sample in bin order,
-// weights computed once for all coils, global atomics. The scatter is bound
-// by the L2's atomic-operation rate, which is the same for 8- and 16-byte
-// vector atomics: so the six x-taps of a sample (at most 7 consecutive cells
-// of a grid row) are laid into an 8-cell window starting at an even cell,
-// and each (z, y) row takes up to 4 float4 atomics (two cells each) instead
-// of 6 float2 ones. Windows that wrap around the row fall back to one float2
-// atomic per tap. Float sums in another order than the per-tap form: the
-// result is the same up to rounding (the atomics' order is arbitrary anyway).
-template <int TZ>
-__global__ void __launch_bounds__(BIN_THREADS, 2) k_grid6_atomic(const float4* __restrict__ traj_sorted,
-		const int* __restrict__ perm, long M, GridGeom g, int C,
-		const float2* __restrict__ ksp, float2* __restrict__ grid, const float* __restrict__ kbg)
-{
-	__shared__ float kb[KB_TABLE_N + 1];
-
-	for (int i = threadIdx.x; i <= KB_TABLE_N; i += blockDim.x)
-		kb[i] = kbg[i];
-
-	__syncthreads();
-
-	long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
-
-	if (i >= M)
-		return;
-
-	float4 k = traj_sorted[i];
-	Taps6 tx, ty, tz;
-	axis_taps6<0>(k.x, g.N[0], g.periodic, kb, 0, tx);
-	axis_taps6<0>(k.y, g.N[1], g.periodic, kb, 0, ty);
-	axis_taps6<0>(k.z, g.N[2], g.periodic, kb, 0, tz);
-	const long m = perm[i];
-
-	// the x window: taps with weight, their lowest and highest cell
-	int lo = INT_MAX, hi = INT_MIN;
-#pragma unroll
-	for (int e = 0; e < 6; e++) {
-
-		if (0.f != tx.w[e]) {
-
-			lo = min(lo, tx.cell[e]);
-			hi = max(hi, tx.cell[e]);
-		}
-	}
-
-	const int base = lo & ~1;
-	const bool vec = (lo <= hi) && (hi - base < 8);
-	float wx8[8];
-#pragma unroll
-	for (int j = 0; j < 8; j++) {
-
-		// only taps with weight: a clipped tap (weight 0) of a non-periodic
-		// grid may sit on the same cell as a valid one
-		float w = 0.f;
-#pragma unroll
-		for (int e = 0; e < 6; e++)
-			w = ((0.f != tx.w[e]) && (tx.cell[e] == base + j)) ? tx.w[e] : w;
-
-		wx8[j] = vec ? w : 0.f;
-	}
-
-	for (int c = 0; c < C; c++) {
-
-		float2 val = ksp[m + M * c];
-
-		if ((0.f == val.x) && (0.f == val.y))
-			continue;
-
-		float2* gc = grid + g.gsz * c;
-#pragma unroll 1
-		for (int a = 0; a < TZ; a++) {
-
-			float dz = tz.w[a];
-			long oz = (long)tz.cell[a] * g.G[1];
-#pragma unroll
-			for (int b = 0; b < 6; b++) {
-
-				float dzy = __fmul_rn(dz, ty.w[b]);
-				long oy = (oz + ty.cell[b]) * g.G[0];
-
-				if (0.f == dzy)
-					continue;
-
-				if (vec) {
-#pragma unroll
-					for (int q = 0; q < 4; q++) {
-
-						float d0 = __fmul_rn(dzy, wx8[2 * q]);
-						float d1 = __fmul_rn(dzy, wx8[2 * q + 1]);
-
-						if ((0.f != d0) || (0.f != d1))
-							atomicAdd((float4*)(gc + oy + base + 2 * q),
-								make_float4(val.x * d0, val.y * d0, val.x * d1, val.y * d1));
-					}
-
-				} else {
-#pragma unroll
-					for (int e = 0; e < 6; e++) {
-
-						float d = __fmul_rn(dzy, tx.w[e]);
-
-						if (0.f != d)
-							atomicAdd(&gc[oy + tx.cell[e]], make_float2(val.x * d, val.y * d));
-					}
-				}
-			}
-		}
-	}
-}
-
 // Footprint record of a sorted sample (built once per trajectory by
 // k_foot): float4 0 holds the centred start cells lo of the x, y, z taps
 // (as int bits); float4s 1..5 the weights of cells lo .. lo + 5 per axis,
@@ -534,9 +424,10 @@ __device__ __forceinline__ void foot6_w(float k, int N, int periodic, const floa
 }
 
 // footprints of all sorted samples (the weights as axis_taps6 computes them:
-// the same kb_lookup of the same float32 distances)
+// the same kb_lookup of the same float32 distances), a thread per sample and
+// axis; lo4 (if given): their start cells once more, for k_tile_hits
 __global__ void k_foot(const float4* __restrict__ traj_sorted, long M, GridGeom g, const float* __restrict__ kbg,
-		float4* __restrict__ foot)
+		float4* __restrict__ foot, short4* __restrict__ lo4)
 {
 	__shared__ float kb[KB_TABLE_N + 1];
 
@@ -545,29 +436,45 @@ __global__ void k_foot(const float4* __restrict__ traj_sorted, long M, GridGeom 
 
 	__syncthreads();
 
-	for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (long)gridDim.x * blockDim.x) {
+	for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < 3 * M; e += (long)gridDim.x * blockDim.x) {
 
+		const long i = e / 3;
+		const int a = (int)(e - 3 * i);
 		const float4 k = traj_sorted[i];
-		const float kk[3] = { k.x, k.y, k.z };
-		float w[24];
-		int lo[3];
-#pragma unroll
-		for (int a = 0; a < 3; a++) {
+		const float ka = (0 == a) ? k.x : ((1 == a) ? k.y : k.z);
+		const int N = (0 == a) ? g.N[0] : ((1 == a) ? g.N[1] : g.N[2]);
+		float w7[7];
+		const int lo = foot6_lo(ka, N);
+		foot6_w(ka, N, g.periodic, kb, lo, w7);
+		float* f = (float*)(foot + i * FOOT_F4);
+		f[a] = __int_as_float(lo);
 
-			float w7[7];
-			lo[a] = foot6_lo(kk[a], g.N[a]);
-			foot6_w(kk[a], g.N[a], g.periodic, kb, lo[a], w7);
-#pragma unroll
-			for (int t = 0; t < 6; t++)
-				w[6 * a + t] = w7[t];
+		if (lo4) {	// for k_tile_hits: cells further out than the grid's edges meet no tile
+
+			const int G = (1 == N) ? 1 : 2 * N;
+			int l = lo;
+
+			if (g.periodic) {
+
+				l %= G;
+				l = (l < 0) ? l + G : l;
+
+			} else {
+
+				l = min(max(l, -6), G);
+			}
+
+			((short*)(lo4 + i))[a] = (short)l;
 		}
-
-		w[18] = w[19] = w[20] = w[21] = w[22] = w[23] = 0.f;
-		float4* f = foot + i * FOOT_F4;
-		f[0] = make_float4(__int_as_float(lo[0]), __int_as_float(lo[1]), __int_as_float(lo[2]), 0.f);
 #pragma unroll
-		for (int q = 0; q < 5; q++)
-			f[1 + q] = make_float4(w[4 * q], w[4 * q + 1], w[4 * q + 2], w[4 * q + 3]);
+		for (int t = 0; t < 6; t += 2)
+			*(float2*)(f + 4 + 6 * a + t) = make_float2(w7[t], w7[t + 1]);
+
+		if (2 == a) {
+
+			f[3] = 0.f;
+			*(float2*)(f + 22) = make_float2(0.f, 0.f);
+		}
 	}
 }
 
@@ -648,6 +555,53 @@ __device__ __forceinline__ int cell_of(int c, int N, int G, int periodic)
 	return (c >= G) ? c - G : c;
 }
 
+// what a lane of a quad needs of its sample: two x cells and their weights, the
+// row and plane offsets of its taps, the y weights
+template <int TZ>
+struct Quad {
+
+	const float* f;			// the footprint record (z weights at 16)
+	float w0, w1;
+	int row[6], zoff[TZ];		// x cell included in row
+	float wy[6];
+
+	__device__ __forceinline__ Quad(const float4* foot, long i, const GridGeom& g)
+	{
+		const int q = threadIdx.x & 3;
+		const float4 h = foot[i * FOOT_F4];
+		f = (const float*)(foot + i * FOOT_F4);
+
+		// this lane's two cells of the x window
+		int lo = __float_as_int(h.x);
+
+		if (g.periodic) {
+
+			lo %= g.G[0];
+			lo = (lo < 0) ? lo + g.G[0] : lo;
+
+		} else {
+
+			lo = min(max(lo, -6), g.G[0]);	// further out all weights are 0
+		}
+
+		const int u = lo + g.N[0];
+		int e = (u & ~1) + 2 * q;
+		const int t = e - u;			// -1 .. 6
+		e = (e >= g.G[0]) ? e - g.G[0] : e;
+		w0 = ((t >= 0) && (t < 6)) ? f[4 + t] : 0.f;
+		w1 = (t < 5) ? f[5 + t] : 0.f;
+#pragma unroll
+		for (int b = 0; b < 6; b++) {
+
+			row[b] = cell_of(__float_as_int(h.y) + b, g.N[1], g.G[1], g.periodic) * g.G[0] + e;
+			wy[b] = f[10 + b];
+		}
+#pragma unroll
+		for (int a = 0; a < TZ; a++)
+			zoff[a] = (TZ > 1) ? cell_of(__float_as_int(h.z) + a, g.N[2], g.G[2], g.periodic) * g.G[1] * g.G[0] : 0;
+	}
+};
+
 template <int TZ>
 __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* __restrict__ foot,
 		const int* __restrict__ perm, long M, GridGeom g, int C, int cpb, const float2* __restrict__ grid,
@@ -656,43 +610,10 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* 
 	const int q = threadIdx.x & 3;
 	const long s = ((long)blockIdx.x * BIN_THREADS + threadIdx.x) / 4;
 	const long i = min(s, M - 1);		// surplus quads repeat the last sample and write nothing
-	const float4 h = foot[i * FOOT_F4];
-	const float* f = (const float*)(foot + i * FOOT_F4);
 	const long m = perm[i];
-
-	// this lane's two cells of the x window
-	int lo = __float_as_int(h.x);
-
-	if (g.periodic) {
-
-		lo %= g.G[0];
-		lo = (lo < 0) ? lo + g.G[0] : lo;
-
-	} else {
-
-		lo = min(max(lo, -6), g.G[0]);	// further out all weights are 0
-	}
-
-	const int u = lo + g.N[0];
-	int e = (u & ~1) + 2 * q;
-	const int t = e - u;			// -1 .. 6
-	e = (e >= g.G[0]) ? e - g.G[0] : e;
-	const float w0 = ((t >= 0) && (t < 6)) ? f[4 + t] : 0.f;
-	const float w1 = (t < 5) ? f[5 + t] : 0.f;
-	int row[6], zoff[TZ];
-	float wy[6];
-#pragma unroll
-	for (int b = 0; b < 6; b++) {
-
-		row[b] = cell_of(__float_as_int(h.y) + b, g.N[1], g.G[1], g.periodic) * g.G[0] + e;
-		wy[b] = f[10 + b];
-	}
-
-	// planes of up to 2^31 cells (z offsets of larger grids do not fit an int: the launcher checks)
-#pragma unroll
-	for (int a = 0; a < TZ; a++)
-		zoff[a] = (TZ > 1) ? cell_of(__float_as_int(h.z) + a, g.N[2], g.G[2], g.periodic) * g.G[1] * g.G[0] : 0;
-
+	const Quad<TZ> d(foot, i, g);
+	const float* f = d.f;
+	const float w0 = d.w0, w1 = d.w1;
 	const bool act = (0.f != w0) || (0.f != w1);
 	const bool valid = (s < M);
 	const int c0 = blockIdx.y * cpb, c1 = min(C, c0 + cpb);
@@ -701,7 +622,7 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* 
 	for (; c + 3 < c1; c += 4) {
 
 		float2 acc[4];
-		degrid6_quad<4, TZ>(grid + g.gsz * c, g.gsz, f, zoff, row, wy, w0, w1, act, acc);
+		degrid6_quad<4, TZ>(grid + g.gsz * c, g.gsz, f, d.zoff, d.row, d.wy, w0, w1, act, acc);
 		float2 k0 = (q & 2) ? acc[2] : acc[0], k1 = (q & 2) ? acc[3] : acc[1];
 		k0 = cadd(k0, shfl_xor2((q & 2) ? acc[0] : acc[2], 2));
 		k1 = cadd(k1, shfl_xor2((q & 2) ? acc[1] : acc[3], 2));
@@ -719,7 +640,7 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* 
 	for (; c < c1; c++) {
 
 		float2 acc[1];
-		degrid6_quad<1, TZ>(grid + g.gsz * c, g.gsz, f, zoff, row, wy, w0, w1, act, acc);
+		degrid6_quad<1, TZ>(grid + g.gsz * c, g.gsz, f, d.zoff, d.row, d.wy, w0, w1, act, acc);
 		float2 r = cadd(acc[0], shfl_xor2(acc[0], 2));
 		r = cadd(r, shfl_xor2(r, 1));
 
@@ -729,6 +650,56 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* 
 				r = cmul(r, wgt[m + M * (c % wgt_c)]);
 
 			ksp[m + M * c] = r;
+		}
+	}
+}
+
+// Gridding, width 6, with global atomics: a quad per sample in bin order as in
+// the degridding, one 16-byte reduction (two cells) per lane and tap row, so a
+// quad's reductions of a row fall into one 64-byte piece of the grid. Bound by
+// the L2's atomic units. The default for a single channel (one thread per
+// sample with four separate 16-byte reductions per row: 256^2 radial, 402
+// spokes, 51.8 us). The grid must be cleared.
+template <int TZ>
+__global__ void __launch_bounds__(BIN_THREADS) k_grid6_quads(const float4* __restrict__ foot,
+		const int* __restrict__ perm, long M, GridGeom g, int C, const float2* __restrict__ ksp,
+		float2* __restrict__ grid)
+{
+	const long i = ((long)blockIdx.x * BIN_THREADS + threadIdx.x) / 4;
+
+	if (i >= M)
+		return;
+
+	const long m = perm[i];
+	const Quad<TZ> d(foot, i, g);
+
+	if ((0.f == d.w0) && (0.f == d.w1))
+		return;
+
+	for (int c = 0; c < C; c++) {
+
+		const float2 val = ksp[m + M * c];
+
+		if ((0.f == val.x) && (0.f == val.y))
+			continue;	// grid(): samples that are zero are skipped
+
+		float2* gc = grid + g.gsz * c;
+#pragma unroll
+		for (int a = 0; a < TZ; a++) {
+
+			const float dz = d.f[16 + a];
+#pragma unroll
+			for (int b = 0; b < 6; b++) {
+
+				const float dzy = __fmul_rn(dz, d.wy[b]);
+
+				if (0.f == dzy)		// clipped tap
+					continue;
+
+				const float d0 = __fmul_rn(dzy, d.w0), d1 = __fmul_rn(dzy, d.w1);
+				atomicAdd((float4*)(gc + ((long)d.zoff[a] + d.row[b])),
+						make_float4(val.x * d0, val.y * d0, val.x * d1, val.y * d1));
+			}
 		}
 	}
 }
@@ -754,7 +725,8 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* 
 // Work items: tiles with one chunk of hits write their cells with plain stores
 // (empty tiles write zeros, so the grid needs no clearing), tiles with several
 // chunks (the dense k-space centre) add their chunks with atomics into cells
-// that k_zero_tiles cleared. Cells travel in pairs (16 bytes): tile edges and
+// that k_zero_tiles cleared, or in deterministic mode (hits listed in sample
+// order) leave partial tiles that k_sum_tiles adds in chunk order. Cells travel in pairs (16 bytes): tile edges and
 // grid sides are even. Weights are those of axis_taps6 (bit-identical to the
 // reference's grid_point_gen, src/noncart/grid.c:403-465) and the combined
 // weight the same float32 product ((1 * wz) * wy) * wx.
@@ -770,59 +742,127 @@ struct TileWork {
 	const int* nwork_dev;		// number of work items
 	const float4* foot;		// [M][FOOT_F4] footprints of the sorted samples
 	int chunk;			// hits per work item
+	const int* slot;		// deterministic: first partial of each tile with several items
+	float2* part;			// [slots][C][cells of a tile] its chunks' partial tiles (null: atomics)
 };
 
-// The tiles of one axis (nb tiles of edge t) that cells lo .. lo + 5 meet:
-// first tile and count (0: none); tiles past the last one wrap around
-__device__ __forceinline__ int2 axis_tiles(int lo, int t, int nb, int G, int periodic)
-{
-	if (1 == G)
-		return make_int2(0, 1);
+__device__ __forceinline__ int dft_index(int c, int N, int G);
+__device__ __forceinline__ int foot_rel(int lo, int origin, int G, int periodic);
 
-	if (periodic) {
+// The hits of every tile: the samples of its 3^d neighbour bins (bins are tiles;
+// a footprint reaches three cells either side of its sample) whose footprint
+// meets it, in bin order, so the lists are the same every time. A block takes a
+// tile; the x neighbours of a row of bins are one range of the sorted samples
+// (two where a periodic grid wraps). lo: the footprints' start cells.
+// hit_start == nullptr: count into nhits; else fill hits.
+enum { TH_THREADS = 128 };
 
-		lo %= G;
-		lo = (lo < 0) ? lo + G : lo;
-		const int first = lo / t, hi = lo + 5;
-		return make_int2(first, (hi < G) ? hi / t - first + 1 : nb - first + (hi - G) / t + 1);
-	}
-
-	if ((lo < -5) || (lo >= G))
-		return make_int2(0, 0);
-
-	const int first = max(lo, 0) / t;
-	return make_int2(first, min(lo + 5, G - 1) / t - first + 1);
-}
-
-// Hits per tile (hits == nullptr: count into cursor) or the hit lists
-// themselves (cursor starts as the tiles' first positions). The order within
-// a tile's list is that of the atomics.
-__global__ void k_tile_hits(const float4* __restrict__ foot, long M, GridGeom g, BinGeom bg, int* __restrict__ cursor,
+__global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restrict__ lo, const int* __restrict__ bin_start,
+		GridGeom g, BinGeom bg, long ntiles, int* __restrict__ nhits, const int* __restrict__ hit_start,
 		int* __restrict__ hits)
 {
-	for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < M; i += (long)gridDim.x * blockDim.x) {
+	__shared__ int wcount[TH_THREADS / 32];
+	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+	const int ry = (bg.nb[1] > 1) ? 1 : 0, rz = (bg.nb[2] > 1) ? 1 : 0;
 
-		const float4 f = foot[i * FOOT_F4];
-		const int2 ax = axis_tiles(__float_as_int(f.x), bg.bs[0], bg.nb[0], g.G[0], g.periodic);
-		const int2 ay = axis_tiles(__float_as_int(f.y), bg.bs[1], bg.nb[1], g.G[1], g.periodic);
-		const int2 az = axis_tiles(__float_as_int(f.z), bg.bs[2], bg.nb[2], g.G[2], g.periodic);
+	for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
 
-		for (int a = 0; a < az.y; a++) {
+		const int bx = (int)(t % bg.nb[0]), by = (int)((t / bg.nb[0]) % bg.nb[1]), bz = (int)(t / ((long)bg.nb[0] * bg.nb[1]));
+		const int ox = bx * bg.bs[0], oy = by * bg.bs[1], oz = bz * bg.bs[2];
+		int pos = hit_start ? hit_start[t] : 0;
+		int count = 0;
 
-			const int z = (az.x + a) % bg.nb[2];
+		for (int r = 0; r < 2 * (2 * ry + 1) * (2 * rz + 1); r++) {
 
-			for (int b = 0; b < ay.y; b++) {
+			// range r: part (0, or 1 past the periodic edge) of neighbour row (y, z)
+			int y = by + (r / 2) % (2 * ry + 1) - ry, z = bz + (r / 2) / (2 * ry + 1) - rz;
+			int x0 = bx - 1, x1 = bx + 2;
 
-				const int y = (ay.x + b) % bg.nb[1];
+			if (g.periodic) {
 
-				for (int c = 0; c < ax.y; c++) {
+				y = (y < 0) ? y + bg.nb[1] : ((y >= bg.nb[1]) ? y - bg.nb[1] : y);
+				z = (z < 0) ? z + bg.nb[2] : ((z >= bg.nb[2]) ? z - bg.nb[2] : z);
+			}
 
-					const int x = (ax.x + c) % bg.nb[0];
-					const int p = atomicAdd(&cursor[x + bg.nb[0] * (y + bg.nb[1] * z)], 1);
+			if ((y < 0) || (y >= bg.nb[1]) || (z < 0) || (z >= bg.nb[2]))
+				continue;
 
-					if (hits)
-						hits[p] = (int)i;
+			if (0 == r % 2) {
+
+				x0 = max(x0, 0);
+				x1 = min(x1, bg.nb[0]);
+
+			} else {
+
+				if (!g.periodic || ((x0 >= 0) && (x1 <= bg.nb[0])))
+					continue;
+
+				x0 = (x0 < 0) ? bg.nb[0] - 1 : 0;
+				x1 = x0 + 1;
+			}
+
+			const long row = (long)bg.nb[0] * (y + (long)bg.nb[1] * z);
+			const int s0 = bin_start[row + x0], s1 = bin_start[row + x1];
+
+			for (int base = s0; base < s1; base += TH_THREADS) {
+
+				const int i = base + threadIdx.x;
+				bool hit = false;
+
+				if (i < s1) {
+
+					const short4 l = lo[i];
+					const int lx = foot_rel(l.x, ox, g.G[0], g.periodic), ly = foot_rel(l.y, oy, g.G[1], g.periodic);
+					const int lz = foot_rel(l.z, oz, g.G[2], g.periodic);
+					hit = (lx > -6) && (lx < bg.bs[0]) && (ly > -6) && (ly < bg.bs[1]) && (lz > -6) && (lz < bg.bs[2]);
 				}
+
+				if (!hits) {
+
+					count += hit;
+					continue;
+				}
+
+				const unsigned m = __ballot_sync(0xffffffffu, hit);
+				__syncthreads();	// the previous counts have been read
+
+				if (0 == lane)
+					wcount[warp] = __popc(m);
+
+				__syncthreads();
+				int at = pos + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+				for (int w = 0; w < TH_THREADS / 32; w++) {
+
+					at += (w < warp) ? wcount[w] : 0;
+					pos += wcount[w];
+				}
+
+				if (hit)
+					hits[at] = i;
+			}
+		}
+
+		if (!hits) {
+
+			for (int o = 16; o > 0; o >>= 1)
+				count += __shfl_xor_sync(0xffffffffu, count, o);
+
+			__syncthreads();
+
+			if (0 == lane)
+				wcount[warp] = count;
+
+			__syncthreads();
+
+			if (0 == threadIdx.x) {
+
+				int n = 0;
+
+				for (int w = 0; w < TH_THREADS / 32; w++)
+					n += wcount[w];
+
+				nhits[t] = n;
 			}
 		}
 	}
@@ -833,6 +873,50 @@ __global__ void k_tile_work(const int* __restrict__ hit_start, long ntiles, int 
 {
 	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t <= ntiles; t += (long)gridDim.x * blockDim.x)
 		nwork[t] = (t < ntiles) ? max(1, (hit_start[t + 1] - hit_start[t] + chunk - 1) / chunk) : 0;
+}
+
+// partial tiles that deterministic mode needs: the chunks of tiles with several
+__global__ void k_tile_slots(const int* __restrict__ nwork, long ntiles, int* __restrict__ nslot)
+{
+	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t <= ntiles; t += (long)gridDim.x * blockDim.x)
+		nslot[t] = ((t < ntiles) && (nwork[t] > 1)) ? nwork[t] : 0;
+}
+
+// deterministic mode: the tiles with several chunks as the sums of their partial
+// tiles in chunk order; a warp per tile and channel
+__global__ void k_sum_tiles(float2* __restrict__ grid, GridGeom g, BinGeom bg, const int* __restrict__ multi,
+		const int* __restrict__ nmulti, const int* __restrict__ work_start, const int* __restrict__ slot,
+		const float2* __restrict__ part, int C)
+{
+	const int lane = threadIdx.x % 32;
+	const long n = (long)*nmulti * C;
+	const int cells = bg.bs[0] * bg.bs[1] * bg.bs[2];
+
+	for (long j = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32; j < n; j += (long)gridDim.x * blockDim.x / 32) {
+
+		const int t = multi[j / C], c = (int)(j % C);
+		const int bx = t % bg.nb[0], by = (t / bg.nb[0]) % bg.nb[1], bz = t / (bg.nb[0] * bg.nb[1]);
+		const int chunks = work_start[t + 1] - work_start[t];
+
+		for (int e = lane; e < cells; e += 32) {
+
+			const int cx = bx * bg.bs[0] + e % bg.bs[0];
+			const int cy = by * bg.bs[1] + (e / bg.bs[0]) % bg.bs[1];
+			const int cz = bz * bg.bs[2] + e / (bg.bs[0] * bg.bs[1]);
+
+			if ((cx >= g.G[0]) || (cy >= g.G[1]) || (cz >= g.G[2]))
+				continue;
+
+			float2 v = make_float2(0.f, 0.f);
+#pragma unroll 4
+			for (int k = 0; k < chunks; k++)
+				v = cadd(v, part[(((long)slot[t] + k) * C + c) * cells + e]);
+
+			const long cell = dft_index(cx, g.N[0], g.G[0]) + (long)g.G[0] * (dft_index(cy, g.N[1], g.G[1])
+					+ (long)g.G[1] * dft_index(cz, g.N[2], g.G[2]));
+			grid[cell + g.gsz * c] = v;
+		}
+	}
 }
 
 // work item table: tile t owns items work_start[t] .. work_start[t + 1] - 1;
@@ -974,7 +1058,7 @@ struct TgStage {
 
 // TX x-cells per lane, LY x LZ lines per tile (LY * LZ divides 32), CT coils
 // per lane: a warp job covers CW = (32 / (LY * LZ)) * CT coils. ksp: [M][Cp] in
-// bin order, Cp even (1 for one coil), zeros past the last coil.
+// bin order, Cp even unless CW = 1, zeros past the last coil.
 template <int TX, int LY, int LZ, int CT>
 __global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(long M, GridGeom g, BinGeom bg, TileWork tw, int C,
 		int Cp, const float2* __restrict__ ksp, float2* __restrict__ grid)
@@ -1163,10 +1247,12 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(long M, GridGe
 			float4* dst = (float4*)(grid + cell + g.gsz * (c0 + c));
 			const float4 v = make_float4(acc[i][c].x, acc[i][c].y, acc[i + 1][c].x, acc[i + 1][c].y);
 
-			if (add)
-				atomicAdd(dst, v);
-			else
+			if (!add)
 				*dst = v;
+			else if (tw.part)
+				*(float4*)(tw.part + (((long)tw.slot[tile] + tw.work_chunk[wi]) * C + c0 + c) * (TX * NL) + line * TX + i) = v;
+			else
+				atomicAdd(dst, v);
 		}
 	}
 }

@@ -337,6 +337,39 @@ def test_tiled_scatter_matches_atomic(N, spokes, coils, nd, periodic, monkeypatc
     assert rel(outs[0], want.reshape(cd, order="F")) < TOL
 
 
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("dims,samples,spokes,coils,periodic,weights", [
+    ((8, 8, 1), 16, 5, 1, False, False),        # the smallest sides of the quad kernels
+    ((50, 26, 1), 71, 33, 3, False, True),      # tiles cut short on both axes, odd coils, weights
+    ((50, 50, 1), 100, 40, 2, True, False),     # the same, wrapping around
+    ((100, 60, 1), 200, 300, 13, False, False),  # several chunks per tile, two coil jobs, the second partial
+    ((24, 30, 26), 48, 120, 5, False, False),   # 3D, partial tiles
+    ((26, 26, 26), 52, 80, 2, True, False)])    # 3D, wrapping around a partial tile
+def test_gridding_edges_vs_oracle(dims, samples, spokes, coils, periodic, weights, deterministic):
+    """Forward and adjoint where the tile lists, the quads' windows and the coil
+    groups of the width-6 kernels end, with samples beyond the band edge (their
+    taps are clipped or wrap), against the float64 oracle. Sums of at most a few
+    thousand float32 products: TOL covers them as for the other sizes."""
+    rng = np.random.default_rng(sum(dims) + coils)
+    t = rng.uniform(-0.52, 0.52, (3, samples, spokes)) * np.array(dims)[:, None, None]
+    t *= (np.arange(samples) / samples)[None, :, None]      # dense towards the centre
+    t[np.array(dims) == 1] = 0.0
+    t = t.astype(np.complex64)
+    cd, kd = list(dims) + [coils], [1, samples, spokes, coils]
+    w = (rng.uniform(0.5, 1.5, kd[:3]) * np.exp(1j * rng.uniform(0, 6, kd[:3]))).astype(np.complex64) if weights else None
+    op = nufft_create2(kd, cd, list(t.shape), t, None if w is None else list(w.shape), w,
+                       conf=NufftConf(toeplitz=False, periodic=periodic, deterministic=deterministic))
+    o = orc.NufftOracle(t.real.reshape(3, -1, order="F"), dims, periodic=periodic, weights=w)
+    x = (rng.standard_normal(cd) + 1j * rng.standard_normal(cd)).astype(np.complex64)
+    y = (rng.standard_normal(kd) + 1j * rng.standard_normal(kd)).astype(np.complex64)
+    fwd, adj = np.asarray(op.forward(x)), np.asarray(op.adjoint(y))
+    if deterministic:
+        assert np.array_equal(adj, np.asarray(op.adjoint(y)))
+    op.free()
+    assert rel(fwd.reshape(-1, coils, order="F"), o.forward(x)) < TOL
+    assert rel(adj, o.adjoint(y.reshape(-1, coils, order="F"))) < TOL
+
+
 @pytest.mark.parametrize("dims,coils", [
     ((96, 160, 1), 2), ((192, 224, 1), 1), ((288, 320, 1), 1), ((384, 62, 1), 2),      # the mixed lengths
     ((70, 132, 1), 3), ((104, 90, 1), 5), ((154, 54, 1), 1),    # radices 2 to 13
