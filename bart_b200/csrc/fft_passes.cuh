@@ -278,6 +278,7 @@ __device__ __forceinline__ double3 sum_partials3_d(const double* a, int na, cons
 //   stop if rs <= eps2, beta = rs / rs_prev, p = r + beta p_prev.
 // p_prev and p_cur are distinct buffers (blocks of other coils still read
 // p_prev while coil 0 writes p_cur); the CG step copies p_cur back to p_prev.
+// X <= L / 2 unless Bluestein (the grids are oversampled twofold or more).
 // Rows of coil 0 write p and the partial ||p||^2 (for lambda ||p||^2 in
 // p^H (A^H A + lambda) p); every row multiplies by its coil's map and runs the
 // forward transform like k_rows_fwd.
@@ -296,10 +297,36 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 	float2* s = smem;
 	float2* tw = smem + LAY::SMEM;
 
-	if (st->done)
+	const long row = (long)blockIdx.x * B + LAY::seq();
+	const bool valid = (row < R);
+	const long yz = valid ? row % YZ : 0;
+	const long c = valid ? row / YZ : 0;
+
+	// the inputs are on their way before the scalars are summed (their
+	// barriers would otherwise hold the loads back); of a transform that is
+	// zero-padded twofold or more only registers 0, 1, 6, 7 have any, of
+	// Bluestein's (d.n <= (L + 1) / 2) the first five
+	constexpr int NL = BLUE ? 5 : 4;
+	auto reg = [](int l) { return BLUE ? l : ((l < 2) ? l : l + 4); };
+	float2 rv[NL], po[NL], mv[NL];
+	it = cg_iter(it, st);
+	const int done = st->done;
+	const float2* ri = (0 == it) ? bvec : r;
+#pragma unroll
+	for (int l = 0; l < NL; l++) {
+
+		int p = reg_pos<L, LAY>(reg(l));
+		int n = (p < dn) ? unwrap_pos(p, X, dn) : X;
+		const bool in = valid && (n < X);
+		const long i = n + X * yz;
+		rv[l] = in ? ri[i] : make_float2(0.f, 0.f);
+		po[l] = (in && (it > 0)) ? p_prev[i] : make_float2(0.f, 0.f);
+		mv[l] = in ? maps[i + X * YZ * c] : make_float2(0.f, 0.f);
+	}
+
+	if (done)
 		return;
 
-	it = cg_iter(it, st);
 	float beta = 0.f;
 
 	if (it > 0) {
@@ -328,49 +355,43 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 	for (int i = threadIdx.x; i < L; i += NT)
 		tw[i] = twg[i];
 
-	const long row = (long)blockIdx.x * B + LAY::seq();
-	const bool valid = (row < R);
-	const long yz = valid ? row % YZ : 0;
-	const long c = valid ? row / YZ : 0;
 	double pp = 0.;
 	float2 v[8];
-
 #pragma unroll
-	for (int m = 0; m < 8; m++) {
-
-		int p = reg_pos<L, LAY>(m);
-		int n = (p < dn) ? unwrap_pos(p, X, dn) : X;
+	for (int m = 0; m < 8; m++)
 		v[m] = make_float2(0.f, 0.f);
+#pragma unroll
+	for (int l = 0; l < NL; l++) {
+
+		int p = reg_pos<L, LAY>(reg(l));
+		int n = (p < dn) ? unwrap_pos(p, X, dn) : X;
 
 		if (valid && (n < X)) {
 
-			long i = n + X * yz;
-			float2 pv;
+			float2 pv = rv[l];
 
-			if (0 == it) {
+			if (it > 0) {
 
-				pv = bvec[i];
-
-			} else {
-
-				float2 rv = r[i];
-				float2 po = p_prev[i];
-				pv.x = fmaf(beta, po.x, rv.x);
-				pv.y = fmaf(beta, po.y, rv.y);
+				pv.x = fmaf(beta, po[l].x, pv.x);
+				pv.y = fmaf(beta, po[l].y, pv.y);
 			}
 
 			if (0 == c) {
 
-				p_cur[i] = pv;
+				p_cur[n + X * yz] = pv;
 				pp += (double)pv.x * (double)pv.x + (double)pv.y * (double)pv.y;
 			}
 
-			float2 w = cmul(pv, maps[i + X * YZ * c]);
-			v[m] = ax ? cscale(w, ax[n] * ayz[yz]) : w;
+			float2 w = cmul(pv, mv[l]);
+			v[reg(l)] = ax ? cscale(w, ax[n] * ayz[yz]) : w;
 		}
 	}
 
-	double t = block_sum_d(pp, red);
+	// rows of coil 0 only are in the first blocks
+	double t = 0.;
+
+	if ((long)blockIdx.x * B < YZ)
+		t = block_sum_d(pp, red);
 
 	if (0 == threadIdx.x)
 		pp_part[blockIdx.x] = t;
@@ -410,8 +431,7 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 	float2* s = smem;
 	float2* tw = smem + LAY::SMEM;
 
-	if (done && *done)
-		return;
+	const int stop = done ? *done : 0;	// tested once the loads are under way
 
 	for (int i = threadIdx.x; i < L; i += NT)
 		tw[i] = twg[i];
@@ -436,6 +456,9 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 			v[m] = ax ? cscale(w, ax[n] * ayz[yz]) : w;
 		}
 	}
+
+	if (stop)
+		return;
 
 	float2 w[out_regs(L, BLUE)];
 	dft_fwd<L, LAY, BLUE>(v, w, s, tw, d, 2 * X <= L);
@@ -486,8 +509,7 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 	float2* s = smem;
 	float2* tw = smem + (DB ? 2 : 1) * LAY::SMEM;
 
-	if (done && *done)
-		return;
+	const int stop = done ? *done : 0;	// tested once the loads are under way
 
 	for (int i = threadIdx.x; i < L; i += NT)
 		tw[i] = twg[i];
@@ -512,6 +534,9 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 		int n = (p >= dn) ? n_in : (wrap_in ? unwrap_pos(p, n_in, dn) : p);
 		x[m] = (valid && (n < n_in)) ? inp[n * ies] : make_float2(0.f, 0.f);
 	}
+
+	if (stop)
+		return;
 
 	const bool half = wrap_in && (2 * n_in <= L);
 
@@ -610,8 +635,7 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 	float2* s = smem;
 	float2* tw = smem + LAY::SMEM;
 
-	if (done && *done)
-		return;
+	const int stop = done ? *done : 0;	// tested once the loads are under way
 
 	for (int i = threadIdx.x; i < L; i += NT)
 		tw[i] = twg[i];
@@ -639,6 +663,9 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 			int p = out_pos<L, LAY, BLUE>(m);
 			w[m] = (valid && (p < dn)) ? in[p + (long)dn * (yz + YZ * c)] : make_float2(0.f, 0.f);
 		}
+
+		if (stop)
+			return;
 
 		dft_inv<L, LAY, BLUE>(w, v, s, tw, d);
 

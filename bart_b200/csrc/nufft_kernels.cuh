@@ -40,8 +40,7 @@ __global__ void __launch_bounds__(TOE512_B * 16, 2) k_cols_toe512(const float2* 
 	float2* s = smem;
 	float2* tw = smem + L * SB;
 
-	if (done && *done)
-		return;
+	const int stop = done ? *done : 0;	// tested once the loads are under way
 
 	for (int i = threadIdx.x; i < L; i += blockDim.x)
 		tw[i] = twg[i];
@@ -60,6 +59,9 @@ __global__ void __launch_bounds__(TOE512_B * 16, 2) k_cols_toe512(const float2* 
 		const int n = wrap_in ? unwrap_pos(p, n_in, L) : p;
 		v[m] = (valid && (n < n_in)) ? inp[n * ies] : make_float2(0.f, 0.f);
 	}
+
+	if (stop)
+		return;
 
 	__syncthreads();	// the twiddle table is complete
 
