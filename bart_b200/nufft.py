@@ -11,6 +11,7 @@ place on the current torch stream.
 from __future__ import annotations
 
 import ctypes
+import math
 from dataclasses import dataclass
 
 import numpy as np
@@ -73,7 +74,7 @@ def _ptr_out(a, n: int):
 
 
 def _alloc_like(src, dims):
-    n = int(np.prod(dims))
+    n = math.prod(dims)
     if _is_torch(src):
         import torch
         return torch.empty(n, dtype=torch.complex64, device=src.device)
@@ -92,7 +93,7 @@ class Linop:
     def _call(self, fn, src, dst, in_dims, out_dims):
         if self._h is None:
             raise RuntimeError("linop was freed")
-        nin, nout = int(np.prod(in_dims)), int(np.prod(out_dims))
+        nin, nout = math.prod(in_dims), math.prod(out_dims)
         if dst is None:
             dst = _alloc_like(src, out_dims)
         ps, keep = _ptr_in(src, nin)
@@ -119,7 +120,7 @@ class Linop:
         preconditioner (needs the Toeplitz PSF)."""
         if self._h is None:
             raise RuntimeError("linop was freed")
-        nin, nout = int(np.prod(self.codomain_dims)), int(np.prod(self.domain_dims))
+        nin, nout = math.prod(self.codomain_dims), math.prod(self.domain_dims)
         if dst is None:
             dst = _alloc_like(ksp, self.domain_dims)
         pk, keep = _ptr_in(ksp, nin)
@@ -145,7 +146,7 @@ class Linop:
         lib = _lib.load()
         t = np.asarray(traj) if not _is_torch(traj) else traj
         tdims = dims16(t.shape) if not _is_torch(traj) else self._traj_dims
-        pt, keep = _ptr_in(t, int(np.prod(tdims)))
+        pt, keep = _ptr_in(t, math.prod(tdims))
         _lib.check(lib.bnufft_update_traj(self._h, len(tdims), _lib.dims_array(tdims), pt, _stream_of(traj)))
         del keep
 
@@ -177,17 +178,17 @@ def nufft_create2(ksp_dims, cim_dims, traj_dims, traj, wgh_dims=None, weights=No
     lib = _lib.load()
     conf = conf or NufftConf()
     kd, cd, td = dims16(ksp_dims), dims16(cim_dims), dims16(traj_dims)
-    pt, keep = _ptr_in(traj, int(np.prod(td)))
+    pt, keep = _ptr_in(traj, math.prod(td))
     wd_arr, pw, keep_w = None, None, None
     if weights is not None:
         wd = dims16(wgh_dims if wgh_dims is not None else np.shape(weights))
         wd_arr = _lib.dims_array(wd)
-        pw, keep_w = _ptr_in(weights, int(np.prod(wd)))
+        pw, keep_w = _ptr_in(weights, math.prod(wd))
     bd_arr, pb, keep_b = None, None, None
     if basis is not None:
         bd = dims16(bas_dims if bas_dims is not None else np.shape(basis))
         bd_arr = _lib.dims_array(bd)
-        pb, keep_b = _ptr_in(basis, int(np.prod(bd)))
+        pb, keep_b = _ptr_in(basis, math.prod(bd))
     h = ctypes.c_void_p()
     cc = conf.c()
     _lib.check(lib.bnufft_create2(ctypes.byref(h), 16, _lib.dims_array(kd), _lib.dims_array(cd),
@@ -216,7 +217,7 @@ class Nudft:
     def __init__(self, ksp_dims, cim_dims, traj_dims, traj):
         lib = _lib.load()
         kd, cd, td = dims16(ksp_dims), dims16(cim_dims), dims16(traj_dims)
-        pt, keep = _ptr_in(traj, int(np.prod(td)))
+        pt, keep = _ptr_in(traj, math.prod(td))
         h = ctypes.c_void_p()
         _lib.check(lib.bnufft_nudft_create(ctypes.byref(h), 16, _lib.dims_array(kd), _lib.dims_array(cd),
                                            _lib.dims_array(td), pt, _stream_of(traj)))
@@ -225,7 +226,7 @@ class Nudft:
         self.domain_dims, self.codomain_dims = cd, kd
 
     def _call(self, fn, src, dst, in_dims, out_dims):
-        nin, nout = int(np.prod(in_dims)), int(np.prod(out_dims))
+        nin, nout = math.prod(in_dims), math.prod(out_dims)
         if dst is None:
             dst = _alloc_like(src, out_dims)
         ps, keep = _ptr_in(src, nin)

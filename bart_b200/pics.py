@@ -10,6 +10,7 @@ libbnufft.
 from __future__ import annotations
 
 import ctypes
+import math
 from dataclasses import dataclass
 
 import numpy as np
@@ -53,8 +54,8 @@ class Pics:
         kd = dims16(ksp_dims)
         self.img_dims = sd[:3] + [1] * 13
         self.ksp_dims = kd
-        pt, k1 = _ptr_in(traj, int(np.prod(td)))
-        ps, k2 = _ptr_in(sens, int(np.prod(sd)))
+        pt, k1 = _ptr_in(traj, math.prod(td))
+        ps, k2 = _ptr_in(sens, math.prod(sd))
         h = ctypes.c_void_p()
         cc = self.conf.c()
         _lib.check(lib.bnufft_pics_create(ctypes.byref(h), 16, _lib.dims_array(kd), _lib.dims_array(sd),
@@ -63,8 +64,8 @@ class Pics:
 
     def run(self, ksp, out=None):
         """One reconstruction of ``ksp`` -> image [X, Y, Z]."""
-        n_in = int(np.prod(self.ksp_dims))
-        n_out = int(np.prod(self.img_dims))
+        n_in = math.prod(self.ksp_dims)
+        n_out = math.prod(self.img_dims)
         if out is None:
             out = _alloc_like(ksp, self.img_dims)
         pk, keep = _ptr_in(ksp, n_in)
@@ -75,7 +76,7 @@ class Pics:
 
     def normal(self, x, out=None):
         """A^H A x."""
-        n = int(np.prod(self.img_dims))
+        n = math.prod(self.img_dims)
         if out is None:
             out = _alloc_like(x, self.img_dims)
         px, keep = _ptr_in(x, n)
@@ -97,8 +98,8 @@ class Pics:
 
     def rhs(self, ksp, out=None):
         """b = A^H y / scale, the right-hand side of the solve."""
-        n_in = int(np.prod(self.ksp_dims))
-        n_out = int(np.prod(self.img_dims))
+        n_in = math.prod(self.ksp_dims)
+        n_out = math.prod(self.img_dims)
         if out is None:
             out = _alloc_like(ksp, self.img_dims)
         pk, keep = _ptr_in(ksp, n_in)
@@ -108,7 +109,7 @@ class Pics:
 
     def precond(self, r, out=None):
         """z = M(r) with the model's preconditioner (precond 1, 2 or 3)."""
-        n = int(np.prod(self.img_dims))
+        n = math.prod(self.img_dims)
         if out is None:
             out = _alloc_like(r, self.img_dims)
         pr, keep = _ptr_in(r, n)
