@@ -26,8 +26,36 @@
 
 namespace bn {
 
-__device__ __forceinline__ float2 cadd(float2 a, float2 b) { return make_float2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ float2 csub(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// Complex sums as one packed instruction each (the same two IEEE operations):
+// the transforms are bound by instruction issue, not by the FP32 pipes.
+__device__ __forceinline__ float2 cadd(float2 a, float2 b)
+{
+	float2 r;
+	asm("{\n\t.reg .b64 a, b, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+		"add.rn.f32x2 r, a, b;\n\tmov.b64 {%0, %1}, r;\n\t}"
+		: "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+	return r;
+}
+
+__device__ __forceinline__ float2 csub(float2 a, float2 b)
+{
+	float2 r;
+	asm("{\n\t.reg .b64 a, b, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\t"
+		"sub.rn.f32x2 r, a, b;\n\tmov.b64 {%0, %1}, r;\n\t}"
+		: "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+	return r;
+}
+
+// (a.x b.x + c.x, a.y b.y + c.y)
+__device__ __forceinline__ float2 cfma(float2 a, float2 b, float2 c)
+{
+	float2 r;
+	asm("{\n\t.reg .b64 a, b, c, r;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %5};\n\tmov.b64 c, {%6, %7};\n\t"
+		"fma.rn.f32x2 r, a, b, c;\n\tmov.b64 {%0, %1}, r;\n\t}"
+		: "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y), "f"(c.x), "f"(c.y));
+	return r;
+}
+
 __device__ __forceinline__ float2 cmul(float2 a, float2 b)
 {
 	return make_float2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);

@@ -978,13 +978,10 @@ __device__ __forceinline__ void tg_accum_x(float2 (&acc)[TX][CT], const float (&
 
 		if ((RX + t >= 0) && (RX + t < TX)) {
 
-			float d = __fmul_rn(wyz, wx[t]);
+			const float d = __fmul_rn(wyz, wx[t]);
 #pragma unroll
-			for (int c = 0; c < CT; c++) {
-
-				acc[RX + t][c].x = fmaf(v[c].x, d, acc[RX + t][c].x);
-				acc[RX + t][c].y = fmaf(v[c].y, d, acc[RX + t][c].y);
-			}
+			for (int c = 0; c < CT; c++)
+				acc[RX + t][c] = cfma(v[c], make_float2(d, d), acc[RX + t][c]);
 		}
 	}
 }
@@ -1192,29 +1189,23 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(long M, GridGe
 			}
 		};
 
-		float wyz, wx[6];
-		int rx;
-		float2 v[CT];
-		load(0, wyz, wx, rx, v);
+		// two sets of inputs in turn: one is loaded while the other is added
+		float wyz[2], wx[2][6];
+		int rx[2];
+		float2 v[2][CT];
+		load(0, wyz[0], wx[0], rx[0], v[0]);
 
-		for (int q = 0; q < n; q++) {
+		for (int q = 0; q < n; q += 2) {
 
-			float wyzn, wxn[6];
-			int rxn;
-			float2 vn[CT];
-			load(min(q + 1, n - 1), wyzn, wxn, rxn, vn);
+			load(min(q + 1, n - 1), wyz[1], wx[1], rx[1], v[1]);
 
-			if (0.f != wyz)
-				tg_switch<TX, CT>(rx, acc, wx, wyz, v);
+			if (0.f != wyz[0])
+				tg_switch<TX, CT>(rx[0], acc, wx[0], wyz[0], v[0]);
 
-			wyz = wyzn;
-			rx = rxn;
-#pragma unroll
-			for (int t = 0; t < 6; t++)
-				wx[t] = wxn[t];
-#pragma unroll
-			for (int c = 0; c < CT; c++)
-				v[c] = vn[c];
+			load(min(q + 2, n - 1), wyz[0], wx[0], rx[0], v[0]);
+
+			if ((0.f != wyz[1]) && (q + 1 < n))
+				tg_switch<TX, CT>(rx[1], acc, wx[1], wyz[1], v[1]);
 		}
 
 		__syncwarp();	// before the batch after next overwrites this buffer
