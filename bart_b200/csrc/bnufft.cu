@@ -329,7 +329,7 @@ static int choose_B(int L, long nseq)
 {
 	int B = 16;
 
-	while (B * L > 8192)
+	while (B * L > (is_mix(L) ? 3584 : 8192))	// mixed lengths: at most 448 threads, so two or three blocks per SM
 		B /= 2;
 
 	int Bmin = std::min(16, std::max(4, 256 / L));	// at least one warp per block
