@@ -3907,35 +3907,36 @@ extern "C" int bnufft_pics_normal(bnufft_pics_t ps, void* dst, const void* src, 
 	return stage_out_copy(o, dst, b, st);
 }
 
-// b = A^H y / scale into ps->b: adjoint (coil-sum partials, then combine) and
-// the data scaling of src/pics.c:499-530 (y /= scale  <=>  A^H y /= scale)
+// A^H y into ps->b (adjoint as coil-sum partials, then combined) and the data
+// scaling of src/pics.c:499-530 into the scalars; the solve starts from
+// b / scale (y /= scale  <=>  A^H y /= scale), divided by k_cg_init
 static int pics_prologue(bnufft_pics_s* ps, const float2* ksp, cudaStream_t st)
 {
 	OpCtx& op = ps->nufft->op;
 	unsigned nb = (unsigned)ps->nparts;
 	TRY(op_adjoint(op, ksp, ps->sens, ps->C, ps->cpg, ps->part, st));
-	k_combine<<<nb, RED_THREADS, 0, st>>>(ps->b, ps->part, ps->groups, ps->npix, nullptr, 0.f, nullptr, nullptr);
-	LAUNCHED();
 
 	if (0.f == ps->conf.scaling) {
 
-		// three order statistics of |b| by radix select (estimate_scaling_norm)
+		// three order statistics of |b| by radix select (estimate_scaling_norm);
+		// the first pass sums b from its coil groups
 		const unsigned sb = (unsigned)std::max(1L, std::min<long>((ps->npix + 4 * SEL_THREADS - 1) / (4 * SEL_THREADS), 2 * 148));
-		k_select_pass<0><<<sb, SEL_THREADS, 0, st>>>(ps->b, ps->mag, ps->npix, ps->sel, ps->scal);
+		const unsigned sb0 = (unsigned)std::max(1L, std::min<long>((ps->npix + SEL_THREADS - 1) / SEL_THREADS, 2 * 148));
+		k_select_pass<0><<<sb0, SEL_THREADS, 0, st>>>(ps->b, ps->part, ps->groups, ps->mag, ps->npix, ps->sel, ps->scal);
 		LAUNCHED();
-		k_select_pass<1><<<sb, SEL_THREADS, 0, st>>>(ps->b, ps->mag, ps->npix, ps->sel, ps->scal);
+		k_select_pass<1><<<sb, SEL_THREADS, 0, st>>>(ps->b, nullptr, 0, ps->mag, ps->npix, ps->sel, ps->scal);
 		LAUNCHED();
-		k_select_pass<2><<<sb, SEL_THREADS, 0, st>>>(ps->b, ps->mag, ps->npix, ps->sel, ps->scal);
+		k_select_pass<2><<<sb, SEL_THREADS, 0, st>>>(ps->b, nullptr, 0, ps->mag, ps->npix, ps->sel, ps->scal);
 		LAUNCHED();
 
 	} else {
 
+		k_combine<<<nb, RED_THREADS, 0, st>>>(ps->b, ps->part, ps->groups, ps->npix, nullptr, 0.f, nullptr, nullptr);
+		LAUNCHED();
 		k_set_scaling<<<1, 1, 0, st>>>(ps->scal, ps->conf.scaling);
 		LAUNCHED();
 	}
 
-	k_scale_dev<<<nb, RED_THREADS, 0, st>>>(ps->b, ps->b, ps->npix, &ps->scal->inv_scale);
-	LAUNCHED();
 	return BNUFFT_OK;
 }
 
@@ -4492,7 +4493,7 @@ static int pics_solve(bnufft_pics_s* ps, const float2* ksp, float2* out, cudaStr
 	TRY(pics_prologue(ps, ksp, st));
 
 	// CG from zero (conjgrad, src/iter/italgos.c:497-572)
-	k_cg_init<<<nb, RED_THREADS, 0, st>>>(ps->x, ps->r, ps->pbuf[1], ps->b, ps->npix, ps->rs_part);
+	k_cg_init<<<nb, RED_THREADS, 0, st>>>(ps->x, ps->r, ps->pbuf[1], ps->b, ps->npix, ps->rs_part, &ps->scal->inv_scale);
 	LAUNCHED();
 	k_cg_start<<<1, RED_THREADS, 0, st>>>(ps->scal, ps->rs_part, ps->nparts, ps->conf.tol, ps->conf.maxiter,
 			(0 == ps->conf.precond) && ps->conf.ref_scalars, (2 == ps->conf.precond) ? ps->conf.net_iters : 0);
@@ -4771,7 +4772,8 @@ extern "C" int bnufft_pics_rhs(bnufft_pics_t ps, void* b, const void* ksp, void*
 	TRY(stage_in(ki, ksp, kb, st));
 	TRY(stage_out_alloc(bo, b, ib, st));
 	TRY(pics_prologue(ps, (const float2*)ki.dev, st));
-	CUDA_TRY(cudaMemcpyAsync(bo.dev, ps->b, ib, cudaMemcpyDeviceToDevice, st));
+	k_scale_dev<<<(unsigned)ps->nparts, RED_THREADS, 0, st>>>((float2*)bo.dev, ps->b, ps->npix, &ps->scal->inv_scale);
+	LAUNCHED();
 	return stage_out_copy(bo, b, ib, st);
 }
 

@@ -107,8 +107,9 @@ __global__ void k_combine(float2* __restrict__ dst, const float2* __restrict__ p
 }
 
 // CG start from x = 0: x = 0, r = p = b; partial ||b||^2.
+// inv_scale: b is multiplied by it first.
 __global__ void k_cg_init(float2* __restrict__ x, float2* __restrict__ r, float2* __restrict__ p,
-		const float2* __restrict__ b, long n, double* __restrict__ part)
+		float2* __restrict__ b, long n, double* __restrict__ part, const float* inv_scale = nullptr)
 {
 	__shared__ double sh[32];
 	double acc = 0.;
@@ -116,6 +117,13 @@ __global__ void k_cg_init(float2* __restrict__ x, float2* __restrict__ r, float2
 	for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
 
 		float2 v = b[i];
+
+		if (inv_scale) {
+
+			v = cscale(v, *inv_scale);
+			b[i] = v;
+		}
+
 		x[i] = make_float2(0.f, 0.f);
 		r[i] = v;
 		p[i] = v;
@@ -175,14 +183,28 @@ __global__ void k_cg_start(CgScalars* st, const double* part, int nparts, float 
 // element Ap = sum_g part_g + lambda p, x += alpha p, r -= alpha Ap, and
 // partial ||r||^2 for the next iteration's direction update. p is also
 // copied to p_keep (the next iteration's previous direction) when given.
+// The first element's inputs are loaded before the partial sums are.
 __global__ void k_cg_step(float2* __restrict__ x, float2* __restrict__ r, const float2* __restrict__ p,
 		const float2* __restrict__ part, int groups, long n, float lam, CgScalars* st, int it,
 		const double* __restrict__ pap_part, int npap, const double* __restrict__ pp_part, int npp,
 		double* __restrict__ rs_part, float2* __restrict__ p_keep)
 {
 	__shared__ double sh[96];
+	const long stride = (long)gridDim.x * blockDim.x;
+	long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+	const int done = st->done;
+	float2 pv, av, xv, rv;
+	pv = av = xv = rv = make_float2(0.f, 0.f);
 
-	if (st->done)
+	if (i < n) {
+
+		pv = p[i];
+		av = group_sum(part, i, n, groups);
+		xv = x[i];
+		rv = r[i];
+	}
+
+	if (done)
 		return;
 
 	it = cg_iter(it, st);
@@ -203,19 +225,13 @@ __global__ void k_cg_step(float2* __restrict__ x, float2* __restrict__ r, const 
 	float a = cg_ratio(st, st->rs[it & 1], pAp);
 	double acc = 0.;
 
-	for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-
-		float2 pv = p[i];
-		float2 av = group_sum(part, i, n, groups);
+	while (i < n) {
 
 		if (p_keep)
 			p_keep[i] = pv;
 
 		av.x = fmaf(lam, pv.x, av.x);
 		av.y = fmaf(lam, pv.y, av.y);
-
-		float2 xv = x[i];
-		float2 rv = r[i];
 		xv.x = fmaf(a, pv.x, xv.x);
 		xv.y = fmaf(a, pv.y, xv.y);
 		rv.x = fmaf(-a, av.x, rv.x);
@@ -223,6 +239,15 @@ __global__ void k_cg_step(float2* __restrict__ x, float2* __restrict__ r, const 
 		x[i] = xv;
 		r[i] = rv;
 		acc += (double)rv.x * (double)rv.x + (double)rv.y * (double)rv.y;
+		i += stride;
+
+		if (i < n) {
+
+			pv = p[i];
+			av = group_sum(part, i, n, groups);
+			xv = x[i];
+			rv = r[i];
+		}
 	}
 
 	double s = block_sum(acc, sh);
@@ -458,8 +483,21 @@ __global__ void k_fcg_step(float2* __restrict__ x, float2* __restrict__ r, const
 		const double* __restrict__ pr_part, int npr, double* __restrict__ rs_part)
 {
 	__shared__ double sh[96];
+	const long stride = (long)gridDim.x * blockDim.x;
+	long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
+	const int done = st->done;
+	float2 pv, av, xv, rv;
+	pv = av = xv = rv = make_float2(0.f, 0.f);
 
-	if (st->done)
+	if (i < n) {	// on their way before the partial sums
+
+		pv = p[i];
+		av = group_sum(part, i, n, groups);
+		xv = x[i];
+		rv = r[i];
+	}
+
+	if (done)
 		return;
 
 	it = cg_iter(it, st);
@@ -481,17 +519,11 @@ __global__ void k_fcg_step(float2* __restrict__ x, float2* __restrict__ r, const
 	float2* Ap = ap_ring + (long)(it % ring) * n;
 	double acc = 0.;
 
-	for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-
-		float2 pv = p[i];
-		float2 av = group_sum(part, i, n, groups);
+	while (i < n) {
 
 		av.x = fmaf(lam, pv.x, av.x);
 		av.y = fmaf(lam, pv.y, av.y);
 		Ap[i] = av;
-
-		float2 xv = x[i];
-		float2 rv = r[i];
 		xv.x = fmaf(a, pv.x, xv.x);
 		xv.y = fmaf(a, pv.y, xv.y);
 		rv.x = fmaf(-a, av.x, rv.x);
@@ -499,15 +531,26 @@ __global__ void k_fcg_step(float2* __restrict__ x, float2* __restrict__ r, const
 		x[i] = xv;
 		r[i] = rv;
 		acc += (double)rv.x * (double)rv.x + (double)rv.y * (double)rv.y;
+		i += stride;
+
+		if (i < n) {
+
+			pv = p[i];
+			av = group_sum(part, i, n, groups);
+			xv = x[i];
+			rv = r[i];
+		}
 	}
 
 	double s = block_sum(acc, sh);
 
-	if (0 == threadIdx.x)
+	if (0 == threadIdx.x) {
+
 		rs_part[blockIdx.x] = s;
 
-	if ((0 == blockIdx.x) && (0 == threadIdx.x))
-		st->pap_hist[it % ring] = pAp;
+		if (0 == blockIdx.x)
+			st->pap_hist[it % ring] = pAp;
+	}
 }
 
 // FCG convergence test after step it: ||r||^2 <= eps2 stops with it + 1
@@ -661,8 +704,8 @@ struct SelDigit {
 };
 
 template <int P>
-__global__ void __launch_bounds__(SEL_THREADS) k_select_pass(const float2* __restrict__ b, float* __restrict__ mag,
-		long n, SelectState* ss, CgScalars* st)
+__global__ void __launch_bounds__(SEL_THREADS) k_select_pass(float2* __restrict__ b, const float2* __restrict__ part, int groups,
+		float* __restrict__ mag, long n, SelectState* ss, CgScalars* st)
 {
 	constexpr int SHIFT = SelDigit<P>::SHIFT;
 	constexpr int W = SelDigit<P>::W;
@@ -686,7 +729,8 @@ __global__ void __launch_bounds__(SEL_THREADS) k_select_pass(const float2* __res
 
 		if (0 == P) {
 
-			float2 v = b[i];
+			const float2 v = group_sum(part, i, n, groups);
+			b[i] = v;
 			m = hypotf(v.x, v.y);	// cabsf
 			mag[i] = m;
 

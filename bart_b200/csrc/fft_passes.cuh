@@ -617,11 +617,11 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 // rows and coils [c0, c1) (a thread keeps its output pixels in registers
 // across the coil loop): inverse FFT per row, keep x < X from
 // wrap_pos(x, X, L), scale by ax[x]*ayz[yz] (optional) and either
-//   maps != 0: accumulate sum_c conj(maps[x + X*yz + X*YZ*c]) * row
+//   MAPS:      accumulate sum_c conj(maps[x + X*yz + X*YZ*c]) * row
 //              into out[x + X*yz + X*YZ*g] (g = blockIdx.y, partial per group)
-//   maps == 0: write out[x + X*yz + X*YZ*c] per coil.
+//   else:      write out[x + X*yz + X*YZ*c] per coil.
 // grid (ceil(YZ/B), groups); coils per group cpg.
-template <int L, int B, bool BLUE>
+template <int L, int B, bool BLUE, bool MAPS>
 __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (B * L / 8) : 1) k_rows_inv(const float2* __restrict__ in, const float2* __restrict__ maps,
 		const float* __restrict__ ax, const float* __restrict__ ayz,
 		int X, long YZ, int C, int cpg, float2* __restrict__ out, const float2* __restrict__ twg,
@@ -630,6 +630,14 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 	using LAY = RowLayout<L, B>;
 	const int dn = BLUE ? d.n : L;	// logical DFT length (compile-time for the FFT itself)
 	constexpr int NT = B * L / 8;
+	constexpr int NW = out_regs(L, BLUE);
+	// the coil sums belong to images of at most half the grid's side: all in
+	// registers 0, 1, 6 and 7 (the last stage computes no others)
+	constexpr int NA = (MAPS && !BLUE) ? 4 : 8;
+	auto reg = [](int l) { return ((4 == NA) && (l >= 2)) ? l + 4 : l; };
+	// the next coil's row is loaded while this one is transformed, where the
+	// registers allow
+	constexpr bool AHEAD = MAPS && !BLUE && !is_mix(L);
 	extern __shared__ float2 smem[];
 	__shared__ double red[32];
 	float2* s = smem;
@@ -647,22 +655,32 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 	const int c1 = min(C, c0 + cpg);
 
 	// this thread's output pixels: x = unwrap(jt + (L/8) m) where < X
-	float2 acc[8];
+	float2 acc[NA];
 #pragma unroll
-	for (int m = 0; m < 8; m++)
-		acc[m] = make_float2(0.f, 0.f);
+	for (int l = 0; l < NA; l++)
+		acc[l] = make_float2(0.f, 0.f);
 
 	double dot = 0.;
+	float2 w[NW], nx[NW], v[8];
+
+	auto load = [&](float2 (&u)[NW], int c) {
+#pragma unroll
+		for (int m = 0; m < NW; m++) {
+
+			int p = out_pos<L, LAY, BLUE>(m);
+			u[m] = (valid && (p < dn)) ? in[p + (long)dn * (yz + YZ * c)] : make_float2(0.f, 0.f);
+		}
+	};
+
+	if (AHEAD)
+		load(w, c0);
 
 	for (int c = c0; c < c1; c++) {
 
-		float2 w[out_regs(L, BLUE)], v[8];
-#pragma unroll
-		for (int m = 0; m < out_regs(L, BLUE); m++) {
-
-			int p = out_pos<L, LAY, BLUE>(m);
-			w[m] = (valid && (p < dn)) ? in[p + (long)dn * (yz + YZ * c)] : make_float2(0.f, 0.f);
-		}
+		if (!AHEAD)
+			load(w, c);
+		else if (c + 1 < c1)
+			load(nx, c + 1);
 
 		if (stop)
 			return;
@@ -671,22 +689,22 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 
 		if (valid) {
 #pragma unroll
-			for (int m = 0; m < 8; m++) {
+			for (int l = 0; l < NA; l++) {
 
-				int p = reg_pos<L, LAY>(m);
+				int p = reg_pos<L, LAY>(reg(l));
 				int x = (p < dn) ? unwrap_pos(p, X, dn) : X;
 
 				if (x >= X)
 					continue;
 
-				float2 t = v[m];
+				float2 t = v[reg(l)];
 
 				if (ax)
 					t = cscale(t, ax[x] * ayz[yz]);
 
-				if (maps) {
+				if (MAPS) {
 
-					acc[m] = cadd(acc[m], cmulc(t, maps[x + X * yz + X * YZ * c]));
+					acc[l] = cadd(acc[l], cmulc(t, maps[x + X * yz + X * YZ * c]));
 
 				} else {
 
@@ -700,26 +718,32 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 				}
 			}
 		}
+
+		if (AHEAD) {
+#pragma unroll
+			for (int m = 0; m < NW; m++)
+				w[m] = nx[m];
+		}
 	}
 
-	if (maps) {
+	if (MAPS) {
 
 		if (valid) {
 #pragma unroll
-			for (int m = 0; m < 8; m++) {
+			for (int l = 0; l < NA; l++) {
 
-				int p = reg_pos<L, LAY>(m);
+				int p = reg_pos<L, LAY>(reg(l));
 				int x = (p < dn) ? unwrap_pos(p, X, dn) : X;
 
 				if (x >= X)
 					continue;
 
-				out[x + X * yz + X * YZ * g] = acc[m];
+				out[x + X * yz + X * YZ * g] = acc[l];
 
 				if (pdot) {	// Re<p, partial> for the CG step length
 
 					float2 pv = pdot[x + X * yz];
-					dot += (double)pv.x * (double)acc[m].x + (double)pv.y * (double)acc[m].y;
+					dot += (double)pv.x * (double)acc[l].x + (double)pv.y * (double)acc[l].y;
 				}
 			}
 		}

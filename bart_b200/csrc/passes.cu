@@ -58,7 +58,8 @@ int launch_rows_inv_LB(const float2* in, const float2* maps, const float* ax, co
 	TRY(get_twiddles(L, &tw));
 	int groups = (C + cpg - 1) / cpg;
 	size_t smem = rows_smem(L, B);
-	auto kern = (d.n == L) ? k_rows_inv<L, B, false> : k_rows_inv<L, B, true>;
+	auto kern = (d.n == L) ? (maps ? k_rows_inv<L, B, false, true> : k_rows_inv<L, B, false, false>)
+			: (maps ? k_rows_inv<L, B, true, true> : k_rows_inv<L, B, true, false>);
 	TRY(prep_kernel(kern, smem));
 	dim3 grid((unsigned)((YZ + B - 1) / B), (unsigned)groups);
 	cudaEvent_t pe = prof_begin("rows_inv", st);
