@@ -1311,7 +1311,7 @@ static int grid_adj(OpCtx& op, const float2* ksp, long C, float2* grid, cudaStre
 
 		if (b.det) {
 
-			k_sum_tiles<<<(unsigned)std::min<long>((b.ntiles * C + 7) / 8, 8 * 148), 256, 0, st>>>(grid, gg, b.bg, b.multi,
+			k_sum_tiles<<<(unsigned)std::min<long>(b.ntiles * C, 16 * 148), TG_DET_CELLS, 0, st>>>(grid, gg, b.bg, b.multi,
 					b.multi + b.ntiles, b.work_start, b.slot, b.part, (int)C);
 			LAUNCHED();
 		}
@@ -1338,7 +1338,7 @@ static int grid_adj(OpCtx& op, const float2* ksp, long C, float2* grid, cudaStre
 		return BNUFFT_OK;
 	}
 
-	if (op.bins.perm && (6.f == op.g.width) && (0 == gridding_kind())) {
+	if (op.bins.perm && (6.f == op.g.width) && op.bins.sub_bin && (0 == gridding_kind())) {
 
 		const Bins& b = op.bins;
 		int cc = (int)std::min<long>(b.cc, C);
@@ -1466,6 +1466,70 @@ static long tg_max_hits(const Geom& g, const BinGeom& bg)
 	return n;
 }
 
+// exclusive sums of n ints into out[0 .. n]: one block, or CUB for many
+static int scan_ints(const int* in, int n, int* out, cudaStream_t st)
+{
+	if (n <= 16384) {
+
+		k_scan<<<1, 1024, 0, st>>>(in, n, out);
+		LAUNCHED();
+		return BNUFFT_OK;
+	}
+
+	// (the last input, past the n counts, is the caller's zero)
+	void* tmp = nullptr;
+	size_t bytes = 0;
+	CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, n + 1, st));
+	CUDA_TRY(cudaMallocAsync(&tmp, bytes, st));
+	CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp, bytes, in, out, n + 1, st));
+	g_launches.fetch_add(1, std::memory_order_relaxed);
+	cudaFreeAsync(tmp, st);
+	return BNUFFT_OK;
+}
+
+// The sub-blocks of the shared-memory tile scatter and its sorted trajectory
+static int build_sub_blocks(OpCtx& op, const int* bin_start, long nbins, cudaStream_t st)
+{
+	Bins& b = op.bins;
+	const long M = op.g.M;
+	int *nsub = nullptr, *sub_start = nullptr;
+	CUDA_TRY(cudaMallocAsync(&nsub, sizeof(int) * (nbins + 1), st));
+	CUDA_TRY(cudaMallocAsync(&sub_start, sizeof(int) * (nbins + 1), st));
+
+	// sub-blocks per bin: ceil(count / sub); their start indices. A
+	// sub-block is one block of the tile scatter, which clears and flushes
+	// its tile once: large sub-blocks amortise that, small ones balance the
+	// dense bins at the k-space centre
+	int sub = BIN_SUB;
+
+	if (const char* e = getenv("BNUFFT_GRID_SUB"))
+		sub = std::max(64, std::min(1 << 20, atoi(e)));
+
+	k_bin_nsub<<<vec_blocks(nbins + 1), RED_THREADS, 0, st>>>(bin_start, (int)nbins, sub, nsub);
+	LAUNCHED();
+	TRY(scan_ints(nsub, (int)nbins, sub_start, st));
+
+	// the number of sub-blocks stays on the device (no host round trip);
+	// launches use the upper bound nbins + M / BIN_SUB and surplus blocks exit
+	const long total = nbins + M / sub + 1;
+	b.nsub = (int)total;
+	b.sub_start = sub_start;
+	b.nsub_dev = sub_start + nbins;
+	CUDA_TRY(cudaMallocAsync(&b.sub_bin, sizeof(int) * total, st));
+	CUDA_TRY(cudaMallocAsync(&b.sub_first, sizeof(int) * total, st));
+	CUDA_TRY(cudaMallocAsync(&b.sub_count, sizeof(int) * total, st));
+	CUDA_TRY(cudaMallocAsync(&b.traj, sizeof(float4) * M, st));
+	k_sub_fill<<<vec_blocks(nbins), RED_THREADS, 0, st>>>(bin_start, sub_start, (int)nbins, sub, b.sub_bin, b.sub_first, b.sub_count);
+	LAUNCHED();
+	k_gather_traj<<<vec_blocks(M), RED_THREADS, 0, st>>>(b.traj, op.traj, b.perm, M);
+	LAUNCHED();
+	cudaFreeAsync(nsub, st);
+
+	// coil tiles per pass: as many as fit in ~110 KB of shared memory
+	b.cc = (int)std::max(1L, std::min(8L, (110L * 1024) / (long)(sizeof(float2) * b.bg.ncells)));
+	return BNUFFT_OK;
+}
+
 // Sort the samples by bin and cut bins into sub-blocks (plan time). det: the
 // scatter is deterministic.
 static int build_bins(OpCtx& op, cudaStream_t st, bool det)
@@ -1529,21 +1593,24 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		b.tg_cfg = -1;
 
 	unsigned *keys = nullptr, *keys2 = nullptr;
-	int *vals = nullptr, *counts = nullptr, *bin_start = nullptr, *nsub = nullptr, *sub_start = nullptr;
+	int *vals = nullptr, *counts = nullptr, *bin_start = nullptr;
 	void* tmp = nullptr;
-	size_t tmp_bytes = 0, tmp2 = 0;
+	size_t tmp_bytes = 0;
 	long M = g.M;
+	const bool binned = (0 == gridding_kind()) && (6.f == g.width);	// the shared-memory tile scatter
+	const bool starts = binned || (b.tg_cfg >= 0);			// the bins' sample ranges are needed
 
 	CUDA_TRY(cudaMallocAsync(&keys, sizeof(unsigned) * M, st));
 	CUDA_TRY(cudaMallocAsync(&keys2, sizeof(unsigned) * M, st));
 	CUDA_TRY(cudaMallocAsync(&vals, sizeof(int) * M, st));
 	CUDA_TRY(cudaMallocAsync(&b.perm, sizeof(int) * M, st));
-	CUDA_TRY(cudaMallocAsync(&b.traj, sizeof(float4) * M, st));
-	CUDA_TRY(cudaMallocAsync(&counts, sizeof(int) * (nbins + 1), st));
-	CUDA_TRY(cudaMallocAsync(&bin_start, sizeof(int) * (nbins + 1), st));
-	CUDA_TRY(cudaMallocAsync(&nsub, sizeof(int) * (nbins + 1), st));
-	CUDA_TRY(cudaMallocAsync(&sub_start, sizeof(int) * (nbins + 1), st));
-	CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (nbins + 1), st));
+
+	if (starts) {
+
+		CUDA_TRY(cudaMallocAsync(&counts, sizeof(int) * (nbins + 1), st));
+		CUDA_TRY(cudaMallocAsync(&bin_start, sizeof(int) * (nbins + 1), st));
+		CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (nbins + 1), st));
+	}
 
 	k_bin_keys<<<vec_blocks(M), RED_THREADS, 0, st>>>(op.traj, M, grid_geom(g), bg, keys, vals, counts);
 	LAUNCHED();
@@ -1554,44 +1621,15 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		end_bit++;
 
 	CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, vals, b.perm, (int)M, 0, end_bit, st));
-	CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, tmp2, counts, bin_start, (int)(nbins + 1), st));
-	tmp_bytes = std::max(tmp_bytes, tmp2);
 	CUDA_TRY(cudaMallocAsync(&tmp, tmp_bytes, st));
 	CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, vals, b.perm, (int)M, 0, end_bit, st));
-	CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, counts, bin_start, (int)(nbins + 1), st));
-	g_launches.fetch_add(2, std::memory_order_relaxed);
-
-	// sub-blocks per bin: ceil(count / sub); their start indices. A
-	// sub-block is one block of the tile scatter, which clears and flushes
-	// its tile once: large sub-blocks amortise that, small ones balance the
-	// dense bins at the k-space centre
-	int sub = BIN_SUB;
-
-	if (const char* e = getenv("BNUFFT_GRID_SUB"))
-		sub = std::max(64, std::min(1 << 20, atoi(e)));
-
-	k_bin_nsub<<<vec_blocks(nbins + 1), RED_THREADS, 0, st>>>(bin_start, (int)nbins, sub, nsub);
-	LAUNCHED();
-	CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, nsub, sub_start, (int)(nbins + 1), st));
 	g_launches.fetch_add(1, std::memory_order_relaxed);
 
-	// the number of sub-blocks stays on the device (no host round trip);
-	// launches use the upper bound nbins + M / BIN_SUB and surplus blocks exit
-	long total = nbins + M / sub + 1;
-	b.nsub = (int)total;
-	b.sub_start = sub_start;
-	b.nsub_dev = sub_start + nbins;
+	if (starts)
+		TRY(scan_ints(counts, (int)nbins, bin_start, st));
 
-	CUDA_TRY(cudaMallocAsync(&b.sub_bin, sizeof(int) * total, st));
-	CUDA_TRY(cudaMallocAsync(&b.sub_first, sizeof(int) * total, st));
-	CUDA_TRY(cudaMallocAsync(&b.sub_count, sizeof(int) * total, st));
-	k_sub_fill<<<vec_blocks(nbins), RED_THREADS, 0, st>>>(bin_start, sub_start, (int)nbins, sub, b.sub_bin, b.sub_first, b.sub_count);
-	LAUNCHED();
-	k_gather_traj<<<vec_blocks(M), RED_THREADS, 0, st>>>(b.traj, op.traj, b.perm, M);
-	LAUNCHED();
-
-	// coil tiles per pass: as many as fit in ~110 KB of shared memory
-	b.cc = (int)std::max(1L, std::min(8L, (110L * 1024) / (long)(sizeof(float2) * bg.ncells)));
+	if (binned)
+		TRY(build_sub_blocks(op, bin_start, nbins, st));
 
 	// the samples' footprints (start cells and weights): they depend on
 	// the trajectory only, so every apply reads them instead of recomputing
@@ -1611,7 +1649,7 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		if (b.tg_cfg >= 0)
 			CUDA_TRY(cudaMallocAsync(&lo4, sizeof(short4) * M, st));
 
-		k_foot<<<vec_blocks(3 * M, 256, 8 * 148), 256, 0, st>>>(b.traj, M, grid_geom(g), op.kb, b.foot, lo4);
+		k_foot<<<vec_blocks(3 * M, 256, 8 * 148), 256, 0, st>>>(op.traj, b.perm, M, grid_geom(g), op.kb, b.foot, lo4);
 		LAUNCHED();
 	}
 
@@ -1620,60 +1658,55 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 	if (b.tg_cfg >= 0) {
 
 		const long nt = nbins;
-		int *nwork = nullptr, *cursor = nullptr;
-		void* wtmp = nullptr;
-		size_t wtmp_bytes = 0;
+		int* nhits = nullptr;
 		b.ntiles = nt;
-		b.chunk = (g.G[2] > 1) ? 256 : 64;
+
+		// hits per work item. 3D: 512 (128^3, 8 coils: 13.5 ms with 256, 13.2
+		// with 512). 2D: 64, and 32 where that leaves fewer jobs (about 2.1 hits
+		// per sample, eight coils per job) than the GPU holds at once, 16 warps
+		// on 148 SMs (192^2, 8 coils, 64 spokes: 486 us a solve with 64, 469 with
+		// 32; 256^2, 16 coils, 96 spokes: 47 us a scatter with 64, 53 with 48).
+		// Deterministic: twice that, for fewer partial tiles
+		// (by one group of coils: the sums of a channel do not depend on the others)
+		const long jobs64 = (long)(2.1 * (double)M) * (det ? 1 : (op.coils + 7) / 8) / 64;
+		b.chunk = (g.G[2] > 1) ? 512 : ((det ? 2 : 1) * ((jobs64 < 16 * 148) ? 32 : 64));
 
 		if (const char* e = getenv("BNUFFT_GRID_CHUNK"))	// tuning knob: hits per work item
 			b.chunk = std::max(32, std::min(4096, atoi(e)));
 
 		b.nwork_max = nt + (M * tg_max_hits(g, bg) + b.chunk - 1) / b.chunk;
-		CUDA_TRY(cudaMallocAsync(&nwork, sizeof(int) * (nt + 1), st));
-		CUDA_TRY(cudaMallocAsync(&cursor, sizeof(int) * (nt + 1), st));
+		CUDA_TRY(cudaMallocAsync(&nhits, sizeof(int) * nt, st));
 		CUDA_TRY(cudaMallocAsync(&b.hit_start, sizeof(int) * (nt + 1), st));
 		CUDA_TRY(cudaMallocAsync(&b.hits, sizeof(int) * M * tg_max_hits(g, bg), st));
 		CUDA_TRY(cudaMallocAsync(&b.work_start, sizeof(int) * (nt + 1), st));
 		CUDA_TRY(cudaMallocAsync(&b.multi, sizeof(int) * (nt + 1), st));
 		CUDA_TRY(cudaMallocAsync(&b.work_tile, sizeof(int) * b.nwork_max, st));
 		CUDA_TRY(cudaMallocAsync(&b.work_chunk, sizeof(int) * b.nwork_max, st));
-		CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, wtmp_bytes, cursor, b.hit_start, (int)(nt + 1), st));
-		CUDA_TRY(cudaMallocAsync(&wtmp, wtmp_bytes, st));
-		CUDA_TRY(cudaMemsetAsync(cursor + nt, 0, sizeof(int), st));
-		CUDA_TRY(cudaMemsetAsync(b.multi + nt, 0, sizeof(int), st));
+
+		if (det)
+			CUDA_TRY(cudaMallocAsync(&b.slot, sizeof(int) * (nt + 1), st));
+
 		const unsigned hb = (unsigned)std::min<long>(nt, 16 * 148);
-		k_tile_hits<<<hb, TH_THREADS, 0, st>>>(lo4, bin_start, grid_geom(g), bg, nt, cursor, nullptr, nullptr);
+		k_tile_hits<<<hb, TH_THREADS, 0, st>>>(lo4, bin_start, grid_geom(g), bg, nt, nhits, nullptr, nullptr, nullptr,
+				nullptr, nullptr);
 		LAUNCHED();
-		CUDA_TRY(cub::DeviceScan::ExclusiveSum(wtmp, wtmp_bytes, cursor, b.hit_start, (int)(nt + 1), st));
-		k_tile_hits<<<hb, TH_THREADS, 0, st>>>(lo4, bin_start, grid_geom(g), bg, nt, nullptr, b.hit_start, b.hits);
+		k_tile_plan<<<1, 1024, 0, st>>>(nhits, (int)nt, b.chunk, b.hit_start, b.work_start, b.slot, b.multi);
+		LAUNCHED();
+		k_tile_hits<<<hb, TH_THREADS, 0, st>>>(lo4, bin_start, grid_geom(g), bg, nt, nullptr, b.hit_start, b.hits,
+				b.work_start, b.work_tile, b.work_chunk);
 		LAUNCHED();
 		cudaFreeAsync(lo4, st);
-		k_tile_work<<<vec_blocks(nt + 1), RED_THREADS, 0, st>>>(b.hit_start, nt, b.chunk, nwork);
-		LAUNCHED();
-		CUDA_TRY(cub::DeviceScan::ExclusiveSum(wtmp, wtmp_bytes, nwork, b.work_start, (int)(nt + 1), st));
-		g_launches.fetch_add(2, std::memory_order_relaxed);
-		k_work_fill<<<vec_blocks(nt), RED_THREADS, 0, st>>>(b.work_start, nt, b.work_tile, b.work_chunk, b.multi,
-				b.multi + nt);
-		LAUNCHED();
+		cudaFreeAsync(nhits, st);
 
 		if (det) {
 
 			b.det = true;
-			CUDA_TRY(cudaMallocAsync(&b.slot, sizeof(int) * (nt + 1), st));
-			k_tile_slots<<<vec_blocks(nt + 1), RED_THREADS, 0, st>>>(nwork, nt, cursor);
-			LAUNCHED();
-			CUDA_TRY(cub::DeviceScan::ExclusiveSum(wtmp, wtmp_bytes, cursor, b.slot, (int)(nt + 1), st));
 			int total = 0;
 			CUDA_TRY(cudaMemcpyAsync(&total, b.slot + nt, sizeof(int), cudaMemcpyDeviceToHost, st));
 			CUDA_TRY(cudaStreamSynchronize(st));
 			b.nslots = total;
 			TRY(alloc_partials(b, op.coils, st));
 		}
-
-		cudaFreeAsync(nwork, st);
-		cudaFreeAsync(cursor, st);
-		cudaFreeAsync(wtmp, st);
 
 		// the bin-ordered k-space of the applies, allocated here so that
 		// applies allocate nothing (their solves can then be captured into
@@ -1682,7 +1715,7 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		CUDA_TRY(cudaMallocAsync(&b.kperm, sizeof(float2) * M * b.kperm_c, st));
 	}
 
-	void* frees[] = { keys, keys2, vals, counts, bin_start, nsub, tmp };
+	void* frees[] = { keys, keys2, vals, counts, bin_start, tmp };
 
 	for (void* q : frees)
 		if (q)

@@ -57,7 +57,7 @@ __device__ __forceinline__ int bin_of(float k, int N, int bs, int nb, int period
 	return min(max(b, 0), nb - 1);
 }
 
-// key = bin id of sample m, value = m
+// key = bin id of sample m, value = m; samples per bin if wanted
 __global__ void k_bin_keys(const float4* __restrict__ traj, long M, GridGeom g, BinGeom bg,
 		unsigned* __restrict__ keys, int* __restrict__ vals, int* __restrict__ counts)
 {
@@ -70,7 +70,9 @@ __global__ void k_bin_keys(const float4* __restrict__ traj, long M, GridGeom g, 
 		unsigned key = (unsigned)(bx + bg.nb[0] * (by + bg.nb[1] * bz));
 		keys[m] = key;
 		vals[m] = (int)m;
-		atomicAdd(&counts[key], 1);
+
+		if (counts)
+			atomicAdd(&counts[key], 1);
 	}
 }
 
@@ -426,7 +428,7 @@ __device__ __forceinline__ void foot6_w(float k, int N, int periodic, const floa
 // footprints of all sorted samples (the weights as axis_taps6 computes them:
 // the same kb_lookup of the same float32 distances), a thread per sample and
 // axis; lo4 (if given): their start cells once more, for k_tile_hits
-__global__ void k_foot(const float4* __restrict__ traj_sorted, long M, GridGeom g, const float* __restrict__ kbg,
+__global__ void k_foot(const float4* __restrict__ traj, const int* __restrict__ perm, long M, GridGeom g, const float* __restrict__ kbg,
 		float4* __restrict__ foot, short4* __restrict__ lo4)
 {
 	__shared__ float kb[KB_TABLE_N + 1];
@@ -440,7 +442,7 @@ __global__ void k_foot(const float4* __restrict__ traj_sorted, long M, GridGeom 
 
 		const long i = e / 3;
 		const int a = (int)(e - 3 * i);
-		const float4 k = traj_sorted[i];
+		const float4 k = traj[perm[i]];
 		const float ka = (0 == a) ? k.x : ((1 == a) ? k.y : k.z);
 		const int N = (0 == a) ? g.N[0] : ((1 == a) ? g.N[1] : g.N[2]);
 		float w7[7];
@@ -753,28 +755,31 @@ __device__ __forceinline__ int foot_rel(int lo, int origin, int G, int periodic)
 // a footprint reaches three cells either side of its sample) whose footprint
 // meets it, in bin order, so the lists are the same every time. A block takes a
 // tile; the x neighbours of a row of bins are one range of the sorted samples
-// (two where a periodic grid wraps). lo: the footprints' start cells.
-// hit_start == nullptr: count into nhits; else fill hits.
-enum { TH_THREADS = 128 };
+// (two where a periodic grid wraps), and the block walks all ranges as one
+// list. lo: the footprints' start cells. work_start == nullptr: count into
+// nhits; else fill hits from hit_start on, and the tile's work items.
+enum { TH_THREADS = 256, TH_RANGES = 18 };
 
 __global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restrict__ lo, const int* __restrict__ bin_start,
 		GridGeom g, BinGeom bg, long ntiles, int* __restrict__ nhits, const int* __restrict__ hit_start,
-		int* __restrict__ hits)
+		int* __restrict__ hits, const int* __restrict__ work_start, int* __restrict__ work_tile,
+		int* __restrict__ work_chunk)
 {
 	__shared__ int wcount[TH_THREADS / 32];
+	__shared__ int rs[TH_RANGES], rn[TH_RANGES];	// ranges: first sample, samples
 	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 	const int ry = (bg.nb[1] > 1) ? 1 : 0, rz = (bg.nb[2] > 1) ? 1 : 0;
+	const int nr = 2 * (2 * ry + 1) * (2 * rz + 1);
 
 	for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
 
 		const int bx = (int)(t % bg.nb[0]), by = (int)((t / bg.nb[0]) % bg.nb[1]), bz = (int)(t / ((long)bg.nb[0] * bg.nb[1]));
 		const int ox = bx * bg.bs[0], oy = by * bg.bs[1], oz = bz * bg.bs[2];
-		int pos = hit_start ? hit_start[t] : 0;
-		int count = 0;
 
-		for (int r = 0; r < 2 * (2 * ry + 1) * (2 * rz + 1); r++) {
+		if ((int)threadIdx.x < nr) {
 
 			// range r: part (0, or 1 past the periodic edge) of neighbour row (y, z)
+			const int r = threadIdx.x;
 			int y = by + (r / 2) % (2 * ry + 1) - ry, z = bz + (r / 2) / (2 * ry + 1) - rz;
 			int x0 = bx - 1, x1 = bx + 2;
 
@@ -784,8 +789,7 @@ __global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restri
 				z = (z < 0) ? z + bg.nb[2] : ((z >= bg.nb[2]) ? z - bg.nb[2] : z);
 			}
 
-			if ((y < 0) || (y >= bg.nb[1]) || (z < 0) || (z >= bg.nb[2]))
-				continue;
+			bool ok = (y >= 0) && (y < bg.nb[1]) && (z >= 0) && (z < bg.nb[2]);
 
 			if (0 == r % 2) {
 
@@ -794,61 +798,88 @@ __global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restri
 
 			} else {
 
-				if (!g.periodic || ((x0 >= 0) && (x1 <= bg.nb[0])))
-					continue;
-
+				ok = ok && g.periodic && ((x0 < 0) || (x1 > bg.nb[0]));
 				x0 = (x0 < 0) ? bg.nb[0] - 1 : 0;
 				x1 = x0 + 1;
 			}
 
 			const long row = (long)bg.nb[0] * (y + (long)bg.nb[1] * z);
-			const int s0 = bin_start[row + x0], s1 = bin_start[row + x1];
-
-			for (int base = s0; base < s1; base += TH_THREADS) {
-
-				const int i = base + threadIdx.x;
-				bool hit = false;
-
-				if (i < s1) {
-
-					const short4 l = lo[i];
-					const int lx = foot_rel(l.x, ox, g.G[0], g.periodic), ly = foot_rel(l.y, oy, g.G[1], g.periodic);
-					const int lz = foot_rel(l.z, oz, g.G[2], g.periodic);
-					hit = (lx > -6) && (lx < bg.bs[0]) && (ly > -6) && (ly < bg.bs[1]) && (lz > -6) && (lz < bg.bs[2]);
-				}
-
-				if (!hits) {
-
-					count += hit;
-					continue;
-				}
-
-				const unsigned m = __ballot_sync(0xffffffffu, hit);
-				__syncthreads();	// the previous counts have been read
-
-				if (0 == lane)
-					wcount[warp] = __popc(m);
-
-				__syncthreads();
-				int at = pos + __popc(m & ((1u << lane) - 1u));
-#pragma unroll
-				for (int w = 0; w < TH_THREADS / 32; w++) {
-
-					at += (w < warp) ? wcount[w] : 0;
-					pos += wcount[w];
-				}
-
-				if (hit)
-					hits[at] = i;
-			}
+			const int s0 = ok ? bin_start[row + x0] : 0;
+			rs[r] = s0;
+			rn[r] = ok ? bin_start[row + x1] - s0 : 0;
 		}
 
-		if (!hits) {
+		__syncthreads();
+		int total = 0;
+
+		for (int r = 0; r < nr; r++)
+			total += rn[r];
+
+		int pos = work_start ? hit_start[t] : 0;
+		int count = 0, r = 0, r0 = 0;	// this thread's range and its first candidate
+
+		// candidate c of the list (the thread's next one is loaded ahead)
+		auto cand = [&](int c, int& i, short4& l) {
+			if (c >= total) {
+
+				i = -1;
+				return;
+			}
+
+			while (c - r0 >= rn[r])
+				r0 += rn[r++];
+
+			i = rs[r] + c - r0;
+			l = lo[i];
+		};
+
+		int in = -1;
+		short4 ln = make_short4(0, 0, 0, 0);
+		cand(threadIdx.x, in, ln);
+
+		for (int base = 0; base < total; base += TH_THREADS) {
+
+			const int i = in;
+			const short4 l = ln;
+			cand(base + TH_THREADS + threadIdx.x, in, ln);
+			bool hit = false;
+
+			if (i >= 0) {
+
+				const int lx = foot_rel(l.x, ox, g.G[0], g.periodic), ly = foot_rel(l.y, oy, g.G[1], g.periodic);
+				const int lz = foot_rel(l.z, oz, g.G[2], g.periodic);
+				hit = (lx > -6) && (lx < bg.bs[0]) && (ly > -6) && (ly < bg.bs[1]) && (lz > -6) && (lz < bg.bs[2]);
+			}
+
+			if (!work_start) {
+
+				count += hit;
+				continue;
+			}
+
+			const unsigned m = __ballot_sync(0xffffffffu, hit);
+			__syncthreads();	// the previous counts have been read
+
+			if (0 == lane)
+				wcount[warp] = __popc(m);
+
+			__syncthreads();
+			int at = pos + __popc(m & ((1u << lane) - 1u));
+#pragma unroll
+			for (int w = 0; w < TH_THREADS / 32; w++) {
+
+				at += (w < warp) ? wcount[w] : 0;
+				pos += wcount[w];
+			}
+
+			if (hit)
+				hits[at] = i;
+		}
+
+		if (!work_start) {
 
 			for (int o = 16; o > 0; o >>= 1)
 				count += __shfl_xor_sync(0xffffffffu, count, o);
-
-			__syncthreads();
 
 			if (0 == lane)
 				wcount[warp] = count;
@@ -864,78 +895,169 @@ __global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restri
 
 				nhits[t] = n;
 			}
+
+		} else {
+
+			const int w0 = work_start[t], w1 = work_start[t + 1];
+
+			for (int w = w0 + threadIdx.x; w < w1; w += TH_THREADS) {
+
+				work_tile[w] = (int)t;
+				work_chunk[w] = w - w0;
+			}
 		}
+
+		__syncthreads();	// before the next tile's ranges
 	}
 }
 
-// work items (chunks of hits) per tile
-__global__ void k_tile_work(const int* __restrict__ hit_start, long ntiles, int chunk, int* __restrict__ nwork)
+// exclusive sum of one value per thread over the block (sh: 33 ints), the total
+// in every thread
+__device__ __forceinline__ int block_scan(int v, int* sh, int& total)
 {
-	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t <= ntiles; t += (long)gridDim.x * blockDim.x)
-		nwork[t] = (t < ntiles) ? max(1, (hit_start[t + 1] - hit_start[t] + chunk - 1) / chunk) : 0;
+	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+	int incl = v;
+
+	for (int o = 1; o < 32; o <<= 1) {
+
+		const int u = __shfl_up_sync(0xffffffffu, incl, o);
+		incl += (lane >= o) ? u : 0;
+	}
+
+	if (31 == lane)
+		sh[warp] = incl;
+
+	__syncthreads();
+
+	if (0 == warp) {
+
+		const int n = (lane < (int)(blockDim.x / 32)) ? sh[lane] : 0;
+		int s = n;
+
+		for (int o = 1; o < 32; o <<= 1) {
+
+			const int u = __shfl_up_sync(0xffffffffu, s, o);
+			s += (lane >= o) ? u : 0;
+		}
+
+		sh[lane] = s - n;
+
+		if (31 == lane)
+			sh[32] = s;
+	}
+
+	__syncthreads();
+	const int r = sh[warp] + incl - v;
+	total = sh[32];
+	__syncthreads();
+	return r;
 }
 
-// partial tiles that deterministic mode needs: the chunks of tiles with several
-__global__ void k_tile_slots(const int* __restrict__ nwork, long ntiles, int* __restrict__ nslot)
+// exclusive sums of n values by one block: out[0 .. n], out[n] the total
+__global__ void __launch_bounds__(1024) k_scan(const int* __restrict__ in, int n, int* __restrict__ out)
 {
-	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t <= ntiles; t += (long)gridDim.x * blockDim.x)
-		nslot[t] = ((t < ntiles) && (nwork[t] > 1)) ? nwork[t] : 0;
+	__shared__ int sh[33];
+	int sum = 0;
+
+	for (int base = 0; base < n; base += 1024) {
+
+		const int t = base + threadIdx.x;
+		int total;
+		const int e = block_scan((t < n) ? in[t] : 0, sh, total);
+
+		if (t < n)
+			out[t] = sum + e;
+
+		sum += total;
+	}
+
+	if (0 == threadIdx.x)
+		out[n] = sum;
+}
+
+// From the hits per tile, in one block: where each tile's hits, work items
+// (chunks of hits, at least one) and, for tiles with several items, partial
+// tiles begin (slot; deterministic mode), and the list of those tiles.
+__global__ void __launch_bounds__(1024) k_tile_plan(const int* __restrict__ nhits, int ntiles, int chunk,
+		int* __restrict__ hit_start, int* __restrict__ work_start, int* __restrict__ slot, int* __restrict__ multi)
+{
+	__shared__ int sh[33];
+	int hsum = 0, wsum = 0, ssum = 0, msum = 0;
+
+	for (int base = 0; base < ntiles; base += 1024) {
+
+		const int t = base + threadIdx.x;
+		const bool in = (t < ntiles);
+		const int n = in ? nhits[t] : 0;
+		const int k = in ? max(1, (n + chunk - 1) / chunk) : 0;
+		const bool several = (k > 1);
+		int th, tw, ts, tm;
+		const int h = block_scan(n, sh, th), w = block_scan(k, sh, tw);
+		const int s = block_scan(several ? k : 0, sh, ts), m = block_scan(several ? 1 : 0, sh, tm);
+
+		if (in) {
+
+			hit_start[t] = hsum + h;
+			work_start[t] = wsum + w;
+
+			if (slot)
+				slot[t] = ssum + s;
+
+			if (several)
+				multi[msum + m] = t;
+		}
+
+		hsum += th;
+		wsum += tw;
+		ssum += ts;
+		msum += tm;
+	}
+
+	if (0 == threadIdx.x) {
+
+		hit_start[ntiles] = hsum;
+		work_start[ntiles] = wsum;
+
+		if (slot)
+			slot[ntiles] = ssum;
+
+		multi[ntiles] = msum;
+	}
 }
 
 // deterministic mode: the tiles with several chunks as the sums of their partial
-// tiles in chunk order; a warp per tile and channel
-__global__ void k_sum_tiles(float2* __restrict__ grid, GridGeom g, BinGeom bg, const int* __restrict__ multi,
-		const int* __restrict__ nmulti, const int* __restrict__ work_start, const int* __restrict__ slot,
-		const float2* __restrict__ part, int C)
-{
-	const int lane = threadIdx.x % 32;
-	const long n = (long)*nmulti * C;
-	const int cells = bg.bs[0] * bg.bs[1] * bg.bs[2];
+// tiles in chunk order; a block per tile and channel, a thread per cell (all
+// tile shapes of this mode have 128 cells)
+enum { TG_DET_CELLS = 128 };
 
-	for (long j = ((long)blockIdx.x * blockDim.x + threadIdx.x) / 32; j < n; j += (long)gridDim.x * blockDim.x / 32) {
+__global__ void __launch_bounds__(TG_DET_CELLS) k_sum_tiles(float2* __restrict__ grid, GridGeom g, BinGeom bg,
+		const int* __restrict__ multi, const int* __restrict__ nmulti, const int* __restrict__ work_start,
+		const int* __restrict__ slot, const float2* __restrict__ part, int C)
+{
+	const int e = threadIdx.x;
+	const long n = (long)*nmulti * C;
+
+	for (long j = blockIdx.x; j < n; j += gridDim.x) {
 
 		const int t = multi[j / C], c = (int)(j % C);
 		const int bx = t % bg.nb[0], by = (t / bg.nb[0]) % bg.nb[1], bz = t / (bg.nb[0] * bg.nb[1]);
 		const int chunks = work_start[t + 1] - work_start[t];
+		const int cx = bx * bg.bs[0] + e % bg.bs[0];
+		const int cy = by * bg.bs[1] + (e / bg.bs[0]) % bg.bs[1];
+		const int cz = bz * bg.bs[2] + e / (bg.bs[0] * bg.bs[1]);
 
-		for (int e = lane; e < cells; e += 32) {
+		if ((cx >= g.G[0]) || (cy >= g.G[1]) || (cz >= g.G[2]))
+			continue;
 
-			const int cx = bx * bg.bs[0] + e % bg.bs[0];
-			const int cy = by * bg.bs[1] + (e / bg.bs[0]) % bg.bs[1];
-			const int cz = bz * bg.bs[2] + e / (bg.bs[0] * bg.bs[1]);
+		const float2* p = part + ((long)slot[t] * C + c) * TG_DET_CELLS + e;
+		float2 v = make_float2(0.f, 0.f);
+#pragma unroll 8
+		for (int k = 0; k < chunks; k++)
+			v = cadd(v, p[(long)k * C * TG_DET_CELLS]);
 
-			if ((cx >= g.G[0]) || (cy >= g.G[1]) || (cz >= g.G[2]))
-				continue;
-
-			float2 v = make_float2(0.f, 0.f);
-#pragma unroll 4
-			for (int k = 0; k < chunks; k++)
-				v = cadd(v, part[(((long)slot[t] + k) * C + c) * cells + e]);
-
-			const long cell = dft_index(cx, g.N[0], g.G[0]) + (long)g.G[0] * (dft_index(cy, g.N[1], g.G[1])
-					+ (long)g.G[1] * dft_index(cz, g.N[2], g.G[2]));
-			grid[cell + g.gsz * c] = v;
-		}
-	}
-}
-
-// work item table: tile t owns items work_start[t] .. work_start[t + 1] - 1;
-// tiles with several are listed in multi (count nmulti, cleared before)
-__global__ void k_work_fill(const int* __restrict__ work_start, long ntiles, int* __restrict__ work_tile,
-		int* __restrict__ work_chunk, int* __restrict__ multi, int* __restrict__ nmulti)
-{
-	for (long t = (long)blockIdx.x * blockDim.x + threadIdx.x; t < ntiles; t += (long)gridDim.x * blockDim.x) {
-
-		const int w0 = work_start[t], w1 = work_start[t + 1];
-
-		for (int w = w0; w < w1; w++) {
-
-			work_tile[w] = (int)t;
-			work_chunk[w] = w - w0;
-		}
-
-		if (w1 - w0 > 1)
-			multi[atomicAdd(nmulti, 1)] = (int)t;
+		const long cell = dft_index(cx, g.N[0], g.G[0]) + (long)g.G[0] * (dft_index(cy, g.N[1], g.G[1])
+				+ (long)g.G[1] * dft_index(cz, g.N[2], g.G[2]));
+		grid[cell + g.gsz * c] = v;
 	}
 }
 
