@@ -3242,8 +3242,42 @@ static int sm_count()
 	return n;
 }
 
-// One 32 -> 32 layer: the tcgen05 kernel (default; work tiles of two rows
-// of 128 pixels) or the mma.sync kernel (BNUFFT_NET_TC=0). wtc: the layer's
+// the tcgen05 kernel with work tiles of R rows of 128 pixels
+template <int MODE, int R>
+static int launch_conv32_tc(const bnufft_precnet_s* n, const bf16* in, const bf16* wtc, const float* bias, const bf16* mask,
+		bf16* out, int X, int Y, long nimg, const int* done, const int* skip, cudaStream_t st)
+{
+	auto enc = tensor_map_encoder();
+
+	if (!enc)
+		return fail(BNUFFT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+
+	// activations [nimg][Y][X][32] bf16; box {8 channels, 130 pixels, R + 2 rows, 1 image}
+	CUtensorMap map;
+	const cuuint64_t gdim[4] = { (cuuint64_t)NET_C, (cuuint64_t)X, (cuuint64_t)Y, (cuuint64_t)nimg };
+	const cuuint64_t gstr[3] = { (cuuint64_t)NET_C * 2, (cuuint64_t)NET_C * 2 * X, (cuuint64_t)NET_C * 2 * X * Y };
+	const cuuint32_t box[4] = { 8, TC_HX, R + 2, 1 };
+	const cuuint32_t estr[4] = { 1, 1, 1, 1 };
+	CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)in, gdim, gstr, box, estr,
+			CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+			CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+
+	if (CUDA_SUCCESS != r)
+		return fail(BNUFFT_ERR_CUDA, "cuTensorMapEncodeTiled: error %d", (int)r);
+
+	const size_t smem = conv_tc_smem(R);
+	TRY(prep_kernel(k_conv32_tc<MODE, R>, smem));
+	const long tiles = (long)((X + TC_M - 1) / TC_M) * ((Y + R - 1) / R) * nimg;
+	const int per_sm = (int)std::max<size_t>(1, (227 * 1024) / (smem + 1024));
+	const long blocks = std::min<long>(tiles, (long)sm_count() * std::min(per_sm, 4));
+	k_conv32_tc<MODE, R><<<(unsigned)blocks, 128, smem, st>>>(map, wtc, bias, mask, out, X, Y, (int)nimg, done,
+			skip, n->tc_status);
+	LAUNCHED();
+	return BNUFFT_OK;
+}
+
+// One 32 -> 32 layer: the tcgen05 kernel (default) or the mma.sync kernel
+// (BNUFFT_NET_TC=0). wtc: the layer's
 // weights in the tensor-core kernel's plane order; w: the same in the
 // mma.sync kernel's order.
 template <int MODE>
@@ -3252,37 +3286,14 @@ static int launch_conv32(const bnufft_precnet_s* n, const bf16* in, const bf16* 
 		cudaStream_t st)
 {
 	const char* e = getenv("BNUFFT_NET_TC");
-	constexpr int R = 2;
 
 	if (!(e && (0 == strcmp(e, "0")))) {
 
-		auto enc = tensor_map_encoder();
-
-		if (!enc)
-			return fail(BNUFFT_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
-
-		// activations [nimg][Y][X][32] bf16; box {8 channels, 130 pixels, R + 2 rows, 1 image}
-		CUtensorMap map;
-		const cuuint64_t gdim[4] = { (cuuint64_t)NET_C, (cuuint64_t)X, (cuuint64_t)Y, (cuuint64_t)nimg };
-		const cuuint64_t gstr[3] = { (cuuint64_t)NET_C * 2, (cuuint64_t)NET_C * 2 * X, (cuuint64_t)NET_C * 2 * X * Y };
-		const cuuint32_t box[4] = { 8, TC_HX, R + 2, 1 };
-		const cuuint32_t estr[4] = { 1, 1, 1, 1 };
-		CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, (void*)in, gdim, gstr, box, estr,
-				CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
-				CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-
-		if (CUDA_SUCCESS != r)
-			return fail(BNUFFT_ERR_CUDA, "cuTensorMapEncodeTiled: error %d", (int)r);
-
-		const size_t smem = conv_tc_smem(R);
-		TRY(prep_kernel(k_conv32_tc<MODE, R>, smem));
-		const long tiles = (long)((X + TC_M - 1) / TC_M) * ((Y + R - 1) / R) * nimg;
-		const int per_sm = (int)std::max<size_t>(1, (227 * 1024) / (smem + 1024));
-		const long blocks = std::min<long>(tiles, (long)sm_count() * std::min(per_sm, 4));
-		k_conv32_tc<MODE, R><<<(unsigned)blocks, 128, smem, st>>>(map, wtc, bias, mask, out, X, Y, (int)nimg, done,
-				skip, n->tc_status);
-		LAUNCHED();
-		return BNUFFT_OK;
+		// four rows per tile (1.5 times the rows loaded instead of 2) where
+		// that still leaves a few tiles per SM
+		const long t4 = (long)((X + TC_M - 1) / TC_M) * ((Y + 3) / 4) * nimg;
+		return (t4 >= 4 * 148) ? launch_conv32_tc<MODE, 4>(n, in, wtc, bias, mask, out, X, Y, nimg, done, skip, st)
+				: launch_conv32_tc<MODE, 2>(n, in, wtc, bias, mask, out, X, Y, nimg, done, skip, st);
 	}
 
 	TRY(prep_kernel(k_conv32<MODE>, NET_CONV_SMEM));
@@ -3375,7 +3386,7 @@ enum { NET_WG_BLOCKS = 4 * 148 };
 static int net_wgrad_reduce(bnufft_precnet_s* n, int l, unsigned nblk, cudaStream_t st)
 {
 	const int O = NetLayout::size(l);
-	k_wgrad_reduce<<<(O + 31) / 32, 256, 0, st>>>(n->part, (int)nblk, O, n->grad + NetLayout::woff(l));
+	k_wgrad_reduce<<<(O + 31) / 32, 32 * WR_SLICES, 0, st>>>(n->part, (int)nblk, O, n->grad + NetLayout::woff(l));
 	LAUNCHED();
 	return BNUFFT_OK;
 }

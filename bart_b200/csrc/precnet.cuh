@@ -196,7 +196,68 @@ __global__ void __launch_bounds__(NET_THREADS) k_conv32(const bf16* __restrict__
 	}
 }
 
-// Layer 1 (2 -> 32), one thread per pixel: act = bf16(relu(conv(s * in) + b)),
+// The thin layers (2 channels on one side) take a quad of lanes per four
+// consecutive pixels: lane q holds channels 8 q .. 8 q + 7 of all four, so the
+// 64 bytes of a pixel's activation are one access of the quad and a weight
+// vector read from shared memory serves four pixels. (One thread per pixel
+// read or wrote sixteen lines per warp access and reloaded the weights for
+// every pixel: seven 256^2 images took 34 us in layer 1, 54 us in layer 6 and
+// 52 us in its backward pass.) Blocks cover 256 pixels.
+struct NetPix {
+
+	long p0;		// first of the quad's pixels
+	int q;			// lane in the quad
+	unsigned in[4];		// bit per tap: the neighbour is inside the image
+
+	__device__ __forceinline__ NetPix(int X, int Y, long P)
+	{
+		q = threadIdx.x & 3;
+		p0 = ((long)blockIdx.x * NET_THREADS + threadIdx.x) / 4 * 4;
+		const long XY = (long)X * Y;
+		const int rest = (int)(min(p0, P - 1) % XY);
+		int y = rest / X, x = rest - y * X;
+#pragma unroll
+		for (int i = 0; i < 4; i++) {
+
+			// columns x - 1, x, x + 1 of a row, the three rows
+			const unsigned row = ((x > 0) ? 1u : 0u) | 2u | ((x + 1 < X) ? 4u : 0u);
+			in[i] = (p0 + i < P) ? (((y > 0) ? row : 0u) | (row << 3) | ((y + 1 < Y) ? row << 6 : 0u)) : 0u;
+
+			if (++x == X) {
+
+				x = 0;
+				y = (y + 1 == Y) ? 0 : y + 1;
+			}
+		}
+	}
+
+	// pixel i has a neighbour at this tap
+	__device__ __forceinline__ bool has(int i, int tap) const { return 0 != ((in[i] >> tap) & 1u); }
+
+	// first pixel plus the tap's offset
+	__device__ __forceinline__ long base(int tap, int X) const { return p0 + (long)(tap / 3 - 1) * X + tap % 3 - 1; }
+};
+
+__device__ __forceinline__ void net_bf16x8(const uint4& u, float (&f)[8])
+{
+	const bf162* h = (const bf162*)&u;
+#pragma unroll
+	for (int j = 0; j < 4; j++) {
+
+		const float2 v = __bfloat1622float2(h[j]);
+		f[2 * j] = v.x;
+		f[2 * j + 1] = v.y;
+	}
+}
+
+__device__ __forceinline__ void net_lds8(const float* s, float (&f)[8])
+{
+	const float4 a = *(const float4*)s, b = *(const float4*)(s + 4);
+	f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w;
+	f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
+}
+
+// Layer 1 (2 -> 32): act = bf16(relu(conv(s * in) + b)),
 // in complex [nimg][Y][X], s = *scale, or 1 / sqrt(sum of norm_part) (the
 // input's norm from the partials of the pass that wrote it), or 1. w: float
 // [32][9][2] (values already rounded to bf16), b: [32]. Nothing is done when
@@ -205,14 +266,14 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_in(const float2* __restrict
 		const float* __restrict__ w, const float* __restrict__ b, const float* scale, const double* norm_part,
 		int nnorm, bf16* __restrict__ out, const int* done, const int* skip)
 {
-	__shared__ float sw[NET_C * 18 + NET_C];
+	__shared__ __align__(16) float sw[19 * NET_C];	// [2 tap + channel][cout], then the biases
 	__shared__ double red[32];
 
 	if ((done && *done) || (skip && *skip))
 		return;
 
-	for (int i = threadIdx.x; i < NET_C * 18 + NET_C; i += NET_THREADS)
-		sw[i] = (i < NET_C * 18) ? w[i] : b[i - NET_C * 18];
+	for (int i = threadIdx.x; i < 19 * NET_C; i += NET_THREADS)
+		sw[i] = (i < 18 * NET_C) ? w[(i % NET_C) * 18 + i / NET_C] : b[i - 18 * NET_C];
 
 	float s = 1.f;
 
@@ -228,92 +289,61 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_in(const float2* __restrict
 
 	__syncthreads();
 
-	const long p = (long)blockIdx.x * NET_THREADS + threadIdx.x;
-
-	if (p >= P)
-		return;
-
-	const long XY = (long)X * Y;
-	const long base = (p / XY) * XY;
-	const int y = (int)((p % XY) / X);
-	const int x = (int)(p % X);
-	float v[18];
+	const NetPix px(X, Y, P);
+	float acc[4][8], wv[8];
+	net_lds8(sw + 18 * NET_C + 8 * px.q, wv);
 #pragma unroll
+	for (int i = 0; i < 4; i++)
+#pragma unroll
+		for (int c = 0; c < 8; c++)
+			acc[i][c] = wv[c];
+
+#pragma unroll 3
 	for (int tap = 0; tap < 9; tap++) {
 
-		int yy = y + tap / 3 - 1;
-		int xx = x + tap % 3 - 1;
-		float2 u = make_float2(0.f, 0.f);
-
-		if ((yy >= 0) && (yy < Y) && (xx >= 0) && (xx < X))
-			u = in[base + (long)yy * X + xx];
-
-		v[2 * tap] = u.x * s;
-		v[2 * tap + 1] = u.y * s;
-	}
-
-	// the pixel's 32 channels leave as four 16-byte stores
-	uint32_t pk[16];
+		const float2* nb = in + px.base(tap, X);
+		float2 v[4];
 #pragma unroll
-	for (int co = 0; co < NET_C; co += 2) {
+		for (int i = 0; i < 4; i++) {
 
-		float a0 = sw[NET_C * 18 + co];
-		float a1 = sw[NET_C * 18 + co + 1];
-#pragma unroll
-		for (int k = 0; k < 18; k++) {
-
-			a0 = fmaf(sw[co * 18 + k], v[k], a0);
-			a1 = fmaf(sw[(co + 1) * 18 + k], v[k], a1);
+			v[i] = px.has(i, tap) ? nb[i] : make_float2(0.f, 0.f);
+			v[i].x *= s;
+			v[i].y *= s;
 		}
 
-		const bf162 h = __floats2bfloat162_rn(fmaxf(a0, 0.f), fmaxf(a1, 0.f));
-		pk[co / 2] = *(const uint32_t*)&h;
+		net_lds8(sw + 2 * tap * NET_C + 8 * px.q, wv);
+#pragma unroll
+		for (int i = 0; i < 4; i++)
+#pragma unroll
+			for (int c = 0; c < 8; c++)
+				acc[i][c] = fmaf(wv[c], v[i].x, acc[i][c]);
+
+		net_lds8(sw + (2 * tap + 1) * NET_C + 8 * px.q, wv);
+#pragma unroll
+		for (int i = 0; i < 4; i++)
+#pragma unroll
+			for (int c = 0; c < 8; c++)
+				acc[i][c] = fmaf(wv[c], v[i].y, acc[i][c]);
 	}
 
-	uint4* o = (uint4*)(out + p * NET_C);
 #pragma unroll
-	for (int q = 0; q < 4; q++)
-		o[q] = make_uint4(pk[4 * q], pk[4 * q + 1], pk[4 * q + 2], pk[4 * q + 3]);
-}
+	for (int i = 0; i < 4; i++) {
 
-// sum over the 3x3 neighbourhood of a 32-channel bf16 activation with
-// weights w[co][tap][ci] (float), co in {0, 1}
-__device__ __forceinline__ float2 net_out_pixel(const bf16* __restrict__ act, long base, int x, int y, int X, int Y,
-		const float* sw)
-{
-	float o0 = 0.f, o1 = 0.f;
-#pragma unroll 1
-	for (int tap = 0; tap < 9; tap++) {
-
-		int yy = y + tap / 3 - 1;
-		int xx = x + tap % 3 - 1;
-
-		if ((yy < 0) || (yy >= Y) || (xx < 0) || (xx >= X))
-			continue;
-
-		const uint4* a = (const uint4*)(act + (base + (long)yy * X + xx) * NET_C);
+		uint4 o;
+		uint32_t* pk = (uint32_t*)&o;
 #pragma unroll
-		for (int q = 0; q < 4; q++) {
+		for (int j = 0; j < 4; j++) {
 
-			uint4 u = a[q];
-			const bf162* h = (const bf162*)&u;
-#pragma unroll
-			for (int j = 0; j < 4; j++) {
-
-				float2 f = __bfloat1622float2(h[j]);
-				int ci = q * 8 + 2 * j;
-				o0 = fmaf(sw[tap * NET_C + ci], f.x, o0);
-				o0 = fmaf(sw[tap * NET_C + ci + 1], f.y, o0);
-				o1 = fmaf(sw[9 * NET_C + tap * NET_C + ci], f.x, o1);
-				o1 = fmaf(sw[9 * NET_C + tap * NET_C + ci + 1], f.y, o1);
-			}
+			const bf162 h = __floats2bfloat162_rn(fmaxf(acc[i][2 * j], 0.f), fmaxf(acc[i][2 * j + 1], 0.f));
+			pk[j] = *(const uint32_t*)&h;
 		}
-	}
 
-	return make_float2(o0, o1);
+		if (px.p0 + i < P)
+			*(uint4*)(out + (px.p0 + i) * NET_C + 8 * px.q) = o;
+	}
 }
 
-// Layer 6 (32 -> 2), one thread per pixel:
+// Layer 6 (32 -> 2):
 //   out = zc + s * (conv(act, w) + b)   (zc = 0 if null),
 // s = *scale, or sqrt(sum of norm_part) (the norm of zc, from the partials
 // of the pass that wrote it), or 1; out = zc when *net_off (the stall
@@ -323,7 +353,7 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out(const bf16* __restrict_
 		int nnorm, const float2* zc, float2* out, const float2* __restrict__ pdot, double* __restrict__ dot_part,
 		const int* done, const int* net_off)
 {
-	__shared__ float sw[2 * 9 * NET_C + 2];
+	__shared__ __align__(16) float sw[2 * 9 * NET_C + 2];
 	__shared__ double red[32];
 
 	if (done && *done)
@@ -335,18 +365,62 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out(const bf16* __restrict_
 	const float s = scale ? *scale : (norm_part ? (float)sqrt(sum_partials_d(norm_part, nnorm, red)) : 1.f);
 	__syncthreads();
 
-	const long p = (long)blockIdx.x * NET_THREADS + threadIdx.x;
 	const bool off = net_off && *net_off;
+	const NetPix px(X, Y, P);
+	const long p = px.p0 + px.q;		// the pixel this lane writes
+	float2 o = make_float2(0.f, 0.f);
+
+	if (!off) {	// block-uniform
+
+		float2 acc[4];
+#pragma unroll
+		for (int i = 0; i < 4; i++)
+			acc[i] = make_float2(0.f, 0.f);
+#pragma unroll 3
+		for (int tap = 0; tap < 9; tap++) {
+
+			const bf16* nb = act + px.base(tap, X) * NET_C + 8 * px.q;
+			uint4 u[4];
+#pragma unroll
+			for (int i = 0; i < 4; i++) {
+
+				u[i] = px.has(i, tap) ? *(const uint4*)(nb + i * NET_C) : make_uint4(0u, 0u, 0u, 0u);
+			}
+
+			float w0[8], w1[8], f[8];
+			net_lds8(sw + tap * NET_C + 8 * px.q, w0);
+			net_lds8(sw + 9 * NET_C + tap * NET_C + 8 * px.q, w1);
+#pragma unroll
+			for (int i = 0; i < 4; i++) {
+
+				net_bf16x8(u[i], f);
+#pragma unroll
+				for (int c = 0; c < 8; c++) {
+
+					acc[i].x = fmaf(w0[c], f[c], acc[i].x);
+					acc[i].y = fmaf(w1[c], f[c], acc[i].y);
+				}
+			}
+		}
+
+		// sums over the quad's channels; lane q keeps pixel q
+		auto shfl = [](float2 v, int m) {
+			return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+		};
+		float2 k0 = (px.q & 2) ? acc[2] : acc[0], k1 = (px.q & 2) ? acc[3] : acc[1];
+		k0 = cadd(k0, shfl((px.q & 2) ? acc[0] : acc[2], 2));
+		k1 = cadd(k1, shfl((px.q & 2) ? acc[1] : acc[3], 2));
+		o = cadd((px.q & 1) ? k1 : k0, shfl((px.q & 1) ? k0 : k1, 1));
+	}
+
 	double dot = 0.;
 
 	if (p < P) {
 
-		const long XY = (long)X * Y;
 		float2 v = zc ? zc[p] : make_float2(0.f, 0.f);
 
 		if (!off) {
 
-			float2 o = net_out_pixel(act, (p / XY) * XY, (int)(p % X), (int)((p % XY) / X), X, Y, sw);
 			v.x = fmaf(s, o.x + sw[2 * 9 * NET_C], v.x);
 			v.y = fmaf(s, o.y + sw[2 * 9 * NET_C + 1], v.y);
 		}
@@ -374,49 +448,64 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out(const bf16* __restrict_
 __global__ void __launch_bounds__(NET_THREADS) k_net_out_bwd(const float2* __restrict__ gout, const bf16* __restrict__ act5,
 		int X, int Y, long P, const float* __restrict__ w, bf16* __restrict__ gu5)
 {
-	__shared__ float sw[2 * 9 * NET_C];
+	__shared__ __align__(16) float sw[2 * 9 * NET_C];
 
 	for (int i = threadIdx.x; i < 2 * 9 * NET_C; i += NET_THREADS)
 		sw[i] = w[i];
 
 	__syncthreads();
 
-	const long q = (long)blockIdx.x * NET_THREADS + threadIdx.x;
-
-	if (q >= P)
-		return;
-
-	const long XY = (long)X * Y;
-	const long base = (q / XY) * XY;
-	const int y = (int)((q % XY) / X);
-	const int x = (int)(q % X);
-	float2 gn[9];
+	const NetPix px(X, Y, P);
+	float acc[4][8];
 #pragma unroll
+	for (int i = 0; i < 4; i++)
+#pragma unroll
+		for (int c = 0; c < 8; c++)
+			acc[i][c] = 0.f;
+
+#pragma unroll 3
 	for (int tap = 0; tap < 9; tap++) {
 
-		int yy = y + tap / 3 - 1;
-		int xx = x + tap % 3 - 1;
-		gn[tap] = ((yy >= 0) && (yy < Y) && (xx >= 0) && (xx < X)) ? gout[base + (long)yy * X + xx] : make_float2(0.f, 0.f);
-	}
-
-	const bf162* m = (const bf162*)(act5 + q * NET_C);
-	bf162* o = (bf162*)(gu5 + q * NET_C);
-#pragma unroll 2
-	for (int ci = 0; ci < NET_C; ci += 2) {
-
-		float a0 = 0.f, a1 = 0.f;
+		const float2* nb = gout + px.base(tap, X);
+		float2 g[4];
 #pragma unroll
-		for (int tap = 0; tap < 9; tap++) {
+		for (int i = 0; i < 4; i++) {
 
-			int ft = 8 - tap;
-			a0 = fmaf(sw[ft * NET_C + ci], gn[tap].x, a0);
-			a0 = fmaf(sw[9 * NET_C + ft * NET_C + ci], gn[tap].y, a0);
-			a1 = fmaf(sw[ft * NET_C + ci + 1], gn[tap].x, a1);
-			a1 = fmaf(sw[9 * NET_C + ft * NET_C + ci + 1], gn[tap].y, a1);
+			g[i] = px.has(i, tap) ? nb[i] : make_float2(0.f, 0.f);
 		}
 
-		float2 mk = __bfloat1622float2(m[ci / 2]);
-		o[ci / 2] = __floats2bfloat162_rn((mk.x > 0.f) ? a0 : 0.f, (mk.y > 0.f) ? a1 : 0.f);
+		float w0[8], w1[8];
+		net_lds8(sw + (8 - tap) * NET_C + 8 * px.q, w0);
+		net_lds8(sw + 9 * NET_C + (8 - tap) * NET_C + 8 * px.q, w1);
+#pragma unroll
+		for (int i = 0; i < 4; i++)
+#pragma unroll
+			for (int c = 0; c < 8; c++) {
+
+				acc[i][c] = fmaf(w0[c], g[i].x, acc[i][c]);
+				acc[i][c] = fmaf(w1[c], g[i].y, acc[i][c]);
+			}
+	}
+
+#pragma unroll
+	for (int i = 0; i < 4; i++) {
+
+		if (px.p0 + i >= P)
+			break;
+
+		float m[8];
+		net_bf16x8(*(const uint4*)(act5 + (px.p0 + i) * NET_C + 8 * px.q), m);
+		uint4 o;
+		uint32_t* pk = (uint32_t*)&o;
+#pragma unroll
+		for (int j = 0; j < 4; j++) {
+
+			const bf162 h = __floats2bfloat162_rn((m[2 * j] > 0.f) ? acc[i][2 * j] : 0.f,
+					(m[2 * j + 1] > 0.f) ? acc[i][2 * j + 1] : 0.f);
+			pk[j] = *(const uint32_t*)&h;
+		}
+
+		*(uint4*)(gu5 + (px.p0 + i) * NET_C + 8 * px.q) = o;
 	}
 }
 
@@ -711,17 +800,19 @@ __global__ void __launch_bounds__(32 * WT_WARPS) k_wgrad_thin(const bf16* __rest
 }
 
 // grad[o] = sum over blocks of part[blk][o] in float64: 32 outputs per block,
-// eight slices of the partials, combined in a fixed order
-__global__ void __launch_bounds__(256) k_wgrad_reduce(const float* __restrict__ part, int nblk, int O,
+// WR_SLICES slices of the partials, combined in a fixed order
+enum { WR_SLICES = 32 };
+
+__global__ void __launch_bounds__(32 * WR_SLICES) k_wgrad_reduce(const float* __restrict__ part, int nblk, int O,
 		float* __restrict__ grad)
 {
-	__shared__ double sh[8][32];
+	__shared__ double sh[WR_SLICES][32];
 	const int o = blockIdx.x * 32 + threadIdx.x % 32, sl = threadIdx.x / 32;
 	double acc = 0.;
 
 	if (o < O) {
 #pragma unroll 4
-		for (int k = sl; k < nblk; k += 8)
+		for (int k = sl; k < nblk; k += WR_SLICES)
 			acc += part[(long)k * O + o];
 	}
 
@@ -729,8 +820,8 @@ __global__ void __launch_bounds__(256) k_wgrad_reduce(const float* __restrict__ 
 	__syncthreads();
 
 	if ((0 == sl) && (o < O)) {
-
-		for (int k = 1; k < 8; k++)
+#pragma unroll
+		for (int k = 1; k < WR_SLICES; k++)
 			acc += sh[k][threadIdx.x];
 
 		grad[o] = (float)acc;

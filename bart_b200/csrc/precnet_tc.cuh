@@ -22,8 +22,9 @@
 //  * B: the weights prepacked as 36 planes of 32 rows x 16 B (plane =
 //    tap * 4 + cin / 8, row = cout), one bulk copy of 18 KB per block.
 // Blocks are persistent: each loads the weights once and walks the tiles
-// blockIdx.x, + gridDim.x, ...; several blocks share an SM, so one block's
-// loads overlap another's MMAs and epilogue.
+// blockIdx.x, + gridDim.x, ...; the next tile's planes are loaded while this
+// one's epilogue runs (its MMAs have read theirs), and several blocks share an
+// SM, so one block's loads overlap another's MMAs.
 //
 // Epilogue: warp w reads TMEM lanes 32w .. 32w + 31 (= pixels), 32 columns
 // (= output channels) per thread; MODE 0 adds the bias and applies the ReLU,
@@ -46,8 +47,9 @@ namespace bn {
 
 enum { TC_M = 128, TC_HX = TC_M + 2, TC_SPIN_LIMIT = 1 << 22, TC_W_BYTES = 36 * 512 };
 
-// bytes of one A channel plane
-__host__ __device__ constexpr uint32_t conv_tc_plane(int R) { return (uint32_t)(R + 2) * TC_HX * 16; }
+// bytes of one A channel plane, and its stride (the TMA writes to 128-byte boundaries)
+__host__ __device__ constexpr uint32_t conv_tc_box(int R) { return (uint32_t)(R + 2) * TC_HX * 16; }
+__host__ __device__ constexpr uint32_t conv_tc_plane(int R) { return (conv_tc_box(R) + 127) / 128 * 128; }
 
 // shared-memory bytes: A planes, B planes, two mbarriers and the TMEM slot
 __host__ __device__ constexpr size_t conv_tc_smem(int R) { return (size_t)4 * conv_tc_plane(R) + TC_W_BYTES + 32; }
@@ -202,26 +204,30 @@ __global__ void __launch_bounds__(128) k_conv32_tc(const __grid_constant__ CUten
 	uint32_t phase = 0;	// uses of each barrier so far (parity of the next wait)
 	bool mma_pending = false, load_pending = false;
 
+	// thread 0: tile t's halo planes (and the weights with the first one)
+	auto load = [&](long t, bool first) {
+		const int rem = (int)(t % ((long)tx * ty));
+		mbar_expect_tx(lbar, 4 * conv_tc_box(R) + (first ? TC_W_BYTES : 0));
+
+		if (first)
+			bulk_load(b0, wp, TC_W_BYTES, lbar);
+
+		for (int j = 0; j < 4; j++)
+			tma_load_4d(a0 + j * PLANE, &in, 8 * j, (rem % tx) * TC_M - 1, (rem / tx) * R - 1, (int)(t / ((long)tx * ty)),
+					lbar);
+	};
+
+	if (0 == tid)
+		load(blockIdx.x, true);
+
+	load_pending = true;
+
 	for (long t = blockIdx.x; t < ntiles; t += gridDim.x, phase ^= 1u) {
 
 		const int img = (int)(t / ((long)tx * ty));
 		const int rem = (int)(t % ((long)tx * ty));
 		const int x0 = (rem % tx) * TC_M;
 		const int y0 = (rem / tx) * R;
-
-		if (0 == tid) {	// halo planes (and the weights with the first tile)
-
-			const bool first = ((long)blockIdx.x == t);
-			mbar_expect_tx(lbar, 4 * PLANE + (first ? TC_W_BYTES : 0));
-
-			if (first)
-				bulk_load(b0, wp, TC_W_BYTES, lbar);
-
-			for (int j = 0; j < 4; j++)
-				tma_load_4d(a0 + j * PLANE, &in, 8 * j, x0 - 1, y0 - 1, img, lbar);
-		}
-
-		load_pending = true;
 		bool ok = mbar_wait_bounded(lbar, phase);
 
 		if (!__syncthreads_and(ok ? 1 : 0)) {
@@ -267,6 +273,15 @@ __global__ void __launch_bounds__(128) k_conv32_tc(const __grid_constant__ CUten
 
 		mma_pending = false;
 		asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+
+		if (t + gridDim.x < ntiles) {
+
+			if (0 == tid)
+				load(t + gridDim.x, false);
+
+			load_pending = true;
+		}
+
 		const int px = x0 + tid;	// this thread's pixel (TMEM lane = tid)
 #pragma unroll 1
 		for (int r = 0; r < R; r++) {
@@ -280,6 +295,13 @@ __global__ void __launch_bounds__(128) k_conv32_tc(const __grid_constant__ CUten
 
 			const long o = (((long)img * Y + gy) * X + px) * NET_C;
 			uint32_t pk[16];
+			uint4 mk[4];
+
+			if (1 == MODE) {
+#pragma unroll
+				for (int q = 0; q < 4; q++)
+					mk[q] = ((const uint4*)(mask + o))[q];
+			}
 #pragma unroll
 			for (int c = 0; c < 32; c += 2) {
 
@@ -292,7 +314,7 @@ __global__ void __launch_bounds__(128) k_conv32_tc(const __grid_constant__ CUten
 
 				} else {
 
-					const bf162 m = *(const bf162*)(mask + o + c);
+					const bf162 m = ((const bf162*)mk)[c / 2];
 					v0 = (__bfloat162float(m.x) > 0.f) ? v0 : 0.f;
 					v1 = (__bfloat162float(m.y) > 0.f) ? v1 : 0.f;
 				}

@@ -41,12 +41,13 @@ def test_forward_vs_oracle(X, Y, n):
     assert rel(out, po.from_channels(ref)) < 3e-3
 
 
-@pytest.mark.parametrize("X,Y,n", [(256, 256, 1), (200, 131, 2), (128, 9, 1)])
+@pytest.mark.parametrize("X,Y,n", [(256, 256, 1), (200, 131, 2), (128, 9, 1), (130, 131, 9)])
 def test_tensor_core_layers_match_mma_sync(X, Y, n, monkeypatch):
     """The tcgen05 layers (default) against the mma.sync ones: both sum the
     same exact bf16 products in float32, in another order, so outputs and
     gradients differ only where an activation rounds to the other bf16
-    neighbour. Covers partial 128-pixel tiles, an odd row count and a batch."""
+    neighbour. Covers partial 128-pixel tiles, an odd row count, a batch, and
+    the four-row tiles of large batches."""
     rng = np.random.default_rng(X * Y + n)
     p = _params(rng)
     x, t = _img(rng, X, Y, n), _img(rng, X, Y, n)
