@@ -238,6 +238,43 @@ struct NetPix {
 	__device__ __forceinline__ long base(int tap, int X) const { return p0 + (long)(tap / 3 - 1) * X + tap % 3 - 1; }
 };
 
+// Position of a work item among nx x ny per image, advanced by a fixed step
+// without a division per item.
+struct NetWalk {
+
+	int x, y, nx, ny, sx, sy;
+	long z, sz;		// image
+
+	__device__ __forceinline__ NetWalk(long first, long step, int nx_, int ny_) : nx(nx_), ny(ny_)
+	{
+		x = (int)(first % nx);
+		y = (int)((first / nx) % ny);
+		z = first / nx / ny;
+		sx = (int)(step % nx);
+		sy = (int)((step / nx) % ny);
+		sz = step / nx / ny;
+	}
+
+	__device__ __forceinline__ void next()
+	{
+		x += sx;
+		y += sy;
+		z += sz;
+
+		if (x >= nx) {
+
+			x -= nx;
+			y++;
+		}
+
+		if (y >= ny) {
+
+			y -= ny;
+			z++;
+		}
+	}
+};
+
 __device__ __forceinline__ void net_bf16x8(const uint4& u, float (&f)[8])
 {
 	const bf162* h = (const bf162*)&u;
@@ -250,11 +287,12 @@ __device__ __forceinline__ void net_bf16x8(const uint4& u, float (&f)[8])
 	}
 }
 
-__device__ __forceinline__ void net_lds8(const float* s, float (&f)[8])
+// eight floats as pairs (two-wide arithmetic)
+__device__ __forceinline__ void net_lds8(const float* s, float2 (&f)[4])
 {
 	const float4 a = *(const float4*)s, b = *(const float4*)(s + 4);
-	f[0] = a.x, f[1] = a.y, f[2] = a.z, f[3] = a.w;
-	f[4] = b.x, f[5] = b.y, f[6] = b.z, f[7] = b.w;
+	f[0] = make_float2(a.x, a.y), f[1] = make_float2(a.z, a.w);
+	f[2] = make_float2(b.x, b.y), f[3] = make_float2(b.z, b.w);
 }
 
 // Layer 1 (2 -> 32): act = bf16(relu(conv(s * in) + b)),
@@ -290,12 +328,12 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_in(const float2* __restrict
 	__syncthreads();
 
 	const NetPix px(X, Y, P);
-	float acc[4][8], wv[8];
+	float2 acc[4][4], wv[4];	// pixel, channel pair
 	net_lds8(sw + 18 * NET_C + 8 * px.q, wv);
 #pragma unroll
 	for (int i = 0; i < 4; i++)
 #pragma unroll
-		for (int c = 0; c < 8; c++)
+		for (int c = 0; c < 4; c++)
 			acc[i][c] = wv[c];
 
 #pragma unroll 3
@@ -315,15 +353,15 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_in(const float2* __restrict
 #pragma unroll
 		for (int i = 0; i < 4; i++)
 #pragma unroll
-			for (int c = 0; c < 8; c++)
-				acc[i][c] = fmaf(wv[c], v[i].x, acc[i][c]);
+			for (int c = 0; c < 4; c++)
+				acc[i][c] = cfma(wv[c], make_float2(v[i].x, v[i].x), acc[i][c]);
 
 		net_lds8(sw + (2 * tap + 1) * NET_C + 8 * px.q, wv);
 #pragma unroll
 		for (int i = 0; i < 4; i++)
 #pragma unroll
-			for (int c = 0; c < 8; c++)
-				acc[i][c] = fmaf(wv[c], v[i].y, acc[i][c]);
+			for (int c = 0; c < 4; c++)
+				acc[i][c] = cfma(wv[c], make_float2(v[i].y, v[i].y), acc[i][c]);
 	}
 
 #pragma unroll
@@ -334,7 +372,7 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_in(const float2* __restrict
 #pragma unroll
 		for (int j = 0; j < 4; j++) {
 
-			const bf162 h = __floats2bfloat162_rn(fmaxf(acc[i][2 * j], 0.f), fmaxf(acc[i][2 * j + 1], 0.f));
+			const bf162 h = __floats2bfloat162_rn(fmaxf(acc[i][j].x, 0.f), fmaxf(acc[i][j].y, 0.f));
 			pk[j] = *(const uint32_t*)&h;
 		}
 
@@ -353,14 +391,14 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out(const bf16* __restrict_
 		int nnorm, const float2* zc, float2* out, const float2* __restrict__ pdot, double* __restrict__ dot_part,
 		const int* done, const int* net_off)
 {
-	__shared__ __align__(16) float sw[2 * 9 * NET_C + 2];
+	__shared__ __align__(16) float sw[2 * 9 * NET_C + 2];	// [tap][channel][output], then the biases
 	__shared__ double red[32];
 
 	if (done && *done)
 		return;
 
 	for (int i = threadIdx.x; i < 2 * 9 * NET_C + 2; i += NET_THREADS)
-		sw[i] = (i < 2 * 9 * NET_C) ? w[i] : b[i - 2 * 9 * NET_C];
+		sw[i] = (i < 2 * 9 * NET_C) ? w[(i % 2) * 9 * NET_C + i / 2] : b[i - 2 * 9 * NET_C];
 
 	const float s = scale ? *scale : (norm_part ? (float)sqrt(sum_partials_d(norm_part, nnorm, red)) : 1.f);
 	__syncthreads();
@@ -387,19 +425,20 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out(const bf16* __restrict_
 				u[i] = px.has(i, tap) ? *(const uint4*)(nb + i * NET_C) : make_uint4(0u, 0u, 0u, 0u);
 			}
 
-			float w0[8], w1[8], f[8];
-			net_lds8(sw + tap * NET_C + 8 * px.q, w0);
-			net_lds8(sw + 9 * NET_C + tap * NET_C + 8 * px.q, w1);
+			float2 wa[4], wb[4];	// channels 0-3 and 4-7 of the lane
+			net_lds8(sw + 2 * (tap * NET_C + 8 * px.q), wa);
+			net_lds8(sw + 2 * (tap * NET_C + 8 * px.q) + 8, wb);
 #pragma unroll
 			for (int i = 0; i < 4; i++) {
 
+				float f[8];
 				net_bf16x8(u[i], f);
 #pragma unroll
-				for (int c = 0; c < 8; c++) {
-
-					acc[i].x = fmaf(w0[c], f[c], acc[i].x);
-					acc[i].y = fmaf(w1[c], f[c], acc[i].y);
-				}
+				for (int c = 0; c < 4; c++)
+					acc[i] = cfma(wa[c], make_float2(f[c], f[c]), acc[i]);
+#pragma unroll
+				for (int c = 0; c < 4; c++)
+					acc[i] = cfma(wb[c], make_float2(f[4 + c], f[4 + c]), acc[i]);
 			}
 		}
 
@@ -456,12 +495,12 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out_bwd(const float2* __res
 	__syncthreads();
 
 	const NetPix px(X, Y, P);
-	float acc[4][8];
+	float2 acc[4][4];	// pixel, channel pair
 #pragma unroll
 	for (int i = 0; i < 4; i++)
 #pragma unroll
-		for (int c = 0; c < 8; c++)
-			acc[i][c] = 0.f;
+		for (int c = 0; c < 4; c++)
+			acc[i][c] = make_float2(0.f, 0.f);
 
 #pragma unroll 3
 	for (int tap = 0; tap < 9; tap++) {
@@ -474,16 +513,16 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out_bwd(const float2* __res
 			g[i] = px.has(i, tap) ? nb[i] : make_float2(0.f, 0.f);
 		}
 
-		float w0[8], w1[8];
+		float2 w0[4], w1[4];
 		net_lds8(sw + (8 - tap) * NET_C + 8 * px.q, w0);
 		net_lds8(sw + 9 * NET_C + (8 - tap) * NET_C + 8 * px.q, w1);
 #pragma unroll
 		for (int i = 0; i < 4; i++)
 #pragma unroll
-			for (int c = 0; c < 8; c++) {
+			for (int c = 0; c < 4; c++) {
 
-				acc[i][c] = fmaf(w0[c], g[i].x, acc[i][c]);
-				acc[i][c] = fmaf(w1[c], g[i].y, acc[i][c]);
+				acc[i][c] = cfma(w0[c], make_float2(g[i].x, g[i].x), acc[i][c]);
+				acc[i][c] = cfma(w1[c], make_float2(g[i].y, g[i].y), acc[i][c]);
 			}
 	}
 
@@ -500,8 +539,8 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out_bwd(const float2* __res
 #pragma unroll
 		for (int j = 0; j < 4; j++) {
 
-			const bf162 h = __floats2bfloat162_rn((m[2 * j] > 0.f) ? acc[i][2 * j] : 0.f,
-					(m[2 * j + 1] > 0.f) ? acc[i][2 * j + 1] : 0.f);
+			const bf162 h = __floats2bfloat162_rn((m[2 * j] > 0.f) ? acc[i][j].x : 0.f,
+					(m[2 * j + 1] > 0.f) ? acc[i][j].y : 0.f);
 			pk[j] = *(const uint32_t*)&h;
 		}
 
@@ -557,12 +596,14 @@ __global__ void __launch_bounds__(WG_THREADS, 2) k_wgrad32(const bf16* __restric
 	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
 	const int ky = warp / 3, kx = warp % 3;
 
-	auto load = [&](long tile, int buf) {
-		const int x0 = (int)(tile % tx) * NET_TILE_X;
-		const int y0 = (int)((tile / tx) % ty) * NET_TILE_Y;
-		const long ibase = (tile / ((long)tx * ty)) * (long)X * Y;
-		const uint32_t sa = s0 + buf * STAGE, sg = sa + HALO * PIX;
+	NetWalk pos(blockIdx.x, gridDim.x, tx, ty);	// the tile to load next
 
+	auto load = [&](int buf) {
+		const int x0 = pos.x * NET_TILE_X, y0 = pos.y * NET_TILE_Y;
+		const long ibase = pos.z * ((long)X * Y);
+		const uint32_t sa = s0 + buf * STAGE, sg = sa + HALO * PIX;
+		pos.next();
+#pragma unroll
 		for (int i = threadIdx.x; i < HALO * 4; i += WG_THREADS) {
 
 			const int q = i & 3, pix = i >> 2;
@@ -571,6 +612,7 @@ __global__ void __launch_bounds__(WG_THREADS, 2) k_wgrad32(const bf16* __restric
 			cp_async16_zfill(sa + pix * PIX + q * 16, ok ? a + (ibase + (long)gy * X + gx) * NET_C + q * 8 : a, ok);
 		}
 
+#pragma unroll
 		for (int i = threadIdx.x; i < NET_TILE_X * NET_TILE_Y * 4; i += WG_THREADS) {
 
 			const int q = i & 3, pix = i >> 2;
@@ -604,21 +646,17 @@ __global__ void __launch_bounds__(WG_THREADS, 2) k_wgrad32(const bf16* __restric
 	int buf = 0;
 
 	if (blockIdx.x < ntiles)
-		load(blockIdx.x, 0);
+		load(0);
 
 	for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
 
-		if (tile + gridDim.x < ntiles) {
-
-			load(tile + gridDim.x, buf ^ 1);
-			asm volatile("cp.async.wait_group 1;\n" ::: "memory");
-
-		} else {
-
-			asm volatile("cp.async.wait_group 0;\n" ::: "memory");
-		}
-
+		// this tile has arrived and the other buffer has been read by all
+		asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 		__syncthreads();
+
+		if (tile + gridDim.x < ntiles)
+			load(buf ^ 1);
+
 		const uint32_t sa = s0 + buf * STAGE + aoff, sg = s0 + buf * STAGE + HALO * PIX + goff;
 #pragma unroll 2
 		for (int k = 0; k < NET_TILE_X * NET_TILE_Y / 16; k++) {
@@ -641,7 +679,6 @@ __global__ void __launch_bounds__(WG_THREADS, 2) k_wgrad32(const bf16* __restric
 			}
 		}
 
-		__syncthreads();	// before the next load overwrites this buffer
 		buf ^= 1;
 	}
 
@@ -691,12 +728,12 @@ __global__ void __launch_bounds__(32 * WT_WARPS) k_wgrad_thin(const bf16* __rest
 		acc[k] = make_float2(0.f, 0.f);
 
 	// work rows: 32 pixels of one image row; tx of them per image row
-	for (long row = (long)blockIdx.x * WT_WARPS + warp; row < nrows; row += (long)gridDim.x * WT_WARPS) {
+	NetWalk pos((long)blockIdx.x * WT_WARPS + warp, (long)gridDim.x * WT_WARPS, tx, Y);
 
-		const int x0 = (int)(row % tx) * NET_TILE_X;
-		const long iy = row / tx;			// image row over all images
-		const int y = (int)(iy % Y);
-		const long base = (iy - y) * X;
+	for (long row = (long)blockIdx.x * WT_WARPS + warp; row < nrows; row += (long)gridDim.x * WT_WARPS, pos.next()) {
+
+		const int x0 = pos.x * NET_TILE_X, y = pos.y;
+		const long base = pos.z * ((long)X * Y);
 		__syncwarp();
 
 		for (int i = lane; i < 3 * (NET_TILE_X + 2); i += 32) {
@@ -730,12 +767,9 @@ __global__ void __launch_bounds__(32 * WT_WARPS) k_wgrad_thin(const bf16* __rest
 				const int r0 = OUT6 ? 3 * (2 - d) + 2 : 3 * d;		// the tap that meets row d, column x - 1
 				const int r1 = OUT6 ? 3 * (2 - d) + 1 : 3 * d + 1;
 				const int r2 = OUT6 ? 3 * (2 - d) : 3 * d + 2;
-				acc[r0].x = fmaf(v, c0[d].x, acc[r0].x);
-				acc[r0].y = fmaf(v, c0[d].y, acc[r0].y);
-				acc[r1].x = fmaf(v, c1[d].x, acc[r1].x);
-				acc[r1].y = fmaf(v, c1[d].y, acc[r1].y);
-				acc[r2].x = fmaf(v, c2[d].x, acc[r2].x);
-				acc[r2].y = fmaf(v, c2[d].y, acc[r2].y);
+				acc[r0] = cfma(make_float2(v, v), c0[d], acc[r0]);
+				acc[r1] = cfma(make_float2(v, v), c1[d], acc[r1]);
+				acc[r2] = cfma(make_float2(v, v), c2[d], acc[r2]);
 			}
 
 			if (!OUT6)
