@@ -38,6 +38,7 @@ using namespace bn;
 // ----------------------------------------------------------------------------
 
 static thread_local std::string g_err;
+thread_local bool bn::g_chain = false;
 std::atomic<long> bn::g_launches{0};
 
 int bn::fail(int code, const char* fmt, ...)
@@ -696,7 +697,7 @@ static int cols(int n, int mode, const float2* in, long ies, long ios, int n_in,
 			TRY(prep_kernel(k_cols_toe512, smem));
 			dim3 grid((unsigned)((W + TOE512_B - 1) / TOE512_B), (unsigned)O);
 			cudaEvent_t pe = prof_begin("cols_toeplitz", st);
-			k_cols_toe512<<<grid, TOE512_B * 16, smem, st>>>(in, ies, ios, n_in, wrap_in, out, oes, oos, n_out,
+			launch_chained(k_cols_toe512, grid, TOE512_B * 16, smem, st, in, ies, ios, n_in, wrap_in, out, oes, oos, n_out,
 					wrap_out, W, psf, pes, pmod, pos, tw, done);
 			prof_end(pe, st);
 			LAUNCHED();
@@ -4025,7 +4026,7 @@ static int pics_iteration(bnufft_pics_s* ps, int it, cudaStream_t st)
 	if ((npp > ps->max_row_blocks) || (npap > ps->max_row_blocks))
 		return fail(BNUFFT_ERR_ARG, "internal: partial arrays too small");
 
-	k_cg_step<<<(unsigned)ps->nparts, RED_THREADS, 0, st>>>(ps->x, ps->r, p_cur, ps->part, ps->groups, ps->npix,
+	launch_chained(k_cg_step, (unsigned)ps->nparts, RED_THREADS, 0, st, ps->x, ps->r, p_cur, ps->part, ps->groups, ps->npix,
 			ps->conf.lambda, ps->scal, it, ps->pap_part, npap, ps->pp_part, npp, ps->rs_part, p_prev);
 	LAUNCHED();
 	return BNUFFT_OK;
@@ -4316,7 +4317,7 @@ static int pics_fcg_iteration(bnufft_pics_s* ps, int it, cudaStream_t st)
 		if (npap > ps->max_row_blocks)
 			return fail(BNUFFT_ERR_ARG, "internal: partial arrays too small");
 
-		k_fcg_step<<<nb, RED_THREADS, 0, st>>>(ps->x, ps->r, p, ps->ap_ring, 1, ps->part, ps->groups, ps->npix,
+		launch_chained(k_fcg_step, nb, RED_THREADS, 0, st, ps->x, ps->r, p, ps->ap_ring, 1, ps->part, ps->groups, ps->npix,
 				ps->conf.lambda, ps->scal, it, ps->pap_part, npap, ps->pp_part, ps->ndir, ps->pr_part, ps->ndir,
 				ps->rs_part);
 		LAUNCHED();
@@ -4336,7 +4337,7 @@ static int pics_fcg_iteration(bnufft_pics_s* ps, int it, cudaStream_t st)
 		LAUNCHED();
 	}
 
-	k_fcgm_dir<<<nb, RED_THREADS, 0, st>>>(p, ps->p_ring, ps->z, ps->r, ps->npix, ps->scal, it, ps->fcg_m, ring,
+	launch_chained(k_fcgm_dir, nb, RED_THREADS, 0, st, p, ps->p_ring, ps->z, ps->r, ps->npix, ps->scal, it, ps->fcg_m, ring,
 			ps->dots_part, folded ? ps->ndots : ps->nparts, ps->pr_part, ps->pp_part,
 			folded ? ps->rs_part : nullptr, ps->nparts);
 	LAUNCHED();
@@ -4348,7 +4349,7 @@ static int pics_fcg_iteration(bnufft_pics_s* ps, int it, cudaStream_t st)
 	if (npap > ps->max_row_blocks)
 		return fail(BNUFFT_ERR_ARG, "internal: partial arrays too small");
 
-	k_fcg_step<<<nb, RED_THREADS, 0, st>>>(ps->x, ps->r, p, ps->ap_ring, ring, ps->part, ps->groups, ps->npix,
+	launch_chained(k_fcg_step, nb, RED_THREADS, 0, st, ps->x, ps->r, p, ps->ap_ring, ring, ps->part, ps->groups, ps->npix,
 			ps->conf.lambda, ps->scal, it, ps->pap_part, npap, ps->pp_part, ps->nparts, ps->pr_part, ps->nparts,
 			ps->rs_part);
 	LAUNCHED();
@@ -4397,11 +4398,12 @@ static int capture_body(bnufft_pics_s* ps, cudaStream_t cap, cudaGraph_t body, c
 {
 	CUDA_TRY(cudaStreamBeginCaptureToGraph(cap, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
 	long before = g_launches.load();
+	ChainScope chain;
 	int s = pics_any_iteration(ps, -1, cap);
 
 	if (BNUFFT_OK == s) {
 
-		k_cg_advance<<<1, 1, 0, cap>>>(ps->scal, loop);
+		launch_chained(k_cg_advance, 1, 1, 0, cap, ps->scal, loop);
 		cudaError_t e = cudaGetLastError();
 
 		if (cudaSuccess != e)

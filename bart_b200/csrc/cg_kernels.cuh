@@ -184,11 +184,12 @@ __global__ void k_cg_start(CgScalars* st, const double* part, int nparts, float 
 // partial ||r||^2 for the next iteration's direction update. p is also
 // copied to p_keep (the next iteration's previous direction) when given.
 // The first element's inputs are loaded before the partial sums are.
-__global__ void k_cg_step(float2* __restrict__ x, float2* __restrict__ r, const float2* __restrict__ p,
-		const float2* __restrict__ part, int groups, long n, float lam, CgScalars* st, int it,
-		const double* __restrict__ pap_part, int npap, const double* __restrict__ pp_part, int npp,
-		double* __restrict__ rs_part, float2* __restrict__ p_keep)
+__global__ void k_cg_step(float2* x, float2* r, const float2* p,
+		const float2* part, int groups, long n, float lam, CgScalars* st, int it,
+		const double* pap_part, int npap, const double* pp_part, int npp,
+		double* rs_part, float2* p_keep)
 {
+	pdl_wait();
 	__shared__ double sh[96];
 	const long stride = (long)gridDim.x * blockDim.x;
 	long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -385,10 +386,11 @@ __global__ void k_fcgm_dots(const float2* __restrict__ z, const float2* __restri
 
 // direction: p = z - sum_q beta_q p_{it-w+q}; p into p_cur and ring slot
 // it % FCG_RING; partials <p, r> and ||p||^2 (lambda ||p||^2 in <p, A p>)
-__global__ void k_fcgm_dir(float2* __restrict__ p_cur, float2* __restrict__ p_ring, const float2* __restrict__ z,
-		const float2* __restrict__ r, long n, CgScalars* st, int it, int m, int ring, const double* __restrict__ dots,
-		int ndots, double* __restrict__ pr_part, double* __restrict__ pp_part, const double* __restrict__ rs_part, int nrs)
+__global__ void k_fcgm_dir(float2* p_cur, float2* p_ring, const float2* z,
+		const float2* r, long n, CgScalars* st, int it, int m, int ring, const double* dots,
+		int ndots, double* pr_part, double* pp_part, const double* rs_part, int nrs)
 {
+	pdl_wait();
 	__shared__ double sh[96];
 	__shared__ float beta[FCG_MAX_M];
 
@@ -477,11 +479,12 @@ __global__ void k_fcgm_dir(float2* __restrict__ p_cur, float2* __restrict__ p_ri
 // FCG step: <p, A p> (coil-sum row-pass partials + lambda ||p||^2), alpha =
 // <p, r> / <p, A p>; per element A p = sum_g part_g + lambda p (into ring
 // slot it % FCG_RING), x += alpha p, r -= alpha A p, partial ||r||^2.
-__global__ void k_fcg_step(float2* __restrict__ x, float2* __restrict__ r, const float2* __restrict__ p,
-		float2* __restrict__ ap_ring, int ring, const float2* __restrict__ part, int groups, long n, float lam, CgScalars* st, int it,
-		const double* __restrict__ pap_part, int npap, const double* __restrict__ pp_part, int npp,
-		const double* __restrict__ pr_part, int npr, double* __restrict__ rs_part)
+__global__ void k_fcg_step(float2* x, float2* r, const float2* p,
+		float2* ap_ring, int ring, const float2* part, int groups, long n, float lam, CgScalars* st, int it,
+		const double* pap_part, int npap, const double* pp_part, int npp,
+		const double* pr_part, int npr, double* rs_part)
 {
+	pdl_wait();
 	__shared__ double sh[96];
 	const long stride = (long)gridDim.x * blockDim.x;
 	long i = (long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -638,6 +641,7 @@ __global__ void k_norm_scalars(const float2* __restrict__ v, long n, CgScalars* 
 // counter and continue the enclosing while node unless converged or at maxiter.
 __global__ void k_cg_advance(CgScalars* st, cudaGraphConditionalHandle loop)
 {
+	pdl_wait();
 	int it = st->it + 1;
 	st->it = it;
 	cudaGraphSetConditional(loop, (!st->done && (it < st->maxiter)) ? 1u : 0u);

@@ -283,12 +283,13 @@ __device__ __forceinline__ double3 sum_partials3_d(const double* a, int na, cons
 // p^H (A^H A + lambda) p); every row multiplies by its coil's map and runs the
 // forward transform like k_rows_fwd.
 template <int L, int B, bool BLUE>
-__global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (B * L / 8) : 1) k_rows_fwd_cg(const float2* __restrict__ bvec, const float2* __restrict__ r,
-		const float2* __restrict__ p_prev, float2* __restrict__ p_cur, const float2* __restrict__ maps,
+__global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (B * L / 8) : 1) k_rows_fwd_cg(const float2* __restrict__ bvec, const float2* r,
+		const float2* p_prev, float2* p_cur, const float2* __restrict__ maps,
 		const float* __restrict__ ax, const float* __restrict__ ayz,
-		int X, long YZ, long R, float2* __restrict__ out, const float2* __restrict__ twg,
-		CgScalars* st, int it, const double* __restrict__ rs_part, int nrs, double* __restrict__ pp_part, Dft d)
+		int X, long YZ, long R, float2* out, const float2* __restrict__ twg,
+		CgScalars* st, int it, const double* rs_part, int nrs, double* pp_part, Dft d)
 {
+	pdl_wait();
 	using LAY = RowLayout<L, B>;
 	const int dn = BLUE ? d.n : L;	// logical DFT length (compile-time for the FFT itself)
 	constexpr int NT = B * L / 8;
@@ -420,10 +421,11 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 // One block: B rows, B*L/8 threads; a warp reads and writes consecutive
 // elements of one row straight from / into the FFT's registers.
 template <int L, int B, bool BLUE>
-__global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (B * L / 8) : 1) k_rows_fwd(const float2* __restrict__ img, const float2* __restrict__ maps,
+__global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (B * L / 8) : 1) k_rows_fwd(const float2* img, const float2* __restrict__ maps,
 		const float* __restrict__ ax, const float* __restrict__ ayz,
-		int X, long YZ, long R, float2* __restrict__ out, const float2* __restrict__ twg, const int* done, Dft d)
+		int X, long YZ, long R, float2* out, const float2* __restrict__ twg, const int* done, Dft d)
 {
+	pdl_wait();
 	using LAY = RowLayout<L, B>;
 	const int dn = BLUE ? d.n : L;	// logical DFT length (compile-time for the FFT itself)
 	constexpr int NT = B * L / 8;
@@ -496,11 +498,12 @@ __host__ __device__ constexpr bool cols_double_buffered(int MODE, bool BLUE, int
 }
 
 template <int L, int B, int MODE, bool BLUE>
-__global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (B * L / 8) : 1) k_cols(const float2* __restrict__ in, long ies, long ios, int n_in, int wrap_in,
-		float2* __restrict__ out, long oes, long oos, int n_out, int wrap_out,
+__global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (B * L / 8) : 1) k_cols(const float2* in, long ies, long ios, int n_in, int wrap_in,
+		float2* out, long oes, long oos, int n_out, int wrap_out,
 		int W, const float2* __restrict__ psf, long pes, long pmod, long pos,
 		const float2* __restrict__ twg, const int* done, Dft d)
 {
+	pdl_wait();
 	using LAY = ColLayout<L, B>;
 	const int dn = BLUE ? d.n : L;	// logical DFT length (compile-time for the FFT itself)
 	constexpr int NT = B * L / 8;
@@ -622,11 +625,12 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 //   else:      write out[x + X*yz + X*YZ*c] per coil.
 // grid (ceil(YZ/B), groups); coils per group cpg.
 template <int L, int B, bool BLUE, bool MAPS>
-__global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (B * L / 8) : 1) k_rows_inv(const float2* __restrict__ in, const float2* __restrict__ maps,
+__global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (B * L / 8) : 1) k_rows_inv(const float2* in, const float2* __restrict__ maps,
 		const float* __restrict__ ax, const float* __restrict__ ayz,
-		int X, long YZ, int C, int cpg, float2* __restrict__ out, const float2* __restrict__ twg,
-		const float2* __restrict__ pdot, double* __restrict__ dot_part, const int* done, Dft d)
+		int X, long YZ, int C, int cpg, float2* out, const float2* __restrict__ twg,
+		const float2* pdot, double* dot_part, const int* done, Dft d)
 {
+	pdl_wait();
 	using LAY = RowLayout<L, B>;
 	const int dn = BLUE ? d.n : L;	// logical DFT length (compile-time for the FFT itself)
 	constexpr int NT = B * L / 8;

@@ -4,6 +4,8 @@
 #pragma once
 
 #include <atomic>
+#include <utility>
+
 #include <cuda_runtime.h>
 
 #include "../../include/bnufft.h"
@@ -29,6 +31,39 @@ template <typename K>
 int prep_kernel(K kernel, size_t)
 {
 	return opt_in_smem((const void*)kernel);
+}
+
+// While a solver's loop body is captured (by this thread), its kernels are
+// launched so that one may start while the previous one drains (pdl_wait).
+extern thread_local bool g_chain;
+
+struct ChainScope {
+
+	bool before;
+	ChainScope() : before(g_chain) { g_chain = true; }
+	~ChainScope() { g_chain = before; }
+};
+
+template <typename... P, typename... A>
+void launch_chained(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args)
+{
+	if (!g_chain) {
+
+		kern<<<grid, block, smem, st>>>(std::forward<A>(args)...);
+		return;
+	}
+
+	cudaLaunchAttribute at = {};
+	at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+	at.val.programmaticStreamSerializationAllowed = 1;
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = grid;
+	cfg.blockDim = block;
+	cfg.dynamicSmemBytes = smem;
+	cfg.stream = st;
+	cfg.attrs = &at;
+	cfg.numAttrs = 1;
+	cudaLaunchKernelEx(&cfg, kern, P(args)...);
 }
 
 } // namespace bn

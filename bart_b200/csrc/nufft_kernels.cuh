@@ -30,11 +30,12 @@ enum { KB_TABLE_N = 1000 };	// kb_size_max, src/noncart/grid.c:38
 // barrier for the twiddle table and the one between the two transforms.
 enum { TOE512_B = 16 };
 
-__global__ void __launch_bounds__(TOE512_B * 16, 2) k_cols_toe512(const float2* __restrict__ in, long ies, long ios,
-		int n_in, int wrap_in, float2* __restrict__ out, long oes, long oos, int n_out, int wrap_out,
+__global__ void __launch_bounds__(TOE512_B * 16, 2) k_cols_toe512(const float2* in, long ies, long ios,
+		int n_in, int wrap_in, float2* out, long oes, long oos, int n_out, int wrap_out,
 		int W, const float2* __restrict__ psf, long pes, long pmod, long pos,
 		const float2* __restrict__ twg, const int* done)
 {
+	pdl_wait();
 	constexpr int L = 512, SB = TOE512_B;
 	extern __shared__ float2 smem[];
 	float2* s = smem;

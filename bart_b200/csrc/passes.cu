@@ -16,7 +16,7 @@ int launch_rows_fwd_LB(const float2* img, const float2* maps, const float* ax, c
 	auto kern = (d.n == L) ? k_rows_fwd<L, B, false> : k_rows_fwd<L, B, true>;
 	TRY(prep_kernel(kern, smem));
 	cudaEvent_t pe = prof_begin("rows_fwd", st);
-	kern<<<(unsigned)((R + B - 1) / B), B * L / 8, smem, st>>>(img, maps, ax, ayz, X, YZ, R, out, tw, done, d);
+	launch_chained(kern, (unsigned)((R + B - 1) / B), B * L / 8, smem, st, img, maps, ax, ayz, X, YZ, R, out, tw, done, d);
 	prof_end(pe, st);
 	LAUNCHED();
 	return BNUFFT_OK;
@@ -42,7 +42,7 @@ int launch_cols_LB(const float2* in, long ies, long ios, int n_in, int wrap_in,
 
 	dim3 grid((unsigned)((W + B - 1) / B), (unsigned)O);
 	cudaEvent_t pe = prof_begin((2 == MODE) ? "cols_toeplitz" : ((1 == MODE) ? "cols_inv" : "cols_fwd"), st);
-	kern<<<grid, B * L / 8, smem, st>>>(in, ies, ios, n_in, wrap_in, out, oes, oos, n_out, wrap_out,
+	launch_chained(kern, grid, B * L / 8, smem, st, in, ies, ios, n_in, wrap_in, out, oes, oos, n_out, wrap_out,
 			W, psf, pes, pmod, pos, tw, done, d);
 	prof_end(pe, st);
 	LAUNCHED();
@@ -63,7 +63,7 @@ int launch_rows_inv_LB(const float2* in, const float2* maps, const float* ax, co
 	TRY(prep_kernel(kern, smem));
 	dim3 grid((unsigned)((YZ + B - 1) / B), (unsigned)groups);
 	cudaEvent_t pe = prof_begin("rows_inv", st);
-	kern<<<grid, B * L / 8, smem, st>>>(in, maps, ax, ayz, X, YZ, C, cpg, out, tw, pdot, dot_part, done, d);
+	launch_chained(kern, grid, B * L / 8, smem, st, in, maps, ax, ayz, X, YZ, C, cpg, out, tw, pdot, dot_part, done, d);
 	prof_end(pe, st);
 	LAUNCHED();
 	return BNUFFT_OK;
@@ -80,7 +80,7 @@ int launch_rows_fwd_cg_LB(const float2* bvec, const float2* r, const float2* p_p
 	auto kern = (d.n == L) ? k_rows_fwd_cg<L, B, false> : k_rows_fwd_cg<L, B, true>;
 	TRY(prep_kernel(kern, smem));
 	cudaEvent_t pe = prof_begin("rows_fwd", st);
-	kern<<<(unsigned)((R + B - 1) / B), B * L / 8, smem, st>>>(bvec, r, p_prev, p_cur, maps, ax, ayz,
+	launch_chained(kern, (unsigned)((R + B - 1) / B), B * L / 8, smem, st, bvec, r, p_prev, p_cur, maps, ax, ayz,
 			X, YZ, R, out, tw, stt, it, rs_part, nrs, pp_part, d);
 	prof_end(pe, st);
 	LAUNCHED();
