@@ -1069,6 +1069,24 @@ static int init_rolloff(OpCtx& op, cudaStream_t st)
 	return BNUFFT_OK;
 }
 
+// Whether the forward grid of C channels holds four channels of a cell side by
+// side (k_degrid6_by4): volumes whose z transform runs on 16 columns a block
+// (4 x-cells of 4 coils: 32-byte pieces in, whole lines out). 2D gathers are
+// short beside their transforms and keep the plain grid. 128^3, 8 coils, 5.12 M
+// samples, forward and adjoint: 11.87 ms so, 13.21 ms on the plain grid.
+static bool grid_by4(const OpCtx& op, long C)
+{
+	const int n = op.g.G[2];
+	SmoothPlan sp;
+	Dft d;
+	int L;
+
+	if (!op.bins.quads || (1 == n) || (0 != C % 4) || (C / 4 > 65535) || smooth_plan(n, &sp))
+		return false;
+
+	return (BNUFFT_OK == get_dft(n, &d, &L)) && (d.n == L) && (L >= 16) && (L <= 512);
+}
+
 // column passes of the forward spectrum: row-transformed t1 -> grid
 static int op_spectrum_cols(OpCtx& op, long C, float2* grid, cudaStream_t st)
 {
@@ -1090,6 +1108,15 @@ static int op_spectrum_cols(OpCtx& op, long C, float2* grid, cudaStream_t st)
 			op.w.t2, g.G[0], (long)g.G[0] * g.G[1], g.G[1], 0, g.G[0], (long)g.N[2] * C, nullptr, 0, 1, 0, st));
 
 	long plane = (long)g.G[0] * g.G[1];
+
+	if (grid_by4(op, C)) {
+
+		Dft d;
+		int L;
+		TRY(get_dft(g.G[2], &d, &L));
+		return pass_table(L)->cols(L, 16, 3, op.w.t2, plane, plane * g.N[2], g.N[2], 1,
+				grid, plane, plane * g.G[2], g.G[2], 0, (int)plane, C / 4, nullptr, 0, 1, 0, nullptr, st, d);
+	}
 
 	return cols(g.G[2], 0, op.w.t2, plane, plane * g.N[2], g.N[2], 1,
 			grid, plane, plane * g.G[2], g.G[2], 0, (int)plane, C, nullptr, 0, 1, 0, st);
@@ -1165,7 +1192,10 @@ static int degrid(OpCtx& op, const float2* grid, long C, float2* ksp, cudaStream
 
 		const dim3 blocks((unsigned)nb, (unsigned)((C + cpb - 1) / cpb));
 
-		if (op.g.G[2] > 1)
+		if (grid_by4(op, C))
+			k_degrid6_by4<<<blocks, BIN_THREADS, 0, st>>>(b.foot, b.perm, M, grid_geom(op.g), (int)C, cpb, grid, ksp,
+					op.wgt, (int)op.wgt_c);
+		else if (op.g.G[2] > 1)
 			k_degrid6_quads<6><<<blocks, BIN_THREADS, 0, st>>>(b.foot, b.perm, M, grid_geom(op.g), (int)C, cpb, grid, ksp,
 					op.wgt, (int)op.wgt_c);
 		else

@@ -517,18 +517,19 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 	for (int i = threadIdx.x; i < L; i += NT)
 		tw[i] = twg[i];
 
-	const int cx = blockIdx.x * B + LAY::seq();
+	constexpr bool BY4 = (3 == MODE), FWD = (0 == MODE) || BY4;
+	const int cx = BY4 ? blockIdx.x * (B / 4) + LAY::seq() % (B / 4) : blockIdx.x * B + LAY::seq();
 	const bool valid = (cx < W);
-	const long o = blockIdx.y;
+	const long o = BY4 ? 4 * (long)blockIdx.y + LAY::seq() / (B / 4) : blockIdx.y;
 	const float2* inp = in + o * ios + cx;
 
 	// the input side holds reg_pos positions, the spectrum side out_pos ones:
 	// MODE 0 loads the former and stores the latter, MODE 1 the reverse, MODE 2
 	// loads and stores the former
 	constexpr int NW = out_regs(L, BLUE);
-	constexpr int NI = (1 == MODE) ? NW : 8, NO = (0 == MODE) ? NW : 8;
+	constexpr int NI = (1 == MODE) ? NW : 8, NO = FWD ? NW : 8;
 	auto ipos = [](int m) { return (1 == MODE) ? out_pos<L, LAY, BLUE>(m) : reg_pos<L, LAY>(m); };
-	auto opos = [](int m) { return (0 == MODE) ? out_pos<L, LAY, BLUE>(m) : reg_pos<L, LAY>(m); };
+	auto opos = [](int m) { return FWD ? out_pos<L, LAY, BLUE>(m) : reg_pos<L, LAY>(m); };
 	float2 x[NI], y[NO];
 #pragma unroll
 	for (int m = 0; m < NI; m++) {
@@ -543,7 +544,7 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 
 	const bool half = wrap_in && (2 * n_in <= L);
 
-	if constexpr (MODE == 0) {
+	if constexpr (FWD) {
 
 		dft_fwd<L, LAY, BLUE>(x, y, s, tw, d, half);
 
@@ -599,7 +600,8 @@ __global__ void __launch_bounds__(B * L / 8, (1024 / (B * L / 8)) > 0 ? 1024 / (
 		dft_inv<L, LAY, BLUE>(w, y, s, tw, d);
 	}
 
-	float2* outp = out + o * oos + cx;
+	float2* outp = BY4 ? out + 4 * (blockIdx.y * oos + cx) + o % 4 : out + o * oos + cx;
+	oes *= BY4 ? 4 : 1;
 
 	if (valid) {
 #pragma unroll

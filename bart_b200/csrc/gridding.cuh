@@ -656,6 +656,110 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* 
 	}
 }
 
+// Degridding from a grid with four channels of a cell side by side (32 bytes;
+// written so by the last column pass): lane q of a sample's quad takes channels
+// 2 (q & 1) and the next one, of the even or odd x taps (q >> 1), so a row is
+// three 64-byte accesses for four channels, without the window's unused cells
+// and mostly within one cache line: 27 lines per sample and channel instead
+// of 50 (the gather is bound by the L1's lines per request).
+template <int NP>
+__device__ __forceinline__ void degrid6_by4(const float4* __restrict__ gp, long plane, const float* __restrict__ f,
+		const int (&zoff)[6], const int (&row)[6], const float (&wy)[6], const int (&xo)[3], const float (&wx)[3],
+		float2 (&acc)[NP][2])
+{
+#pragma unroll
+	for (int p = 0; p < NP; p++)
+		acc[p][0] = acc[p][1] = make_float2(0.f, 0.f);
+#pragma unroll 1
+	for (int a = 0; a < 6; a++) {
+
+		const float dz = f[16 + a];
+		int zo = zoff[0];
+#pragma unroll
+		for (int k = 1; k < 6; k++)
+			zo = (k == a) ? zoff[k] : zo;
+#pragma unroll
+		for (int b = 0; b < 6; b++) {
+
+			const float dzy = __fmul_rn(dz, wy[b]);
+			const float4* r = gp + 2 * (long)(zo + row[b]);
+#pragma unroll
+			for (int k = 0; k < 3; k++) {
+
+				const float d = __fmul_rn(dzy, wx[k]);
+#pragma unroll
+				for (int p = 0; p < NP; p++) {
+
+					const float4 v = r[plane * p + xo[k]];
+					acc[p][0] = cfma(make_float2(v.x, v.y), make_float2(d, d), acc[p][0]);
+					acc[p][1] = cfma(make_float2(v.z, v.w), make_float2(d, d), acc[p][1]);
+				}
+			}
+		}
+	}
+}
+
+__global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_by4(const float4* __restrict__ foot,
+		const int* __restrict__ perm, long M, GridGeom g, int C, int cpb, const float2* __restrict__ grid,
+		float2* __restrict__ ksp, const float2* __restrict__ wgt, int wgt_c)
+{
+	const int q = threadIdx.x & 3, h = q & 1, odd = q >> 1;
+	const long s = ((long)blockIdx.x * BIN_THREADS + threadIdx.x) / 4;
+	const long i = min(s, M - 1);		// surplus quads repeat the last sample and write nothing
+	const long m = perm[i];
+	const float4 lo = foot[i * FOOT_F4];
+	const float* f = (const float*)(foot + i * FOOT_F4);
+	int zoff[6], row[6], xo[3];
+	float wy[6], wx[3];
+#pragma unroll
+	for (int t = 0; t < 6; t++) {
+
+		row[t] = cell_of(__float_as_int(lo.y) + t, g.N[1], g.G[1], g.periodic) * g.G[0];
+		zoff[t] = cell_of(__float_as_int(lo.z) + t, g.N[2], g.G[2], g.periodic) * g.G[1] * g.G[0];
+		wy[t] = f[10 + t];
+	}
+#pragma unroll
+	for (int k = 0; k < 3; k++) {
+
+		xo[k] = 2 * cell_of(__float_as_int(lo.x) + 2 * k + odd, g.N[0], g.G[0], g.periodic);
+		wx[k] = f[4 + 2 * k + odd];
+	}
+
+	const int c1 = min(C, (int)blockIdx.y * cpb + cpb);
+	const long plane = 2 * g.gsz;		// in 16-byte words
+
+	// the quad's two halves of a sum are exchanged: lane q keeps channel 2 h + odd
+	auto store = [&](const float2 (&a)[2], int c) {
+		float2 r = cadd(odd ? a[1] : a[0], shfl_xor2(odd ? a[0] : a[1], 2));
+		c += 2 * h + odd;
+
+		if (s < M) {
+
+			if (wgt)
+				r = cmul(r, wgt[m + M * (c % wgt_c)]);
+
+			ksp[m + M * c] = r;
+		}
+	};
+
+	int c = blockIdx.y * cpb;
+
+	for (; c + 7 < c1; c += 8) {
+
+		float2 acc[2][2];
+		degrid6_by4<2>((const float4*)grid + plane * (c / 4) + h, plane, f, zoff, row, wy, xo, wx, acc);
+		store(acc[0], c);
+		store(acc[1], c + 4);
+	}
+
+	if (c < c1) {
+
+		float2 acc[1][2];
+		degrid6_by4<1>((const float4*)grid + plane * (c / 4) + h, plane, f, zoff, row, wy, xo, wx, acc);
+		store(acc[0], c);
+	}
+}
+
 // Gridding, width 6, with global atomics: a quad per sample in bin order as in
 // the degridding, one 16-byte reduction (two cells) per lane and tap row, so a
 // quad's reductions of a row fall into one 64-byte piece of the grid. Bound by

@@ -27,26 +27,37 @@ int launch_cols_LB(const float2* in, long ies, long ios, int n_in, int wrap_in,
 		float2* out, long oes, long oos, int n_out, int wrap_out, int W, long O,
 		const float2* psf, long pes, long pmod, long pos, const int* done, cudaStream_t st, const Dft& d)
 {
-	const float2* tw;
-	TRY(get_twiddles(L, &tw));
-	size_t smem = pass_smem(L, B);
+	if constexpr ((3 == MODE) && (16 != B)) {
 
-	if ((d.n == L) && cols_double_buffered(MODE, false, L, B))
-		smem += sizeof(float2) * (size_t)L * (size_t)smem_stride(B);	// the second exchange buffer
+		return fail(BNUFFT_ERR_ARG, "internal: outputs by four images take 16 columns a block");
 
-	auto kern = (d.n == L) ? k_cols<L, B, MODE, false> : k_cols<L, B, MODE, true>;
-	TRY(prep_kernel(kern, smem));
+	} else {
 
-	if (O > 65535)
-		return fail(BNUFFT_ERR_UNSUPPORTED, "column pass with %ld outer sequences", O);
+		const float2* tw;
+		TRY(get_twiddles(L, &tw));
+		size_t smem = pass_smem(L, B);
 
-	dim3 grid((unsigned)((W + B - 1) / B), (unsigned)O);
-	cudaEvent_t pe = prof_begin((2 == MODE) ? "cols_toeplitz" : ((1 == MODE) ? "cols_inv" : "cols_fwd"), st);
-	launch_chained(kern, grid, B * L / 8, smem, st, in, ies, ios, n_in, wrap_in, out, oes, oos, n_out, wrap_out,
-			W, psf, pes, pmod, pos, tw, done, d);
-	prof_end(pe, st);
-	LAUNCHED();
-	return BNUFFT_OK;
+		if ((d.n == L) && cols_double_buffered(MODE, false, L, B))
+			smem += sizeof(float2) * (size_t)L * (size_t)smem_stride(B);	// the second exchange buffer
+
+		auto kern = k_cols<L, B, MODE, false>;
+
+		if constexpr (3 != MODE)
+			kern = (d.n == L) ? kern : k_cols<L, B, MODE, true>;
+
+		TRY(prep_kernel(kern, smem));
+
+		if (O > 65535)
+			return fail(BNUFFT_ERR_UNSUPPORTED, "column pass with %ld outer sequences", O);
+
+		dim3 grid((unsigned)((3 == MODE) ? (W + B / 4 - 1) / (B / 4) : (W + B - 1) / B), (unsigned)O);
+		cudaEvent_t pe = prof_begin((2 == MODE) ? "cols_toeplitz" : ((1 == MODE) ? "cols_inv" : "cols_fwd"), st);
+		launch_chained(kern, grid, B * L / 8, smem, st, in, ies, ios, n_in, wrap_in, out, oes, oos, n_out, wrap_out,
+				W, psf, pes, pmod, pos, tw, done, d);
+		prof_end(pe, st);
+		LAUNCHED();
+		return BNUFFT_OK;
+	}
 }
 
 template <int L, int B>
@@ -131,7 +142,7 @@ int cols(int L, int B, int mode, const float2* in, long ies, long ios, int n_in,
 		long oos, int n_out, int wrap_out, int W, long O, const float2* psf, long pes, long pmod, long pos,
 		const int* done, cudaStream_t st, const Dft& d)
 {
-	auto f = (0 == mode) ? cols_mode<0> : ((1 == mode) ? cols_mode<1> : cols_mode<2>);
+	auto f = (0 == mode) ? cols_mode<0> : ((1 == mode) ? cols_mode<1> : ((2 == mode) ? cols_mode<2> : cols_mode<3>));
 	return f(L, B, in, ies, ios, n_in, wrap_in, out, oes, oos, n_out, wrap_out, W, O, psf, pes, pmod, pos, done, st, d);
 }
 

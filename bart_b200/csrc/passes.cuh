@@ -6,7 +6,8 @@
 
 namespace bn {
 
-// L: FFT length, B: sequences per block; mode: 0 forward, 1 inverse, 2 Toeplitz
+// L: FFT length, B: sequences per block; mode: 0 forward, 1 inverse, 2 Toeplitz, 3
+// forward with the outputs of four outer sequences (coils) side by side (O: fours)
 struct PassTable {
 
 	int (*rows_fwd)(int L, int B, const float2* img, const float2* maps, const float* ax, const float* ayz, int X, long YZ,
