@@ -373,7 +373,7 @@ def test_gridding_edges_vs_oracle(dims, samples, spokes, coils, periodic, weight
 @pytest.mark.parametrize("dims,coils,periodic,weights", [
     ((8, 8, 8), 4, False, False),       # the shortest z transform, one group of four
     ((10, 14, 16), 8, True, True),      # two groups at once, wrapping around, weights
-    ((9, 22, 32), 12, False, True),     # two groups and one more, odd image side
+    ((18, 22, 32), 12, False, True),     # two groups and one more
     ((16, 12, 96), 20, False, False),   # a mixed z length, several groups
     ((12, 10, 64), 6, True, False)])    # coils not in fours: the plain grid
 def test_forward_of_coil_fours_vs_oracle(dims, coils, periodic, weights):
