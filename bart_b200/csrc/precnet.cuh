@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(NET_THREADS) k_conv32(const bf16* __restrict__
 // vector read from shared memory serves four pixels. (One thread per pixel
 // read or wrote sixteen lines per warp access and reloaded the weights for
 // every pixel: seven 256^2 images took 34 us in layer 1, 54 us in layer 6 and
-// 52 us in its backward pass.) Blocks cover 256 pixels.
+// 52 us in its backward pass; 25, 42 and 33 us so.) Blocks cover 256 pixels.
 struct NetPix {
 
 	long p0;		// first of the quad's pixels
@@ -562,11 +562,11 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out_bwd(const float2* __res
 // Per tile of 32 x 8 pixels the gradient rows and the activations' halo lie
 // in shared memory pixel by pixel; ldmatrix.trans reads both as MMA operands
 // with the pixels as K. Warp w owns tap w: its 32 x 32 sums are 32 registers.
-// The next tile arrives by cp.async while this one is summed. Bound by the
-// tile traffic (1.33 x 64 + 64 B per pixel) and shared-memory reads; the
-// FP32-pipe kernel it replaces took two shared-memory loads per FMA (1019 us
-// per layer of seven 256^2 images; their whole gradient pass 5.37 -> 0.74 ms,
-// with the thin layers and the reduction below).
+// The next tile arrives by cp.async while this one is summed, one barrier per
+// tile. Bound by the mma.sync rate (half of the tensor cycles at 39 us a layer of
+// seven 256^2 images); the FP32-pipe kernel it replaced took two shared-memory
+// loads per FMA (1019 us a layer; the whole forward and gradient pass 5.37 ms
+// then, 0.65 ms now).
 constexpr int WG_WARPS = 9;
 constexpr int WG_THREADS = 32 * WG_WARPS;
 constexpr int WG_STAGE = (NET_HALO_X * NET_HALO_Y + NET_TILE_X * NET_TILE_Y) * NET_SA_STRIDE;	// bf16 per buffer
