@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(NET_THREADS) k_conv32(const bf16* __restrict__
 // vector read from shared memory serves four pixels. (One thread per pixel
 // read or wrote sixteen lines per warp access and reloaded the weights for
 // every pixel: seven 256^2 images took 34 us in layer 1, 54 us in layer 6 and
-// 52 us in its backward pass; 25, 42 and 33 us so.) Blocks cover 256 pixels.
+// 52 us in its backward pass; 27, 37 and 33 us so.) Blocks cover 256 pixels.
 struct NetPix {
 
 	long p0;		// first of the quad's pixels
@@ -391,14 +391,14 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out(const bf16* __restrict_
 		int nnorm, const float2* zc, float2* out, const float2* __restrict__ pdot, double* __restrict__ dot_part,
 		const int* done, const int* net_off)
 {
-	__shared__ __align__(16) float sw[2 * 9 * NET_C + 2];	// [tap][channel][output], then the biases
+	__shared__ __align__(16) float sw[2 * 9 * NET_C + 2];
 	__shared__ double red[32];
 
 	if (done && *done)
 		return;
 
 	for (int i = threadIdx.x; i < 2 * 9 * NET_C + 2; i += NET_THREADS)
-		sw[i] = (i < 2 * 9 * NET_C) ? w[(i % 2) * 9 * NET_C + i / 2] : b[i - 2 * 9 * NET_C];
+		sw[i] = (i < 2 * 9 * NET_C) ? w[i] : b[i - 2 * 9 * NET_C];
 
 	const float s = scale ? *scale : (norm_part ? (float)sqrt(sum_partials_d(norm_part, nnorm, red)) : 1.f);
 	__syncthreads();
@@ -425,20 +425,24 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out(const bf16* __restrict_
 				u[i] = px.has(i, tap) ? *(const uint4*)(nb + i * NET_C) : make_uint4(0u, 0u, 0u, 0u);
 			}
 
-			float2 wa[4], wb[4];	// channels 0-3 and 4-7 of the lane
-			net_lds8(sw + 2 * (tap * NET_C + 8 * px.q), wa);
-			net_lds8(sw + 2 * (tap * NET_C + 8 * px.q) + 8, wb);
+			// (pairs of outputs in two-wide sums would spend the instructions
+			// saved on doubling the activations: 42 against 37 us)
+			float2 w0[4], w1[4];
+			net_lds8(sw + tap * NET_C + 8 * px.q, w0);
+			net_lds8(sw + 9 * NET_C + tap * NET_C + 8 * px.q, w1);
 #pragma unroll
 			for (int i = 0; i < 4; i++) {
 
 				float f[8];
 				net_bf16x8(u[i], f);
 #pragma unroll
-				for (int c = 0; c < 4; c++)
-					acc[i] = cfma(wa[c], make_float2(f[c], f[c]), acc[i]);
-#pragma unroll
-				for (int c = 0; c < 4; c++)
-					acc[i] = cfma(wb[c], make_float2(f[4 + c], f[4 + c]), acc[i]);
+				for (int c = 0; c < 4; c++) {
+
+					acc[i].x = fmaf(w0[c].x, f[2 * c], acc[i].x);
+					acc[i].y = fmaf(w1[c].x, f[2 * c], acc[i].y);
+					acc[i].x = fmaf(w0[c].y, f[2 * c + 1], acc[i].x);
+					acc[i].y = fmaf(w1[c].y, f[2 * c + 1], acc[i].y);
+				}
 			}
 		}
 
@@ -563,10 +567,10 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out_bwd(const float2* __res
 // in shared memory pixel by pixel; ldmatrix.trans reads both as MMA operands
 // with the pixels as K. Warp w owns tap w: its 32 x 32 sums are 32 registers.
 // The next tile arrives by cp.async while this one is summed, one barrier per
-// tile. Bound by the mma.sync rate (half of the tensor cycles at 39 us a layer of
+// tile. Bound by the mma.sync rate (half of the tensor cycles at 42 us a layer of
 // seven 256^2 images); the FP32-pipe kernel it replaced took two shared-memory
 // loads per FMA (1019 us a layer; the whole forward and gradient pass 5.37 ms
-// then, 0.65 ms now).
+// then, 0.64 ms now).
 constexpr int WG_WARPS = 9;
 constexpr int WG_THREADS = 32 * WG_WARPS;
 constexpr int WG_STAGE = (NET_HALO_X * NET_HALO_Y + NET_TILE_X * NET_TILE_Y) * NET_SA_STRIDE;	// bf16 per buffer
@@ -713,7 +717,7 @@ __global__ void __launch_bounds__(WG_THREADS, 2) k_wgrad32(const bf16* __restric
 constexpr int WT_WARPS = 8;
 
 template <bool OUT6>
-__global__ void __launch_bounds__(32 * WT_WARPS) k_wgrad_thin(const bf16* __restrict__ w, const float2* __restrict__ t,
+__global__ void __launch_bounds__(32 * WT_WARPS, 4) k_wgrad_thin(const bf16* __restrict__ w, const float2* __restrict__ t,
 		int X, int Y, int tx, long nrows, float* __restrict__ part)
 {
 	constexpr int O = 2 * 9 * NET_C;
