@@ -1578,10 +1578,10 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 	b.tg_cfg = -1;
 
 	// measured on B200: it wins for multi-channel problems (8-coil 128^3
-	// kooshball: 10.5 against 28.2 ms; 16-coil 256^2 radial: 122 against
-	// 144 us), while single-channel problems (little work per candidate
-	// sample) are faster with the global-atomic scatter (256^2, 402 spokes:
-	// 55 against 122 us); BNUFFT_GRIDDING=lines selects it everywhere
+	// kooshball: 5.9 against 18.4 ms; 16-coil 256^2 radial: 55 against
+	// 79 us), while single-channel problems (little work per listed hit)
+	// are faster with the quads' reductions (256^2, 402 spokes: 30 against
+	// 55 us); BNUFFT_GRIDDING=lines selects it everywhere
 	// (deterministic: tiles for single channels too, and of one shape, so that a
 	// channel's sums do not depend on how many are gridded at once)
 	const bool tg_want = (2 == gridding_kind()) ? (det || (op.coils >= 2)) : (3 == gridding_kind());
@@ -1971,6 +1971,28 @@ static bool on_device(const void* p)
 	}
 
 	return (cudaMemoryTypeDevice == a.type) || (cudaMemoryTypeManaged == a.type);
+}
+
+// The device's default pool returns unused memory at every host
+// synchronisation, and a new plan's first call would map its work space again:
+// plans let the pool keep up to this much, a few volumes' worth (set-ups with
+// auxiliary streams, which allocate per model, let it keep all). 200 x 180, 12
+// coils: first call of a new plan 430 -> 216 us, creation 1.9 -> 1.2 ms.
+static void keep_in_pool()
+{
+	const uint64_t keep = 4UL << 30;
+	uint64_t now = 0;
+	int dev;
+	cudaMemPool_t pool;
+
+	if ((cudaSuccess == cudaGetDevice(&dev)) && (cudaSuccess == cudaDeviceGetDefaultMemPool(&pool, dev))
+	    && (cudaSuccess == cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &now)) && (now < keep)) {
+
+		uint64_t k = keep;
+		cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &k);
+	}
+
+	cudaGetLastError();
 }
 
 // per thread and device: an auxiliary compute stream with a fork / join
@@ -2442,6 +2464,8 @@ extern "C" int bnufft_create2(bnufft_plan_t* plan, int N, const long ksp_dims[],
 
 	if ((N < 4) || (nullptr == traj))
 		return fail(BNUFFT_ERR_ARG, "need N >= 4 dims and a trajectory");
+
+	keep_in_pool();
 
 	// subspace basis [1, 1, 1, 1, 1, T, K] (nufft_set_traj,
 	// src/noncart/nufft.c:1018-1042): cim [X, Y, Z, ..., 1 (TE), K (COEFF)],
