@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(NET_THREADS) k_conv32(const bf16* __restrict__
 // vector read from shared memory serves four pixels. (One thread per pixel
 // read or wrote sixteen lines per warp access and reloaded the weights for
 // every pixel: seven 256^2 images took 34 us in layer 1, 54 us in layer 6 and
-// 52 us in its backward pass; 27, 37 and 33 us so.) Blocks cover 256 pixels.
+// 52 us in its backward pass; 25, 37 and 33 us so.) Blocks cover 256 pixels.
 struct NetPix {
 
 	long p0;		// first of the quad's pixels
@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out_bwd(const float2* __res
 // in shared memory pixel by pixel; ldmatrix.trans reads both as MMA operands
 // with the pixels as K. Warp w owns tap w: its 32 x 32 sums are 32 registers.
 // The next tile arrives by cp.async while this one is summed, one barrier per
-// tile. Bound by the mma.sync rate (half of the tensor cycles at 42 us a layer of
+// tile. Bound by the mma.sync rate (half of the tensor cycles at 39 us a layer of
 // seven 256^2 images); the FP32-pipe kernel it replaced took two shared-memory
 // loads per FMA (1019 us a layer; the whole forward and gradient pass 5.37 ms
 // then, 0.64 ms now).
