@@ -429,6 +429,28 @@ def test_grid_lengths_vs_oracle(dims, coils):
     assert rel(nrm, o.normal_toeplitz(x)) < TOL
 
 
+@pytest.mark.parametrize("N", [96, 160, 192, 224])
+def test_mixed_lengths_are_as_exact_as_their_roundings(N):
+    """Toeplitz normal on sides of 2N = 192, 320, 384 and 448 points (no
+    embedding) against the float64 oracle, tighter than TOL: the transforms of
+    the mixed lengths round no more often than their stages do. With u = 2^-24
+    a float32 transform of L points with rounded twiddles has an rms error of
+    about 0.7 u sqrt(log2 L). The normal has four of them along the two axes,
+    the PSF four more (of 2L points) and its 36-product sums, about 2 u: together
+    u sqrt(8 * 0.49 log2 L + 4), at most 2.12 u sqrt(log2 L) here. Bound: a tenth
+    more, 2.35."""
+    rng = np.random.default_rng(N)
+    ang = np.arange(60) * np.pi * (np.sqrt(5.0) - 1.0) / 2.0
+    r = ((np.arange(2 * N) + 0.5) / (2 * N) - 0.5) * N
+    t = np.stack([r[:, None] * np.cos(ang), r[:, None] * np.sin(ang), 0.0 * r[:, None] * ang]).astype(np.complex64)
+    op = nufft_create2([1, 2 * N, 60, 4], [N, N, 1, 4], list(t.shape), t, conf=NufftConf(toeplitz=True, deterministic=True))
+    x = (rng.standard_normal((N, N, 1, 4)) + 1j * rng.standard_normal((N, N, 1, 4))).astype(np.complex64)
+    y = np.asarray(op.normal(x)).copy()
+    op.free()
+    want = orc.NufftOracle(t.real.reshape(3, -1, order="F"), (N, N, 1)).normal_toeplitz(x)
+    assert rel(y, want) < 2.35 * 2.0 ** -24 * np.sqrt(np.log2(2 * N))
+
+
 @pytest.mark.parametrize("name", ["nufft2d_n64_chain", "nufft2d_n64_chain_weights", "nufft3d_n16_chain"])
 def test_chain_vs_reference(name):
     """Oversampling other than 2 (nufft -o 1.25 / 1.5 / 2.5: the reference's
