@@ -3242,7 +3242,7 @@ struct bnufft_precnet_s {
 	float *m = nullptr, *v = nullptr, *grad = nullptr;	// Adam moments, gradient
 	int step = 0;
 	// training workspace, sized for P pixels and nblk tiles
-	long ws_P = 0, ws_nblk = 0;
+	long ws_P = 0, ws_part = 0;
 	bf16* act[5] = { nullptr, nullptr, nullptr, nullptr, nullptr };
 	bf16 *gu0 = nullptr, *gu1 = nullptr;
 	float2 *out = nullptr, *gout = nullptr;
@@ -3408,12 +3408,13 @@ static void net_free_ws(bnufft_precnet_s* n)
 	n->out = n->gout = nullptr;
 	n->part = nullptr;
 	n->loss_part = nullptr;
-	n->ws_P = n->ws_nblk = 0;
+	n->ws_P = n->ws_part = 0;
 }
 
-static int net_ensure_ws(bnufft_precnet_s* n, long P, long nblk)
+// work space for images of P pixels in all and np floats of gradient partials
+static int net_ensure_ws(bnufft_precnet_s* n, long P, long np)
 {
-	if ((P <= n->ws_P) && (nblk <= n->ws_nblk))
+	if ((P <= n->ws_P) && (np <= n->ws_part))
 		return BNUFFT_OK;
 
 	CUDA_TRY(cudaDeviceSynchronize());	// buffers may be in use by earlier steps
@@ -3427,21 +3428,29 @@ static int net_ensure_ws(bnufft_precnet_s* n, long P, long nblk)
 	CUDA_TRY(cudaMalloc(&n->gu1, ab));
 	CUDA_TRY(cudaMalloc(&n->out, sizeof(float2) * P));
 	CUDA_TRY(cudaMalloc(&n->gout, sizeof(float2) * P));
-	CUDA_TRY(cudaMalloc(&n->part, sizeof(float) * nblk * NetLayout::size(1)));
+	CUDA_TRY(cudaMalloc(&n->part, sizeof(float) * np));
 	CUDA_TRY(cudaMalloc(&n->loss_part, sizeof(double) * NET_LOSS_BLOCKS));
 	n->ws_P = P;
-	n->ws_nblk = nblk;
+	n->ws_part = np;
 	return BNUFFT_OK;
 }
 
-// most blocks of a weight-gradient launch (persistent, two to four per SM):
-// the partial vectors to reduce
+// most blocks of a weight-gradient launch (persistent, two to four per SM)
 enum { NET_WG_BLOCKS = 4 * 148 };
 
-static int net_wgrad_reduce(bnufft_precnet_s* n, int l, unsigned nblk, cudaStream_t st)
+// floats of the partial vectors of an image batch's largest gradient launch
+static long net_part_floats(int X, int Y, long nimg)
+{
+	const dim3 t = net_tiles(X, Y, nimg);
+	const long tiles = (long)t.x * t.y * t.z, rows = ((long)((X + NET_TILE_X - 1) / NET_TILE_X) * Y * nimg + WT_WARPS - 1) / WT_WARPS;
+	return std::max(wg_slots(tiles, std::min<long>(tiles, NET_WG_BLOCKS / 2)) * NetLayout::size(1),
+			wg_slots(rows, std::min<long>(rows, NET_WG_BLOCKS)) * std::max(NetLayout::size(0), NetLayout::size(5)));
+}
+
+static int net_wgrad_reduce(bnufft_precnet_s* n, int l, long slots, cudaStream_t st)
 {
 	const int O = NetLayout::size(l);
-	k_wgrad_reduce<<<(O + 31) / 32, 32 * WR_SLICES, 0, st>>>(n->part, (int)nblk, O, n->grad + NetLayout::woff(l));
+	k_wgrad_reduce<<<(O + 31) / 32, 32 * WR_SLICES, 0, st>>>(n->part, (int)slots, O, n->grad + NetLayout::woff(l));
 	LAUNCHED();
 	return BNUFFT_OK;
 }
@@ -3455,7 +3464,7 @@ static int net_wgrad32(bnufft_precnet_s* n, int l, const bf16* a, const bf16* g,
 	TRY(prep_kernel(k_wgrad32, WG_SMEM));
 	k_wgrad32<<<nblk, WG_THREADS, WG_SMEM, st>>>(a, g, X, Y, (int)t.x, (int)t.y, ntiles, n->part);
 	LAUNCHED();
-	return net_wgrad_reduce(n, l, nblk, st);
+	return net_wgrad_reduce(n, l, wg_slots(ntiles, nblk), st);
 }
 
 // the same for the layers with 2 channels on one side (OUT6: layer 6, else
@@ -3465,10 +3474,11 @@ static int net_wgrad_thin(bnufft_precnet_s* n, const bf16* w, const float2* t, i
 {
 	const int tx = (X + NET_TILE_X - 1) / NET_TILE_X;
 	const long nrows = (long)tx * Y * nimg;
-	const unsigned nblk = (unsigned)std::min<long>((nrows + WT_WARPS - 1) / WT_WARPS, NET_WG_BLOCKS);
+	const long units = (nrows + WT_WARPS - 1) / WT_WARPS;
+	const unsigned nblk = (unsigned)std::min<long>(units, NET_WG_BLOCKS);
 	k_wgrad_thin<OUT6><<<nblk, 32 * WT_WARPS, 0, st>>>(w, t, X, Y, tx, nrows, n->part);
 	LAUNCHED();
-	return net_wgrad_reduce(n, OUT6 ? 5 : 0, nblk, st);
+	return net_wgrad_reduce(n, OUT6 ? 5 : 0, wg_slots(units, nblk), st);
 }
 
 extern "C" int bnufft_precnet_nparams(void) { return NET_N; }
@@ -3572,8 +3582,7 @@ extern "C" int bnufft_precnet_forward(bnufft_precnet_t n, void* out, const void*
 		return fail(BNUFFT_ERR_ARG, "bad precnet image size");
 
 	const long P = X * Y * nimg;
-	dim3 grid = net_tiles((int)X, (int)Y, nimg);
-	TRY(net_ensure_ws(n, P, std::min<long>((long)grid.x * grid.y * grid.z, NET_WG_BLOCKS)));
+	TRY(net_ensure_ws(n, P, net_part_floats((int)X, (int)Y, nimg)));
 	size_t b = sizeof(float2) * P;
 	Staged i, o;
 	TRY(stage_in(i, in, b, st));
@@ -3609,8 +3618,7 @@ static int net_train(bnufft_precnet_t n, const void* in, const void* target, con
 
 	const long P = X * Y * nimg;
 	const int x = (int)X, y = (int)Y;
-	dim3 grid = net_tiles(x, y, nimg);
-	TRY(net_ensure_ws(n, P, std::min<long>((long)grid.x * grid.y * grid.z, NET_WG_BLOCKS)));
+	TRY(net_ensure_ws(n, P, net_part_floats(x, y, nimg)));
 	size_t b = sizeof(float2) * P;
 	Staged si, stg;
 	TRY(stage_in(si, in, b, st));

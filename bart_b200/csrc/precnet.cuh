@@ -242,17 +242,16 @@ struct NetPix {
 // without a division per item.
 struct NetWalk {
 
-	int x, y, nx, ny, sx, sy;
-	long z, sz;		// image
+	int x, y, z, nx, ny, sx, sy, sz;	// z: image
 
 	__device__ __forceinline__ NetWalk(long first, long step, int nx_, int ny_) : nx(nx_), ny(ny_)
 	{
 		x = (int)(first % nx);
 		y = (int)((first / nx) % ny);
-		z = first / nx / ny;
+		z = (int)(first / nx / ny);
 		sx = (int)(step % nx);
 		sy = (int)((step / nx) % ny);
-		sz = step / nx / ny;
+		sz = (int)(step / nx / ny);
 	}
 
 	__device__ __forceinline__ void next()
@@ -554,23 +553,37 @@ __global__ void __launch_bounds__(NET_THREADS) k_net_out_bwd(const float2* __res
 
 // Weight and bias gradients -----------------------------------------------------
 //
-// Both kernels are persistent: a block takes image tiles blockIdx.x,
-// blockIdx.x + gridDim.x, ... and keeps its sums in registers over all of
-// them, so it writes one partial vector of the layer's parameters at the end
-// (a few hundred vectors to reduce instead of one per tile), in a fixed order:
-// the gradients are the same bits every run.
-//   part[blk][(co * 9 + tap) * CIN + ci] = sum_p g[p][co] a[p + off(tap)][ci]
-//   part[blk][COUT * 9 * CIN + co]       = sum_p g[p][co]
+// Both kernels are persistent: a block takes units of 256 pixels (image tiles, or
+// rows of its warps) blockIdx.x, blockIdx.x + gridDim.x, ..., sums each in float32
+// as before and leaves a partial vector of the layer's parameters after every
+// WG_RUN units, which k_wgrad_reduce adds in float64. So no float32 sum grows with
+// the number of images, there are a few hundred vectors to reduce instead of one
+// per tile, and the order is fixed: the gradients are the same bits every run.
+// Partial f of block b is vector b + f gridDim.x (slots):
+//   part[slot][(co * 9 + tap) * CIN + ci] = sum_p g[p][co] a[p + off(tap)][ci]
+//   part[slot][COUT * 9 * CIN + co]       = sum_p g[p][co]
+enum { WG_RUN = 8 };
+
+// partial vectors of nblk <= units blocks
+inline long wg_slots(long units, long nblk)
+{
+	const long most = (units + nblk - 1) / nblk;			// units of the first blocks; the others one less
+	const long full = (most - 1) / WG_RUN;				// partials before the first blocks' last
+	const bool all = (most - 1 > full * WG_RUN);			// the other blocks have one more too
+	return nblk * full + (all ? nblk : units - nblk * (most - 1));
+}
 
 // 32 -> 32 channels on the tensor cores (mma.sync, bf16 in, float32 sums).
 // Per tile of 32 x 8 pixels the gradient rows and the activations' halo lie
 // in shared memory pixel by pixel; ldmatrix.trans reads both as MMA operands
-// with the pixels as K. Warp w owns tap w: its 32 x 32 sums are 32 registers.
+// with the pixels as K. Warp w owns tap w: its 32 x 32 sums are 32 registers, and
+// 32 more for the run's (one set over a whole block's tiles took 39 us a layer of
+// seven 256^2 images instead of 42, but its error grew with the images: equal terms
+// of 128 of 250^2 were off by 2.9e-4, now by 6e-8).
 // The next tile arrives by cp.async while this one is summed, one barrier per
-// tile. Bound by the mma.sync rate (half of the tensor cycles at 39 us a layer of
-// seven 256^2 images); the FP32-pipe kernel it replaced took two shared-memory
+// tile. Bound by the mma.sync rate (half of the tensor cycles); the FP32-pipe kernel it replaced took two shared-memory
 // loads per FMA (1019 us a layer; the whole forward and gradient pass 5.37 ms
-// then, 0.64 ms now).
+// then, 0.65 ms now).
 constexpr int WG_WARPS = 9;
 constexpr int WG_THREADS = 32 * WG_WARPS;
 constexpr int WG_STAGE = (NET_HALO_X * NET_HALO_Y + NET_TILE_X * NET_TILE_Y) * NET_SA_STRIDE;	// bf16 per buffer
@@ -628,18 +641,22 @@ __global__ void __launch_bounds__(WG_THREADS, 2) k_wgrad32(const bf16* __restric
 		asm volatile("cp.async.commit_group;\n" ::: "memory");
 	};
 
-	float acc[2][4][4], bacc[2][4];
-#pragma unroll
-	for (int mt = 0; mt < 2; mt++) {
-#pragma unroll
-		for (int e = 0; e < 4; e++) {
+	float sum[2][4][4], bsum[2][2];		// over the run's tiles
 
-			bacc[mt][e] = 0.f;
+	auto clear = [&]() {
+#pragma unroll
+		for (int mt = 0; mt < 2; mt++) {
+
+			bsum[mt][0] = bsum[mt][1] = 0.f;
 #pragma unroll
 			for (int nt = 0; nt < 4; nt++)
-				acc[mt][nt][e] = 0.f;
+#pragma unroll
+				for (int e = 0; e < 4; e++)
+					sum[mt][nt][e] = 0.f;
 		}
-	}
+	};
+
+	clear();
 
 	// lane's row of the 8x8 matrices of one ldmatrix: gradient matrices are
 	// (pixels 0-7, co 0-7), (0-7, 8-15), (8-15, 0-7), (8-15, 8-15) of a 16 x 16
@@ -647,19 +664,33 @@ __global__ void __launch_bounds__(WG_THREADS, 2) k_wgrad32(const bf16* __restric
 	const int mrow = lane & 7, msel = lane >> 3;
 	const uint32_t goff = ((msel >> 1) * 8 + mrow) * PIX + (msel & 1) * 16;
 	const uint32_t aoff = ((msel & 1) * 8 + mrow + ky * NET_HALO_X + kx) * PIX + (msel >> 1) * 16;
-	int buf = 0;
+	int buf = 0, run = 0, slot = blockIdx.x;
+	int left = (int)((ntiles - blockIdx.x + gridDim.x - 1) / gridDim.x);	// the block's tiles
 
-	if (blockIdx.x < ntiles)
+	if (left > 0)
 		load(0);
 
-	for (long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
+	for (; left > 0; left--) {
 
 		// this tile has arrived and the other buffer has been read by all
 		asm volatile("cp.async.wait_group 0;\n" ::: "memory");
 		__syncthreads();
 
-		if (tile + gridDim.x < ntiles)
+		if (left > 1)
 			load(buf ^ 1);
+
+		float acc[2][4][4], bacc[2][4];		// over this tile
+#pragma unroll
+		for (int mt = 0; mt < 2; mt++) {
+#pragma unroll
+			for (int e = 0; e < 4; e++) {
+
+				bacc[mt][e] = 0.f;
+#pragma unroll
+				for (int nt = 0; nt < 4; nt++)
+					acc[mt][nt][e] = 0.f;
+			}
+		}
 
 		const uint32_t sa = s0 + buf * STAGE + aoff, sg = s0 + buf * STAGE + HALO * PIX + goff;
 #pragma unroll 2
@@ -684,24 +715,42 @@ __global__ void __launch_bounds__(WG_THREADS, 2) k_wgrad32(const bf16* __restric
 		}
 
 		buf ^= 1;
-	}
-
-	float* dst = part + (long)blockIdx.x * (NET_C * 9 * NET_C + NET_C);
-	const int r = lane >> 2, t = lane & 3;
 #pragma unroll
-	for (int mt = 0; mt < 2; mt++) {
-#pragma unroll
-		for (int hh = 0; hh < 2; hh++) {
+		for (int mt = 0; mt < 2; mt++) {
 
-			const int co = mt * 16 + hh * 8 + r;
+			bsum[mt][0] += bacc[mt][0];
+			bsum[mt][1] += bacc[mt][2];
 #pragma unroll
 			for (int nt = 0; nt < 4; nt++)
-				*(float2*)(dst + (co * 9 + warp) * NET_C + nt * 8 + 2 * t)
-					= make_float2(acc[mt][nt][2 * hh], acc[mt][nt][2 * hh + 1]);
-
-			if ((4 == warp) && (0 == t))
-				dst[NET_C * 9 * NET_C + co] = bacc[mt][2 * hh];
+#pragma unroll
+				for (int e = 0; e < 4; e++)
+					sum[mt][nt][e] += acc[mt][nt][e];
 		}
+
+		if ((++run < WG_RUN) && (left > 1))
+			continue;
+
+		float* dst = part + (long)slot * (NET_C * 9 * NET_C + NET_C);
+		const int r = lane >> 2, t = lane & 3;
+#pragma unroll
+		for (int mt = 0; mt < 2; mt++) {
+#pragma unroll
+			for (int hh = 0; hh < 2; hh++) {
+
+				const int co = mt * 16 + hh * 8 + r;
+#pragma unroll
+				for (int nt = 0; nt < 4; nt++)
+					*(float2*)(dst + (co * 9 + warp) * NET_C + nt * 8 + 2 * t)
+						= make_float2(sum[mt][nt][2 * hh], sum[mt][nt][2 * hh + 1]);
+
+				if ((4 == warp) && (0 == t))
+					dst[NET_C * 9 * NET_C + co] = bsum[mt][hh];
+			}
+		}
+
+		slot += gridDim.x;
+		run = 0;
+		clear();
 	}
 }
 
@@ -725,119 +774,131 @@ __global__ void __launch_bounds__(32 * WT_WARPS, 4) k_wgrad_thin(const bf16* __r
 	__shared__ float red[WT_WARPS][O + NET_C];
 	__shared__ float2 win[WT_WARPS][3][NET_TILE_X + 2];
 	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-	float2 acc[9];
-	float2 bsum = make_float2(0.f, 0.f);
-#pragma unroll
-	for (int k = 0; k < 9; k++)
-		acc[k] = make_float2(0.f, 0.f);
+	float* dst = part + (long)blockIdx.x * (O + OB);
 
 	// work rows: 32 pixels of one image row; tx of them per image row
 	NetWalk pos((long)blockIdx.x * WT_WARPS + warp, (long)gridDim.x * WT_WARPS, tx, Y);
 
-	for (long row = (long)blockIdx.x * WT_WARPS + warp; row < nrows; row += (long)gridDim.x * WT_WARPS, pos.next()) {
+	// units of the block (a row per warp) and rows of this warp
+	int units = (int)(((nrows + WT_WARPS - 1) / WT_WARPS - blockIdx.x + gridDim.x - 1) / gridDim.x);
+	int rows = (int)((nrows - (long)blockIdx.x * WT_WARPS - warp + (long)gridDim.x * WT_WARPS - 1) / ((long)gridDim.x * WT_WARPS));
 
-		const int x0 = pos.x * NET_TILE_X, y = pos.y;
-		const long base = pos.z * ((long)X * Y);
-		__syncwarp();
+	for (; units > 0; units -= WG_RUN, rows -= WG_RUN) {	// a run
 
-		for (int i = lane; i < 3 * (NET_TILE_X + 2); i += 32) {
-
-			const int dy = i / (NET_TILE_X + 2), dx = i % (NET_TILE_X + 2);
-			const int yy = y + dy - 1, xx = x0 + dx - 1;
-			win[warp][dy][dx] = ((yy >= 0) && (yy < Y) && (xx >= 0) && (xx < X)) ? t[base + (long)yy * X + xx]
-					: make_float2(0.f, 0.f);
-		}
-
-		__syncwarp();
-		const bf16* wp = w + (base + (long)y * X + x0) * NET_C + lane;
-		const int n = min(NET_TILE_X, X - x0);
-		float2 c0[3], c1[3], c2[3];			// window columns x - 1, x, x + 1
+		float2 acc[9];
+		float2 bsum = make_float2(0.f, 0.f);
 #pragma unroll
-		for (int d = 0; d < 3; d++) {
+		for (int k = 0; k < 9; k++)
+			acc[k] = make_float2(0.f, 0.f);
 
-			c0[d] = win[warp][d][0];
-			c1[d] = win[warp][d][1];
-		}
+		for (int u = 0; u < min(rows, (int)WG_RUN); u++, pos.next()) {
+
+			const int x0 = pos.x * NET_TILE_X, y = pos.y;
+			const long base = pos.z * ((long)X * Y);
+			__syncwarp();
+
+			for (int i = lane; i < 3 * (NET_TILE_X + 2); i += 32) {
+
+				const int dy = i / (NET_TILE_X + 2), dx = i % (NET_TILE_X + 2);
+				const int yy = y + dy - 1, xx = x0 + dx - 1;
+				win[warp][dy][dx] = ((yy >= 0) && (yy < Y) && (xx >= 0) && (xx < X)) ? t[base + (long)yy * X + xx]
+						: make_float2(0.f, 0.f);
+			}
+
+			__syncwarp();
+			const bf16* wp = w + (base + (long)y * X + x0) * NET_C + lane;
+			const int n = min(NET_TILE_X, X - x0);
+			float2 c0[3], c1[3], c2[3];			// window columns x - 1, x, x + 1
+#pragma unroll
+			for (int d = 0; d < 3; d++) {
+
+				c0[d] = win[warp][d][0];
+				c1[d] = win[warp][d][1];
+			}
 #pragma unroll 8
-		for (int px = 0; px < NET_TILE_X; px++) {
+			for (int px = 0; px < NET_TILE_X; px++) {
 
-			const float v = (px < n) ? __bfloat162float(wp[(long)px * NET_C]) : 0.f;
+				const float v = (px < n) ? __bfloat162float(wp[(long)px * NET_C]) : 0.f;
 #pragma unroll
-			for (int d = 0; d < 3; d++)
-				c2[d] = win[warp][d][px + 2];
+				for (int d = 0; d < 3; d++)
+					c2[d] = win[warp][d][px + 2];
 #pragma unroll
-			for (int d = 0; d < 3; d++) {
+				for (int d = 0; d < 3; d++) {
 
-				const int r0 = OUT6 ? 3 * (2 - d) + 2 : 3 * d;		// the tap that meets row d, column x - 1
-				const int r1 = OUT6 ? 3 * (2 - d) + 1 : 3 * d + 1;
-				const int r2 = OUT6 ? 3 * (2 - d) : 3 * d + 2;
-				acc[r0] = cfma(make_float2(v, v), c0[d], acc[r0]);
-				acc[r1] = cfma(make_float2(v, v), c1[d], acc[r1]);
-				acc[r2] = cfma(make_float2(v, v), c2[d], acc[r2]);
+					const int r0 = OUT6 ? 3 * (2 - d) + 2 : 3 * d;		// the tap that meets row d, column x - 1
+					const int r1 = OUT6 ? 3 * (2 - d) + 1 : 3 * d + 1;
+					const int r2 = OUT6 ? 3 * (2 - d) : 3 * d + 2;
+					acc[r0] = cfma(make_float2(v, v), c0[d], acc[r0]);
+					acc[r1] = cfma(make_float2(v, v), c1[d], acc[r1]);
+					acc[r2] = cfma(make_float2(v, v), c2[d], acc[r2]);
+				}
+
+				if (!OUT6)
+					bsum.x += v;
+#pragma unroll
+				for (int d = 0; d < 3; d++) {
+
+					c0[d] = c1[d];
+					c1[d] = c2[d];
+				}
 			}
 
-			if (!OUT6)
-				bsum.x += v;
-#pragma unroll
-			for (int d = 0; d < 3; d++) {
+			if (OUT6) {	// lane's pixel of the row: the bias gradient (summed over lanes below)
 
-				c0[d] = c1[d];
-				c1[d] = c2[d];
+				const float2 v = win[warp][1][lane + 1];
+
+				if (lane < n) {
+
+					bsum.x += v.x;
+					bsum.y += v.y;
+				}
 			}
 		}
 
-		if (OUT6) {	// lane's pixel of the row: the bias gradient (summed over lanes below)
+#pragma unroll
+		for (int k = 0; k < 9; k++) {
 
-			const float2 v = win[warp][1][lane + 1];
+			red[warp][OUT6 ? k * NET_C + lane : (lane * 9 + k) * 2] = acc[k].x;
+			red[warp][OUT6 ? (9 + k) * NET_C + lane : (lane * 9 + k) * 2 + 1] = acc[k].y;
+		}
 
-			if (lane < n) {
+		if (OUT6) {
 
-				bsum.x += v.x;
-				bsum.y += v.y;
+			for (int o = 16; o > 0; o >>= 1) {
+
+				bsum.x += __shfl_xor_sync(0xffffffffu, bsum.x, o);
+				bsum.y += __shfl_xor_sync(0xffffffffu, bsum.y, o);
 			}
-		}
-	}
 
+			if (0 == lane) {
+
+				red[warp][O] = bsum.x;
+				red[warp][O + 1] = bsum.y;
+			}
+
+		} else {
+
+			red[warp][O + lane] = bsum.x;
+		}
+
+		__syncthreads();
+
+		for (int o = threadIdx.x; o < O + OB; o += 32 * WT_WARPS) {
+
+			float s = 0.f;
 #pragma unroll
-	for (int k = 0; k < 9; k++) {
+			for (int k = 0; k < WT_WARPS; k++)
+				s += red[k][o];
 
-		red[warp][OUT6 ? k * NET_C + lane : (lane * 9 + k) * 2] = acc[k].x;
-		red[warp][OUT6 ? (9 + k) * NET_C + lane : (lane * 9 + k) * 2 + 1] = acc[k].y;
-	}
-
-	if (OUT6) {
-
-		for (int o = 16; o > 0; o >>= 1) {
-
-			bsum.x += __shfl_xor_sync(0xffffffffu, bsum.x, o);
-			bsum.y += __shfl_xor_sync(0xffffffffu, bsum.y, o);
+			dst[o] = s;
 		}
 
-		if (0 == lane) {
-
-			red[warp][O] = bsum.x;
-			red[warp][O + 1] = bsum.y;
-		}
-
-	} else {
-
-		red[warp][O + lane] = bsum.x;
-	}
-
-	__syncthreads();
-
-	for (int o = threadIdx.x; o < O + OB; o += 32 * WT_WARPS) {
-
-		float s = 0.f;
-#pragma unroll
-		for (int k = 0; k < WT_WARPS; k++)
-			s += red[k][o];
-
-		part[(long)blockIdx.x * (O + OB) + o] = s;
+		__syncthreads();	// before the next run's sums
+		dst += (long)gridDim.x * (O + OB);
 	}
 }
 
-// grad[o] = sum over blocks of part[blk][o] in float64: 32 outputs per block,
+// grad[o] = sum over the partial vectors part[slot][o] in float64: 32 outputs per block,
 // WR_SLICES slices of the partials, combined in a fixed order
 enum { WR_SLICES = 32 };
 

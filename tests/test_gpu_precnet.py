@@ -88,7 +88,8 @@ def test_gradients_vs_oracle():
 def test_gradients_tile_edges(X, Y, n):
     """Weight and bias gradients where the 32 x 8 pixel tiles and 32-pixel rows
     of the persistent kernels end: one pixel, a tile exactly and one pixel
-    more, several images, more tiles (320) than blocks. The kernels sum exact
+    more, several images, more tiles (320) than the tensor-core kernel has
+    blocks. The kernels sum exact
     bf16 products in float32, so they differ from the oracle only where an
     activation or gradient rounds to its other bf16 neighbour (2^-8 relative);
     a layer's gradient has up to five such roundings behind it, and few pixels
@@ -105,6 +106,66 @@ def test_gradients_tile_edges(X, Y, n):
     for li, (wo, bo, e) in enumerate(po.offsets()):
         assert rel(g[wo:bo], go[wo:bo]) < 5 * 2.0 ** -8, li
         assert rel(g[bo:e], go[bo:e]) < 5 * 2.0 ** -8, li
+
+
+def test_gradients_of_many_images_sum_in_float64():
+    """Weight and bias gradients of 128 images, every parameter against its
+    exact value: no float32 sum covers more than a tile's 256 pixels, however
+    many images there are. With weights on the centre tap only and constant
+    images all activations and gradients are constant, so a gradient is one
+    pixel's (the oracle's) times the number of pixels that have the tap's
+    neighbour. Equal terms round the same way every time, the worst case: 256
+    additions by up to half an ulp each, 128 * 2^-24 of the sum (the tensor
+    cores' 16 additions per tile, which may truncate, stay below that), eight
+    tiles or warps added up, one rounding of the product and the sum each:
+    138 * 2^-24."""
+    X, Y, n = 250, 250, 128
+    rng = np.random.default_rng(9)
+    p = np.zeros(po.NPARAMS, dtype=np.float32)
+    for li, (wo, bo, e) in enumerate(po.offsets()):
+        ci, co = 2 if 0 == li else 32, 2 if 5 == li else 32
+        w = np.zeros((co, 9, ci), dtype=np.float32)
+        w[:, 4] = rng.uniform(0.02, 0.06, (co, ci))
+        p[wo:bo] = w.ravel()
+        p[bo:e] = rng.uniform(0.1, 0.9, e - bo)
+    one = np.full((1, 1, 1), 0.37 + 0.81j, dtype=np.complex64)
+    aim = np.full((1, 1, 1), -1.3 - 2.1j, dtype=np.complex64)
+    net = precnet.PrecNet(p)
+    g = np.zeros(po.NPARAMS, dtype=np.float32)
+    net.train_step(np.full((X, Y, n), one[0, 0, 0], order="F"), np.full((X, Y, n), aim[0, 0, 0], order="F"), X, Y, n, 0.0,
+                   grads=g)
+    net.free()
+    _, g1 = po.loss_and_grad(p, po.to_channels(one), po.to_channels(aim), bf16_mode=True)
+    count = np.array([(X - abs(t % 3 - 1)) * (Y - abs(t // 3 - 1)) for t in range(9)], dtype=np.float64)
+    for li, (wo, bo, e) in enumerate(po.offsets()):
+        ci, co = 2 if 0 == li else 32, 2 if 5 == li else 32
+        want = g1[wo:bo].reshape(co, 9, ci)[:, 4:5] * count[:, None]
+        assert np.max(np.abs(g[wo:bo].reshape(co, 9, ci) / want - 1)) < 138 * 2.0 ** -24, li
+        assert np.max(np.abs(g[bo:e] / (g1[bo:e] * X * Y) - 1)) < 138 * 2.0 ** -24, li
+
+
+def test_gradients_of_a_batch_are_those_of_its_parts():
+    """64 uneven images at once against eight batches of eight. At once, a block
+    takes up to six tiles and a warp three rows, across columns, rows and images
+    and with every buffer used again; a part's tiles and rows (192 and 1464) all
+    have their own. The gradients of the outputs differ by exactly eight, so do
+    all bf16 roundings, and only the order of float32 sums is left: 256 products
+    at a time, so 16 * 2^-24 for independent roundings. Twice the same bits."""
+    X, Y, n = 70, 61, 64
+    rng = np.random.default_rng(12)
+    x, t = _img(rng, X, Y, n), _img(rng, X, Y, n)
+    net = precnet.PrecNet(_params(rng))
+    g, again, part, total = (np.zeros(po.NPARAMS, dtype=d) for d in (np.float32, np.float32, np.float32, np.float64))
+    net.train_step(x, t, X, Y, n, 0.0, grads=g)
+    net.train_step(x, t, X, Y, n, 0.0, grads=again)
+    for i in range(0, n, 8):
+        net.train_step(np.asfortranarray(x[..., i:i + 8]), np.asfortranarray(t[..., i:i + 8]), X, Y, 8, 0.0, grads=part)
+        total += part / 8.0
+    net.free()
+    assert np.array_equal(g.view(np.uint32), again.view(np.uint32))
+    for li, (wo, bo, e) in enumerate(po.offsets()):
+        assert rel(g[wo:bo], total[wo:bo]) < 16 * 2.0 ** -24, li
+        assert rel(g[bo:e], total[bo:e]) < 16 * 2.0 ** -24, li
 
 
 def test_gradients_bit_reproducible():
