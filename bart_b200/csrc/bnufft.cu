@@ -822,7 +822,7 @@ struct Bins {
 	// output-stationary scatter (k_grid6_tiles): bins are its tiles
 	int tg_cfg = -1;		// kernel shape (TG_*), -1: not used
 	long ntiles = 0;
-	int* hit_start = nullptr;	// [ntiles + 1]
+	long* hit_start = nullptr;	// [ntiles + 1]
 	int* hits = nullptr;		// samples that meet each tile
 	int* work_tile = nullptr;	// [nwork_max]
 	int* work_chunk = nullptr;
@@ -1483,6 +1483,9 @@ static int build_csr(OpCtx& op, cudaStream_t st)
 	return BNUFFT_OK;
 }
 
+// fewest hits of a work item, and the longest hit lists made without counting first
+enum { TG_MIN_CHUNK = 32, TG_LIST_BYTES = 64 << 20 };
+
 // tiles that one sample can meet at most: its six cells per axis meet two
 // tiles of at least six cells, three shorter ones, and on periodic grids one
 // more where the last tile is cut short
@@ -1620,7 +1623,7 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 	if ((g.M >= (1L << 31)) || (nbins >= (1L << 31)))
 		return fail(BNUFFT_ERR_UNSUPPORTED, "binning: %ld samples, %ld bins", g.M, nbins);
 
-	if ((b.tg_cfg >= 0) && (g.M * tg_max_hits(g, bg) >= (1L << 31)))	// hit lists are indexed with ints
+	if ((b.tg_cfg >= 0) && (nbins + g.M * tg_max_hits(g, bg) / TG_MIN_CHUNK >= (1L << 31)))	// work items are counted with ints
 		b.tg_cfg = -1;
 
 	unsigned *keys = nullptr, *keys2 = nullptr;
@@ -1703,16 +1706,12 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		b.chunk = (g.G[2] > 1) ? 512 : ((det ? 2 : 1) * ((jobs64 < 16 * 148) ? 32 : 64));
 
 		if (const char* e = getenv("BNUFFT_GRID_CHUNK"))	// tuning knob: hits per work item
-			b.chunk = std::max(32, std::min(4096, atoi(e)));
+			b.chunk = std::max((int)TG_MIN_CHUNK, std::min(4096, atoi(e)));
 
-		b.nwork_max = nt + (M * tg_max_hits(g, bg) + b.chunk - 1) / b.chunk;
 		CUDA_TRY(cudaMallocAsync(&nhits, sizeof(int) * nt, st));
-		CUDA_TRY(cudaMallocAsync(&b.hit_start, sizeof(int) * (nt + 1), st));
-		CUDA_TRY(cudaMallocAsync(&b.hits, sizeof(int) * M * tg_max_hits(g, bg), st));
+		CUDA_TRY(cudaMallocAsync(&b.hit_start, sizeof(long) * (nt + 1), st));
 		CUDA_TRY(cudaMallocAsync(&b.work_start, sizeof(int) * (nt + 1), st));
 		CUDA_TRY(cudaMallocAsync(&b.multi, sizeof(int) * (nt + 1), st));
-		CUDA_TRY(cudaMallocAsync(&b.work_tile, sizeof(int) * b.nwork_max, st));
-		CUDA_TRY(cudaMallocAsync(&b.work_chunk, sizeof(int) * b.nwork_max, st));
 
 		if (det)
 			CUDA_TRY(cudaMallocAsync(&b.slot, sizeof(int) * (nt + 1), st));
@@ -1723,21 +1722,49 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		LAUNCHED();
 		k_tile_plan<<<1, 1024, 0, st>>>(nhits, (int)nt, b.chunk, b.hit_start, b.work_start, b.slot, b.multi);
 		LAUNCHED();
+
+		// lists and work items: at most so many; the lists are made as long as
+		// counted where the bound (18 hits a sample in 3D, 8.2 on average) would
+		// cost more than the host's wait for the count, some 20 us
+		long total = M * tg_max_hits(g, bg);
+		b.nwork_max = nt + (total + b.chunk - 1) / b.chunk;
+		cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+		CUDA_TRY(cudaStreamIsCapturing(st, &cs));
+		const bool count = (sizeof(int) * total > TG_LIST_BYTES) && (cudaStreamCaptureStatusNone == cs);
+
+		if (count || det) {
+
+			int slots = 0, work = 0;
+
+			if (count) {
+
+				CUDA_TRY(cudaMemcpyAsync(&total, b.hit_start + nt, sizeof(long), cudaMemcpyDeviceToHost, st));
+				CUDA_TRY(cudaMemcpyAsync(&work, b.work_start + nt, sizeof(int), cudaMemcpyDeviceToHost, st));
+			}
+
+			if (det)
+				CUDA_TRY(cudaMemcpyAsync(&slots, b.slot + nt, sizeof(int), cudaMemcpyDeviceToHost, st));
+
+			CUDA_TRY(cudaStreamSynchronize(st));
+
+			if (count)
+				b.nwork_max = work;
+
+			b.det = det;
+			b.nslots = slots;
+		}
+
+		CUDA_TRY(cudaMallocAsync(&b.hits, sizeof(int) * std::max(1L, total), st));
+		CUDA_TRY(cudaMallocAsync(&b.work_tile, sizeof(int) * b.nwork_max, st));
+		CUDA_TRY(cudaMallocAsync(&b.work_chunk, sizeof(int) * b.nwork_max, st));
 		k_tile_hits<<<hb, TH_THREADS, 0, st>>>(lo4, bin_start, grid_geom(g), bg, nt, nullptr, b.hit_start, b.hits,
 				b.work_start, b.work_tile, b.work_chunk);
 		LAUNCHED();
 		cudaFreeAsync(lo4, st);
 		cudaFreeAsync(nhits, st);
 
-		if (det) {
-
-			b.det = true;
-			int total = 0;
-			CUDA_TRY(cudaMemcpyAsync(&total, b.slot + nt, sizeof(int), cudaMemcpyDeviceToHost, st));
-			CUDA_TRY(cudaStreamSynchronize(st));
-			b.nslots = total;
+		if (det)
 			TRY(alloc_partials(b, op.coils, st));
-		}
 
 		// the bin-ordered k-space of the applies, allocated here so that
 		// applies allocate nothing (their solves can then be captured into

@@ -843,7 +843,7 @@ enum { TG_WARPS = 4 };
 
 struct TileWork {
 
-	const int* hit_start;		// [ntiles + 1]
+	const long* hit_start;		// [ntiles + 1]
 	const int* hits;		// sorted-sample indices by tile
 	const int* work_tile;		// [nwork] tile of a work item
 	const int* work_chunk;		// [nwork] chunk of the tile's hits
@@ -867,7 +867,7 @@ __device__ __forceinline__ int foot_rel(int lo, int origin, int G, int periodic)
 enum { TH_THREADS = 256, TH_RANGES = 18 };
 
 __global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restrict__ lo, const int* __restrict__ bin_start,
-		GridGeom g, BinGeom bg, long ntiles, int* __restrict__ nhits, const int* __restrict__ hit_start,
+		GridGeom g, BinGeom bg, long ntiles, int* __restrict__ nhits, const long* __restrict__ hit_start,
 		int* __restrict__ hits, const int* __restrict__ work_start, int* __restrict__ work_tile,
 		int* __restrict__ work_chunk)
 {
@@ -921,7 +921,8 @@ __global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restri
 		for (int r = 0; r < nr; r++)
 			total += rn[r];
 
-		int pos = work_start ? hit_start[t] : 0;
+		int* dst = work_start ? hits + hit_start[t] : nullptr;	// the tile's list
+		int pos = 0;
 		int count = 0, r = 0, r0 = 0;	// this thread's range and its first candidate
 
 		// candidate c of the list (the thread's next one is loaded ahead)
@@ -979,7 +980,7 @@ __global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restri
 			}
 
 			if (hit)
-				hits[at] = i;
+				dst[at] = i;
 		}
 
 		if (!work_start) {
@@ -1085,10 +1086,11 @@ __global__ void __launch_bounds__(1024) k_scan(const int* __restrict__ in, int n
 // (chunks of hits, at least one) and, for tiles with several items, partial
 // tiles begin (slot; deterministic mode), and the list of those tiles.
 __global__ void __launch_bounds__(1024) k_tile_plan(const int* __restrict__ nhits, int ntiles, int chunk,
-		int* __restrict__ hit_start, int* __restrict__ work_start, int* __restrict__ slot, int* __restrict__ multi)
+		long* __restrict__ hit_start, int* __restrict__ work_start, int* __restrict__ slot, int* __restrict__ multi)
 {
 	__shared__ int sh[33];
-	int hsum = 0, wsum = 0, ssum = 0, msum = 0;
+	long hsum = 0;
+	int wsum = 0, ssum = 0, msum = 0;
 
 	for (int base = 0; base < ntiles; base += 1024) {
 
@@ -1097,13 +1099,14 @@ __global__ void __launch_bounds__(1024) k_tile_plan(const int* __restrict__ nhit
 		const int n = in ? nhits[t] : 0;
 		const int k = in ? max(1, (n + chunk - 1) / chunk) : 0;
 		const bool several = (k > 1);
-		int th, tw, ts, tm;
-		const int h = block_scan(n, sh, th), w = block_scan(k, sh, tw);
+		int tl, th, tw, ts, tm;
+		const int l = block_scan(n & 0xfffff, sh, tl), h = block_scan(n >> 20, sh, th);	// 1024 counts below 2^31
+		const int w = block_scan(k, sh, tw);
 		const int s = block_scan(several ? k : 0, sh, ts), m = block_scan(several ? 1 : 0, sh, tm);
 
 		if (in) {
 
-			hit_start[t] = hsum + h;
+			hit_start[t] = hsum + l + ((long)h << 20);
 			work_start[t] = wsum + w;
 
 			if (slot)
@@ -1113,7 +1116,7 @@ __global__ void __launch_bounds__(1024) k_tile_plan(const int* __restrict__ nhit
 				multi[msum + m] = t;
 		}
 
-		hsum += th;
+		hsum += tl + ((long)th << 20);
 		wsum += tw;
 		ssum += ts;
 		msum += tm;
@@ -1312,8 +1315,10 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(long M, GridGe
 	const int line = lane % NL, grp = lane / NL;
 	const int cw0 = cq * CW;		// first coil of the job
 	const int c0 = cw0 + grp * CT;		// first coil of this lane
-	const int h0 = tw.hit_start[tile], h1 = tw.hit_start[tile + 1];
-	const int first = h0 + tw.work_chunk[wi] * tw.chunk, last = min(h1, first + tw.chunk);
+	const long h0 = tw.hit_start[tile];
+	const int nh = (int)(tw.hit_start[tile + 1] - h0);	// (a sample is in a tile's list once)
+	const int* hits = tw.hits + h0;
+	const int first = tw.work_chunk[wi] * tw.chunk, last = min(nh, first + tw.chunk);
 
 	float2 acc[TX][CT];
 #pragma unroll
@@ -1358,14 +1363,14 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(long M, GridGe
 	};
 
 	int buf = 0;
-	int inext = (first + lane < last) ? tw.hits[first + lane] : -1;
+	int inext = (first + lane < last) ? hits[first + lane] : -1;
 	fetch(inext, 0);
-	inext = (first + 32 + lane < last) ? tw.hits[first + 32 + lane] : -1;
+	inext = (first + 32 + lane < last) ? hits[first + 32 + lane] : -1;
 
 	for (int base = first; base < last; base += 32) {
 
 		fetch(inext, buf ^ 1);
-		inext = (base + 64 + lane < last) ? tw.hits[base + 64 + lane] : -1;
+		inext = (base + 64 + lane < last) ? hits[base + 64 + lane] : -1;
 		asm volatile("cp.async.wait_group 1;\n" ::: "memory");
 		float* rb = rec + buf * 32 * ST::REC;
 		const int n = min(32, last - base);
@@ -1446,7 +1451,7 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(long M, GridGe
 	if ((cy >= g.G[1]) || (cz >= g.G[2]))
 		return;
 
-	const bool add = (h1 - h0 > tw.chunk);
+	const bool add = (nh > tw.chunk);
 	const long row = (long)g.G[0] * (dft_index(cy, g.N[1], g.G[1]) + (long)g.G[1] * dft_index(cz, g.N[2], g.G[2]));
 #pragma unroll
 	for (int i = 0; i < TX; i += 2) {

@@ -9,6 +9,9 @@ default (output-stationary) scatter against the global-atomic scatter to
 """
 
 import hashlib
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -105,3 +108,34 @@ def test_kooshball_full_size_properties(monkeypatch):
     finally:
         op.free()
         ref.free()
+
+
+_MEMORY = """
+import sys
+import torch
+from bart_b200.nufft import NufftConf, nufft_create2
+M, C, N = int(sys.argv[1]), int(sys.argv[2]), 64
+t = ((torch.rand(M, 3, device="cuda") - 0.5) * N).to(torch.complex64)
+torch.cuda.synchronize()
+free = torch.cuda.mem_get_info()[0]
+op = nufft_create2([1, 1024, M // 1024, C], [N, N, N, C], [3, 1024, M // 1024], t, conf=NufftConf(toeplitz=False))
+torch.cuda.synchronize()
+print((free - torch.cuda.mem_get_info()[0]) / M)
+"""
+
+
+def _plan_bytes_per_sample(M, C):
+    """Device memory that a new process's first plan takes, per sample."""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", _MEMORY, str(M), str(C)], cwd=root, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stderr
+    return float(r.stdout)
+
+
+def test_plan_memory_of_many_samples():
+    """Hit lists as long as counted: of 2^23 uniform samples a footprint of six
+    cells a side meets (8 + 5)(4 + 5)(4 + 5) / 128 = 8.2 tiles, 33 bytes, and a
+    sample further holds 96 bytes of footprint, 4 of order, 16 of trajectory and
+    16 of two channels' k-space: 165. The set-up's own arrays (order, its sort and
+    the start cells) stay below 32. (At the bound of 18 hits: 204 and those.)"""
+    assert _plan_bytes_per_sample(1 << 23, 2) < 165 + 32
