@@ -835,7 +835,8 @@ struct Bins {
 	long nslots = 0;
 	float2* part = nullptr;		// [nslots][part_c][cells of a tile]
 	long part_c = 0;
-	float4* foot = nullptr;		// [M][FOOT_F4] footprints of the sorted samples
+	float4* foot = nullptr;		// [foot_n][FOOT_F4] footprints of the sorted samples: of all M, or
+	long foot_n = 0;		// room for a part of them, filled part by part in every apply
 	bool quads = false;		// they serve the quad kernels (degridding, single-channel scatter)
 	float2* kperm = nullptr;	// [M][kperm_c] k-space in bin order, a sample's coils side by side
 	long kperm_c = 0;
@@ -1173,6 +1174,22 @@ static int op_spectrum_adjoint(OpCtx& op, const float2* grid, const float2* maps
 			dh.p, dh.part, dh.done, dh.nblocks);
 }
 
+// the footprints of sorted samples i0 .. i0 + n - 1: kept by the plan, or made now
+static int footprints(const OpCtx& op, long i0, long n, const float4** foot, cudaStream_t st)
+{
+	const Bins& b = op.bins;
+	*foot = b.foot + FOOT_F4 * i0;
+
+	if (b.foot_n < op.g.M) {
+
+		k_foot<<<vec_blocks(3 * n, 256, 8 * 148), 256, 0, st>>>(op.traj, b.perm + i0, n, grid_geom(op.g), op.kb, b.foot, nullptr);
+		LAUNCHED();
+		*foot = b.foot;
+	}
+
+	return BNUFFT_OK;
+}
+
 // grid -> k-space of C channels, times the plan's weights
 static int degrid(OpCtx& op, const float2* grid, long C, float2* ksp, cudaStream_t st)
 {
@@ -1182,28 +1199,37 @@ static int degrid(OpCtx& op, const float2* grid, long C, float2* ksp, cudaStream
 
 		const Bins& b = op.bins;
 		cudaEvent_t pe = prof_begin("degrid", st);
-		const long nb = (4 * M + BIN_THREADS - 1) / BIN_THREADS;
-		// channels per block: all of them (the weights are read once), fewer
-		// (in fours) when the samples alone give less than a few blocks per SM
-		int cpb = (int)C;
 
-		while ((cpb > 4) && (nb * ((C + cpb - 1) / cpb) < 8 * 148))
-			cpb = std::max(4, (cpb / 2 + 3) / 4 * 4);
+		for (long i0 = 0; i0 < M; i0 += b.foot_n) {
 
-		const dim3 blocks((unsigned)nb, (unsigned)((C + cpb - 1) / cpb));
+			const long n = std::min(b.foot_n, M - i0), nb = (4 * n + BIN_THREADS - 1) / BIN_THREADS;
+			const int* perm = b.perm + i0;
+			const float4* foot;
+			TRY(footprints(op, i0, n, &foot, st));
 
-		if (grid_by4(op, C))
-			k_degrid6_by4<<<blocks, BIN_THREADS, 0, st>>>(b.foot, b.perm, M, grid_geom(op.g), (int)C, cpb, grid, ksp,
-					op.wgt, (int)op.wgt_c);
-		else if (op.g.G[2] > 1)
-			k_degrid6_quads<6><<<blocks, BIN_THREADS, 0, st>>>(b.foot, b.perm, M, grid_geom(op.g), (int)C, cpb, grid, ksp,
-					op.wgt, (int)op.wgt_c);
-		else
-			k_degrid6_quads<1><<<blocks, BIN_THREADS, 0, st>>>(b.foot, b.perm, M, grid_geom(op.g), (int)C, cpb, grid, ksp,
-					op.wgt, (int)op.wgt_c);
+			// channels per block: all of them (the weights are read once), fewer
+			// (in fours) when the samples alone give less than a few blocks per SM
+			int cpb = (int)C;
+
+			while ((cpb > 4) && (nb * ((C + cpb - 1) / cpb) < 8 * 148))
+				cpb = std::max(4, (cpb / 2 + 3) / 4 * 4);
+
+			const dim3 blocks((unsigned)nb, (unsigned)((C + cpb - 1) / cpb));
+
+			if (grid_by4(op, C))
+				k_degrid6_by4<<<blocks, BIN_THREADS, 0, st>>>(foot, perm, n, M, grid_geom(op.g), (int)C, cpb, grid, ksp,
+						op.wgt, (int)op.wgt_c);
+			else if (op.g.G[2] > 1)
+				k_degrid6_quads<6><<<blocks, BIN_THREADS, 0, st>>>(foot, perm, n, M, grid_geom(op.g), (int)C, cpb, grid,
+						ksp, op.wgt, (int)op.wgt_c);
+			else
+				k_degrid6_quads<1><<<blocks, BIN_THREADS, 0, st>>>(foot, perm, n, M, grid_geom(op.g), (int)C, cpb, grid,
+						ksp, op.wgt, (int)op.wgt_c);
+
+			LAUNCHED();
+		}
 
 		prof_end(pe, st);
-		LAUNCHED();
 		return BNUFFT_OK;
 	}
 
@@ -1357,15 +1383,23 @@ static int grid_adj(OpCtx& op, const float2* ksp, long C, float2* grid, cudaStre
 
 		const Bins& b = op.bins;
 		cudaEvent_t pe = prof_begin("grid", st);
-		const unsigned nb = (unsigned)((4 * op.g.M + BIN_THREADS - 1) / BIN_THREADS);
 
-		if (op.g.G[2] > 1)
-			k_grid6_quads<6><<<nb, BIN_THREADS, 0, st>>>(b.foot, b.perm, op.g.M, grid_geom(op.g), (int)C, ksp, grid);
-		else
-			k_grid6_quads<1><<<nb, BIN_THREADS, 0, st>>>(b.foot, b.perm, op.g.M, grid_geom(op.g), (int)C, ksp, grid);
+		for (long i0 = 0; i0 < op.g.M; i0 += b.foot_n) {
+
+			const long n = std::min(b.foot_n, op.g.M - i0);
+			const unsigned nb = (unsigned)((4 * n + BIN_THREADS - 1) / BIN_THREADS);
+			const float4* foot;
+			TRY(footprints(op, i0, n, &foot, st));
+
+			if (op.g.G[2] > 1)
+				k_grid6_quads<6><<<nb, BIN_THREADS, 0, st>>>(foot, b.perm + i0, n, op.g.M, grid_geom(op.g), (int)C, ksp, grid);
+			else
+				k_grid6_quads<1><<<nb, BIN_THREADS, 0, st>>>(foot, b.perm + i0, n, op.g.M, grid_geom(op.g), (int)C, ksp, grid);
+
+			LAUNCHED();
+		}
 
 		prof_end(pe, st);
-		LAUNCHED();
 		return BNUFFT_OK;
 	}
 
@@ -1482,6 +1516,9 @@ static int build_csr(OpCtx& op, cudaStream_t st)
 	cudaFreeAsync(scan_tmp, st);
 	return BNUFFT_OK;
 }
+
+// most footprints kept by plans without tiles
+enum { FOOT_MOST = 1 << 25 };
 
 // fewest hits of a work item, and the longest hit lists made without counting first
 enum { TG_MIN_CHUNK = 32, TG_LIST_BYTES = 64 << 20 };
@@ -1667,7 +1704,9 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 
 	// the samples' footprints (start cells and weights): they depend on
 	// the trajectory only, so every apply reads them instead of recomputing
-	// 18 table lookups per sample. The quad kernels need sides of at least 16
+	// 18 table lookups per sample. Tiles need all of them (they read in hit
+	// order); plans without tiles keep those of up to FOOT_MOST samples, 3.2 GB,
+	// and of more samples make them again, FOOT_MOST at a time. The quad kernels need sides of at least 16
 	// cells and z offsets that fit an int; other sizes take the generic ones.
 	b.quads = (6.f == g.width) && (g.gsz < (1L << 31));
 
@@ -1678,13 +1717,17 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 
 	if ((b.tg_cfg >= 0) || b.quads) {
 
-		CUDA_TRY(cudaMallocAsync(&b.foot, sizeof(float4) * FOOT_F4 * M, st));
+		b.foot_n = (b.tg_cfg >= 0) ? M : std::min(M, (long)FOOT_MOST);
+		CUDA_TRY(cudaMallocAsync(&b.foot, sizeof(float4) * FOOT_F4 * b.foot_n, st));
 
 		if (b.tg_cfg >= 0)
 			CUDA_TRY(cudaMallocAsync(&lo4, sizeof(short4) * M, st));
 
-		k_foot<<<vec_blocks(3 * M, 256, 8 * 148), 256, 0, st>>>(op.traj, b.perm, M, grid_geom(g), op.kb, b.foot, lo4);
-		LAUNCHED();
+		if (b.foot_n == M) {
+
+			k_foot<<<vec_blocks(3 * M, 256, 8 * 148), 256, 0, st>>>(op.traj, b.perm, M, grid_geom(g), op.kb, b.foot, lo4);
+			LAUNCHED();
+		}
 	}
 
 	// the output-stationary scatter: the samples that meet each tile, and the

@@ -490,6 +490,7 @@ __global__ void k_foot(const float4* __restrict__ traj, const int* __restrict__ 
 // alone do not fill the GPU). Four channels are summed side by side and
 // exchanged within the quad so that lane q ends up with channel c + q. The
 // optional weights multiply (wgt, wgt_c channels) happens on the way out.
+// foot, perm: of n samples; M: samples of a channel of ksp.
 // Needs even grid sides of at least 16 cells (2N grids of N >= 8).
 // One B200, 8-coil 128^3 kooshball, 5.12 M samples: 9.17 ms a thread per
 // sample, 5.3 ms by quads (3.9 ms from the grid in fours of coils below).
@@ -607,18 +608,18 @@ struct Quad {
 
 template <int TZ>
 __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* __restrict__ foot,
-		const int* __restrict__ perm, long M, GridGeom g, int C, int cpb, const float2* __restrict__ grid,
+		const int* __restrict__ perm, long n, long M, GridGeom g, int C, int cpb, const float2* __restrict__ grid,
 		float2* __restrict__ ksp, const float2* __restrict__ wgt, int wgt_c)
 {
 	const int q = threadIdx.x & 3;
 	const long s = ((long)blockIdx.x * BIN_THREADS + threadIdx.x) / 4;
-	const long i = min(s, M - 1);		// surplus quads repeat the last sample and write nothing
+	const long i = min(s, n - 1);		// surplus quads repeat the last sample and write nothing
 	const long m = perm[i];
 	const Quad<TZ> d(foot, i, g);
 	const float* f = d.f;
 	const float w0 = d.w0, w1 = d.w1;
 	const bool act = (0.f != w0) || (0.f != w1);
-	const bool valid = (s < M);
+	const bool valid = (s < n);
 	const int c0 = blockIdx.y * cpb, c1 = min(C, c0 + cpb);
 	int c = c0;
 
@@ -701,12 +702,12 @@ __device__ __forceinline__ void degrid6_by4(const float4* __restrict__ gp, long 
 }
 
 __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_by4(const float4* __restrict__ foot,
-		const int* __restrict__ perm, long M, GridGeom g, int C, int cpb, const float2* __restrict__ grid,
+		const int* __restrict__ perm, long n, long M, GridGeom g, int C, int cpb, const float2* __restrict__ grid,
 		float2* __restrict__ ksp, const float2* __restrict__ wgt, int wgt_c)
 {
 	const int q = threadIdx.x & 3, h = q & 1, odd = q >> 1;
 	const long s = ((long)blockIdx.x * BIN_THREADS + threadIdx.x) / 4;
-	const long i = min(s, M - 1);		// surplus quads repeat the last sample and write nothing
+	const long i = min(s, n - 1);		// surplus quads repeat the last sample and write nothing
 	const long m = perm[i];
 	const float4 lo = foot[i * FOOT_F4];
 	const float* f = (const float*)(foot + i * FOOT_F4);
@@ -734,7 +735,7 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_by4(const float4* __
 		float2 r = cadd(odd ? a[1] : a[0], shfl_xor2(odd ? a[0] : a[1], 2));
 		c += 2 * h + odd;
 
-		if (s < M) {
+		if (s < n) {
 
 			if (wgt)
 				r = cmul(r, wgt[m + M * (c % wgt_c)]);
@@ -769,12 +770,12 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_by4(const float4* __
 // spokes, 51.8 us; 27 us by quads). The grid must be cleared.
 template <int TZ>
 __global__ void __launch_bounds__(BIN_THREADS) k_grid6_quads(const float4* __restrict__ foot,
-		const int* __restrict__ perm, long M, GridGeom g, int C, const float2* __restrict__ ksp,
+		const int* __restrict__ perm, long n, long M, GridGeom g, int C, const float2* __restrict__ ksp,
 		float2* __restrict__ grid)
 {
 	const long i = ((long)blockIdx.x * BIN_THREADS + threadIdx.x) / 4;
 
-	if (i >= M)
+	if (i >= n)
 		return;
 
 	const long m = perm[i];

@@ -139,3 +139,44 @@ def test_plan_memory_of_many_samples():
     16 of two channels' k-space: 165. The set-up's own arrays (order, its sort and
     the start cells) stay below 32. (At the bound of 18 hits: 204 and those.)"""
     assert _plan_bytes_per_sample(1 << 23, 2) < 165 + 32
+
+
+def test_plan_memory_of_many_samples_one_channel():
+    """Plans without tiles keep the footprints of 2^25 samples, 96 bytes each: of
+    2^26 samples 48 bytes a sample, and 4 of order, 16 of trajectory and less
+    than 28 of the set-up's own arrays. (96 with all footprints.)"""
+    assert _plan_bytes_per_sample(1 << 26, 1) < 68 + 28
+
+
+def test_more_samples_than_footprints():
+    """2^25 + 3 * 2^20 samples in one channel, with weights, more than a plan keeps
+    footprints of: forward has the same bits as a plan of the last 2^21 samples,
+    and the adjoint is the sum of those of the first and the other 2^25. Some
+    1200 terms in a cell of the grid: 1200^(1/2) 2^-24 = 2.1e-6."""
+    import torch
+    N, M, last, first = 512, (1 << 25) + 3 * (1 << 20), 1 << 21, 1 << 25
+    gen = torch.Generator(device="cuda").manual_seed(5)
+    t = torch.zeros(M, 3, dtype=torch.complex64, device="cuda")
+    t[:, :2] = (torch.rand(M, 2, generator=gen, device="cuda") - 0.5) * N
+    y = torch.view_as_complex(torch.randn(M, 2, generator=gen, device="cuda"))
+    w = torch.rand(M, generator=gen, device="cuda").to(torch.complex64)
+    x = torch.view_as_complex(torch.randn(N * N, 2, generator=gen, device="cuda"))
+
+    def plan(sel):
+        n = t[sel].shape[0] // 1024
+        return nufft_create2([1, 1024, n, 1], [N, N, 1, 1], [3, 1024, n], t[sel].contiguous(), [1, 1024, n],
+                             w[sel].contiguous(), conf=NufftConf(toeplitz=False))
+
+    op = plan(slice(0, M))
+    fwd, adj = op.forward(x), op.adjoint(y).to(torch.complex128)
+    op.free()
+    parts = []
+    for sel in (slice(0, first), slice(first, M)):
+        op = plan(sel)
+        parts.append(op.adjoint(y[sel].contiguous()).to(torch.complex128))
+        op.free()
+    op = plan(slice(M - last, M))
+    assert torch.equal(torch.view_as_real(op.forward(x)), torch.view_as_real(fwd[M - last:].contiguous()))
+    op.free()
+    want = parts[0] + parts[1]
+    assert float(torch.linalg.vector_norm(adj - want) / torch.linalg.vector_norm(want)) < 2.1e-6
