@@ -1706,13 +1706,8 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 	// the trajectory only, so every apply reads them instead of recomputing
 	// 18 table lookups per sample. Tiles need all of them (they read in hit
 	// order); plans without tiles keep those of up to FOOT_MOST samples, 3.2 GB,
-	// and of more samples make them again, FOOT_MOST at a time. The quad kernels need sides of at least 16
-	// cells and z offsets that fit an int; other sizes take the generic ones.
-	b.quads = (6.f == g.width) && (g.gsz < (1L << 31));
-
-	for (int a = 0; a < 3; a++)
-		b.quads = b.quads && ((1 == g.G[a]) || (g.G[a] >= 16));
-
+	// and of more samples make them again, FOOT_MOST at a time.
+	b.quads = (6.f == g.width);
 	short4* lo4 = nullptr;
 
 	if ((b.tg_cfg >= 0) || b.quads) {

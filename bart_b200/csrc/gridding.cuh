@@ -491,13 +491,13 @@ __global__ void k_foot(const float4* __restrict__ traj, const int* __restrict__ 
 // exchanged within the quad so that lane q ends up with channel c + q. The
 // optional weights multiply (wgt, wgt_c channels) happens on the way out.
 // foot, perm: of n samples; M: samples of a channel of ksp.
-// Needs even grid sides of at least 16 cells (2N grids of N >= 8).
+// Grid sides are even (2N, N even), so the pairs are aligned.
 // One B200, 8-coil 128^3 kooshball, 5.12 M samples: 9.17 ms a thread per
 // sample, 5.3 ms by quads (3.9 ms from the grid in fours of coils below).
 template <int CC, int TZ>
-__device__ __forceinline__ void degrid6_quad(const float2* __restrict__ gc, long gsz, const float* __restrict__ f,
-		const int (&zoff)[TZ], const int (&row)[6], const float (&wy)[6], float w0, float w1, bool act,
-		float2 (&acc)[CC])
+__device__ __forceinline__ void degrid6_quad(const float2* __restrict__ gc, long gsz, long plane,
+		const float* __restrict__ f, const int (&zc)[TZ], const int (&row)[6], const float (&wy)[6], float w0, float w1,
+		bool act, float2 (&acc)[CC])
 {
 #pragma unroll
 	for (int c = 0; c < CC; c++)
@@ -510,20 +510,21 @@ __device__ __forceinline__ void degrid6_quad(const float2* __restrict__ gc, long
 	for (int a = 0; a < TZ; a++) {
 
 		const float dz = f[16 + a];
-		int zo = zoff[0];
+		int z = zc[0];
 #pragma unroll
 		for (int k = 1; k < TZ; k++)
-			zo = (k == a) ? zoff[k] : zo;
+			z = (k == a) ? zc[k] : z;
+
+		const float2* gz = gc + z * plane;
 #pragma unroll
 		for (int b = 0; b < 6; b++) {
 
 			const float dzy = __fmul_rn(dz, wy[b]);
 			const float d0 = __fmul_rn(dzy, w0), d1 = __fmul_rn(dzy, w1);
-			const long o = (long)zo + row[b];
 #pragma unroll
 			for (int c = 0; c < CC; c++) {
 
-				const float4 v = *(const float4*)(gc + gsz * c + o);
+				const float4 v = *(const float4*)(gz + gsz * c + row[b]);
 				acc[c].x = fmaf(v.x, d0, acc[c].x);
 				acc[c].y = fmaf(v.y, d0, acc[c].y);
 				acc[c].x = fmaf(v.z, d1, acc[c].x);
@@ -560,13 +561,13 @@ __device__ __forceinline__ int cell_of(int c, int N, int G, int periodic)
 }
 
 // what a lane of a quad needs of its sample: two x cells and their weights, the
-// row and plane offsets of its taps, the y weights
+// row offsets and z cells of its taps, the y weights
 template <int TZ>
 struct Quad {
 
 	const float* f;			// the footprint record (z weights at 16)
 	float w0, w1;
-	int row[6], zoff[TZ];		// x cell included in row
+	int row[6], zc[TZ];		// x cell included in row
 	float wy[6];
 
 	__device__ __forceinline__ Quad(const float4* foot, long i, const GridGeom& g)
@@ -588,10 +589,14 @@ struct Quad {
 			lo = min(max(lo, -6), g.G[0]);	// further out all weights are 0
 		}
 
+		// (sides below eight cells hold the window more than once)
 		const int u = lo + g.N[0];
 		int e = (u & ~1) + 2 * q;
 		const int t = e - u;			// -1 .. 6
-		e = (e >= g.G[0]) ? e - g.G[0] : e;
+		e = (e < 0) ? e + 2 * g.G[0] : e;
+
+		while (e >= g.G[0])
+			e -= g.G[0];
 		w0 = ((t >= 0) && (t < 6)) ? f[4 + t] : 0.f;
 		w1 = (t < 5) ? f[5 + t] : 0.f;
 #pragma unroll
@@ -602,7 +607,7 @@ struct Quad {
 		}
 #pragma unroll
 		for (int a = 0; a < TZ; a++)
-			zoff[a] = (TZ > 1) ? cell_of(__float_as_int(h.z) + a, g.N[2], g.G[2], g.periodic) * g.G[1] * g.G[0] : 0;
+			zc[a] = (TZ > 1) ? cell_of(__float_as_int(h.z) + a, g.N[2], g.G[2], g.periodic) : 0;
 	}
 };
 
@@ -620,13 +625,14 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* 
 	const float w0 = d.w0, w1 = d.w1;
 	const bool act = (0.f != w0) || (0.f != w1);
 	const bool valid = (s < n);
+	const long plane = (long)g.G[0] * g.G[1];
 	const int c0 = blockIdx.y * cpb, c1 = min(C, c0 + cpb);
 	int c = c0;
 
 	for (; c + 3 < c1; c += 4) {
 
 		float2 acc[4];
-		degrid6_quad<4, TZ>(grid + g.gsz * c, g.gsz, f, d.zoff, d.row, d.wy, w0, w1, act, acc);
+		degrid6_quad<4, TZ>(grid + g.gsz * c, g.gsz, plane, f, d.zc, d.row, d.wy, w0, w1, act, acc);
 		float2 k0 = (q & 2) ? acc[2] : acc[0], k1 = (q & 2) ? acc[3] : acc[1];
 		k0 = cadd(k0, shfl_xor2((q & 2) ? acc[0] : acc[2], 2));
 		k1 = cadd(k1, shfl_xor2((q & 2) ? acc[1] : acc[3], 2));
@@ -644,7 +650,7 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* 
 	for (; c < c1; c++) {
 
 		float2 acc[1];
-		degrid6_quad<1, TZ>(grid + g.gsz * c, g.gsz, f, d.zoff, d.row, d.wy, w0, w1, act, acc);
+		degrid6_quad<1, TZ>(grid + g.gsz * c, g.gsz, plane, f, d.zc, d.row, d.wy, w0, w1, act, acc);
 		float2 r = cadd(acc[0], shfl_xor2(acc[0], 2));
 		r = cadd(r, shfl_xor2(r, 1));
 
@@ -665,8 +671,8 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_quads(const float4* 
 // and mostly within one cache line: 27 lines per sample and channel instead
 // of 50 (the gather is bound by the L1's lines per request).
 template <int NP>
-__device__ __forceinline__ void degrid6_by4(const float4* __restrict__ gp, long plane, const float* __restrict__ f,
-		const int (&zoff)[6], const int (&row)[6], const float (&wy)[6], const int (&xo)[3], const float (&wx)[3],
+__device__ __forceinline__ void degrid6_by4(const float4* __restrict__ gp, long group, long plane,
+		const float* __restrict__ f, const int (&zc)[6], const int (&row)[6], const float (&wy)[6], const int (&xo)[3], const float (&wx)[3],
 		float2 (&acc)[NP][2])
 {
 #pragma unroll
@@ -676,15 +682,17 @@ __device__ __forceinline__ void degrid6_by4(const float4* __restrict__ gp, long 
 	for (int a = 0; a < 6; a++) {
 
 		const float dz = f[16 + a];
-		int zo = zoff[0];
+		int z = zc[0];
 #pragma unroll
 		for (int k = 1; k < 6; k++)
-			zo = (k == a) ? zoff[k] : zo;
+			z = (k == a) ? zc[k] : z;
+
+		const float4* gz = gp + z * plane;
 #pragma unroll
 		for (int b = 0; b < 6; b++) {
 
 			const float dzy = __fmul_rn(dz, wy[b]);
-			const float4* r = gp + 2 * (long)(zo + row[b]);
+			const float4* r = gz + 2 * row[b];
 #pragma unroll
 			for (int k = 0; k < 3; k++) {
 
@@ -692,7 +700,7 @@ __device__ __forceinline__ void degrid6_by4(const float4* __restrict__ gp, long 
 #pragma unroll
 				for (int p = 0; p < NP; p++) {
 
-					const float4 v = r[plane * p + xo[k]];
+					const float4 v = r[group * p + xo[k]];
 					acc[p][0] = cfma(make_float2(v.x, v.y), make_float2(d, d), acc[p][0]);
 					acc[p][1] = cfma(make_float2(v.z, v.w), make_float2(d, d), acc[p][1]);
 				}
@@ -711,13 +719,13 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_by4(const float4* __
 	const long m = perm[i];
 	const float4 lo = foot[i * FOOT_F4];
 	const float* f = (const float*)(foot + i * FOOT_F4);
-	int zoff[6], row[6], xo[3];
+	int zc[6], row[6], xo[3];
 	float wy[6], wx[3];
 #pragma unroll
 	for (int t = 0; t < 6; t++) {
 
 		row[t] = cell_of(__float_as_int(lo.y) + t, g.N[1], g.G[1], g.periodic) * g.G[0];
-		zoff[t] = cell_of(__float_as_int(lo.z) + t, g.N[2], g.G[2], g.periodic) * g.G[1] * g.G[0];
+		zc[t] = cell_of(__float_as_int(lo.z) + t, g.N[2], g.G[2], g.periodic);
 		wy[t] = f[10 + t];
 	}
 #pragma unroll
@@ -728,7 +736,7 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_by4(const float4* __
 	}
 
 	const int c1 = min(C, (int)blockIdx.y * cpb + cpb);
-	const long plane = 2 * g.gsz;		// in 16-byte words
+	const long group = 2 * g.gsz, plane = 2L * g.G[0] * g.G[1];		// in 16-byte words
 
 	// the quad's two halves of a sum are exchanged: lane q keeps channel 2 h + odd
 	auto store = [&](const float2 (&a)[2], int c) {
@@ -749,7 +757,7 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_by4(const float4* __
 	for (; c + 7 < c1; c += 8) {
 
 		float2 acc[2][2];
-		degrid6_by4<2>((const float4*)grid + plane * (c / 4) + h, plane, f, zoff, row, wy, xo, wx, acc);
+		degrid6_by4<2>((const float4*)grid + group * (c / 4) + h, group, plane, f, zc, row, wy, xo, wx, acc);
 		store(acc[0], c);
 		store(acc[1], c + 4);
 	}
@@ -757,7 +765,7 @@ __global__ void __launch_bounds__(BIN_THREADS, 3) k_degrid6_by4(const float4* __
 	if (c < c1) {
 
 		float2 acc[1][2];
-		degrid6_by4<1>((const float4*)grid + plane * (c / 4) + h, plane, f, zoff, row, wy, xo, wx, acc);
+		degrid6_by4<1>((const float4*)grid + group * (c / 4) + h, group, plane, f, zc, row, wy, xo, wx, acc);
 		store(acc[0], c);
 	}
 }
@@ -792,6 +800,7 @@ __global__ void __launch_bounds__(BIN_THREADS) k_grid6_quads(const float4* __res
 			continue;	// grid(): samples that are zero are skipped
 
 		float2* gc = grid + g.gsz * c;
+		const long plane = (long)g.G[0] * g.G[1];
 #pragma unroll
 		for (int a = 0; a < TZ; a++) {
 
@@ -805,7 +814,7 @@ __global__ void __launch_bounds__(BIN_THREADS) k_grid6_quads(const float4* __res
 					continue;
 
 				const float d0 = __fmul_rn(dzy, d.w0), d1 = __fmul_rn(dzy, d.w1);
-				atomicAdd((float4*)(gc + ((long)d.zoff[a] + d.row[b])),
+				atomicAdd((float4*)(gc + (d.zc[a] * plane + d.row[b])),
 						make_float4(val.x * d0, val.y * d0, val.x * d1, val.y * d1));
 			}
 		}

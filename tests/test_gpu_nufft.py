@@ -339,7 +339,13 @@ def test_tiled_scatter_matches_atomic(N, spokes, coils, nd, periodic, monkeypatc
 
 @pytest.mark.parametrize("deterministic", [False, True])
 @pytest.mark.parametrize("dims,samples,spokes,coils,periodic,weights", [
-    ((8, 8, 1), 16, 5, 1, False, False),        # the smallest sides of the quad kernels
+    ((8, 8, 1), 16, 5, 1, False, False),        # a side of the quads' window twice over
+    ((2, 4, 1), 16, 5, 1, False, False),        # shorter than the window, the smallest of all
+    ((2, 4, 1), 16, 5, 3, True, False),         # the same, wrapping around several times
+    ((6, 40, 1), 60, 9, 2, True, True),
+    ((40, 6, 4), 60, 30, 4, False, True),       # a thin volume
+    ((40, 4, 2), 60, 30, 3, True, False),       # the same, the footprint longer than an axis
+    ((4, 6, 16), 40, 30, 8, True, False),       # four coils side by side on a short x
     ((50, 26, 1), 71, 33, 3, False, True),      # tiles cut short on both axes, odd coils, weights
     ((50, 50, 1), 100, 40, 2, True, False),     # the same, wrapping around
     ((100, 60, 1), 200, 300, 13, False, False),  # several chunks per tile, two coil jobs, the second partial
