@@ -1558,6 +1558,56 @@ static int scan_ints(const int* in, int n, int* out, cudaStream_t st)
 	return BNUFFT_OK;
 }
 
+// Count or fill the tiles' hits. large: room for the number and the list of the tiles
+// with many candidates (made by the count); none: a block for every tile.
+static int tile_hits(const OpCtx& op, const short4* lo4, const int* bin_start, const TileHits& th, int* large, cudaStream_t st)
+{
+	const Bins& b = op.bins;
+	const GridGeom gg = grid_geom(op.g);
+
+	if (large) {
+
+		if (!th.work_start)
+			CUDA_TRY(cudaMemsetAsync(large, 0, sizeof(int), st));
+
+		k_tile_hits_warp<<<(unsigned)std::min<long>((b.ntiles + 7) / 8, 8 * 148), TH_THREADS, 0, st>>>(lo4, bin_start, gg, b.bg,
+				b.ntiles, th, large + 1, large);
+		LAUNCHED();
+	}
+
+	auto kern = large ? k_tile_hits<true> : k_tile_hits<false>;
+	kern<<<(unsigned)std::min<long>(b.ntiles, 16 * 148), TH_THREADS, 0, st>>>(lo4, bin_start, gg, b.bg, b.ntiles, th,
+			large ? large + 1 : nullptr, large);
+	LAUNCHED();
+	return BNUFFT_OK;
+}
+
+// The tiles' starts from their hits: one block for few tiles, else segments
+// of at least 8192 tiles, at most 1024 of them, summed first (one block walking the
+// 131072 tiles of a 256^3 grid took 0.27 ms, the two launches take 0.03)
+static int plan_tiles(const Bins& b, const int* nhits, cudaStream_t st)
+{
+	const long nt = b.ntiles;
+	const long seg = std::max(8192L, ((nt + 1023) / 1024 + 1023) / 1024 * 1024);
+	const unsigned nseg = (unsigned)((nt + seg - 1) / seg);
+	TileSums* sums = nullptr;
+
+	if (nseg > 1) {
+
+		CUDA_TRY(cudaMallocAsync(&sums, sizeof(TileSums) * nseg, st));
+		k_tile_sums<<<nseg, 1024, 0, st>>>(nhits, (int)nt, b.chunk, (int)seg, sums);
+		LAUNCHED();
+	}
+
+	k_tile_plan<<<nseg, 1024, 0, st>>>(nhits, (int)nt, b.chunk, (int)seg, sums, b.hit_start, b.work_start, b.slot, b.multi);
+	LAUNCHED();
+
+	if (sums)
+		cudaFreeAsync(sums, st);
+
+	return BNUFFT_OK;
+}
+
 // The sub-blocks of the shared-memory tile scatter and its sorted trajectory
 static int build_sub_blocks(OpCtx& op, const int* bin_start, long nbins, cudaStream_t st)
 {
@@ -1754,12 +1804,14 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		if (det)
 			CUDA_TRY(cudaMallocAsync(&b.slot, sizeof(int) * (nt + 1), st));
 
-		const unsigned hb = (unsigned)std::min<long>(nt, 16 * 148);
-		k_tile_hits<<<hb, TH_THREADS, 0, st>>>(lo4, bin_start, grid_geom(g), bg, nt, nhits, nullptr, nullptr, nullptr,
-				nullptr, nullptr);
-		LAUNCHED();
-		k_tile_plan<<<1, 1024, 0, st>>>(nhits, (int)nt, b.chunk, b.hit_start, b.work_start, b.slot, b.multi);
-		LAUNCHED();
+		TileHits th = { nhits, nullptr, nullptr, nullptr, nullptr, nullptr };
+		int* large = nullptr;
+
+		if (27 * M < TH_MEAN * nt)
+			CUDA_TRY(cudaMallocAsync(&large, sizeof(int) * (1 + std::min(nt, 27 * M / TH_WARP_MOST + 1)), st));
+
+		TRY(tile_hits(op, lo4, bin_start, th, large, st));
+		TRY(plan_tiles(b, nhits, st));
 
 		// lists and work items: at most so many; the lists are made as long as
 		// counted where the bound (18 hits a sample in 3D, 8.2 on average) would
@@ -1795,9 +1847,12 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		CUDA_TRY(cudaMallocAsync(&b.hits, sizeof(int) * std::max(1L, total), st));
 		CUDA_TRY(cudaMallocAsync(&b.work_tile, sizeof(int) * b.nwork_max, st));
 		CUDA_TRY(cudaMallocAsync(&b.work_chunk, sizeof(int) * b.nwork_max, st));
-		k_tile_hits<<<hb, TH_THREADS, 0, st>>>(lo4, bin_start, grid_geom(g), bg, nt, nullptr, b.hit_start, b.hits,
-				b.work_start, b.work_tile, b.work_chunk);
-		LAUNCHED();
+		th = { nullptr, b.hit_start, b.hits, b.work_start, b.work_tile, b.work_chunk };
+		TRY(tile_hits(op, lo4, bin_start, th, large, st));
+
+		if (large)
+			cudaFreeAsync(large, st);
+
 		cudaFreeAsync(lo4, st);
 		cudaFreeAsync(nhits, st);
 

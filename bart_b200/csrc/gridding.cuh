@@ -869,60 +869,163 @@ __device__ __forceinline__ int foot_rel(int lo, int origin, int G, int periodic)
 
 // The hits of every tile: the samples of its 3^d neighbour bins (bins are tiles;
 // a footprint reaches three cells either side of its sample) whose footprint
-// meets it, in bin order, so the lists are the same every time. A block takes a
-// tile; the x neighbours of a row of bins are one range of the sorted samples
-// (two where a periodic grid wraps), and the block walks all ranges as one
-// list. lo: the footprints' start cells. work_start == nullptr: count into
-// nhits; else fill hits from hit_start on, and the tile's work items.
-enum { TH_THREADS = 256, TH_RANGES = 18 };
+// meets it, in bin order, so the lists are the same every time. The x neighbours
+// of a row of bins are one range of the sorted samples (two where a periodic grid
+// wraps), and all ranges are walked as one list of candidates. lo: the footprints'
+// start cells. work_start == nullptr: count into nhits; else fill hits from
+// hit_start on, and the tile's work items.
+// k_tile_hits: a block per tile. k_tile_hits_warp: a warp per tile of at most
+// TH_WARP_MOST candidates, the other ones into a list for k_tile_hits. The warps
+// serve grids whose tiles have less than TH_MEAN candidates on average (uniform
+// samples, two coils, plan creation by blocks and by warps: 5.12 M on a 1024^3 grid,
+// 16 candidates, 47.4 and 11.1 ms; on 512^3, 132, 7.1 and 4.0 ms; on 256^3, 1054,
+// 2.6 and 3.4 ms).
+enum { TH_THREADS = 256, TH_RANGES = 18, TH_WARP_MOST = 1024, TH_MEAN = 256 };
 
-__global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restrict__ lo, const int* __restrict__ bin_start,
-		GridGeom g, BinGeom bg, long ntiles, int* __restrict__ nhits, const long* __restrict__ hit_start,
-		int* __restrict__ hits, const int* __restrict__ work_start, int* __restrict__ work_tile,
-		int* __restrict__ work_chunk)
+struct TileHits {
+
+	int* nhits;			// count
+	const long* hit_start;		// fill
+	int* hits;
+	const int* work_start;
+	int* work_tile;
+	int* work_chunk;
+};
+
+__device__ __forceinline__ int hit_ranges(const BinGeom& bg) { return 2 * ((bg.nb[1] > 1) ? 3 : 1) * ((bg.nb[2] > 1) ? 3 : 1); }
+
+// range r (first sample, samples) of tile (bx, by, bz): part (0, or 1 past the
+// periodic edge) of a neighbour row
+__device__ __forceinline__ int2 hit_range(int r, int bx, int by, int bz, const int* bin_start, const GridGeom& g, const BinGeom& bg)
+{
+	const int ry = (bg.nb[1] > 1) ? 1 : 0, rz = (bg.nb[2] > 1) ? 1 : 0;
+	int y = by + (r / 2) % (2 * ry + 1) - ry, z = bz + (r / 2) / (2 * ry + 1) - rz;
+	int x0 = bx - 1, x1 = bx + 2;
+
+	if (g.periodic) {
+
+		y = (y < 0) ? y + bg.nb[1] : ((y >= bg.nb[1]) ? y - bg.nb[1] : y);
+		z = (z < 0) ? z + bg.nb[2] : ((z >= bg.nb[2]) ? z - bg.nb[2] : z);
+	}
+
+	bool ok = (y >= 0) && (y < bg.nb[1]) && (z >= 0) && (z < bg.nb[2]);
+
+	if (0 == r % 2) {
+
+		x0 = max(x0, 0);
+		x1 = min(x1, bg.nb[0]);
+
+	} else {
+
+		ok = ok && g.periodic && ((x0 < 0) || (x1 > bg.nb[0]));
+		x0 = (x0 < 0) ? bg.nb[0] - 1 : 0;
+		x1 = x0 + 1;
+	}
+
+	const long row = (long)bg.nb[0] * (y + (long)bg.nb[1] * z);
+	const int s0 = ok ? bin_start[row + x0] : 0;
+	return make_int2(s0, ok ? bin_start[row + x1] - s0 : 0);
+}
+
+// a sample's footprint meets the tile at (ox, oy, oz)
+__device__ __forceinline__ bool is_hit(short4 l, int ox, int oy, int oz, const GridGeom& g, const BinGeom& bg)
+{
+	const int lx = foot_rel(l.x, ox, g.G[0], g.periodic), ly = foot_rel(l.y, oy, g.G[1], g.periodic);
+	const int lz = foot_rel(l.z, oz, g.G[2], g.periodic);
+	return (lx > -6) && (lx < bg.bs[0]) && (ly > -6) && (ly < bg.bs[1]) && (lz > -6) && (lz < bg.bs[2]);
+}
+
+__global__ void __launch_bounds__(TH_THREADS) k_tile_hits_warp(const short4* __restrict__ lo, const int* __restrict__ bin_start,
+		GridGeom g, BinGeom bg, long ntiles, TileHits th, int* __restrict__ large, int* __restrict__ nlarge)
+{
+	const int lane = threadIdx.x % 32, nr = hit_ranges(bg);
+
+	for (long t = ((long)blockIdx.x * TH_THREADS + threadIdx.x) / 32; t < ntiles; t += (long)gridDim.x * (TH_THREADS / 32)) {
+
+		const int bx = (int)(t % bg.nb[0]), by = (int)((t / bg.nb[0]) % bg.nb[1]), bz = (int)(t / ((long)bg.nb[0] * bg.nb[1]));
+		const int ox = bx * bg.bs[0], oy = by * bg.bs[1], oz = bz * bg.bs[2];
+		const int2 range = (lane < nr) ? hit_range(lane, bx, by, bz, bin_start, g, bg) : make_int2(0, 0);
+		int end = range.y;		// candidates up to this lane's range
+
+		for (int o = 1; o < 32; o <<= 1) {
+
+			const int u = __shfl_up_sync(0xffffffffu, end, o);
+			end += (lane >= o) ? u : 0;
+		}
+
+		const int total = __shfl_sync(0xffffffffu, end, 31);
+
+		if (total > TH_WARP_MOST) {
+
+			if (!th.work_start && (0 == lane))
+				large[atomicAdd(nlarge, 1)] = (int)t;
+
+			continue;
+		}
+
+		int* dst = th.work_start ? th.hits + th.hit_start[t] : nullptr;
+		int n = 0;
+
+		for (int base = 0; base < total; base += 32) {
+
+			const int c = base + lane;
+			int i = -1;
+
+			for (int r = 0; r < nr; r++) {
+
+				const int e = __shfl_sync(0xffffffffu, end, r), k = __shfl_sync(0xffffffffu, range.y, r);
+				const int s = __shfl_sync(0xffffffffu, range.x, r);
+				i = ((c < e) && (c >= e - k)) ? s + c - (e - k) : i;
+			}
+
+			const bool hit = (i >= 0) && is_hit(lo[i], ox, oy, oz, g, bg);
+			const unsigned m = __ballot_sync(0xffffffffu, hit);
+
+			if (hit && dst)
+				dst[n + __popc(m & ((1u << lane) - 1u))] = i;
+
+			n += __popc(m);
+		}
+
+		if (!th.work_start) {
+
+			if (0 == lane)
+				th.nhits[t] = n;
+
+		} else {
+
+			const int w0 = th.work_start[t], w1 = th.work_start[t + 1];
+
+			for (int w = w0 + lane; w < w1; w += 32) {
+
+				th.work_tile[w] = (int)t;
+				th.work_chunk[w] = w - w0;
+			}
+		}
+	}
+}
+
+// LIST: takes the *nlist tiles of list instead of all
+template <bool LIST>
+__global__ void __launch_bounds__(TH_THREADS, 6) k_tile_hits(const short4* __restrict__ lo, const int* __restrict__ bin_start,
+		GridGeom g, BinGeom bg, long ntiles, TileHits th, const int* __restrict__ list, const int* __restrict__ nlist)
 {
 	__shared__ int wcount[TH_THREADS / 32];
 	__shared__ int rs[TH_RANGES], rn[TH_RANGES];	// ranges: first sample, samples
-	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-	const int ry = (bg.nb[1] > 1) ? 1 : 0, rz = (bg.nb[2] > 1) ? 1 : 0;
-	const int nr = 2 * (2 * ry + 1) * (2 * rz + 1);
+	const int warp = threadIdx.x / 32, lane = threadIdx.x % 32, nr = hit_ranges(bg);
+	const long n = LIST ? *nlist : ntiles;
 
-	for (long t = blockIdx.x; t < ntiles; t += gridDim.x) {
+	for (long j = blockIdx.x; j < n; j += gridDim.x) {
 
+		const long t = LIST ? list[j] : j;
 		const int bx = (int)(t % bg.nb[0]), by = (int)((t / bg.nb[0]) % bg.nb[1]), bz = (int)(t / ((long)bg.nb[0] * bg.nb[1]));
 		const int ox = bx * bg.bs[0], oy = by * bg.bs[1], oz = bz * bg.bs[2];
 
 		if ((int)threadIdx.x < nr) {
 
-			// range r: part (0, or 1 past the periodic edge) of neighbour row (y, z)
-			const int r = threadIdx.x;
-			int y = by + (r / 2) % (2 * ry + 1) - ry, z = bz + (r / 2) / (2 * ry + 1) - rz;
-			int x0 = bx - 1, x1 = bx + 2;
-
-			if (g.periodic) {
-
-				y = (y < 0) ? y + bg.nb[1] : ((y >= bg.nb[1]) ? y - bg.nb[1] : y);
-				z = (z < 0) ? z + bg.nb[2] : ((z >= bg.nb[2]) ? z - bg.nb[2] : z);
-			}
-
-			bool ok = (y >= 0) && (y < bg.nb[1]) && (z >= 0) && (z < bg.nb[2]);
-
-			if (0 == r % 2) {
-
-				x0 = max(x0, 0);
-				x1 = min(x1, bg.nb[0]);
-
-			} else {
-
-				ok = ok && g.periodic && ((x0 < 0) || (x1 > bg.nb[0]));
-				x0 = (x0 < 0) ? bg.nb[0] - 1 : 0;
-				x1 = x0 + 1;
-			}
-
-			const long row = (long)bg.nb[0] * (y + (long)bg.nb[1] * z);
-			const int s0 = ok ? bin_start[row + x0] : 0;
-			rs[r] = s0;
-			rn[r] = ok ? bin_start[row + x1] - s0 : 0;
+			const int2 range = hit_range(threadIdx.x, bx, by, bz, bin_start, g, bg);
+			rs[threadIdx.x] = range.x;
+			rn[threadIdx.x] = range.y;
 		}
 
 		__syncthreads();
@@ -931,7 +1034,7 @@ __global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restri
 		for (int r = 0; r < nr; r++)
 			total += rn[r];
 
-		int* dst = work_start ? hits + hit_start[t] : nullptr;	// the tile's list
+		int* dst = th.work_start ? th.hits + th.hit_start[t] : nullptr;	// the tile's list
 		int pos = 0;
 		int count = 0, r = 0, r0 = 0;	// this thread's range and its first candidate
 
@@ -959,16 +1062,9 @@ __global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restri
 			const int i = in;
 			const short4 l = ln;
 			cand(base + TH_THREADS + threadIdx.x, in, ln);
-			bool hit = false;
+			const bool hit = (i >= 0) && is_hit(l, ox, oy, oz, g, bg);
 
-			if (i >= 0) {
-
-				const int lx = foot_rel(l.x, ox, g.G[0], g.periodic), ly = foot_rel(l.y, oy, g.G[1], g.periodic);
-				const int lz = foot_rel(l.z, oz, g.G[2], g.periodic);
-				hit = (lx > -6) && (lx < bg.bs[0]) && (ly > -6) && (ly < bg.bs[1]) && (lz > -6) && (lz < bg.bs[2]);
-			}
-
-			if (!work_start) {
+			if (!th.work_start) {
 
 				count += hit;
 				continue;
@@ -993,7 +1089,7 @@ __global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restri
 				dst[at] = i;
 		}
 
-		if (!work_start) {
+		if (!th.work_start) {
 
 			for (int o = 16; o > 0; o >>= 1)
 				count += __shfl_xor_sync(0xffffffffu, count, o);
@@ -1005,22 +1101,22 @@ __global__ void __launch_bounds__(TH_THREADS) k_tile_hits(const short4* __restri
 
 			if (0 == threadIdx.x) {
 
-				int n = 0;
+				int sum = 0;
 
 				for (int w = 0; w < TH_THREADS / 32; w++)
-					n += wcount[w];
+					sum += wcount[w];
 
-				nhits[t] = n;
+				th.nhits[t] = sum;
 			}
 
 		} else {
 
-			const int w0 = work_start[t], w1 = work_start[t + 1];
+			const int w0 = th.work_start[t], w1 = th.work_start[t + 1];
 
 			for (int w = w0 + threadIdx.x; w < w1; w += TH_THREADS) {
 
-				work_tile[w] = (int)t;
-				work_chunk[w] = w - w0;
+				th.work_tile[w] = (int)t;
+				th.work_chunk[w] = w - w0;
 			}
 		}
 
@@ -1092,22 +1188,102 @@ __global__ void __launch_bounds__(1024) k_scan(const int* __restrict__ in, int n
 		out[n] = sum;
 }
 
-// From the hits per tile, in one block: where each tile's hits, work items
-// (chunks of hits, at least one) and, for tiles with several items, partial
-// tiles begin (slot; deterministic mode), and the list of those tiles.
-__global__ void __launch_bounds__(1024) k_tile_plan(const int* __restrict__ nhits, int ntiles, int chunk,
-		long* __restrict__ hit_start, int* __restrict__ work_start, int* __restrict__ slot, int* __restrict__ multi)
+// What precedes a tile: hits, work items, partial tiles (of tiles with several
+// items) and tiles with several items.
+struct TileSums {
+
+	long hits;
+	int work, slots, multi;
+};
+
+// work items of a tile: chunks of its hits, at least one
+__device__ __forceinline__ int tile_items(int n, int chunk) { return (n > 0) ? (n - 1) / chunk + 1 : 1; }
+
+// the sums over the block's threads, in every thread (sh: one per warp)
+__device__ __forceinline__ TileSums block_sums(TileSums v, TileSums* sh)
+{
+	for (int o = 16; o > 0; o >>= 1) {
+
+		v.hits += __shfl_xor_sync(0xffffffffu, v.hits, o);
+		v.work += __shfl_xor_sync(0xffffffffu, v.work, o);
+		v.slots += __shfl_xor_sync(0xffffffffu, v.slots, o);
+		v.multi += __shfl_xor_sync(0xffffffffu, v.multi, o);
+	}
+
+	if (0 == threadIdx.x % 32)
+		sh[threadIdx.x / 32] = v;
+
+	__syncthreads();
+	TileSums r = { 0, 0, 0, 0 };
+
+	for (int w = 0; w < (int)(blockDim.x / 32); w++) {
+
+		r.hits += sh[w].hits;
+		r.work += sh[w].work;
+		r.slots += sh[w].slots;
+		r.multi += sh[w].multi;
+	}
+
+	__syncthreads();
+	return r;
+}
+
+// the sums of each segment of seg tiles, a block per segment
+__global__ void __launch_bounds__(1024) k_tile_sums(const int* __restrict__ nhits, int ntiles, int chunk, int seg,
+		TileSums* __restrict__ sums)
+{
+	__shared__ TileSums sh[32];
+	const int t0 = blockIdx.x * seg, t1 = min(ntiles - t0, seg) + t0;
+	TileSums v = { 0, 0, 0, 0 };
+
+	for (int t = t0 + threadIdx.x; t < t1; t += 1024) {
+
+		const int n = nhits[t], k = tile_items(n, chunk);
+		v.hits += n;
+		v.work += k;
+		v.slots += (k > 1) ? k : 0;
+		v.multi += (k > 1) ? 1 : 0;
+	}
+
+	v = block_sums(v, sh);
+
+	if (0 == threadIdx.x)
+		sums[blockIdx.x] = v;
+}
+
+// From the hits per tile: where each tile's hits, work items (chunks of hits, at
+// least one) and, for tiles with several items, partial tiles begin (slot;
+// deterministic mode), and the list of those tiles. A block takes a segment of
+// seg tiles; sums: of the segments (not read by a single one).
+__global__ void __launch_bounds__(1024) k_tile_plan(const int* __restrict__ nhits, int ntiles, int chunk, int seg,
+		const TileSums* __restrict__ sums, long* __restrict__ hit_start, int* __restrict__ work_start,
+		int* __restrict__ slot, int* __restrict__ multi)
 {
 	__shared__ int sh[33];
-	long hsum = 0;
-	int wsum = 0, ssum = 0, msum = 0;
+	__shared__ TileSums shs[32];
+	const int t0 = blockIdx.x * seg, t1 = min(ntiles - t0, seg) + t0;
+	TileSums before = { 0, 0, 0, 0 };
 
-	for (int base = 0; base < ntiles; base += 1024) {
+	if (blockIdx.x > 0) {
+
+		for (int b = threadIdx.x; b < (int)blockIdx.x; b += 1024) {
+
+			const TileSums v = sums[b];
+			before.hits += v.hits;
+			before.work += v.work;
+			before.slots += v.slots;
+			before.multi += v.multi;
+		}
+
+		before = block_sums(before, shs);
+	}
+
+	for (int base = t0; base < t1; base += 1024) {
 
 		const int t = base + threadIdx.x;
-		const bool in = (t < ntiles);
+		const bool in = (t < t1);
 		const int n = in ? nhits[t] : 0;
-		const int k = in ? max(1, (n + chunk - 1) / chunk) : 0;
+		const int k = in ? tile_items(n, chunk) : 0;
 		const bool several = (k > 1);
 		int tl, th, tw, ts, tm;
 		const int l = block_scan(n & 0xfffff, sh, tl), h = block_scan(n >> 20, sh, th);	// 1024 counts below 2^31
@@ -1116,31 +1292,31 @@ __global__ void __launch_bounds__(1024) k_tile_plan(const int* __restrict__ nhit
 
 		if (in) {
 
-			hit_start[t] = hsum + l + ((long)h << 20);
-			work_start[t] = wsum + w;
+			hit_start[t] = before.hits + l + ((long)h << 20);
+			work_start[t] = before.work + w;
 
 			if (slot)
-				slot[t] = ssum + s;
+				slot[t] = before.slots + s;
 
 			if (several)
-				multi[msum + m] = t;
+				multi[before.multi + m] = t;
 		}
 
-		hsum += tl + ((long)th << 20);
-		wsum += tw;
-		ssum += ts;
-		msum += tm;
+		before.hits += tl + ((long)th << 20);
+		before.work += tw;
+		before.slots += ts;
+		before.multi += tm;
 	}
 
-	if (0 == threadIdx.x) {
+	if ((t1 == ntiles) && (0 == threadIdx.x)) {
 
-		hit_start[ntiles] = hsum;
-		work_start[ntiles] = wsum;
+		hit_start[ntiles] = before.hits;
+		work_start[ntiles] = before.work;
 
 		if (slot)
-			slot[ntiles] = ssum;
+			slot[ntiles] = before.slots;
 
-		multi[ntiles] = msum;
+		multi[ntiles] = before.multi;
 	}
 }
 

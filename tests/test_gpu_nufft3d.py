@@ -180,3 +180,34 @@ def test_more_samples_than_footprints():
     op.free()
     want = parts[0] + parts[1]
     assert float(torch.linalg.vector_norm(adj - want) / torch.linalg.vector_norm(want)) < 2.1e-6
+
+
+@pytest.mark.parametrize("dims,spokes,chunk,periodic", [((64, 64, 64), 2000, None, False),
+                                                        ((128, 64, 80), 2000, 32, False), ((128, 72, 84), 2000, 32, True)])
+def test_plans_of_many_tiles(dims, spokes, chunk, periodic, monkeypatch):
+    """More tiles than one block plans (16384 in two segments, 40960 in five, 48384
+    in six): the tile scatter and its deterministic form against the
+    single-channel scatter, with hits that fit one work item a tile and with
+    several. Tiles listed by blocks (330 candidates on average) and by warps (130 and
+    110), with more candidates than a warp takes at the centre, and where a
+    periodic grid wraps around tiles cut short. Two orders of the same float32
+    sums of some hundred terms."""
+    rng = np.random.default_rng(dims[0] + spokes)
+    if chunk:
+        monkeypatch.setenv("BNUFFT_GRID_CHUNK", str(chunk))
+    t = rng.uniform(-0.55, 0.55, (3, 100, spokes)) * np.array(dims)[:, None, None]
+    t[:, :, :spokes // 5] *= 0.1            # dense towards the centre
+    t = t.astype(np.complex64)
+    y = _cplx(rng, (1, 100, spokes, 2))
+    kd, cd = [1, 100, spokes, 2], list(dims) + [2]
+    out = []
+    for det in (False, True):
+        op = nufft_create2(kd, cd, list(t.shape), t, conf=NufftConf(toeplitz=False, deterministic=det, periodic=periodic))
+        out.append(np.asarray(op.adjoint(y)).copy().reshape(cd, order="F"))
+        op.free()
+    op = nufft_create2(kd[:3] + [1], list(dims) + [1], list(t.shape), t, conf=NufftConf(toeplitz=False, periodic=periodic))
+    one = [np.asarray(op.adjoint(np.asfortranarray(y[..., c:c + 1]))).copy().reshape(dims, order="F") for c in range(2)]
+    op.free()
+    for c in range(2):
+        assert rel(out[0][..., c], one[c]) < 1e-6
+        assert rel(out[1][..., c], one[c]) < 1e-6
