@@ -114,6 +114,7 @@ def load(path: str = LIB_PATH) -> ctypes.CDLL:
     sig("bnufft_cg_status", i, vp, ctypes.POINTER(i), ctypes.POINTER(i), fp, vp)
     sig("bnufft_cg_free", None, vp)
     sig("bnufft_last_error", ctypes.c_char_p)
+    sig("bnufft_release_memory", i)
     sig("bnufft_launch_count", ctypes.c_long)
     sig("bnufft_prof_start", i, ctypes.c_char_p)
     sig("bnufft_prof_stop", i, ctypes.POINTER(ctypes.c_double), ctypes.POINTER(ctypes.c_long))

@@ -52,6 +52,54 @@ int bn::fail(int code, const char* fmt, ...)
 	return code;
 }
 
+// The library's own stream-ordered memory pool of each device. The device's default
+// pool is the application's: its settings stay as they are. The pool keeps up to an
+// eighth of the device mapped when it is free, so that the next plan or model does
+// not map it again (200 x 180, 12 coils: first call of a new plan 430 us from a pool
+// that gives everything back at each host synchronisation, 215 us so);
+// bnufft_release_memory gives it back.
+static std::atomic<cudaMemPool_t> g_pools[64];
+
+static cudaMemPool_t lib_pool()
+{
+	int dev = 0;
+
+	if ((cudaSuccess != cudaGetDevice(&dev)) || (dev >= 64))
+		return nullptr;
+
+	cudaMemPool_t p = g_pools[dev].load(std::memory_order_acquire);
+
+	if (p)
+		return p;
+
+	static std::mutex mu;
+	std::lock_guard<std::mutex> lock(mu);
+
+	if ((p = g_pools[dev].load(std::memory_order_acquire)))
+		return p;
+
+	cudaMemPoolProps props = {};
+	props.allocType = cudaMemAllocationTypePinned;
+	props.location.type = cudaMemLocationTypeDevice;
+	props.location.id = dev;
+	size_t free_now = 0, total = 0;
+
+	if ((cudaSuccess != cudaMemGetInfo(&free_now, &total)) || (cudaSuccess != cudaMemPoolCreate(&p, &props)))
+		return nullptr;
+
+	uint64_t keep = total / 8;
+	cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+	g_pools[dev].store(p, std::memory_order_release);
+	return p;
+}
+
+template <typename T>
+static cudaError_t pool_malloc(T** p, size_t bytes, cudaStream_t st)
+{
+	cudaMemPool_t pool = lib_pool();
+	return pool ? cudaMallocFromPoolAsync((void**)p, bytes, pool, st) : cudaMallocAsync((void**)p, bytes, st);
+}
+
 // Optional timing of one kernel class (bnufft_prof_start): a pair of CUDA
 // events on the launching stream around every launch of that class.
 static std::mutex g_prof_mutex;
@@ -919,11 +967,11 @@ static int alloc_work(Work& w, const Geom& g, long C, cudaStream_t st)
 	if (w.t2) cudaFreeAsync(w.t2, st);
 	w = Work{};
 
-	CUDA_TRY(cudaMallocAsync(&w.grid, sizeof(float2) * g.gsz * C, st));
-	CUDA_TRY(cudaMallocAsync(&w.t1, sizeof(float2) * (long)g.G[0] * g.N[1] * g.N[2] * C, st));
+	CUDA_TRY(pool_malloc(&w.grid, sizeof(float2) * g.gsz * C, st));
+	CUDA_TRY(pool_malloc(&w.t1, sizeof(float2) * (long)g.G[0] * g.N[1] * g.N[2] * C, st));
 
 	if (g.G[2] > 1)
-		CUDA_TRY(cudaMallocAsync(&w.t2, sizeof(float2) * (long)g.G[0] * g.G[1] * g.N[2] * C, st));
+		CUDA_TRY(pool_malloc(&w.t2, sizeof(float2) * (long)g.G[0] * g.G[1] * g.N[2] * C, st));
 
 	w.cap = C;
 	return BNUFFT_OK;
@@ -1253,7 +1301,7 @@ static int degrid(OpCtx& op, const float2* grid, long C, float2* ksp, cudaStream
 static int alloc_partials(Bins& b, long C, cudaStream_t st)
 {
 	const long cells = (long)b.bg.bs[0] * b.bg.bs[1] * b.bg.bs[2];
-	CUDA_TRY(cudaMallocAsync(&b.part, sizeof(float2) * std::max(1L, b.nslots * C * cells), st));
+	CUDA_TRY(pool_malloc(&b.part, sizeof(float2) * std::max(1L, b.nslots * C * cells), st));
 	b.part_c = C;
 	return BNUFFT_OK;
 }
@@ -1284,7 +1332,7 @@ static int grid_adj(OpCtx& op, const float2* ksp, long C, float2* grid, cudaStre
 	if (op.wgt && !tiles) {
 
 		if (!op.wbuf)
-			CUDA_TRY(cudaMallocAsync(&op.wbuf, sizeof(float2) * op.g.M * C, st));
+			CUDA_TRY(pool_malloc(&op.wbuf, sizeof(float2) * op.g.M * C, st));
 
 		k_weight<<<vec_blocks(op.g.M * C), RED_THREADS, 0, st>>>(op.wbuf, ksp, op.wgt, op.g.M, C, op.wgt_c, 1);
 		LAUNCHED();
@@ -1317,7 +1365,7 @@ static int grid_adj(OpCtx& op, const float2* ksp, long C, float2* grid, cudaStre
 
 			b.kperm = nullptr;
 			b.kperm_c = 0;
-			CUDA_TRY(cudaMallocAsync(&b.kperm, sizeof(float2) * op.g.M * Cp, st));
+			CUDA_TRY(pool_malloc(&b.kperm, sizeof(float2) * op.g.M * Cp, st));
 			b.kperm_c = Cp;
 		}
 
@@ -1467,35 +1515,35 @@ static int build_csr(OpCtx& op, cudaStream_t st)
 	int* counts = nullptr;
 	void* tmp = nullptr;
 	size_t tmp_bytes = 0;
-	CUDA_TRY(cudaMallocAsync(&keys, sizeof(unsigned long long) * n, st));
-	CUDA_TRY(cudaMallocAsync(&keys2, sizeof(unsigned long long) * n, st));
-	CUDA_TRY(cudaMallocAsync(&vals, sizeof(float) * n, st));
-	CUDA_TRY(cudaMallocAsync(&vals2, sizeof(float) * n, st));
+	CUDA_TRY(pool_malloc(&keys, sizeof(unsigned long long) * n, st));
+	CUDA_TRY(pool_malloc(&keys2, sizeof(unsigned long long) * n, st));
+	CUDA_TRY(pool_malloc(&vals, sizeof(float) * n, st));
+	CUDA_TRY(pool_malloc(&vals2, sizeof(float) * n, st));
 
 	k_csr_keys<<<(unsigned)((g.M + 127) / 128), 128, 0, st>>>(op.traj, g.M, grid_geom(g), op.kb, keys, vals, slots_z);
 	LAUNCHED();
 
 	CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, vals, vals2, (int)n, 0, 64, st));
-	CUDA_TRY(cudaMallocAsync(&tmp, tmp_bytes, st));
+	CUDA_TRY(pool_malloc(&tmp, tmp_bytes, st));
 	CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, vals, vals2, (int)n, 0, 64, st));
 	g_launches.fetch_add(1, std::memory_order_relaxed);
 
 	// entries with a valid key come first; count them per cell
 	Csr& c = op.csr;
-	CUDA_TRY(cudaMallocAsync(&counts, sizeof(int) * (g.gsz + 1), st));
+	CUDA_TRY(pool_malloc(&counts, sizeof(int) * (g.gsz + 1), st));
 	CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (g.gsz + 1), st));
-	CUDA_TRY(cudaMallocAsync(&c.row_ptr, sizeof(long) * (g.gsz + 1), st));
+	CUDA_TRY(pool_malloc(&c.row_ptr, sizeof(long) * (g.gsz + 1), st));
 
 	// number of valid entries: taps of every sample (host needs it for sizes)
 	int* col_all = nullptr;
-	CUDA_TRY(cudaMallocAsync(&col_all, sizeof(int) * n, st));
+	CUDA_TRY(pool_malloc(&col_all, sizeof(int) * n, st));
 	k_csr_fill_valid<<<vec_blocks(n), RED_THREADS, 0, st>>>(keys2, n, g.M, g.gsz, col_all, counts);
 	LAUNCHED();
 
 	size_t scan_bytes = 0;
 	void* scan_tmp = nullptr;
 	CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, counts, c.row_ptr, (int)(g.gsz + 1), st));
-	CUDA_TRY(cudaMallocAsync(&scan_tmp, scan_bytes, st));
+	CUDA_TRY(pool_malloc(&scan_tmp, scan_bytes, st));
 	CUDA_TRY(cub::DeviceScan::ExclusiveSum(scan_tmp, scan_bytes, counts, c.row_ptr, (int)(g.gsz + 1), st));
 	g_launches.fetch_add(1, std::memory_order_relaxed);
 
@@ -1551,7 +1599,7 @@ static int scan_ints(const int* in, int n, int* out, cudaStream_t st)
 	void* tmp = nullptr;
 	size_t bytes = 0;
 	CUDA_TRY(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, n + 1, st));
-	CUDA_TRY(cudaMallocAsync(&tmp, bytes, st));
+	CUDA_TRY(pool_malloc(&tmp, bytes, st));
 	CUDA_TRY(cub::DeviceScan::ExclusiveSum(tmp, bytes, in, out, n + 1, st));
 	g_launches.fetch_add(1, std::memory_order_relaxed);
 	cudaFreeAsync(tmp, st);
@@ -1594,7 +1642,7 @@ static int plan_tiles(const Bins& b, const int* nhits, cudaStream_t st)
 
 	if (nseg > 1) {
 
-		CUDA_TRY(cudaMallocAsync(&sums, sizeof(TileSums) * nseg, st));
+		CUDA_TRY(pool_malloc(&sums, sizeof(TileSums) * nseg, st));
 		k_tile_sums<<<nseg, 1024, 0, st>>>(nhits, (int)nt, b.chunk, (int)seg, sums);
 		LAUNCHED();
 	}
@@ -1614,8 +1662,8 @@ static int build_sub_blocks(OpCtx& op, const int* bin_start, long nbins, cudaStr
 	Bins& b = op.bins;
 	const long M = op.g.M;
 	int *nsub = nullptr, *sub_start = nullptr;
-	CUDA_TRY(cudaMallocAsync(&nsub, sizeof(int) * (nbins + 1), st));
-	CUDA_TRY(cudaMallocAsync(&sub_start, sizeof(int) * (nbins + 1), st));
+	CUDA_TRY(pool_malloc(&nsub, sizeof(int) * (nbins + 1), st));
+	CUDA_TRY(pool_malloc(&sub_start, sizeof(int) * (nbins + 1), st));
 
 	// sub-blocks per bin: ceil(count / sub); their start indices. A
 	// sub-block is one block of the tile scatter, which clears and flushes
@@ -1636,10 +1684,10 @@ static int build_sub_blocks(OpCtx& op, const int* bin_start, long nbins, cudaStr
 	b.nsub = (int)total;
 	b.sub_start = sub_start;
 	b.nsub_dev = sub_start + nbins;
-	CUDA_TRY(cudaMallocAsync(&b.sub_bin, sizeof(int) * total, st));
-	CUDA_TRY(cudaMallocAsync(&b.sub_first, sizeof(int) * total, st));
-	CUDA_TRY(cudaMallocAsync(&b.sub_count, sizeof(int) * total, st));
-	CUDA_TRY(cudaMallocAsync(&b.traj, sizeof(float4) * M, st));
+	CUDA_TRY(pool_malloc(&b.sub_bin, sizeof(int) * total, st));
+	CUDA_TRY(pool_malloc(&b.sub_first, sizeof(int) * total, st));
+	CUDA_TRY(pool_malloc(&b.sub_count, sizeof(int) * total, st));
+	CUDA_TRY(pool_malloc(&b.traj, sizeof(float4) * M, st));
 	k_sub_fill<<<vec_blocks(nbins), RED_THREADS, 0, st>>>(bin_start, sub_start, (int)nbins, sub, b.sub_bin, b.sub_first, b.sub_count);
 	LAUNCHED();
 	k_gather_traj<<<vec_blocks(M), RED_THREADS, 0, st>>>(b.traj, op.traj, b.perm, M);
@@ -1721,15 +1769,15 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 	const bool binned = (0 == gridding_kind()) && (6.f == g.width);	// the shared-memory tile scatter
 	const bool starts = binned || (b.tg_cfg >= 0);			// the bins' sample ranges are needed
 
-	CUDA_TRY(cudaMallocAsync(&keys, sizeof(unsigned) * M, st));
-	CUDA_TRY(cudaMallocAsync(&keys2, sizeof(unsigned) * M, st));
-	CUDA_TRY(cudaMallocAsync(&vals, sizeof(int) * M, st));
-	CUDA_TRY(cudaMallocAsync(&b.perm, sizeof(int) * M, st));
+	CUDA_TRY(pool_malloc(&keys, sizeof(unsigned) * M, st));
+	CUDA_TRY(pool_malloc(&keys2, sizeof(unsigned) * M, st));
+	CUDA_TRY(pool_malloc(&vals, sizeof(int) * M, st));
+	CUDA_TRY(pool_malloc(&b.perm, sizeof(int) * M, st));
 
 	if (starts) {
 
-		CUDA_TRY(cudaMallocAsync(&counts, sizeof(int) * (nbins + 1), st));
-		CUDA_TRY(cudaMallocAsync(&bin_start, sizeof(int) * (nbins + 1), st));
+		CUDA_TRY(pool_malloc(&counts, sizeof(int) * (nbins + 1), st));
+		CUDA_TRY(pool_malloc(&bin_start, sizeof(int) * (nbins + 1), st));
 		CUDA_TRY(cudaMemsetAsync(counts, 0, sizeof(int) * (nbins + 1), st));
 	}
 
@@ -1742,7 +1790,7 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		end_bit++;
 
 	CUDA_TRY(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, vals, b.perm, (int)M, 0, end_bit, st));
-	CUDA_TRY(cudaMallocAsync(&tmp, tmp_bytes, st));
+	CUDA_TRY(pool_malloc(&tmp, tmp_bytes, st));
 	CUDA_TRY(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, vals, b.perm, (int)M, 0, end_bit, st));
 	g_launches.fetch_add(1, std::memory_order_relaxed);
 
@@ -1763,10 +1811,10 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 	if ((b.tg_cfg >= 0) || b.quads) {
 
 		b.foot_n = (b.tg_cfg >= 0) ? M : std::min(M, (long)FOOT_MOST);
-		CUDA_TRY(cudaMallocAsync(&b.foot, sizeof(float4) * FOOT_F4 * b.foot_n, st));
+		CUDA_TRY(pool_malloc(&b.foot, sizeof(float4) * FOOT_F4 * b.foot_n, st));
 
 		if (b.tg_cfg >= 0)
-			CUDA_TRY(cudaMallocAsync(&lo4, sizeof(short4) * M, st));
+			CUDA_TRY(pool_malloc(&lo4, sizeof(short4) * M, st));
 
 		if (b.foot_n == M) {
 
@@ -1796,19 +1844,19 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		if (const char* e = getenv("BNUFFT_GRID_CHUNK"))	// tuning knob: hits per work item
 			b.chunk = std::max((int)TG_MIN_CHUNK, std::min(4096, atoi(e)));
 
-		CUDA_TRY(cudaMallocAsync(&nhits, sizeof(int) * nt, st));
-		CUDA_TRY(cudaMallocAsync(&b.hit_start, sizeof(long) * (nt + 1), st));
-		CUDA_TRY(cudaMallocAsync(&b.work_start, sizeof(int) * (nt + 1), st));
-		CUDA_TRY(cudaMallocAsync(&b.multi, sizeof(int) * (nt + 1), st));
+		CUDA_TRY(pool_malloc(&nhits, sizeof(int) * nt, st));
+		CUDA_TRY(pool_malloc(&b.hit_start, sizeof(long) * (nt + 1), st));
+		CUDA_TRY(pool_malloc(&b.work_start, sizeof(int) * (nt + 1), st));
+		CUDA_TRY(pool_malloc(&b.multi, sizeof(int) * (nt + 1), st));
 
 		if (det)
-			CUDA_TRY(cudaMallocAsync(&b.slot, sizeof(int) * (nt + 1), st));
+			CUDA_TRY(pool_malloc(&b.slot, sizeof(int) * (nt + 1), st));
 
 		TileHits th = { nhits, nullptr, nullptr, nullptr, nullptr, nullptr };
 		int* large = nullptr;
 
 		if (27 * M < TH_MEAN * nt)
-			CUDA_TRY(cudaMallocAsync(&large, sizeof(int) * (1 + std::min(nt, 27 * M / TH_WARP_MOST + 1)), st));
+			CUDA_TRY(pool_malloc(&large, sizeof(int) * (1 + std::min(nt, 27 * M / TH_WARP_MOST + 1)), st));
 
 		TRY(tile_hits(op, lo4, bin_start, th, large, st));
 		TRY(plan_tiles(b, nhits, st));
@@ -1844,9 +1892,9 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 			b.nslots = slots;
 		}
 
-		CUDA_TRY(cudaMallocAsync(&b.hits, sizeof(int) * std::max(1L, total), st));
-		CUDA_TRY(cudaMallocAsync(&b.work_tile, sizeof(int) * b.nwork_max, st));
-		CUDA_TRY(cudaMallocAsync(&b.work_chunk, sizeof(int) * b.nwork_max, st));
+		CUDA_TRY(pool_malloc(&b.hits, sizeof(int) * std::max(1L, total), st));
+		CUDA_TRY(pool_malloc(&b.work_tile, sizeof(int) * b.nwork_max, st));
+		CUDA_TRY(pool_malloc(&b.work_chunk, sizeof(int) * b.nwork_max, st));
 		th = { nullptr, b.hit_start, b.hits, b.work_start, b.work_tile, b.work_chunk };
 		TRY(tile_hits(op, lo4, bin_start, th, large, st));
 
@@ -1863,7 +1911,7 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		// applies allocate nothing (their solves can then be captured into
 		// graphs and nested as child graphs)
 		b.kperm_c = tg_row(b.tg_cfg, op.coils);
-		CUDA_TRY(cudaMallocAsync(&b.kperm, sizeof(float2) * M * b.kperm_c, st));
+		CUDA_TRY(pool_malloc(&b.kperm, sizeof(float2) * M * b.kperm_c, st));
 	}
 
 	void* frees[] = { keys, keys2, vals, counts, bin_start, tmp };
@@ -1990,10 +2038,10 @@ static int compute_psf(const Geom& g, const float2* traj_c, const float* kb, flo
 	float2* ones = nullptr;
 	float2* psft = nullptr;
 	float2* psf = nullptr;
-	CUDA_TRY(cudaMallocAsync(&t2, sizeof(float4) * g.M, st));
-	CUDA_TRY(cudaMallocAsync(&ones, sizeof(float2) * g.M * nch, st));
-	CUDA_TRY(cudaMallocAsync(&psft, sizeof(float2) * in.g.npix * nch, st));
-	CUDA_TRY(cudaMallocAsync(&psf, sizeof(float2) * g.gsz * nch, st));
+	CUDA_TRY(pool_malloc(&t2, sizeof(float4) * g.M, st));
+	CUDA_TRY(pool_malloc(&ones, sizeof(float2) * g.M * nch, st));
+	CUDA_TRY(pool_malloc(&psft, sizeof(float2) * in.g.npix * nch, st));
+	CUDA_TRY(pool_malloc(&psf, sizeof(float2) * g.gsz * nch, st));
 
 	k_traj_convert<<<vec_blocks(g.M), RED_THREADS, 0, st>>>(t2, traj_c, g.M, 2.f);
 	LAUNCHED();
@@ -2093,28 +2141,6 @@ static bool on_device(const void* p)
 	return (cudaMemoryTypeDevice == a.type) || (cudaMemoryTypeManaged == a.type);
 }
 
-// The device's default pool returns unused memory at every host
-// synchronisation, and a new plan's first call would map its work space again:
-// plans let the pool keep up to this much, a few volumes' worth (set-ups with
-// auxiliary streams, which allocate per model, let it keep all). 200 x 180, 12
-// coils: first call of a new plan 430 -> 216 us, creation 1.9 -> 1.2 ms.
-static void keep_in_pool()
-{
-	const uint64_t keep = 4UL << 30;
-	uint64_t now = 0;
-	int dev;
-	cudaMemPool_t pool;
-
-	if ((cudaSuccess == cudaGetDevice(&dev)) && (cudaSuccess == cudaDeviceGetDefaultMemPool(&pool, dev))
-	    && (cudaSuccess == cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &now)) && (now < keep)) {
-
-		uint64_t k = keep;
-		cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &k);
-	}
-
-	cudaGetLastError();
-}
-
 // per thread and device: an auxiliary compute stream with a fork / join
 // event pair, and a copy stream with its event
 struct AuxStream {
@@ -2145,18 +2171,6 @@ static const AuxStream* aux_stream(int dev)
 		return nullptr;
 	}
 
-	// the library allocates and frees stream-ordered per model: keep the
-	// device's default pool from returning its memory at every host
-	// synchronisation (it would map it again for the next model)
-	cudaMemPool_t pool;
-
-	if (cudaSuccess == cudaDeviceGetDefaultMemPool(&pool, dev)) {
-
-		uint64_t keep = UINT64_MAX;
-		cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-	}
-
-	cudaGetLastError();
 	return &(aux[dev] = a);
 }
 
@@ -2198,7 +2212,7 @@ static int copy_in(void* dst, const void* src, size_t bytes, cudaStream_t st)
 }
 
 // staging of host data through device buffers (the e2e path)
-// Staging buffers come from the stream-ordered pool (cudaMallocAsync) and go
+// Staging buffers come from the library's stream-ordered pool and go
 // back to it in stream order, so host-pointer calls neither synchronise the
 // device nor pay cudaMalloc. Host inputs are read asynchronously from pinned
 // memory: keep them unchanged until the stream has caught up (as with
@@ -2221,7 +2235,7 @@ static int stage_in(Staged& s, const void* p, size_t bytes, cudaStream_t st)
 	}
 
 	cudaStream_t cs = copy_stream();
-	CUDA_TRY(cudaMallocAsync(&s.dev, bytes, cs ? cs : st));
+	CUDA_TRY(pool_malloc(&s.dev, bytes, cs ? cs : st));
 	s.owned = true;
 	s.st = st;
 	return copy_in(s.dev, p, bytes, st);
@@ -2235,7 +2249,7 @@ static int stage_out_alloc(Staged& s, void* p, size_t bytes, cudaStream_t st = n
 		return BNUFFT_OK;
 	}
 
-	CUDA_TRY(cudaMallocAsync(&s.dev, bytes, st));
+	CUDA_TRY(pool_malloc(&s.dev, bytes, st));
 	s.owned = true;
 	s.st = st;
 	return BNUFFT_OK;
@@ -2384,8 +2398,8 @@ static int embed_psf(bnufft_plan_s* p, const int E[3], OpCtx& ctx, float2** psf_
 	const long ne = (long)E[0] * E[1] * E[2];
 	float2* q = nullptr;
 	float2* qe = nullptr;
-	CUDA_TRY(cudaMallocAsync(&q, sizeof(float2) * g.gsz, st));
-	CUDA_TRY(cudaMallocAsync(&qe, sizeof(float2) * ne, st));
+	CUDA_TRY(pool_malloc(&q, sizeof(float2) * g.gsz, st));
+	CUDA_TRY(pool_malloc(&qe, sizeof(float2) * ne, st));
 
 	// rows of a [L0, rows] array as column-pass sequences (element stride 1),
 	// at most 65535 per launch
@@ -2585,8 +2599,6 @@ extern "C" int bnufft_create2(bnufft_plan_t* plan, int N, const long ksp_dims[],
 	if ((N < 4) || (nullptr == traj))
 		return fail(BNUFFT_ERR_ARG, "need N >= 4 dims and a trajectory");
 
-	keep_in_pool();
-
 	// subspace basis [1, 1, 1, 1, 1, T, K] (nufft_set_traj,
 	// src/noncart/nufft.c:1018-1042): cim [X, Y, Z, ..., 1 (TE), K (COEFF)],
 	// ksp [1, Mr, Ms, ..., T, 1], trajectory per frame or shared
@@ -2690,7 +2702,7 @@ extern "C" int bnufft_create2(bnufft_plan_t* plan, int N, const long ksp_dims[],
 	if (BNUFFT_OK == s)
 		s = init_rolloff(p->op, st);
 
-	if ((BNUFFT_OK == s) && (cudaSuccess != cudaMallocAsync(&p->traj, sizeof(float4) * M, st)))
+	if ((BNUFFT_OK == s) && (cudaSuccess != pool_malloc(&p->traj, sizeof(float4) * M, st)))
 		s = fail(BNUFFT_ERR_NOMEM, "trajectory buffer");
 
 	p->op.traj = p->traj;
@@ -2700,7 +2712,7 @@ extern "C" int bnufft_create2(bnufft_plan_t* plan, int N, const long ksp_dims[],
 		Staged bs;
 		s = stage_in(bs, basis, sizeof(float2) * T * nb, st);
 
-		if ((BNUFFT_OK == s) && (cudaSuccess != cudaMallocAsync(&p->basis, sizeof(float2) * T * nb, st)))
+		if ((BNUFFT_OK == s) && (cudaSuccess != pool_malloc(&p->basis, sizeof(float2) * T * nb, st)))
 			s = fail(BNUFFT_ERR_NOMEM, "basis buffer");
 
 		if ((BNUFFT_OK == s) && (cudaSuccess != cudaMemcpyAsync(p->basis, bs.dev, sizeof(float2) * T * nb, cudaMemcpyDeviceToDevice, st)))
@@ -2723,7 +2735,7 @@ extern "C" int bnufft_create2(bnufft_plan_t* plan, int N, const long ksp_dims[],
 			if (BNUFFT_OK == s)
 				s = stage_in(ws, weights, sizeof(float2) * p->MrMs * wf, st);
 
-			if ((BNUFFT_OK == s) && (cudaSuccess != cudaMallocAsync(&p->wgt, sizeof(float2) * M, st)))
+			if ((BNUFFT_OK == s) && (cudaSuccess != pool_malloc(&p->wgt, sizeof(float2) * M, st)))
 				s = fail(BNUFFT_ERR_NOMEM, "weights buffer");
 
 			for (long t = 0; (BNUFFT_OK == s) && (t < T); t++)
@@ -2756,7 +2768,7 @@ extern "C" int bnufft_create2(bnufft_plan_t* plan, int N, const long ksp_dims[],
 			Staged ws;
 			s = stage_in(ws, weights, sizeof(float2) * M * wc, st);
 
-			if ((BNUFFT_OK == s) && (cudaSuccess != cudaMallocAsync(&p->wgt, sizeof(float2) * M * wc, st)))
+			if ((BNUFFT_OK == s) && (cudaSuccess != pool_malloc(&p->wgt, sizeof(float2) * M * wc, st)))
 				s = fail(BNUFFT_ERR_NOMEM, "weights buffer");
 
 			if ((BNUFFT_OK == s) && (cudaSuccess != cudaMemcpyAsync(p->wgt, ws.dev, sizeof(float2) * M * wc, cudaMemcpyDeviceToDevice, st)))
@@ -2779,7 +2791,7 @@ extern "C" int bnufft_create2(bnufft_plan_t* plan, int N, const long ksp_dims[],
 		Staged ts;
 		s = stage_in(ts, traj, sizeof(float2) * 3 * p->MrMs, st);
 
-		if ((BNUFFT_OK == s) && (cudaSuccess != cudaMallocAsync(&rep, sizeof(float2) * 3 * M, st)))
+		if ((BNUFFT_OK == s) && (cudaSuccess != pool_malloc(&rep, sizeof(float2) * 3 * M, st)))
 			s = fail(BNUFFT_ERR_NOMEM, "trajectory frames");
 
 		for (long t = 0; (BNUFFT_OK == s) && (t < T); t++)
@@ -2836,7 +2848,7 @@ static int basis_forward(bnufft_plan_s* p, const float2* x, float2* y, cudaStrea
 {
 	const long M = p->op.g.M;
 	float2* tmp = nullptr;
-	CUDA_TRY(cudaMallocAsync(&tmp, sizeof(float2) * M * p->C, st));
+	CUDA_TRY(pool_malloc(&tmp, sizeof(float2) * M * p->C, st));
 	int s = op_forward(p->op, x, nullptr, p->C, tmp, st);
 
 	if (BNUFFT_OK == s) {
@@ -2855,7 +2867,7 @@ static int basis_adjoint(bnufft_plan_s* p, const float2* y, float2* x, cudaStrea
 {
 	const long M = p->op.g.M;
 	float2* tmp = nullptr;
-	CUDA_TRY(cudaMallocAsync(&tmp, sizeof(float2) * M * p->C, st));
+	CUDA_TRY(pool_malloc(&tmp, sizeof(float2) * M * p->C, st));
 	k_basis_expand<<<vec_blocks(M * p->C), RED_THREADS, 0, st>>>(tmp, y, p->basis, p->MrMs, p->T, p->Cc, p->nb);
 	cudaError_t e = cudaGetLastError();
 	g_launches.fetch_add(1, std::memory_order_relaxed);
@@ -2929,7 +2941,7 @@ extern "C" int bnufft_apply_normal(bnufft_plan_t p, void* dst, const void* src, 
 		} else {
 
 			float2* k = nullptr;
-			CUDA_TRY(cudaMallocAsync(&k, sizeof(float2) * p->op.g.M * p->Cc, st));
+			CUDA_TRY(pool_malloc(&k, sizeof(float2) * p->op.g.M * p->Cc, st));
 			int s = basis_forward(p, (const float2*)i.dev, k, st);
 
 			if (BNUFFT_OK == s)
@@ -2953,7 +2965,7 @@ extern "C" int bnufft_apply_normal(bnufft_plan_t p, void* dst, const void* src, 
 	} else {
 
 		float2* k = nullptr;
-		CUDA_TRY(cudaMallocAsync(&k, sizeof(float2) * p->op.g.M * p->C, st));
+		CUDA_TRY(pool_malloc(&k, sizeof(float2) * p->op.g.M * p->C, st));
 		TRY(op_forward(p->op, (const float2*)i.dev, nullptr, p->C, k, st));
 		TRY(op_adjoint(p->op, k, nullptr, p->C, 1, (float2*)o.dev, st));
 		cudaFreeAsync(k, st);
@@ -3099,8 +3111,8 @@ static int build_precond(bnufft_plan_s* p, cudaStream_t st)
 	TRY(alloc_work(op.w, g, 1, st));
 	float2* crop = nullptr;
 	float2* F = nullptr;
-	CUDA_TRY(cudaMallocAsync(&crop, sizeof(float2) * g.npix, st));
-	CUDA_TRY(cudaMallocAsync(&F, sizeof(float2) * g.npix, st));
+	CUDA_TRY(pool_malloc(&crop, sizeof(float2) * g.npix, st));
+	CUDA_TRY(pool_malloc(&F, sizeof(float2) * g.npix, st));
 	TRY(op_spectrum_adjoint(op, p->psf, nullptr, false, 1, 1, crop, st));
 
 	// forward N-point transform (no zero padding): a geometry with L = N
@@ -3115,7 +3127,7 @@ static int build_precond(bnufft_plan_s* p, cudaStream_t st)
 	full.traj = nullptr;
 	TRY(alloc_work(full.w, full.g, 1, st));
 	TRY(op_spectrum(full, crop, nullptr, false, 1, F, st));
-	CUDA_TRY(cudaMallocAsync(&p->pinv, sizeof(float2) * g.npix, st));
+	CUDA_TRY(pool_malloc(&p->pinv, sizeof(float2) * g.npix, st));
 	k_precond_from_spectrum<<<vec_blocks(g.npix), RED_THREADS, 0, st>>>(p->pinv, F, g.npix, (float)(1. / sqrt((double)g.npix)));
 	LAUNCHED();
 	free_work(full.w, st);
@@ -3173,12 +3185,12 @@ extern "C" int bnufft_nufft_inverse(bnufft_plan_t p, void* img, const void* ksp,
 	double *pap = nullptr, *rsp = nullptr;
 	CgScalars* sc = nullptr;
 	unsigned nb = vec_blocks(n);
-	CUDA_TRY(cudaMallocAsync(&r, ib, st));
-	CUDA_TRY(cudaMallocAsync(&pv, ib, st));
-	CUDA_TRY(cudaMallocAsync(&Ap, ib, st));
-	CUDA_TRY(cudaMallocAsync(&pap, sizeof(double) * nb, st));
-	CUDA_TRY(cudaMallocAsync(&rsp, sizeof(double) * nb, st));
-	CUDA_TRY(cudaMallocAsync(&sc, sizeof(CgScalars), st));
+	CUDA_TRY(pool_malloc(&r, ib, st));
+	CUDA_TRY(pool_malloc(&pv, ib, st));
+	CUDA_TRY(pool_malloc(&Ap, ib, st));
+	CUDA_TRY(pool_malloc(&pap, sizeof(double) * nb, st));
+	CUDA_TRY(pool_malloc(&rsp, sizeof(double) * nb, st));
+	CUDA_TRY(pool_malloc(&sc, sizeof(CgScalars), st));
 
 	// b = P^-1 N^H y  (into r, then CG start from x = 0)
 	TRY(op_adjoint(op, (const float2*)ki.dev, nullptr, C, 1, Ap, st));
@@ -3201,7 +3213,7 @@ extern "C" int bnufft_nufft_inverse(bnufft_plan_t p, void* img, const void* ksp,
 		} else {
 
 			float2* k = nullptr;
-			CUDA_TRY(cudaMallocAsync(&k, kb, st));
+			CUDA_TRY(pool_malloc(&k, kb, st));
 			TRY(op_forward(op, pv, nullptr, C, k, st));
 			TRY(op_adjoint(op, k, nullptr, C, 1, Ap, st));
 			cudaFreeAsync(k, st);
@@ -3293,7 +3305,7 @@ extern "C" int bnufft_nudft_create(bnufft_nudft_t* out, int N, const long ksp_di
 	cudaError_t e = cudaSuccess;
 
 	if (BNUFFT_OK == s)
-		e = cudaMallocAsync(&p->traj, sizeof(float4) * p->g.M, st);
+		e = pool_malloc(&p->traj, sizeof(float4) * p->g.M, st);
 
 	if ((BNUFFT_OK == s) && (cudaSuccess != e))
 		s = fail(BNUFFT_ERR_NOMEM, "nudft trajectory: %s", cudaGetErrorString(e));
@@ -4035,28 +4047,28 @@ extern "C" int bnufft_pics_create(bnufft_pics_t* out, int N, const long ksp_dims
 	auto ck = [&](cudaError_t e) { if (cudaSuccess != e && BNUFFT_OK == s) s = fail(BNUFFT_ERR_NOMEM, "pics buffers: %s", cudaGetErrorString(e)); };
 	// maps from the host are copied on the copy stream: allocated in its order
 	cudaStream_t mst = on_device(sens) ? st : copy_stream();
-	ck(cudaMallocAsync(&ps->sens, sizeof(float2) * ps->npix * ps->C, mst ? mst : st));
-	ck(cudaMallocAsync(&ps->part, sizeof(float2) * ps->npix * ps->groups, st));
-	ck(cudaMallocAsync(&ps->x, sizeof(float2) * ps->npix, st));
-	ck(cudaMallocAsync(&ps->r, sizeof(float2) * ps->npix, st));
-	ck(cudaMallocAsync(&ps->pbuf[0], sizeof(float2) * ps->npix, st));
-	ck(cudaMallocAsync(&ps->pbuf[1], sizeof(float2) * ps->npix, st));
-	ck(cudaMallocAsync(&ps->b, sizeof(float2) * ps->npix, st));
-	ck(cudaMallocAsync(&ps->mag, sizeof(float) * ps->npix, st));
-	ck(cudaMallocAsync(&ps->sel, sizeof(SelectState), st));
+	ck(pool_malloc(&ps->sens, sizeof(float2) * ps->npix * ps->C, mst ? mst : st));
+	ck(pool_malloc(&ps->part, sizeof(float2) * ps->npix * ps->groups, st));
+	ck(pool_malloc(&ps->x, sizeof(float2) * ps->npix, st));
+	ck(pool_malloc(&ps->r, sizeof(float2) * ps->npix, st));
+	ck(pool_malloc(&ps->pbuf[0], sizeof(float2) * ps->npix, st));
+	ck(pool_malloc(&ps->pbuf[1], sizeof(float2) * ps->npix, st));
+	ck(pool_malloc(&ps->b, sizeof(float2) * ps->npix, st));
+	ck(pool_malloc(&ps->mag, sizeof(float) * ps->npix, st));
+	ck(pool_malloc(&ps->sel, sizeof(SelectState), st));
 
 	if (ps->sel)
 		ck(cudaMemsetAsync(ps->sel, 0, sizeof(SelectState), st));
 	// row-pass blocks hold at least 4 rows: bounds for the partial arrays
 	ps->max_row_blocks = (YZ + 3) / 4 * ps->C + 1;
-	ck(cudaMallocAsync(&ps->pap_part, sizeof(double) * ps->max_row_blocks, st));
+	ck(pool_malloc(&ps->pap_part, sizeof(double) * ps->max_row_blocks, st));
 	// ||p||^2 partials: per first row-pass block (plain CG) or per vector block (flexible CG)
-	ck(cudaMallocAsync(&ps->pp_part, sizeof(double) * std::max<long>(ps->max_row_blocks, ps->nparts), st));
-	ck(cudaMallocAsync(&ps->rs_part, sizeof(double) * ps->nparts, st));
-	ck(cudaMallocAsync(&ps->scal, sizeof(CgScalars), st));
+	ck(pool_malloc(&ps->pp_part, sizeof(double) * std::max<long>(ps->max_row_blocks, ps->nparts), st));
+	ck(pool_malloc(&ps->rs_part, sizeof(double) * ps->nparts, st));
+	ck(pool_malloc(&ps->scal, sizeof(CgScalars), st));
 
 	if (!conf.toeplitz)
-		ck(cudaMallocAsync(&ps->kbuf, sizeof(float2) * ps->M * ps->C, st));
+		ck(pool_malloc(&ps->kbuf, sizeof(float2) * ps->M * ps->C, st));
 
 	if (conf.precond) {
 
@@ -4071,12 +4083,12 @@ extern "C" int bnufft_pics_create(bnufft_pics_t* out, int N, const long ksp_dims
 		if (const char* e = getenv("BNUFFT_FCG_FOLD"))
 			ps->fcg_fold = (0 != strcmp(e, "0"));
 
-		ck(cudaMallocAsync(&ps->z, sizeof(float2) * ps->npix, st));
-		ck(cudaMallocAsync(&ps->p_ring, sizeof(float2) * ps->npix * FCG_RING, st));
-		ck(cudaMallocAsync(&ps->ap_ring, sizeof(float2) * ps->npix * FCG_RING, st));
-		ck(cudaMallocAsync(&ps->dots_part, sizeof(double) * std::max<long>((long)ps->nparts * FCG_MAX_M,
+		ck(pool_malloc(&ps->z, sizeof(float2) * ps->npix, st));
+		ck(pool_malloc(&ps->p_ring, sizeof(float2) * ps->npix * FCG_RING, st));
+		ck(pool_malloc(&ps->ap_ring, sizeof(float2) * ps->npix * FCG_RING, st));
+		ck(pool_malloc(&ps->dots_part, sizeof(double) * std::max<long>((long)ps->nparts * FCG_MAX_M,
 				ps->max_row_blocks), st));
-		ck(cudaMallocAsync(&ps->pr_part, sizeof(double) * ps->nparts, st));
+		ck(pool_malloc(&ps->pr_part, sizeof(double) * ps->nparts, st));
 
 		if (BNUFFT_OK == s) {	// after the PSF, on the stream that builds it
 
@@ -4242,7 +4254,7 @@ static int build_precond_pad(bnufft_pics_s* ps, cudaStream_t st)
 
 	const Geom& g = ps->pre_own ? ps->pre.g : tg;
 	const float mu_lam = (float)(2.5 * ps->conf.lambda * std::pow(4., (double)g.nd) / (double)g.gsz);
-	CUDA_TRY(cudaMallocAsync(&ps->pinv_pad, sizeof(float2) * g.gsz, st));
+	CUDA_TRY(pool_malloc(&ps->pinv_pad, sizeof(float2) * g.gsz, st));
 	k_precond_pad_spectrum<<<vec_blocks(g.gsz), RED_THREADS, 0, st>>>(ps->pinv_pad, psf_e ? psf_e : toe_psf(p, st), g.gsz, mu_lam);
 	LAUNCHED();
 
@@ -4972,10 +4984,10 @@ extern "C" int bnufft_pics_set_precnet(bnufft_pics_t ps, bnufft_precnet_t net, v
 
 	for (auto& a : ps->nact)
 		if (!a)
-			CUDA_TRY(cudaMallocAsync(&a, sizeof(bf16) * NET_C * ps->npix, st));
+			CUDA_TRY(pool_malloc(&a, sizeof(bf16) * NET_C * ps->npix, st));
 
 	if (!ps->mcn_part)
-		CUDA_TRY(cudaMallocAsync(&ps->mcn_part, sizeof(double) * ps->max_row_blocks, st));
+		CUDA_TRY(pool_malloc(&ps->mcn_part, sizeof(double) * ps->max_row_blocks, st));
 
 	return BNUFFT_OK;
 }
@@ -5376,3 +5388,12 @@ extern "C" int bnufft_forward2d_noalloc(long X, long Y, long M, const void* traj
 
 // ESPIRiT calibration (include/bespirit.h)
 #include "espirit.cuh"
+
+extern "C" int bnufft_release_memory(void)
+{
+	for (cudaMemPool_t p : { lib_pool(), ec_pool() })
+		if (p)
+			CUDA_TRY(cudaMemPoolTrimTo(p, 0));
+
+	return BNUFFT_OK;
+}

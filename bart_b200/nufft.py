@@ -73,6 +73,12 @@ def _ptr_out(a, n: int):
     return ctypes.c_void_p(a.ctypes.data)
 
 
+def release_memory() -> None:
+    """Give the current device's memory that freed plans and models left mapped
+    back to the system (synchronise their streams first)."""
+    _lib.check(_lib.load().bnufft_release_memory())
+
+
 def _alloc_like(src, dims):
     n = math.prod(dims)
     if _is_torch(src):

@@ -334,6 +334,14 @@ void bnufft_cg_free(bnufft_cg_t cg);
 /* Message of the last failure on this thread ("" if none). */
 const char* bnufft_last_error(void);
 
+/* Device memory (no counterpart in the reference): plans, models, work space
+ * and staging buffers come from a memory pool of the library's own on each
+ * device (the calibration's from a second one). What is freed stays mapped
+ * for the next ones, up to an eighth of the device for the former; this gives
+ * the current device's unused part back, once the streams that freed it are
+ * synchronised. The device's default pool is not touched. */
+int bnufft_release_memory(void);
+
 /* Number of kernel launches issued by this library since load. */
 long bnufft_launch_count(void);
 

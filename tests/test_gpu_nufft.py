@@ -492,3 +492,36 @@ def test_cli_nufft_basis(tmp_path):
     assert rel(readcfl(p("k")), g["fwd"]) < TOL
     assert 0 == main_nufft(["-a", "-B", p("basis"), "-x", "32:32:1", p("traj"), p("ksp"), p("a")])
     assert rel(readcfl(p("a")), g["adj"]) < TOL
+
+
+def test_memory_pool_is_the_librarys_own(cuda):
+    """Plans and models leave the release threshold of the device's default
+    memory pool as the application set it, and what they leave mapped is given
+    back on request."""
+    import ctypes
+    import torch
+    from bart_b200 import _lib
+    from bart_b200.pics import Pics, PicsConf
+    lib = _lib.load()               # (with the symbols of the CUDA runtime that it links)
+    pool, keep, now, before = ctypes.c_void_p(), ctypes.c_uint64(3 << 20), ctypes.c_uint64(0), ctypes.c_uint64(0)
+    threshold = 4                   # cudaMemPoolAttrReleaseThreshold
+    assert 0 == lib.cudaDeviceGetDefaultMemPool(ctypes.byref(pool), 0)
+    assert 0 == lib.cudaMemPoolGetAttribute(pool, threshold, ctypes.byref(before))
+    try:
+        assert 0 == lib.cudaMemPoolSetAttribute(pool, threshold, ctypes.byref(keep))
+        rng = np.random.default_rng(2)
+        t = synth.radial_traj(128, 60)
+        free = torch.cuda.mem_get_info()[0]
+        op = nufft_create2([1, 256, 60, 64], [128, 128, 1, 64], list(t.shape), t, conf=NufftConf(toeplitz=True))
+        op.normal((rng.standard_normal((128, 128, 1, 64)) + 0j).astype(np.complex64))
+        model = Pics(t, synth.coil_maps(128, 4, rng), conf=PicsConf(maxiter=2))
+        model.run((rng.standard_normal((1, 256, 60, 4)) + 0j).astype(np.complex64))
+        op.free()
+        model.free()
+        torch.cuda.synchronize()
+        assert 0 == lib.cudaMemPoolGetAttribute(pool, threshold, ctypes.byref(now))
+        assert now.value == keep.value
+        _lib.check(lib.bnufft_release_memory())
+        assert free - torch.cuda.mem_get_info()[0] < 64 << 20       # of some 200 MB of grids
+    finally:
+        lib.cudaMemPoolSetAttribute(pool, threshold, ctypes.byref(before))
