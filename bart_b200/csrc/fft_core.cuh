@@ -211,6 +211,7 @@ __device__ __forceinline__ void twiddle(float2* v, int k, const float2* tw)
 template <int L, int Ns, int R, bool INV>
 __device__ __forceinline__ void twiddle_short(float2* v, int k, const float2* tw)
 {
+	static_assert(Ns > 1, "the first stage has no twiddles");
 	const int t = k * (L / (Ns * R));
 	float2 w[R];
 #pragma unroll
@@ -267,7 +268,7 @@ struct RowLayout {
 
 // Stage with Ns = product of earlier radices, Ns > 1: smem -> smem (middle
 // stages) or smem -> registers (the last stage).
-template <int L, typename LAY, int Ns, bool INV>
+template <int L, typename LAY, int Ns, bool INV, bool SHORT>
 __device__ __forceinline__ void fft_tail(float2 (&v)[8], float2* s, int b, int jt, const float2* tw)
 {
 	constexpr int REM = L / Ns;
@@ -294,7 +295,12 @@ __device__ __forceinline__ void fft_tail(float2 (&v)[8], float2* s, int b, int j
 
 		int j = jt + q * T;
 		int k = j % Ns;
-		twiddle<L, Ns, R, INV>(u[q], k, tw);
+
+		if constexpr (SHORT)
+			twiddle_short<L, Ns, R, INV>(u[q], k, tw);
+		else
+			twiddle<L, Ns, R, INV>(u[q], k, tw);
+
 		butterfly<R, INV>(u[q]);
 
 		if constexpr (LAST) {
@@ -315,7 +321,7 @@ __device__ __forceinline__ void fft_tail(float2 (&v)[8], float2* s, int b, int j
 	if constexpr (!LAST) {
 
 		__syncthreads();
-		fft_tail<L, LAY, Ns * R, INV>(v, s, b, jt, tw);
+		fft_tail<L, LAY, Ns * R, INV, SHORT>(v, s, b, jt, tw);
 	}
 }
 
@@ -323,7 +329,8 @@ __device__ __forceinline__ void fft_tail(float2 (&v)[8], float2* s, int b, int j
 // out). Begins with a barrier, so the caller may have been reading s just
 // before; the caller must barrier before writing s after it returns.
 // half_in: registers 2..5 are known zeros (input of length L/2, centred).
-template <int L, typename LAY, bool INV>
+// SHORT: with twiddle_short.
+template <int L, typename LAY, bool INV, bool SHORT = false>
 __device__ __forceinline__ void fft_regs(float2 (&v)[8], float2* s, const float2* tw, bool half_in = false)
 {
 	static_assert(L >= 16 && L <= 4096 && (L & (L - 1)) == 0, "power-of-two length 16..4096");
@@ -341,7 +348,7 @@ __device__ __forceinline__ void fft_regs(float2 (&v)[8], float2* s, const float2
 		s[LAY::idx(8 * jt + i, b)] = v[i];
 	__syncthreads();
 
-	fft_tail<L, LAY, 8, INV>(v, s, b, jt, tw);
+	fft_tail<L, LAY, 8, INV, SHORT>(v, s, b, jt, tw);
 }
 
 // Double-buffered form for transforms of three stages (L = 128, 256, 512):
@@ -756,7 +763,7 @@ __device__ __forceinline__ void mix_inv(float2 (&w)[spec_regs(L)], float2 (&v)[8
 // Forward and inverse transforms of any built length between the input-side
 // set v and the spectrum-side set w (the same registers for powers of two);
 // single exchange buffer, barrier on entry.
-template <int L, typename LAY>
+template <int L, typename LAY, bool SHORT = false>
 __device__ __forceinline__ void fft_fwd(float2 (&v)[8], float2 (&w)[spec_regs(L)], float2* s, const float2* tw,
 		bool half_in = false)
 {
@@ -766,14 +773,14 @@ __device__ __forceinline__ void fft_fwd(float2 (&v)[8], float2 (&w)[spec_regs(L)
 
 	} else {
 
-		fft_regs<L, LAY, false>(v, s, tw, half_in);
+		fft_regs<L, LAY, false, SHORT>(v, s, tw, half_in);
 #pragma unroll
 		for (int m = 0; m < 8; m++)
 			w[m] = v[m];
 	}
 }
 
-template <int L, typename LAY>
+template <int L, typename LAY, bool SHORT = false>
 __device__ __forceinline__ void fft_inv(float2 (&w)[spec_regs(L)], float2 (&v)[8], float2* s, const float2* tw)
 {
 	if constexpr (is_mix(L)) {
@@ -785,7 +792,7 @@ __device__ __forceinline__ void fft_inv(float2 (&w)[spec_regs(L)], float2 (&v)[8
 		for (int m = 0; m < 8; m++)
 			v[m] = w[m];
 
-		fft_regs<L, LAY, true>(v, s, tw);
+		fft_regs<L, LAY, true, SHORT>(v, s, tw);
 	}
 }
 
