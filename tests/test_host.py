@@ -1,7 +1,12 @@
 """Host-side logic: .cfl I/O, synthetic inputs, CLI dimension rules."""
 
-import numpy as np
+import os
+import stat
 
+import numpy as np
+import pytest
+
+from bart_b200 import build as builder
 from bart_b200 import synth
 from bart_b200.__main__ import estimate_im_dims
 from bart_b200.cfl import readcfl, writecfl
@@ -62,3 +67,51 @@ def test_stream_reader_on_the_reference_stream():
         assert np.array_equal(block[..., 0, 0].reshape(block.shape[:4], order="F"),
                               g["ksp"][..., pos[0]].reshape(block.shape[:4], order="F"))
     assert seen == [0, 1, 2]
+
+
+@pytest.fixture
+def fake_nvcc(tmp_path, monkeypatch):
+    """The build with a compiler that logs its arguments and writes its output file;
+    with the word fail among the flags it leaves half a file and fails."""
+    log = tmp_path / "log"
+    nvcc = tmp_path / "nvcc"
+    nvcc.write_text('#!/bin/sh\n[ "$1" = --version ] && echo one && exit\necho "$@" >> ' + str(log) + '\n'
+                    'fail=0\nfor a in "$@"; do [ "$a" = fail ] && fail=1; [ "$p" = -o ] && echo out > "$a"; p="$a"; done\nexit $fail\n')
+    nvcc.chmod(nvcc.stat().st_mode | stat.S_IXUSR)
+    for name, value in (("NVCC", str(nvcc)), ("OBJ", str(tmp_path / "obj")), ("LIB", str(tmp_path / "lib" / "lib.so")),
+                        ("STAMP", str(tmp_path / "obj" / "command")), ("FLAGS", ["-O3"])):
+        monkeypatch.setattr(builder, name, value, raising=False)
+    log.touch()
+    return lambda: log.read_text().splitlines()
+
+
+def test_build_follows_its_command_and_sources(fake_nvcc, monkeypatch):
+    """Objects and the library are made again when a flag, an environment's compiler or
+    a source changed, and not otherwise."""
+    builder.build()
+    n = len(fake_nvcc())
+    assert n == len(builder.UNITS) + 1
+    builder.build()
+    assert len(fake_nvcc()) == n
+    monkeypatch.setattr(builder, "FLAGS", ["-O2"])
+    builder.build()
+    assert len(fake_nvcc()) == 2 * n and all("-O2" in c for c in fake_nvcc()[n:2 * n - 1])
+    later = os.path.getmtime(builder.LIB) + 1000
+    inputs = builder._inputs
+    monkeypatch.setattr(builder, "_inputs", lambda u: inputs(u) + (["changed"] if u == "passes_1" else []))
+    getmtime = os.path.getmtime
+    monkeypatch.setattr(os.path, "getmtime", lambda f: later if f == "changed" else getmtime(f))
+    builder.build()
+    assert len(fake_nvcc()) == 2 * n + 2
+
+
+def test_build_that_fails_leaves_no_object(fake_nvcc, monkeypatch):
+    monkeypatch.setattr(builder, "FLAGS", ["fail"])
+    with pytest.raises(RuntimeError):
+        builder.build()
+    assert not os.path.exists(builder.LIB) and not os.listdir(builder.OBJ)
+
+
+def test_objects_are_kept_in_the_checkout():
+    """No folder of a predictable name that other users of the machine can make first."""
+    assert builder.OBJ.startswith(builder.ROOT + os.sep)
