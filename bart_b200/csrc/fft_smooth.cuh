@@ -7,7 +7,8 @@
 // buffer to the other, the radix a warp-uniform switch. Twiddle powers come
 // from table entries and at most two products each, as in the mixed lengths.
 // The row passes keep each sequence contiguous, the column pass interleaves
-// the block's columns. Same positions, fusions and results (up to rounding) as
+// the block's columns. A block has read its sequences before it writes them, so
+// passes run in place too: in and out (and pdot) may be one array. Same positions, fusions and results (up to rounding) as
 // the passes of fft_passes.cuh.
 #pragma once
 
@@ -165,9 +166,9 @@ enum { SM_THREADS = 256 };
 
 // k_rows_fwd (CG: k_rows_fwd_cg) for a smooth length: B rows per block
 template <bool CG, int B>
-__global__ void __launch_bounds__(SM_THREADS) k_srows_fwd(const float2* __restrict__ img, const float2* __restrict__ r,
+__global__ void __launch_bounds__(SM_THREADS) k_srows_fwd(const float2* img, const float2* __restrict__ r,
 		const float2* __restrict__ p_prev, float2* __restrict__ p_cur, const float2* __restrict__ maps,
-		const float* __restrict__ ax, const float* __restrict__ ayz, int X, long YZ, long R, float2* __restrict__ out,
+		const float* __restrict__ ax, const float* __restrict__ ayz, int X, long YZ, long R, float2* out,
 		const float2* __restrict__ twg, const int* done, CgScalars* st, int it, const double* __restrict__ rs_part,
 		int nrs, double* __restrict__ pp_part, SmoothPlan d)
 {
@@ -282,8 +283,8 @@ __global__ void __launch_bounds__(SM_THREADS) k_srows_fwd(const float2* __restri
 
 // k_cols MODE 0 (forward) or 1 (inverse): B columns of one outer index
 template <bool INV, int B>
-__global__ void __launch_bounds__(SM_THREADS) k_scols(const float2* __restrict__ in, long ies, long ios, int n_in,
-		int wrap_in, float2* __restrict__ out, long oes, long oos, int n_out, int wrap_out, int W,
+__global__ void __launch_bounds__(SM_THREADS) k_scols(const float2* in, long ies, long ios, int n_in,
+		int wrap_in, float2* out, long oes, long oos, int n_out, int wrap_out, int W,
 		const float2* __restrict__ twg, const int* done, SmoothPlan d)
 {
 	extern __shared__ float2 smem[];
@@ -324,9 +325,9 @@ __global__ void __launch_bounds__(SM_THREADS) k_scols(const float2* __restrict__
 // k_rows_inv: B rows and the coils of one group per block; the coil sums of
 // the block's pixels are kept in shared memory, each by its own thread
 template <int B>
-__global__ void __launch_bounds__(SM_THREADS) k_srows_inv(const float2* __restrict__ in, const float2* __restrict__ maps,
+__global__ void __launch_bounds__(SM_THREADS) k_srows_inv(const float2* in, const float2* __restrict__ maps,
 		const float* __restrict__ ax, const float* __restrict__ ayz, int X, long YZ, int C, int cpg,
-		float2* __restrict__ out, const float2* __restrict__ twg, const float2* __restrict__ pdot,
+		float2* out, const float2* __restrict__ twg, const float2* pdot,
 		double* __restrict__ dot_part, const int* done, unsigned x_magic, SmoothPlan d)
 {
 	extern __shared__ float2 smem[];
