@@ -378,8 +378,8 @@ def test_gridding_edges_vs_oracle(dims, samples, spokes, coils, periodic, weight
 
 @pytest.mark.parametrize("dims,coils,periodic,weights", [
     ((8, 8, 8), 4, False, False),       # the shortest z transform, one group of four
-    ((10, 14, 16), 8, True, True),      # two groups at once, wrapping around, weights
-    ((18, 22, 32), 12, False, True),     # two groups and one more
+    ((10, 14, 16), 8, True, True),      # a block for each of two groups, wrapping around, weights
+    ((18, 22, 32), 12, False, True),     # three groups
     ((16, 12, 96), 20, False, False),   # a mixed z length, several groups
     ((12, 10, 64), 6, True, False)])    # coils not in fours: the plain grid
 def test_forward_of_coil_fours_vs_oracle(dims, coils, periodic, weights):
@@ -405,6 +405,27 @@ def test_forward_of_coil_fours_vs_oracle(dims, coils, periodic, weights):
     one.free()
     assert rel(fwd, single) < 9e-7
     assert rel(fwd.reshape(-1, coils, order="F"), o.forward(x)) < TOL
+
+
+@pytest.mark.parametrize("coils,periodic,weights", [(8, True, True), (12, False, True), (12, True, False), (20, False, True)])
+def test_forward_of_two_coil_fours_at_once(coils, periodic, weights):
+    """As above with samples enough (76000 and more) for blocks that take all
+    channels, eight at a time and the last four after them, against the plain
+    grid's gather channel by channel."""
+    dims, M = (12, 14, 16), 400 * 200
+    rng = np.random.default_rng(coils)
+    t = (rng.uniform(-0.55, 0.55, (3, 400, 200)) * np.array(dims)[:, None, None]).astype(np.complex64)
+    w = (rng.uniform(0.5, 2.0, (1, 400, 200)) * np.exp(1j * rng.uniform(0, 6, (1, 400, 200)))).astype(np.complex64) if weights else None
+    wd = list(w.shape) if weights else None
+    conf = NufftConf(toeplitz=False, periodic=periodic)
+    op = nufft_create2([1, 400, 200, coils], list(dims) + [coils], list(t.shape), t, wd, w, conf=conf)
+    one = nufft_create2([1, 400, 200, 1], list(dims) + [1], list(t.shape), t, wd, w, conf=conf)
+    x = (rng.standard_normal(dims + (coils,)) + 1j * rng.standard_normal(dims + (coils,))).astype(np.complex64)
+    fwd = np.asarray(op.forward(x)).reshape(M, coils, order="F")
+    for c in range(coils):
+        assert rel(fwd[:, c], np.asarray(one.forward(np.asfortranarray(x[..., c:c + 1])))) < 9e-7
+    op.free()
+    one.free()
 
 
 @pytest.mark.parametrize("dims,coils", [
