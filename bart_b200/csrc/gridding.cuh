@@ -1503,8 +1503,9 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(long M, GridGe
 	const int c0 = cw0 + grp * CT;		// first coil of this lane
 	const long h0 = tw.hit_start[tile];
 	const int nh = (int)(tw.hit_start[tile + 1] - h0);	// (a sample is in a tile's list once)
-	const int* hits = tw.hits + h0;
-	const int first = tw.work_chunk[wi] * tw.chunk, last = min(nh, first + tw.chunk);
+	const int first = tw.work_chunk[wi] * tw.chunk;
+	const int* hits = tw.hits + h0 + first + lane;		// this lane's next hits are 32 apart
+	int left = min(nh - first, tw.chunk);
 
 	float2 acc[TX][CT];
 #pragma unroll
@@ -1549,17 +1550,17 @@ __global__ void __launch_bounds__(32 * TG_WARPS, 4) k_grid6_tiles(long M, GridGe
 	};
 
 	int buf = 0;
-	int inext = (first + lane < last) ? hits[first + lane] : -1;
+	int inext = (lane < left) ? hits[0] : -1;
 	fetch(inext, 0);
-	inext = (first + 32 + lane < last) ? hits[first + 32 + lane] : -1;
+	inext = (32 + lane < left) ? hits[32] : -1;
 
-	for (int base = first; base < last; base += 32) {
+	for (; left > 0; left -= 32, hits += 32) {
 
 		fetch(inext, buf ^ 1);
-		inext = (base + 64 + lane < last) ? hits[base + 64 + lane] : -1;
+		inext = (64 + lane < left) ? hits[64] : -1;
 		asm volatile("cp.async.wait_group 1;\n" ::: "memory");
 		float* rb = rec + buf * 32 * ST::REC;
-		const int n = min(32, last - base);
+		const int n = min(32, left);
 
 		if (lane < n) {	// this lane's own record: offsets relative to the tile
 
