@@ -1866,9 +1866,14 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		// cost more than the host's wait for the count, some 20 us
 		long total = M * tg_max_hits(g, bg);
 		b.nwork_max = nt + (total + b.chunk - 1) / b.chunk;
-		cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-		CUDA_TRY(cudaStreamIsCapturing(st, &cs));
-		const bool count = (sizeof(int) * total > TG_LIST_BYTES) && (cudaStreamCaptureStatusNone == cs);
+		bool count = (sizeof(int) * total > TG_LIST_BYTES);
+
+		if (count) {	// (not while capturing)
+
+			cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+			CUDA_TRY(cudaStreamIsCapturing(st, &cs));
+			count = (cudaStreamCaptureStatusNone == cs);
+		}
 
 		if (count || det) {
 
