@@ -2375,18 +2375,34 @@ __global__ static void k_toe_embed(float2* __restrict__ qe, const float2* __rest
 }
 
 // Embedding lengths E >= 2N per axis: the shortest built FFT lengths (pow2: of
-// the powers of two). Returns whether they differ from 2N; false too where an
-// axis is too long for any.
-static bool embed_lengths(const Geom& g, bool pow2, int E[3])
+// the powers of two). Slices embed on 512 instead of 448 points: 56 threads do the
+// last 64 butterflies of a 448-point transform in two rounds, and columns of 512 have
+// the two-stage kernel. Only rows keep 448 from 24 channels on, where the grid's size
+// counts and the columns are not 512 long. (Normal operator with 16 channels,
+// 198^2 and 210^2 on 448: 51.3 us, on 512: 44.1 and 43.9; 20 CG iterations 1312 and
+// 1162 us. 224 x 160 with 16 and 32: 41.0 and 63.6 us on rows of 448, 39.3 and 68.3
+// on 512. Volumes, bound by the grid's traffic, take the shortest.) 2N = 448 itself
+// needs no embedding, whose two transforms of the PSF would round more.
+// Returns whether they differ from 2N; false too where an axis is too long for any.
+static bool embed_lengths(const Geom& g, long C, bool pow2, int E[3])
 {
 	bool embed = false, ok = true;
+	auto slow = [&](int a) { return (1 == g.G[2]) && (448 == E[a]) && (448 != g.G[a]); };
 
 	for (int a = 0; a < 3; a++) {
 
 		E[a] = (g.G[a] > 1) ? fft_length(g.G[a], pow2) : 1;
 		ok = ok && (E[a] > 0);
-		embed = embed || (E[a] != g.G[a]);
 	}
+
+	if (slow(1))
+		E[1] = 512;
+
+	if (slow(0) && ((512 == E[1]) || (C < 24)))
+		E[0] = 512;
+
+	for (int a = 0; a < 3; a++)
+		embed = embed || (E[a] != g.G[a]);
 
 	return embed && ok;
 }
@@ -2466,7 +2482,7 @@ static int build_toeplitz_embedding(bnufft_plan_s* p, cudaStream_t st)
 	p->embed = false;
 	int E[3];
 
-	if (!embed_lengths(p->op.g, false, E))
+	if (!embed_lengths(p->op.g, p->C, false, E))
 		return BNUFFT_OK;
 
 	TRY(embed_psf(p, E, p->toe, &p->psf_t, st));
@@ -4246,7 +4262,7 @@ static int build_precond_pad(bnufft_pics_s* ps, cudaStream_t st)
 	// the preconditioner is defined on the power-of-two circulant; the normal
 	// operator may run on a shorter one
 	int E[3];
-	const bool embed = embed_lengths(p->op.g, true, E);
+	const bool embed = embed_lengths(p->op.g, p->C, true, E);
 	const Geom& tg = toe_ctx(p).g;
 	float2* psf_e = nullptr;
 

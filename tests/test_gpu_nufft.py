@@ -433,6 +433,7 @@ def test_forward_of_two_coil_fours_at_once(coils, periodic, weights):
     ((70, 132, 1), 3), ((104, 90, 1), 5), ((154, 54, 1), 1),    # radices 2 to 13
     ((228, 34, 1), 1),                                          # 456 = 8 3 19 and 68 = 4 17: Bluestein
     ((250, 500, 1), 1),                                         # four sequences per block
+    ((210, 60, 1), 3), ((210, 60, 1), 25), ((60, 200, 1), 3),   # embedded on 512 points: rows of few channels, columns
     ((36, 40, 50), 2)])
 def test_grid_lengths_vs_oracle(dims, coils):
     """Forward, adjoint and Toeplitz normal on grids of mixed lengths (64 times

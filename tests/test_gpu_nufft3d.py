@@ -182,15 +182,16 @@ def test_more_samples_than_footprints():
     assert float(torch.linalg.vector_norm(adj - want) / torch.linalg.vector_norm(want)) < 2.1e-6
 
 
-@pytest.mark.parametrize("dims,spokes,chunk,periodic", [((64, 64, 64), 2000, None, False),
+@pytest.mark.parametrize("dims,spokes,chunk,periodic", [((64, 64, 64), 2000, None, False), ((64, 64, 64), 9000, None, True),
                                                         ((128, 64, 80), 2000, 32, False), ((128, 72, 84), 2000, 32, True)])
 def test_plans_of_many_tiles(dims, spokes, chunk, periodic, monkeypatch):
     """More tiles than one block plans (16384 in two segments, 40960 in five, 48384
     in six): the tile scatter and its deterministic form against the
     single-channel scatter, with hits that fit one work item a tile and with
-    several. Tiles listed by blocks (330 candidates on average) and by warps (130 and
-    110), with more candidates than a warp takes at the centre, and where a
-    periodic grid wraps around tiles cut short. Two orders of the same float32
+    several. Tiles listed by blocks (330 and 1500 candidates on average; the latter's
+    lists are counted before they are made) and by warps (130 and 110), with more
+    candidates than a warp takes at the centre, and where a periodic grid wraps
+    around tiles cut short. Two orders of the same float32
     sums of some hundred terms."""
     rng = np.random.default_rng(dims[0] + spokes)
     if chunk:
