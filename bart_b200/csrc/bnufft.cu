@@ -1855,7 +1855,7 @@ static int build_bins(OpCtx& op, cudaStream_t st, bool det)
 		TileHits th = { nhits, nullptr, nullptr, nullptr, nullptr, nullptr };
 		int* large = nullptr;
 
-		if (27 * M < TH_MEAN * nt)
+		if ((nt > TH_TILES) && (27 * M < TH_MEAN * nt))
 			CUDA_TRY(pool_malloc(&large, sizeof(int) * (1 + std::min(nt, 27 * M / TH_WARP_MOST + 1)), st));
 
 		TRY(tile_hits(op, lo4, bin_start, th, large, st));

@@ -876,11 +876,13 @@ __device__ __forceinline__ int foot_rel(int lo, int origin, int G, int periodic)
 // hit_start on, and the tile's work items.
 // k_tile_hits: a block per tile. k_tile_hits_warp: a warp per tile of at most
 // TH_WARP_MOST candidates, the other ones into a list for k_tile_hits. The warps
-// serve grids whose tiles have less than TH_MEAN candidates on average (uniform
-// samples, two coils, plan creation by blocks and by warps: 5.12 M on a 1024^3 grid,
-// 16 candidates, 47.4 and 11.1 ms; on 512^3, 132, 7.1 and 4.0 ms; on 256^3, 1054,
-// 2.6 and 3.4 ms).
-enum { TH_THREADS = 256, TH_RANGES = 18, TH_WARP_MOST = 1024, TH_MEAN = 256 };
+// serve grids of more than TH_TILES tiles (few tiles are latency, and the blocks'
+// form has two launches less) with less than TH_MEAN candidates on average. Plan
+// creation by blocks and by warps, radial samples: 128^3, 384 000 samples (79
+// candidates) 1025 and 419 us; 5.12 million (1055) 3.30 and 2.94 ms; 64^3, 192 000
+// (316) 302 and 267 us; 768 000 (1266) 691 and 712; 256^2, 49 000 in 2048 tiles 101
+// and 127; uniform samples on a 1024^3 grid (16) 47 and 8.2 ms.
+enum { TH_THREADS = 256, TH_RANGES = 18, TH_WARP_MOST = 1024, TH_MEAN = 1200, TH_TILES = 8192 };
 
 struct TileHits {
 
@@ -944,6 +946,18 @@ __global__ void __launch_bounds__(TH_THREADS) k_tile_hits_warp(const short4* __r
 
 		const int bx = (int)(t % bg.nb[0]), by = (int)((t / bg.nb[0]) % bg.nb[1]), bz = (int)(t / ((long)bg.nb[0] * bg.nb[1]));
 		const int ox = bx * bg.bs[0], oy = by * bg.bs[1], oz = bz * bg.bs[2];
+
+		if (th.work_start && (th.hit_start[t] == th.hit_start[t + 1])) {	// no hits: one work item
+
+			if (0 == lane) {
+
+				th.work_tile[th.work_start[t]] = (int)t;
+				th.work_chunk[th.work_start[t]] = 0;
+			}
+
+			continue;
+		}
+
 		const int2 range = (lane < nr) ? hit_range(lane, bx, by, bz, bin_start, g, bg) : make_int2(0, 0);
 		int end = range.y;		// candidates up to this lane's range
 
@@ -969,16 +983,13 @@ __global__ void __launch_bounds__(TH_THREADS) k_tile_hits_warp(const short4* __r
 		for (int base = 0; base < total; base += 32) {
 
 			const int c = base + lane;
-			int i = -1;
+			int r = 0;		// the candidate's range: the first that ends after it
+#pragma unroll
+			for (int step = 16; step > 0; step /= 2)
+				r += (c >= __shfl_sync(0xffffffffu, end, r + step - 1)) ? step : 0;
 
-			for (int r = 0; r < nr; r++) {
-
-				const int e = __shfl_sync(0xffffffffu, end, r), k = __shfl_sync(0xffffffffu, range.y, r);
-				const int s = __shfl_sync(0xffffffffu, range.x, r);
-				i = ((c < e) && (c >= e - k)) ? s + c - (e - k) : i;
-			}
-
-			const bool hit = (i >= 0) && is_hit(lo[i], ox, oy, oz, g, bg);
+			const int i = __shfl_sync(0xffffffffu, range.x + range.y - end, r) + c;
+			const bool hit = (c < total) && is_hit(lo[i], ox, oy, oz, g, bg);
 			const unsigned m = __ballot_sync(0xffffffffu, hit);
 
 			if (hit && dst)

@@ -188,10 +188,9 @@ def test_plans_of_many_tiles(dims, spokes, chunk, periodic, monkeypatch):
     """More tiles than one block plans (16384 in two segments, 40960 in five, 48384
     in six): the tile scatter and its deterministic form against the
     single-channel scatter, with hits that fit one work item a tile and with
-    several. Tiles listed by blocks (330 and 1500 candidates on average; the latter's
-    lists are counted before they are made) and by warps (130 and 110), with more
-    candidates than a warp takes at the centre, and where a periodic grid wraps
-    around tiles cut short. Two orders of the same float32
+    several. Tiles listed by warps (330, 130 and 110 candidates on average, more than
+    a warp takes at the centre, and where a periodic grid wraps around tiles cut
+    short) and by blocks (1500; their lists are counted before they are made). Two orders of the same float32
     sums of some hundred terms."""
     rng = np.random.default_rng(dims[0] + spokes)
     if chunk:
